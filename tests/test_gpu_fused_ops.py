@@ -64,6 +64,36 @@ def test_rope_matches_complex_rotation_and_inverts():
     torch.testing.assert_close(x.grad.float(), x.detach().float(), rtol=3e-2, atol=3e-2)
 
 
+@pytest.mark.parametrize("tokens,heads,hd", [(1, 1, 8), (3, 5, 96), (31, 1, 256), (257, 8, 64), (1025, 4, 128)])
+@pytest.mark.parametrize("layout", ["slice", "transposed", "expanded", "odd_offset"])
+def test_rope_reads_strided_inputs(tokens, heads, hd, layout):
+    from torchcomms_b200.ops import fused
+
+    cos_t, sin_t = fused.rope_tables(2048, hd, 10000.0, "cuda")
+    pos = torch.randint(0, 2048, (tokens,), dtype=torch.int32, device="cuda")
+    if layout == "slice":
+        x = _bf(tokens, (heads + 2) * hd, seed=6)[:, hd : (heads + 1) * hd].reshape(tokens, heads, hd)
+    elif layout == "transposed":
+        x = _bf(heads, tokens, hd, seed=6).transpose(0, 1)
+    elif layout == "expanded":
+        x = _bf(tokens, 1, hd, seed=6).expand(tokens, heads, hd)
+    else:
+        x = _bf(tokens * heads * hd + 1, seed=6)[1:].view(tokens, heads, hd)
+    x = x.detach().requires_grad_(True)
+    y = fused.apply_rope(x, pos, cos_t, sin_t)
+    (dx,) = torch.autograd.grad(y, x, _bf(heads, tokens, hd, seed=7).transpose(0, 1))
+    assert y.is_contiguous()
+
+    def rotate(t, sign):
+        a, b = t.float().unflatten(-1, (-1, 2)).unbind(-1)
+        c, s = cos_t[pos.long()].unsqueeze(1), sign * sin_t[pos.long()].unsqueeze(1)
+        return torch.stack((a * c - b * s, a * s + b * c), dim=-1).flatten(-2)
+
+    # One rounding to bf16 of a two-term fp32 sum: half a unit in the last place (2^-9), plus cancellation noise.
+    torch.testing.assert_close(y.float(), rotate(x.detach(), 1.0), rtol=2**-8, atol=2e-6)
+    torch.testing.assert_close(dx.float(), rotate(_bf(heads, tokens, hd, seed=7).transpose(0, 1), -1.0), rtol=2**-8, atol=2e-6)
+
+
 @pytest.mark.parametrize("rows,vocab", [(7, 1000), (64, 32003), (9, 128256)])
 def test_cross_entropy_loss_and_gradient(rows, vocab):
     from torchcomms_b200 import _comms

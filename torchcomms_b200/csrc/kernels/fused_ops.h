@@ -27,11 +27,14 @@ cudaError_t launch_colsum_bf16(const float* in, __nv_bfloat16* out, int rows, in
 // What a collective degenerates to on a single rank (cast, scale, copy) in one pass.
 cudaError_t launch_cast_scale(const void* in, int in_kind, void* out, int out_kind, size_t n, float scale, cudaStream_t s);
 
-// Rotary embedding in place on [tokens, heads, head_dim] with interleaved
-// pairs; pos[t] indexes the cos/sin tables [max_pos, head_dim/2]. `inverse`
-// rotates by the negative angle (the backward pass).
-cudaError_t launch_rope(__nv_bfloat16* x, const int* pos, const float* cos_t, const float* sin_t, int tokens,
-                        int heads, int head_dim, bool inverse, cudaStream_t s);
+// Rotary embedding of x[tokens, heads, head_dim] with interleaved pairs into the
+// contiguous y; pos[t] indexes the cos/sin tables [max_pos, head_dim/2]. `inverse`
+// rotates by the negative angle (the backward pass). x may be a slice of a wider
+// tensor: element strides of its token and head dimensions, multiples of 8 like
+// head_dim; x, y and the tables 16-byte aligned. y may be x itself if that is contiguous.
+cudaError_t launch_rope(const __nv_bfloat16* x, int64_t stride_t, int64_t stride_h, __nv_bfloat16* y, const int* pos,
+                        const float* cos_t, const float* sin_t, int tokens, int heads, int head_dim, bool inverse,
+                        cudaStream_t s);
 
 // h = silu(gate) * up where gate_up = [rows, 2*ffn] (gate first).
 cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, int rows, int ffn, cudaStream_t s);

@@ -29,6 +29,31 @@ cudaStream_t cur(const at::Tensor& t) {
   return at::cuda::getCurrentCUDAStream(t.device().index()).stream();
 }
 
+// y = x rotated; y contiguous, possibly x itself.
+void rope_into(const at::Tensor& x, at::Tensor& y, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t,
+               bool inverse) {
+  want(pos, at::kInt, "pos");
+  want(cos_t, at::kFloat, "cos");
+  want(sin_t, at::kFloat, "sin");
+  TORCH_CHECK(x.dim() >= 3, "x must be [..., tokens, heads, head_dim]");
+  const int head_dim = static_cast<int>(x.size(-1));
+  const int heads = static_cast<int>(x.size(-2));
+  const int64_t per_token = static_cast<int64_t>(head_dim) * heads;
+  const int tokens = per_token == 0 ? 0 : static_cast<int>(x.numel() / per_token);
+  TORCH_CHECK(pos.numel() == tokens, "pos must have one entry per token");
+  TORCH_CHECK(cos_t.size(-1) == head_dim / 2 && sin_t.size(-1) == head_dim / 2, "cos/sin tables: [max_pos, head_dim/2]");
+  c10::cuda::CUDAGuard g(x.device());
+  // A slice of a wider tensor (queries or keys of a fused projection) is read where it is; layouts that
+  // 16-byte loads cannot follow are made contiguous first.
+  auto aligned = [](const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; };
+  const bool in_place = x.dim() == 3 && x.stride(2) == 1 && x.stride(0) % 8 == 0 && x.stride(1) % 8 == 0 && aligned(x);
+  const at::Tensor src = in_place || x.is_same(y) ? x : x.clone(at::MemoryFormat::Contiguous);
+  const int64_t st = in_place ? src.stride(0) : per_token, sh = in_place ? src.stride(1) : head_dim;
+  const at::Tensor c = aligned(cos_t) ? cos_t : cos_t.clone(), sn = aligned(sin_t) ? sin_t : sin_t.clone();
+  B200C_CUDA_CHECK(launch_rope(bf(src), st, sh, bf_mut(y), pos.data_ptr<int>(), c.data_ptr<float>(), sn.data_ptr<float>(), tokens,
+                               heads, head_dim, inverse, cur(x)));
+}
+
 } // namespace
 
 void bind_ops(py::module_& m) {
@@ -87,19 +112,15 @@ void bind_ops(py::module_& m) {
 
   ops.def("rope_", [](at::Tensor x, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t, bool inverse) {
     want(x, at::kBFloat16, "x");
-    want(pos, at::kInt, "pos");
-    want(cos_t, at::kFloat, "cos");
-    want(sin_t, at::kFloat, "sin");
-    TORCH_CHECK(x.dim() >= 3, "x must be [..., tokens, heads, head_dim]");
-    const int head_dim = static_cast<int>(x.size(-1));
-    const int heads = static_cast<int>(x.size(-2));
-    const int tokens = static_cast<int>(x.numel() / (static_cast<int64_t>(head_dim) * heads));
-    TORCH_CHECK(pos.numel() == tokens, "pos must have one entry per token");
-    TORCH_CHECK(cos_t.size(-1) == head_dim / 2 && sin_t.size(-1) == head_dim / 2, "cos/sin tables: [max_pos, head_dim/2]");
-    c10::cuda::CUDAGuard g(x.device());
-    B200C_CUDA_CHECK(launch_rope(bf_mut(x), pos.data_ptr<int>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), tokens,
-                                 heads, head_dim, inverse, cur(x)));
+    rope_into(x, x, pos, cos_t, sin_t, inverse);
     return x;
+  });
+  // Out of place: x [..., tokens, heads, head_dim] of any strides -> contiguous.
+  ops.def("rope", [](const at::Tensor& x, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t, bool inverse) {
+    TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16, "x: bf16 CUDA tensor expected");
+    at::Tensor y = at::empty_like(x, at::MemoryFormat::Contiguous);
+    rope_into(x, y, pos, cos_t, sin_t, inverse);
+    return y;
   });
 
   ops.def("swiglu_fwd", [](const at::Tensor& gate_up) {

@@ -91,12 +91,12 @@ class _Rope(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, pos, cos_t, sin_t):
         ctx.save_for_backward(pos, cos_t, sin_t)
-        return _k.rope_(x.clone(memory_format=torch.contiguous_format), pos, cos_t, sin_t, False)
+        return _k.rope(x, pos, cos_t, sin_t, False)
 
     @staticmethod
     def backward(ctx, dy):
         pos, cos_t, sin_t = ctx.saved_tensors
-        return _k.rope_(dy.clone(memory_format=torch.contiguous_format), pos, cos_t, sin_t, True), None, None, None
+        return _k.rope(dy, pos, cos_t, sin_t, True), None, None, None
 
 
 def apply_rope(x: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor) -> torch.Tensor:
