@@ -32,6 +32,24 @@ def test_rmsnorm_forward_backward(rows, cols):
         torch.testing.assert_close(w.grad.float(), wf.grad, rtol=3e-2, atol=3e-2 * max(1.0, rows ** 0.5))
 
 
+@pytest.mark.parametrize("cols", [8, 256, 264, 512, 1000, 1024, 1032, 2048, 2056, 4096, 4104, 8192])
+@pytest.mark.parametrize("rows", [1, 9, 1200, 2377])
+def test_rmsnorm_row_layouts(rows, cols):
+    """Every split of a row over threads, at its edges, with fewer and more rows than row groups on the GPU."""
+    from torchcomms_b200 import _comms
+
+    x, dy, w = _bf(rows, cols, seed=1), _bf(rows, cols, seed=2), _bf(cols, seed=3, scale=0.1) + 1
+    y, rstd = _comms.ops.rmsnorm_fwd(x, w, 1e-5)
+    dx, dw = _comms.ops.rmsnorm_bwd(dy, x, w, rstd)
+    xd, wd = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    ref = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd
+    rdx, rdw = torch.autograd.grad(ref, (xd, wd), dy.double())
+    # Half a bf16 ulp (2^-9 relative) and fp32 sums of up to 8192 (dx) or `rows` (dw) terms of unit size before it.
+    torch.testing.assert_close(y.double(), ref.detach(), rtol=2**-8, atol=1e-6)
+    torch.testing.assert_close(dx.double(), rdx, rtol=2**-8, atol=2e-5)
+    torch.testing.assert_close(dw.double(), rdw, rtol=2**-8, atol=1e-6 * rows**0.5 + 2e-5)
+
+
 def test_swiglu_forward_backward():
     from torchcomms_b200.ops import fused
 

@@ -20,7 +20,7 @@ cudaError_t launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* w, _
 cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
                                const float* rstd, __nv_bfloat16* dx, float* dw_partial, int* nblocks, int rows,
                                int cols, cudaStream_t s);
-// out[c] = sum_r in[r, c]  (fp32 in, bf16 or fp32 out)
+// out[c] = sum_r in[r, c]  (fp32 in, 16-byte aligned, cols a multiple of 4; bf16 out)
 cudaError_t launch_colsum_bf16(const float* in, __nv_bfloat16* out, int rows, int cols, cudaStream_t s);
 
 // out[i] = convert(in[i] * scale) for n elements; `in_kind` / `out_kind`: 0 = fp32, 1 = bf16.
