@@ -89,6 +89,40 @@ def _fp8_ref(q_a, s_a, q_b, s_b):
     return (q_a.float() * s_a.unsqueeze(1)) @ (q_b.float() * s_b.unsqueeze(1)).t()
 
 
+@pytest.mark.parametrize("rows,cols,layout", [(1, 16, "plain"), (67, 4096, "plain"), (700, 1024, "plain"), (700, 4096, "plain"),
+                                              (5, 2040, "plain"), (9, 1001, "plain"), (3, 16384, "plain"), (2, 20488, "plain"),
+                                              (33, 512, "slice"), (33, 500, "odd_slice"), (4, 264, "odd_offset")])
+def test_quantize_rows_kernel_matches_operators(rows, cols, layout):
+    """The kernel gives the bits of the operator-by-operator path, special values included."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops.tp import quantize_rows
+
+    if layout == "plain":
+        x = _rand((rows, cols), 3, scale=2.0)
+    elif layout == "slice":
+        x = _rand((rows, 3 * cols), 3)[:, cols : 2 * cols]
+    elif layout == "odd_slice":
+        x = _rand((rows, 2 * cols + 1), 3)[:, 3 : 3 + cols]
+    else:
+        x = _rand((rows * cols + 1,), 3)[1:].view(rows, cols)
+    x[0] *= 1e-12                       # below the smallest scale
+    if rows > 4:
+        x[1, 0], x[2, 0], x[3, 0] = float("inf"), float("-inf"), float("nan")
+        x[4] = 0
+    amax = x.float().abs().amax(dim=1).clamp_min(1e-8)
+    scale = amax / 448.0
+    ref = (x.float() / scale.unsqueeze(1)).to(torch.float8_e4m3fn)
+    q, s = quantize_rows(x)
+    torch.testing.assert_close(s, scale, rtol=0, atol=0, equal_nan=True)
+    assert torch.equal(q.view(torch.uint8), ref.view(torch.uint8))
+    # Calls that autograd or another layer of the dispatcher wants to see do not go to the kernel.
+    assert _comms.ops.quantize_rows(x) is not None
+    assert _comms.ops.quantize_rows(x.detach().requires_grad_(True)) is None
+    assert _comms.ops.quantize_rows(x.float()) is None and _comms.ops.quantize_rows(x.cpu()) is None
+    with torch.no_grad():
+        assert _comms.ops.quantize_rows(x.t()) is None or cols == 1
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 256, 128), (300, 264, 256), (1024, 1792, 2048), (128 * 9, 256 * 5, 1024)])
 def test_gemm_e4m3_rowwise_scales(m, n, k):
     from torchcomms_b200.ops.tp import gemm_e4m3_nt, quantize_rows

@@ -27,6 +27,10 @@ cudaError_t launch_colsum_bf16(const float* in, __nv_bfloat16* out, int rows, in
 // What a collective degenerates to on a single rank (cast, scale, copy) in one pass.
 cudaError_t launch_cast_scale(const void* in, int in_kind, void* out, int out_kind, size_t n, float scale, cudaStream_t s);
 
+// Row-wise e4m3 quantisation of bf16 x [rows, cols] (row stride `ld` elements): scale[r] = max(max|x_r|, 1e-8) / 448,
+// q[r, c] = e4m3(x[r, c] / scale[r]), q contiguous. Any cols; 16-byte accesses where the layout allows them.
+cudaError_t launch_quantize_rows(const __nv_bfloat16* x, int64_t ld, void* q, float* scale, int rows, int cols, cudaStream_t s);
+
 // Rotary embedding of x[tokens, heads, head_dim] with interleaved pairs into the
 // contiguous y; pos[t] indexes the cos/sin tables [max_pos, head_dim/2]. `inverse`
 // rotates by the negative angle (the backward pass). x may be a slice of a wider

@@ -8,6 +8,7 @@
 #include "../kernels/fused_ops.h"
 #include "../kernels/launch_count.h"
 #include "../kernels/tc_gemm.h"
+#include "plain_call.hpp"
 
 namespace b200c {
 
@@ -27,6 +28,15 @@ void want(const at::Tensor& t, at::ScalarType dt, const char* name) {
 
 cudaStream_t cur(const at::Tensor& t) {
   return at::cuda::getCurrentCUDAStream(t.device().index()).stream();
+}
+
+bool quantizable(const at::Tensor& x) {
+  return plain_call(x) && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.numel() > 0 && x.stride(1) == 1 &&
+      x.size(0) <= INT32_MAX && x.size(1) <= INT32_MAX;
+}
+void quantize_into(const at::Tensor& x, at::Tensor& q, at::Tensor& scale) {
+  B200C_CUDA_CHECK(launch_quantize_rows(bf(x), x.stride(0), q.data_ptr(), scale.data_ptr<float>(), static_cast<int>(x.size(0)),
+                                        static_cast<int>(x.size(1)), cur(x)));
 }
 
 // y = x rotated; y contiguous, possibly x itself.
@@ -171,6 +181,26 @@ void bind_ops(py::module_& m) {
                                   static_cast<size_t>(p.numel()), static_cast<float>(lr), static_cast<float>(beta1),
                                   static_cast<float>(beta2), static_cast<float>(eps), static_cast<float>(weight_decay), step,
                                   static_cast<float>(grad_scale), cur(p)));
+  });
+
+  // Row-wise e4m3 quantisation: (q, scale), or None where the kernel does not apply (the caller then takes the
+  // operator-by-operator path, which every device, type and transform understands).
+  ops.def("quantize_rows", [](const at::Tensor& x) -> std::optional<std::pair<at::Tensor, at::Tensor>> {
+    if (!quantizable(x)) return std::nullopt;
+    c10::cuda::CUDAGuard g(x.device());
+    at::Tensor q = at::empty({x.size(0), x.size(1)}, x.options().dtype(at::kFloat8_e4m3fn));
+    at::Tensor scale = at::empty({x.size(0)}, x.options().dtype(at::kFloat));
+    quantize_into(x, q, scale);
+    return std::make_pair(q, scale);
+  });
+  // The same into existing buffers; false where the kernel does not apply.
+  ops.def("quantize_rows_into", [](const at::Tensor& x, at::Tensor q, at::Tensor scale) {
+    if (!quantizable(x) || q.device() != x.device() || scale.device() != x.device()) return false;
+    if (q.sizes() != x.sizes() || q.scalar_type() != at::kFloat8_e4m3fn || !q.is_contiguous()) return false;
+    if (scale.numel() != x.size(0) || scale.scalar_type() != at::kFloat || !scale.is_contiguous()) return false;
+    c10::cuda::CUDAGuard g(x.device());
+    quantize_into(x, q, scale);
+    return true;
   });
 
   ops.def("gemm_bf16_nt", [](const at::Tensor& a, const at::Tensor& b) {

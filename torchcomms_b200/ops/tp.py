@@ -49,6 +49,10 @@ def _impl(comm: Optional[TorchComm]):
 
 def quantize_rows(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """``(q, scale)`` with ``q`` e4m3 ``[rows, cols]`` and ``scale`` fp32 ``[rows]`` such that ``q * scale[:, None] ~ x``."""
+    if type(x) is torch.Tensor and not torch.compiler.is_compiling():
+        out = _comms.ops.quantize_rows(x)
+        if out is not None:
+            return out
     amax = x.float().abs().amax(dim=1).clamp_min(1e-8)
     scale = amax / FP8_MAX
     return (x.float() / scale.unsqueeze(1)).to(torch.float8_e4m3fn), scale
@@ -81,11 +85,15 @@ class AllGatherGemm:
                  scale_x: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``fp8``: ``w`` e4m3 with ``scale_w [n]``; ``x_shard`` e4m3 with ``scale_x [m_local]``, or bf16 (quantised here)."""
         if x_shard is not None:
-            if self.fp8 and x_shard.dtype != torch.float8_e4m3fn:
-                x_shard, scale_x = quantize_rows(x_shard)
-            self.input.copy_(x_shard)
-            if self.fp8:
-                self.input_scales.copy_(scale_x)
+            quantise = self.fp8 and x_shard.dtype != torch.float8_e4m3fn
+            # bf16 rows are quantised straight into the peer-readable buffers where the kernel takes them.
+            if not (quantise and type(x_shard) is torch.Tensor
+                    and _comms.ops.quantize_rows_into(x_shard, self.input, self.input_scales)):
+                if quantise:
+                    x_shard, scale_x = quantize_rows(x_shard)
+                self.input.copy_(x_shard)
+                if self.fp8:
+                    self.input_scales.copy_(scale_x)
         return self._layer.ag_gemm(w, scale_w)
 
     def status(self):
