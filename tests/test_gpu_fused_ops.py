@@ -128,6 +128,57 @@ def test_cross_entropy_loss_and_gradient(rows, vocab):
     torch.testing.assert_close(work.float(), lf.grad, rtol=3e-2, atol=2e-3)
 
 
+@pytest.mark.parametrize("vocab", [1, 7, 9, 16, 23, 4096, 4097, 16384, 16391, 40003])
+@pytest.mark.parametrize("rows", [1, 300, 1300])
+def test_cross_entropy_row_layouts(rows, vocab):
+    """Heads and tails of rows that start off a 16-byte boundary, every block size, targets at both ends, and rows
+    with masked (-inf, lowest finite) logits."""
+    from torchcomms_b200 import _comms
+
+    logits = _bf(rows, vocab, seed=11, scale=3.0)
+    targets = torch.randint(0, vocab, (rows,), device="cuda")
+    targets[-1], targets[0] = vocab - 1, 0
+    if rows > 8 and vocab > 8:
+        logits[1, 1:] = float("-inf")                        # one allowed token
+        targets[1] = 0
+        logits[2, : vocab // 2] = float("-inf")
+        targets[2] = vocab - 1
+        logits[3] = torch.finfo(torch.bfloat16).min          # everything masked with the lowest value
+        logits[4, : vocab // 2] = torch.finfo(torch.bfloat16).min
+        targets[4] = vocab - 1
+        logits[5] -= 30.0
+        targets[6] = -1
+        targets[7] = vocab
+    ld = logits.double()
+    keep = ((targets >= 0) & (targets < vocab)).double()
+    logp = torch.log_softmax(ld, dim=-1)
+    at = targets.clamp(0, vocab - 1).unsqueeze(1)
+    ref_loss = -logp.gather(1, at).squeeze(1) * keep
+    ref = (logp.exp() - torch.zeros_like(ld).scatter_(1, at, 1.0)) * (0.5 * keep).unsqueeze(1)
+    loss = _comms.ops.cross_entropy_fwd_bwd_(logits, targets, 0.5)
+    if rows > 8 and vocab > 8:  # a row without any allowed token has no meaningful value, but stays finite
+        assert torch.isfinite(loss[3]) and torch.isfinite(logits[3].float()).all()
+        loss, ref_loss, logits, ref = (torch.cat((t[:3], t[4:])) for t in (loss, ref_loss, logits, ref))
+    # fp32 sums of up to 40003 exponentials; p - 1 at the target cancels to the sum's error; bf16 results (2^-9).
+    torch.testing.assert_close(loss.double(), ref_loss, rtol=2e-6, atol=1e-5)
+    torch.testing.assert_close(logits.double(), ref, rtol=2**-8, atol=1e-5)
+
+
+@pytest.mark.parametrize("numel", [1, 8, 4099, 3_000_001])
+def test_scale_by_matches_operators(numel):
+    from torchcomms_b200 import _comms
+
+    t = _bf(numel, seed=12)
+    for value in (1.0, -0.3337, 0.0, float("inf")):
+        f = torch.tensor(value, device="cuda")
+        torch.testing.assert_close(_comms.ops.scale_by(t, f), t * f.to(t.dtype), rtol=0, atol=0, equal_nan=True)
+    w = t[: numel // 2 * 2].view(-1, 2).t() if numel > 1 else t.view(1, 1)
+    assert torch.equal(_comms.ops.scale_by(w, torch.tensor(2.0, device="cuda")), w * 2)
+    assert _comms.ops.scale_by(w, torch.tensor(2.0, device="cuda")).stride() == (w * 2).stride()
+    g = torch.tensor(3.0, device="cuda", requires_grad=True)
+    assert _comms.ops.scale_by(t, g).requires_grad  # a gradient of the gradient keeps its graph
+
+
 def test_linear_cross_entropy_matches_unfused():
     from torchcomms_b200.ops import fused
 

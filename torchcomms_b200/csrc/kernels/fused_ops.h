@@ -50,6 +50,9 @@ cudaError_t launch_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate
 cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, const int64_t* targets, float* loss, int rows,
                                          int vocab, float grad_scale, cudaStream_t s);
 
+// out = in * bf16(*factor) on n bf16 values, the factor read from device memory; in and out 16-byte aligned.
+cudaError_t launch_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* factor, size_t n, cudaStream_t s);
+
 // AdamW on flat fp32 tensors. `grad_scale` multiplies the gradient first
 // (loss scaling / averaging); `step` starts at 1.
 cudaError_t launch_adamw(float* p, const float* g, float* m, float* v, size_t n, float lr, float beta1, float beta2,

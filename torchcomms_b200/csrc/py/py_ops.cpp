@@ -169,6 +169,18 @@ void bind_ops(py::module_& m) {
     return loss;
   });
 
+  // t * factor.to(t.dtype) for a 0-d factor on the device (the gradient of a loss).
+  ops.def("scale_by", [](const at::Tensor& t, const at::Tensor& factor) {
+    const bool direct = plain_call(t) && plain_call(factor) && t.scalar_type() == at::kBFloat16 &&
+        t.is_non_overlapping_and_dense() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0 && factor.dim() == 0 &&
+        factor.scalar_type() == at::kFloat && factor.device() == t.device();
+    if (!direct) return t * factor.to(t.scalar_type());
+    c10::cuda::CUDAGuard g(t.device());
+    at::Tensor out = at::empty_like(t);  // same strides: dense tensors map element by element
+    B200C_CUDA_CHECK(launch_scale_bf16(bf(t), bf_mut(out), factor.data_ptr<float>(), static_cast<size_t>(t.numel()), cur(t)));
+    return out;
+  });
+
   ops.def("adamw_step_", [](at::Tensor p, const at::Tensor& grad, at::Tensor mom, at::Tensor var, double lr, double beta1,
                             double beta2, double eps, double weight_decay, int step, double grad_scale) {
     want(p, at::kFloat, "p");

@@ -130,7 +130,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
         # Mean over all rows; rows with a negative target contribute zero.
         scale = 1.0 / max(rows, 1)
         dx = torch.empty_like(x)
-        dw = torch.zeros_like(weight)
+        dw = torch.empty_like(weight) if x.is_cuda and rows else torch.zeros_like(weight)
         loss_sum = torch.zeros((), dtype=torch.float32, device=x.device)
         for r0 in range(0, rows, chunk_rows):
             r1 = min(rows, r0 + chunk_rows)
@@ -145,14 +145,22 @@ class _LinearCrossEntropy(torch.autograd.Function):
                 onehot = F.one_hot(targets[r0:r1].clamp_min(0), lf.shape[-1]).float()
                 dlogits = ((p - onehot) * (targets[r0:r1] >= 0).unsqueeze(-1) * scale).to(x.dtype)
             loss_sum += loss.sum()
-            dx[r0:r1] = dlogits @ weight
-            dw.addmm_(dlogits.t(), x[r0:r1])
+            if x.is_cuda:
+                torch.mm(dlogits, weight, out=dx[r0:r1])
+            else:
+                dx[r0:r1] = dlogits @ weight
+            if x.is_cuda and r0 == 0:
+                torch.mm(dlogits.t(), x[r0:r1], out=dw)  # the first chunk needs no zeroed gradient to add to
+            else:
+                dw.addmm_(dlogits.t(), x[r0:r1])
         ctx.save_for_backward(dx, dw)
         return loss_sum * scale
 
     @staticmethod
     def backward(ctx, dloss):
         dx, dw = ctx.saved_tensors
+        if dx.is_cuda:
+            return _k.scale_by(dx, dloss), _k.scale_by(dw, dloss), None, None
         return dx * dloss.to(dx.dtype), dw * dloss.to(dw.dtype), None, None
 
 
