@@ -20,6 +20,31 @@ def test_gemm_bf16_nt(m, n, k):
     torch.testing.assert_close(c.float(), ref, rtol=2e-2, atol=2e-2 * (k ** 0.5))
 
 
+@pytest.mark.parametrize("m", [1, 67, 128, 129, 300])
+@pytest.mark.parametrize("n,k", [(8, 8), (136, 72), (128, 256), (136, 264), (3584, 4096), (6144, 1928)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_gemm_split_over_clusters(m, n, k, fp8):
+    """Products of fewer tiles than SMs: every number of K shares, ragged edges in all three sizes."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops.tp import quantize_rows
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = (torch.randn(m, k, generator=g, device="cuda") * 0.5).to(torch.bfloat16)
+    b = (torch.randn(n, k, generator=g, device="cuda") * 0.5).to(torch.bfloat16)
+    if fp8:
+        if k % 16:
+            a, b = torch.nn.functional.pad(a, (0, 8)), torch.nn.functional.pad(b, (0, 8))
+        (qa, sa), (qb, sb) = quantize_rows(a), quantize_rows(b)
+        c, status = _comms.ops.gemm_e4m3_nt(qa, qb, sa, sb)
+        ref = (qa.double() * sa.double().unsqueeze(1)) @ (qb.double() * sb.double().unsqueeze(1)).t()
+    else:
+        c, status = _comms.ops.gemm_bf16_nt(a, b)
+        ref = a.double() @ b.double().t()
+    assert int(status[0]) == 0
+    # Half a bf16 ulp (2^-9 relative), and k fp32 additions of terms of size 1/4 before it.
+    torch.testing.assert_close(c.double(), ref, rtol=2**-8, atol=1e-6 * k)
+
+
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (512, 512, 1024), (300, 264, 200), (1024, 7168, 2048), (4096, 4096, 4096),
                                    (8192, 1792, 512)])
 def test_gemm_bf16_nt_cta_pairs(m, n, k):

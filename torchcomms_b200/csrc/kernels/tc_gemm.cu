@@ -597,7 +597,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
     // the tensor cores are still busy with the remaining tiles.
     if (MODE == TpMode::GEMM_RS) {
       const int ct = threadIdx.x - kGemmThreads;
-      const int my_tiles = tiles_per_src * tiles_n;
+      const int my_tiles = c.nranks > 1 ? tiles_per_src * tiles_n : 0;
       const int first_own = (c.nranks - 1) * tiles_per_src;   // ordinal of this rank's first own m-tile
       // First the tiles this CTA computes for other ranks (they come first in the schedule): as soon as the
       // epilogue has put one into the send staging, move it into its owner's receive staging and flag it.
@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(tp_threads<MODE>(), 1) k_tp_gemm_pair(const __
     if (MODE == TpMode::GEMM_RS) {
       const int ct = threadIdx.x - kGemmThreads;
       const int first_own = (c.nranks - 1) * tiles_per_src;
-      const int my_pair_tiles = (tiles_per_src / 2) * tiles_n;
+      const int my_pair_tiles = c.nranks > 1 ? (tiles_per_src / 2) * tiles_n : 0;
       // forward this CTA's half of the pair tiles computed for other ranks (see k_tp_gemm)
       uint32_t handed = 0;
       bool fwd_ok = true;
@@ -1176,6 +1176,9 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) {
     return cudaErrorInvalidValue;
   }
+  bool done = false;
+  const cudaError_t split = launch_gemm_nt_split(a, b, c, m, n, k, scale_a, scale_b, status, stream, &done);
+  if (split != cudaSuccess || done) return split;
   TpMaps maps;
   if (!make_map(&maps.a_local, a, m, k, kBlockM) || !make_map(&maps.b, b, n, k, kTpBN) ||
       !make_map(&maps.out[0], c, m, n, kBlockM)) {
@@ -1262,7 +1265,8 @@ cudaError_t build_rs(const CommDev& comm, const GemmRsArgs& a, bool pairs, TpMap
   // TMA stores stay on this GPU: own rows go into this rank's receive staging (viewed as [m, n]), the other
   // ranks' rows into the local send staging, from where the forward warps push them with plain stores.
   if (comm.nranks > 1 && a.send_stage == nullptr) return cudaErrorInvalidValue;
-  if (!make_map(&maps.out[comm.rank], a.partials[comm.rank], a.m, a.n, kBlockM)) return cudaErrorInvalidValue;
+  // A single rank has nothing to add up: its tiles are the result.
+  if (!make_map(&maps.out[comm.rank], comm.nranks > 1 ? a.partials[comm.rank] : a.out, a.m, a.n, kBlockM)) return cudaErrorInvalidValue;
   for (int r = 0; r < kMaxRanks; ++r) {
     if (r != comm.rank) maps.out[r] = maps.out[comm.rank];
   }
@@ -1320,6 +1324,12 @@ cudaError_t launch_allgather_gemm(const CommDev& comm, const AgGemmArgs& a, cuda
   const bool pairs = a.m_local > 0 && use_pairs(a.m_local);
   cudaError_t e = build_ag(comm, a, pairs, maps, p);
   if (e != cudaSuccess) return e;
+  if (comm.nranks == 1) {  // nothing to gather: the plain product, where that fills the GPU better
+    bool done = false;
+    e = launch_gemm_nt_split(a.x_shards[0], a.w, a.y, a.m_local, a.n, p.k, a.fp8 ? a.scale_x_shards[0] : nullptr, a.scale_w,
+                             const_cast<uint32_t*>(comm.status), stream, &done);
+    if (e != cudaSuccess || done) return e;
+  }
   if (pairs) return tp_launch_pair<TpMode::AG_GEMM>(0, maps, comm, p, stream);
   // All CTAs take part in the copy, so the grid is the whole GPU even when
   // there are fewer tiles than SMs.
@@ -1332,6 +1342,12 @@ cudaError_t launch_gemm_reduce_scatter(const CommDev& comm, const GemmRsArgs& a,
   const bool pairs = a.m > 0 && comm.nranks > 0 && use_pairs(a.m / comm.nranks);
   cudaError_t e = build_rs(comm, a, pairs, maps, p);
   if (e != cudaSuccess) return e;
+  if (comm.nranks == 1) {  // nothing to scatter
+    bool done = false;
+    e = launch_gemm_nt_split(a.h, a.w, a.out, a.m, a.n, p.k, a.fp8 ? a.scale_h : nullptr, a.scale_w,
+                             const_cast<uint32_t*>(comm.status), stream, &done);
+    if (e != cudaSuccess || done) return e;
+  }
   const int tiles = (a.m / kBlockM) * (a.n / kTpBN);
   if (pairs) return tp_launch_pair<TpMode::GEMM_RS>(tiles / 2, maps, comm, p, stream);
   return tp_launch<TpMode::GEMM_RS>(std::min(sm_count(), tiles), maps, comm, p, stream);
