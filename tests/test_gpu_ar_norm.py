@@ -129,3 +129,24 @@ def test_backend_layer_multi_gpu():
     if world < 2:
         pytest.skip("needs 2 GPUs")
     run_ranks(_backend_worker, world, timeout=150)
+
+
+@pytest.mark.parametrize("hidden", [8, 264, 1000, 4096, 8192])
+@pytest.mark.parametrize("rows", [1, 7, 128])
+def test_single_rank_rows_of_every_width(rows, hidden):
+    """Block sizes from one warp to 1024 threads, rows that end inside a warp."""
+    from torchcomms_b200.ops.ar_norm import AllReduceRMSNorm
+
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(rows * 10000 + hidden)
+    layer = AllReduceRMSNorm(None, hidden)
+    weight = (1.0 + 0.1 * torch.randn(hidden, device=dev)).to(torch.bfloat16)
+    x = torch.randn(rows, hidden, device=dev).to(torch.bfloat16)
+    res = torch.randn(rows, hidden, device=dev).to(torch.bfloat16)
+    stored, normed = _reference([x], res, weight, 1e-5)
+    out = layer(x, weight, residual=res)
+    assert torch.equal(res, stored)                          # one rounding of one fp32 sum
+    # Half a bf16 ulp (2^-9 relative) on top of fp32 sums of up to 8192 squares.
+    torch.testing.assert_close(out.float(), normed, rtol=2**-8, atol=1e-6)
+    torch.testing.assert_close(layer(x, weight).float(), _reference([x], None, weight, 1e-5)[1], rtol=2**-8, atol=1e-6)
+    assert layer.status()[0] == 0
