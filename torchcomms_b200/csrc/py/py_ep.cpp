@@ -300,7 +300,7 @@ class EpBuffer {
       return p;
     };
     e.cnt = static_cast<int*>(local(sizeof(int) * kMaxRanks));
-    e.cursor = static_cast<int*>(local(sizeof(int) * kMaxRanks));
+    e.order = static_cast<int*>(local(sizeof(int) * static_cast<size_t>(max_tokens_) * nranks_));
     e.base = static_cast<long long*>(local(sizeof(long long) * kMaxRanks));
     e.recv_info = static_cast<int*>(local(sizeof(int) * (1 + kMaxRanks)));
     e.send_slot = static_cast<int*>(local(sizeof(int) * static_cast<size_t>(max_tokens_) * nranks_));
