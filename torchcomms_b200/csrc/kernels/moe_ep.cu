@@ -269,7 +269,7 @@ __device__ void ep_combine_body(const CommDev& c, const EpDev& e, const CombineA
   const int cap_rows = e.nranks * e.max_tokens;
   const int* send_slot = a.send_slot != nullptr ? a.send_slot : e.send_slot;
   BlockEpoch ep;
-  ep.load(c, kFlagSetEp);
+  if (RANKS > 1) ep.load(c, kFlagSetEp);
   trace_mark(c, 0);
   bool ok = RANKS == 1 || block_barrier(c, kFlagSetEp, ep, 0x93);
   trace_mark(c, 1);
@@ -367,7 +367,7 @@ __device__ void ep_combine_body(const CommDev& c, const EpDev& e, const CombineA
     ok = RANKS == 1 || block_barrier(c, kFlagSetEp, ep, 0x94);
     trace_mark(c, 3);
   }
-  ep.store(c, kFlagSetEp);
+  if (RANKS > 1) ep.store(c, kFlagSetEp);
 }
 
 __global__ void __launch_bounds__(kEpThreads) k_ep_combine(CommDev c, EpDev e, CombineArgs a) {

@@ -55,6 +55,8 @@ struct EpLlRecv {
   int* packed_src;          // [local experts][nranks * max_tokens] source token index
   int* packed_count;        // [local experts]
   long long* layout_range;  // [local experts][nranks]: (first packed row << 32) | rows
+  int* send_slot;           // [tokens][topk] copy of the source-side handle, or null
+  int* begin;               // [num_experts] likewise
 };
 
 cudaError_t launch_ep_ll_dispatch(const CommDev* comms, const EpLlDev* eps, int emu_ranks, const void* const* x,

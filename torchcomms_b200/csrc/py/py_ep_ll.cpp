@@ -84,8 +84,9 @@ class EpLlBuffer {
   int local_experts() const { return num_experts_ / nranks_; }
   int rows_per_expert() const { return nranks_ * max_tokens_; }
 
-  // Outputs per local rank: packed_x, packed_scales (fp8 only, else undefined), packed_src, packed_count, layout_range.
-  std::vector<std::vector<at::Tensor>> dispatch(std::vector<at::Tensor> x, std::vector<at::Tensor> topk_idx) {
+  // Outputs per local rank: packed_x, packed_scales (fp8 only, else undefined), packed_src, packed_count, layout_range;
+  // with `handles` also this call's send_slot and begin (which the views of those names hold until the next call).
+  std::vector<std::vector<at::Tensor>> dispatch(std::vector<at::Tensor> x, std::vector<at::Tensor> topk_idx, bool handles) {
     TORCH_CHECK(static_cast<int>(x.size()) == n_local_ && static_cast<int>(topk_idx.size()) == n_local_,
                 "one tensor per local rank expected");
     const int T = static_cast<int>(x[0].size(0));
@@ -112,8 +113,15 @@ class EpLlBuffer {
       at::Tensor count = at::empty({Le}, opts.dtype(at::kInt));
       at::Tensor range = at::empty({Le, nranks_}, opts.dtype(at::kLong));
       recv[i] = {px.data_ptr(), fp8_ ? ps.data_ptr<float>() : nullptr, src.data_ptr<int>(), count.data_ptr<int>(),
-                 reinterpret_cast<long long*>(range.data_ptr<int64_t>())};
+                 reinterpret_cast<long long*>(range.data_ptr<int64_t>()), nullptr, nullptr};
       outs[i] = {px, ps, src, count, range};
+      if (handles) {
+        at::Tensor slot = at::empty({T, topk_}, opts.dtype(at::kInt)), begin = at::empty({num_experts_}, opts.dtype(at::kInt));
+        recv[i].send_slot = slot.data_ptr<int>();
+        recv[i].begin = begin.data_ptr<int>();
+        outs[i].insert(outs[i].end(), {slot, begin});
+        keep.insert(keep.end(), {slot, begin});
+      }
       keep.insert(keep.end(), {x[i], topk_idx[i], px, src, count, range});
       if (fp8_) keep.push_back(ps);
     }
@@ -284,7 +292,7 @@ void bind_ep_ll(py::module_& m) {
         return std::make_unique<EpLlBuffer>(nranks, max_tokens, hidden, num_experts, topk, fp8, wait_ms);
       }, py::arg("nranks"), py::arg("max_tokens"), py::arg("hidden"), py::arg("num_experts"), py::arg("topk"),
          py::arg("fp8") = true, py::arg("wait_ms") = 2000.0)
-      .def("dispatch", &EpLlBuffer::dispatch)
+      .def("dispatch", &EpLlBuffer::dispatch, py::arg("x"), py::arg("topk_idx"), py::arg("handles") = false)
       .def("combine", &EpLlBuffer::combine, py::arg("out"), py::arg("topk_idx"), py::arg("topk_weights"),
            py::arg("send_slot") = std::vector<at::Tensor>{}, py::arg("begin") = std::vector<at::Tensor>{})
       .def("view", &EpLlBuffer::view, py::arg("local_rank"), py::arg("what"))

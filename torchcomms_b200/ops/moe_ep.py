@@ -244,10 +244,9 @@ class LowLatencyBuffer:
         return self._buf.view(0, "out_x")
 
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor) -> LowLatencyRecv:
-        px, ps, src, count, rng = self._buf.dispatch([x.contiguous()], [topk_idx.to(torch.int32).contiguous()])[0]
-        t = x.shape[0]
-        return LowLatencyRecv(px, ps if self.fp8 else None, count, src, rng,
-                              self._buf.view(0, "send_slot")[:t].clone(), self._buf.view(0, "begin").clone())
+        px, ps, src, count, rng, slot, begin = self._buf.dispatch([x.contiguous()], [topk_idx.to(torch.int32).contiguous()],
+                                                                  True)[0]
+        return LowLatencyRecv(px, ps if self.fp8 else None, count, src, rng, slot, begin)
 
     def combine(self, topk_idx: torch.Tensor, topk_weights: torch.Tensor, recv: Optional[LowLatencyRecv] = None,
                 x: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
