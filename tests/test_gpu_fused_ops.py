@@ -65,6 +65,21 @@ def test_swiglu_forward_backward():
     torch.testing.assert_close(gu.grad.float(), guf.grad, rtol=3e-2, atol=3e-2)
 
 
+@pytest.mark.parametrize("rows,ffn", [(1, 8), (3, 264), (511, 8), (1025, 520), (7, 14336)])
+def test_swiglu_every_vector(rows, ffn):
+    """Row lengths that end anywhere in a block's span of vectors."""
+    from torchcomms_b200 import _comms
+
+    gu, dh = _bf(rows, 2 * ffn, seed=4, scale=3.0), _bf(rows, ffn, seed=5)
+    gud = gu.double().requires_grad_(True)
+    g, u = gud.chunk(2, dim=-1)
+    ref = F.silu(g) * u
+    (rdgu,) = torch.autograd.grad(ref, gud, dh.double())
+    # Half a bf16 ulp (2^-9 relative); the derivative of silu crosses zero, where fp32 terms of size 30 cancel.
+    torch.testing.assert_close(_comms.ops.swiglu_fwd(gu).double(), ref.detach(), rtol=2**-8, atol=1e-6)
+    torch.testing.assert_close(_comms.ops.swiglu_bwd(dh, gu).double(), rdgu, rtol=2**-8, atol=2e-5)
+
+
 def test_rope_matches_complex_rotation_and_inverts():
     from torchcomms_b200.ops import fused
 

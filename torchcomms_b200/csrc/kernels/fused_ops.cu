@@ -387,49 +387,74 @@ __global__ void __launch_bounds__(256) k_rope(const __nv_bfloat16* x, __nv_bfloa
 
 // -------------------------------------------------------------- SwiGLU ------
 
-__global__ void k_swiglu_fwd(const __nv_bfloat16* __restrict__ gate_up, __nv_bfloat16* __restrict__ h, int rows, int ffn) {
-  const int vec_per_row = ffn / 8;
-  const size_t total = static_cast<size_t>(rows) * vec_per_row;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const size_t r = i / vec_per_row;
-    const int v = static_cast<int>(i % vec_per_row);
-    const uint4* row = reinterpret_cast<const uint4*>(gate_up + r * 2 * static_cast<size_t>(ffn));
-    float g[8], u[8], o[8];
-    unpack8(row[v], g);
-    unpack8(row[vec_per_row + v], u);
+// Both directions stream their operands once and are bound by memory: every thread takes kSwigluVecs vectors of
+// each operand, all loads before the first use, and finds its row with a multiply instead of a 64-bit division.
+// [4096, 2 x 14336]: forward 60.8 us, now 53.8 (6.5 TB/s); backward 101.2 us, now 83.5 (7.0 TB/s).
+constexpr int kSwigluVecs = 2;
+
+__device__ __forceinline__ float sigmoid_of(float g) { return 1.0f / (1.0f + __expf(-g)); }
+
+__global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* __restrict__ gate_up, __nv_bfloat16* __restrict__ h,
+                                                    uint32_t total, FastDiv per_row) {
+  const uint32_t base = blockIdx.x * (256u * kSwigluVecs) + threadIdx.x;
+  uint4 gv[kSwigluVecs], uv[kSwigluVecs];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float sig = 1.0f / (1.0f + __expf(-g[k]));
-      o[k] = g[k] * sig * u[k];
+  for (int k = 0; k < kSwigluVecs; ++k) {
+    const uint32_t i = base + k * 256u;
+    if (i < total) {
+      // row r holds 2 x per_row vectors: gate, then up
+      const size_t at = static_cast<size_t>(i) + static_cast<size_t>(fast_div(i, per_row)) * per_row.d;
+      gv[k] = reinterpret_cast<const uint4*>(gate_up)[at];
+      uv[k] = reinterpret_cast<const uint4*>(gate_up)[at + per_row.d];
     }
-    reinterpret_cast<uint4*>(h)[i] = pack8(o);
+  }
+#pragma unroll
+  for (int k = 0; k < kSwigluVecs; ++k) {
+    const uint32_t i = base + k * 256u;
+    if (i < total) {
+      float g[8], u[8], o[8];
+      unpack8(gv[k], g);
+      unpack8(uv[k], u);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoid_of(g[j]) * u[j];
+      reinterpret_cast<uint4*>(h)[i] = pack8(o);
+    }
   }
 }
 
-__global__ void k_swiglu_bwd(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gate_up,
-                             __nv_bfloat16* __restrict__ dgate_up, int rows, int ffn) {
-  const int vec_per_row = ffn / 8;
-  const size_t total = static_cast<size_t>(rows) * vec_per_row;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const size_t r = i / vec_per_row;
-    const int v = static_cast<int>(i % vec_per_row);
-    const uint4* row = reinterpret_cast<const uint4*>(gate_up + r * 2 * static_cast<size_t>(ffn));
-    uint4* drow = reinterpret_cast<uint4*>(dgate_up + r * 2 * static_cast<size_t>(ffn));
-    float g[8], u[8], d[8], dg[8], du[8];
-    unpack8(row[v], g);
-    unpack8(row[vec_per_row + v], u);
-    unpack8(reinterpret_cast<const uint4*>(dh)[i], d);
+__global__ void __launch_bounds__(256) k_swiglu_bwd(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gate_up,
+                                                    __nv_bfloat16* __restrict__ dgate_up, uint32_t total, FastDiv per_row) {
+  const uint32_t base = blockIdx.x * (256u * kSwigluVecs) + threadIdx.x;
+  uint4 gv[kSwigluVecs], uv[kSwigluVecs], dv[kSwigluVecs];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float sig = 1.0f / (1.0f + __expf(-g[k]));
-      const float silu = g[k] * sig;
-      dg[k] = d[k] * u[k] * (sig + silu * (1.0f - sig));
-      du[k] = d[k] * silu;
+  for (int k = 0; k < kSwigluVecs; ++k) {
+    const uint32_t i = base + k * 256u;
+    if (i < total) {
+      const size_t at = static_cast<size_t>(i) + static_cast<size_t>(fast_div(i, per_row)) * per_row.d;
+      gv[k] = reinterpret_cast<const uint4*>(gate_up)[at];
+      uv[k] = reinterpret_cast<const uint4*>(gate_up)[at + per_row.d];
+      dv[k] = reinterpret_cast<const uint4*>(dh)[i];
     }
-    drow[v] = pack8(dg);
-    drow[vec_per_row + v] = pack8(du);
+  }
+#pragma unroll
+  for (int k = 0; k < kSwigluVecs; ++k) {
+    const uint32_t i = base + k * 256u;
+    if (i < total) {
+      const size_t at = static_cast<size_t>(i) + static_cast<size_t>(fast_div(i, per_row)) * per_row.d;
+      float g[8], u[8], d[8], dg[8], du[8];
+      unpack8(gv[k], g);
+      unpack8(uv[k], u);
+      unpack8(dv[k], d);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float sig = sigmoid_of(g[j]);
+        const float silu = g[j] * sig;
+        dg[j] = d[j] * u[j] * (sig + silu * (1.0f - sig));
+        du[j] = d[j] * silu;
+      }
+      reinterpret_cast<uint4*>(dgate_up)[at] = pack8(dg);
+      reinterpret_cast<uint4*>(dgate_up)[at + per_row.d] = pack8(du);
+    }
   }
 }
 
@@ -856,19 +881,39 @@ cudaError_t launch_rope(const __nv_bfloat16* x, int64_t stride_t, int64_t stride
   return cudaGetLastError();
 }
 
+namespace {
+
+// Calls fn(first row, vectors) for slices of whole rows whose vectors fit 32-bit indices (one slice but for tensors
+// of many gigabytes).
+template <typename Fn>
+cudaError_t for_row_slices(int rows, int per_row, Fn fn) {
+  if (rows <= 0 || per_row <= 0) return cudaSuccess;
+  const int slice = std::max(1, (1 << 30) / per_row);
+  for (int r0 = 0; r0 < rows; r0 += std::min(slice, rows - r0)) {
+    const uint32_t total = static_cast<uint32_t>(std::min(slice, rows - r0)) * static_cast<uint32_t>(per_row);
+    fn(static_cast<size_t>(r0), total);
+    note_kernel_launch();
+  }
+  return cudaGetLastError();
+}
+
+} // namespace
+
 cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, int rows, int ffn, cudaStream_t s) {
   if (ffn % 8 != 0) return cudaErrorInvalidValue;
-  k_swiglu_fwd<<<grid_for(static_cast<size_t>(rows) * (ffn / 8), 256), 256, 0, s>>>(gate_up, h, rows, ffn);
-  note_kernel_launch();
-  return cudaGetLastError();
+  return for_row_slices(rows, ffn / 8, [&](size_t r0, uint32_t total) {
+    k_swiglu_fwd<<<(total + 256u * kSwigluVecs - 1) / (256u * kSwigluVecs), 256, 0, s>>>(gate_up + r0 * 2 * ffn, h + r0 * ffn, total,
+                                                                                        make_fast_div(ffn / 8));
+  });
 }
 
 cudaError_t launch_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate_up, __nv_bfloat16* dgate_up, int rows,
                               int ffn, cudaStream_t s) {
   if (ffn % 8 != 0) return cudaErrorInvalidValue;
-  k_swiglu_bwd<<<grid_for(static_cast<size_t>(rows) * (ffn / 8), 256), 256, 0, s>>>(dh, gate_up, dgate_up, rows, ffn);
-  note_kernel_launch();
-  return cudaGetLastError();
+  return for_row_slices(rows, ffn / 8, [&](size_t r0, uint32_t total) {
+    k_swiglu_bwd<<<(total + 256u * kSwigluVecs - 1) / (256u * kSwigluVecs), 256, 0, s>>>(
+        dh + r0 * ffn, gate_up + r0 * 2 * ffn, dgate_up + r0 * 2 * ffn, total, make_fast_div(ffn / 8));
+  });
 }
 
 cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, const int64_t* targets, float* loss, int rows, int vocab,
