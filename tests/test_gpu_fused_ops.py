@@ -5,6 +5,7 @@ import os
 import pytest
 import torch
 import torch.nn.functional as F
+import torch.utils.checkpoint
 
 pytestmark = pytest.mark.gpu
 
@@ -225,6 +226,62 @@ def test_adamw_matches_torch():
         opt.step()
         fused.adamw_step_(p, g, m, v, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=step)
     torch.testing.assert_close(p, ref_p.detach(), rtol=1e-4, atol=1e-5)
+
+
+def _op_calls():
+    from torchcomms_b200.ops import fused
+
+    cos_t, sin_t = fused.rope_tables(64, 64, 10000.0, "cuda")
+    pos = torch.arange(24, dtype=torch.int32, device="cuda")
+    w = (_bf(256, seed=20, scale=0.1) + 1).detach().requires_grad_(True)
+    return {
+        "rms_norm": (lambda x: fused.rms_norm(x, w, 1e-5), (24, 256), fused._RmsNorm, (w, 1e-5)),
+        "swiglu": (lambda x: fused.swiglu(x), (24, 512), fused._SwiGlu, ()),
+        "apply_rope": (lambda x: fused.apply_rope(x, pos, cos_t, sin_t), (24, 4, 64), fused._Rope, (pos, cos_t, sin_t)),
+    }
+
+
+@pytest.mark.parametrize("name", ["rms_norm", "swiglu", "apply_rope"])
+def test_native_autograd_nodes(name):
+    """Same values and gradients as the autograd functions in Python, hooks and graph modes seen alike."""
+    call, shape, function, rest = _op_calls()[name]
+    x = _bf(*shape, seed=21).requires_grad_(True)
+    y, ref = call(x), function.apply(x, *rest)
+    assert y.grad_fn.name() != ref.grad_fn.name()
+    assert torch.equal(y, ref)
+    g = _bf(*y.shape, seed=22)
+    leaves = (x,) + tuple(t for t in rest if isinstance(t, torch.Tensor) and t.requires_grad)
+    for a, b in zip(torch.autograd.grad(y, leaves, g, retain_graph=True), torch.autograd.grad(ref, leaves, g)):
+        assert torch.equal(a, b)
+    for a, b in zip(torch.autograd.grad(y, leaves, g, retain_graph=True), torch.autograd.grad(y, leaves, g)):
+        assert torch.equal(a, b)                                   # a second pass over a retained graph
+    # saved tensors go through hooks (activation checkpointing and offloading rest on them)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.clone(), lambda t: t):
+        z = call(x)
+    (dx,) = torch.autograd.grad(z, x, g)
+    assert packed and torch.equal(dx, torch.autograd.grad(call(x), x, g)[0])
+    c = torch.utils.checkpoint.checkpoint(call, x, use_reentrant=False)
+    assert torch.equal(torch.autograd.grad(c, x, g)[0], dx)
+    with torch.no_grad():
+        assert call(x).grad_fn is None
+    # inputs of any layout, and calls on another stream
+    xt = _bf(*shape[:-2], shape[-1], shape[-2], seed=23).transpose(-1, -2)
+    assert torch.equal(call(xt), call(xt.contiguous()))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        ys = call(x)
+    torch.cuda.current_stream().wait_stream(side)
+    assert torch.equal(ys, y)
+    # forward mode and vmap are refused as by the autograd functions in Python
+    import torch.autograd.forward_ad as fwad
+
+    with fwad.dual_level():
+        with pytest.raises(Exception):
+            call(fwad.make_dual(x.detach(), torch.ones_like(x)))
+    with pytest.raises(Exception):
+        torch.func.vmap(call)(x.detach().unsqueeze(0).expand(2, *shape))
 
 
 def test_engine_step_on_gpu_matches_reference_forward():

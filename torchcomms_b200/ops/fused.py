@@ -30,6 +30,15 @@ def kernel_launch_count() -> int:
     return int(_k.kernel_launch_count())
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _native(*tensors: torch.Tensor) -> bool:
+    """Whether the native autograd nodes may be asked (they look at the rest themselves): no tensor subclasses, no
+    compilation, which traces the autograd functions below."""
+    return all(type(t) in _PLAIN for t in tensors) and not torch.compiler.is_compiling()
+
+
 # ------------------------------------------------------------------ RMSNorm
 
 
@@ -49,7 +58,8 @@ class _RmsNorm(torch.autograd.Function):
 
 def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
     if x.is_cuda:
-        return _RmsNorm.apply(x.contiguous(), w, eps)
+        y = _k.rms_norm(x, w, eps) if _native(x, w) else None
+        return _RmsNorm.apply(x.contiguous(), w, eps) if y is None else y
     xf = x.float()
     y = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps) * w.float()
     return y.to(x.dtype)
@@ -73,7 +83,8 @@ class _SwiGlu(torch.autograd.Function):
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` for ``gate_up = [..., 2*ffn]`` (gate first)."""
     if gate_up.is_cuda:
-        return _SwiGlu.apply(gate_up.contiguous())
+        h = _k.swiglu(gate_up) if _native(gate_up) else None
+        return _SwiGlu.apply(gate_up.contiguous()) if h is None else h
     gate, up = gate_up.float().chunk(2, dim=-1)
     return (F.silu(gate) * up).to(gate_up.dtype)
 
@@ -102,7 +113,8 @@ class _Rope(torch.autograd.Function):
 def apply_rope(x: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor) -> torch.Tensor:
     """Rotates interleaved pairs of ``x = [tokens, heads, head_dim]`` by the angle of ``pos[token]``."""
     if x.is_cuda:
-        return _Rope.apply(x, pos, cos_t, sin_t)
+        y = _k.apply_rope(x, pos, cos_t, sin_t) if _native(x, pos, cos_t, sin_t) else None
+        return _Rope.apply(x, pos, cos_t, sin_t) if y is None else y
     xf = x.float().reshape(*x.shape[:-1], -1, 2)
     c = cos_t[pos.long()].unsqueeze(-2)  # [tokens, 1, hd/2]
     s = sin_t[pos.long()].unsqueeze(-2)
