@@ -228,6 +228,33 @@ def test_adamw_matches_torch():
     torch.testing.assert_close(p, ref_p.detach(), rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("factor", [1.0, 0.37])
+def test_linear_cross_entropy_gradients_are_handed_out_once(factor):
+    """The last backward gives its gradients away in place; retained graphs, hooks and later passes get copies."""
+    from torchcomms_b200.ops import fused
+
+    x, w = _bf(64, 128, seed=30).requires_grad_(True), _bf(1000, 128, seed=31, scale=0.05).requires_grad_(True)
+    t = torch.randint(0, 1000, (64,), device="cuda")
+    g = torch.tensor(factor, device="cuda")
+    first = torch.autograd.grad(fused.linear_cross_entropy(x, w, t), (x, w), g)
+    loss = fused.linear_cross_entropy(x, w, t)
+    a = torch.autograd.grad(loss, (x, w), g, retain_graph=True)
+    b = torch.autograd.grad(loss, (x, w), 2 * g, retain_graph=True)
+    c = torch.autograd.grad(loss, (x, w), g)
+    for f, p, q, r in zip(first, a, b, c):
+        assert torch.equal(f, p) and torch.equal(p, r) and p.data_ptr() != r.data_ptr()
+        torch.testing.assert_close(q.float(), 2 * p.float(), rtol=2**-7, atol=0)   # two bf16 roundings apart
+    kept = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda s: kept.append(s) or s, lambda s: s):
+        loss = fused.linear_cross_entropy(x, w, t)
+    before = [k.clone() for k in kept]
+    d = torch.autograd.grad(loss, (x, w), g)
+    assert all(torch.equal(k, b) for k, b in zip(kept, before)) and all(torch.equal(p, q) for p, q in zip(d, first))
+    loss = fused.linear_cross_entropy(x, w, t) * factor             # reaches .grad the same way
+    loss.backward()
+    assert torch.equal(x.grad, first[0]) and torch.equal(w.grad, first[1])
+
+
 def _op_calls():
     from torchcomms_b200.ops import fused
 

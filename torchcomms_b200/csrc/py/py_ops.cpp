@@ -1,6 +1,7 @@
 // Tensor-level bindings of the fused model kernels (`_comms.ops`).
 #include "py_common.hpp"
 
+#include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -238,17 +239,20 @@ void bind_ops(py::module_& m) {
     return loss;
   });
 
-  // t * factor.to(t.dtype) for a 0-d factor on the device (the gradient of a loss).
-  ops.def("scale_by", [](const at::Tensor& t, const at::Tensor& factor) {
+  // t * factor.to(t.dtype) for a 0-d factor on the device (the gradient of a loss). `consume`: nobody reads t
+  // afterwards, so the product may take its place.
+  ops.def("scale_by", [](const at::Tensor& t, const at::Tensor& factor, bool consume) {
     const bool direct = plain_call(t) && plain_call(factor) && t.scalar_type() == at::kBFloat16 &&
         t.is_non_overlapping_and_dense() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0 && factor.dim() == 0 &&
         factor.scalar_type() == at::kFloat && factor.device() == t.device();
     if (!direct) return t * factor.to(t.scalar_type());
     c10::cuda::CUDAGuard g(t.device());
-    at::Tensor out = at::empty_like(t);  // same strides: dense tensors map element by element
+    at::Tensor out = consume ? t : at::empty_like(t);  // same strides: dense tensors map element by element
     B200C_CUDA_CHECK(launch_scale_bf16(bf(t), bf_mut(out), factor.data_ptr<float>(), static_cast<size_t>(t.numel()), cur(t)));
     return out;
-  });
+  }, py::arg("t"), py::arg("factor"), py::arg("consume") = false);
+  // Whether tensors that autograd saves now go through hooks (which may keep them).
+  ops.def("saved_tensor_hooks_active", []() { return at::SavedTensorDefaultHooks::get_hooks().has_value(); });
 
   ops.def("adamw_step_", [](at::Tensor p, const at::Tensor& grad, at::Tensor mom, at::Tensor var, double lr, double beta1,
                             double beta2, double eps, double weight_decay, int step, double grad_scale) {

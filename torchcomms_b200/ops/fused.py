@@ -166,13 +166,18 @@ class _LinearCrossEntropy(torch.autograd.Function):
             else:
                 dw.addmm_(dlogits.t(), x[r0:r1])
         ctx.save_for_backward(dx, dw)
+        # The gradients belong to this node alone unless a hook was handed them.
+        ctx.own = x.is_cuda and not _k.saved_tensor_hooks_active()
         return loss_sum * scale
 
     @staticmethod
     def backward(ctx, dloss):
         dx, dw = ctx.saved_tensors
-        if dx.is_cuda:
-            return _k.scale_by(dx, dloss), _k.scale_by(dw, dloss), None, None
+        if dx.is_cuda and _native(dx, dw, dloss):
+            # A backward that frees the graph hands them out themselves; the gradient of the weight is the size of the
+            # weight, and a copy of it would take longer than the loss kernel.
+            last = ctx.own and not torch._C._autograd._get_current_graph_task_keep_graph()
+            return _k.scale_by(dx, dloss, last), _k.scale_by(dw, dloss, last), None, None
         return dx * dloss.to(dx.dtype), dw * dloss.to(dw.dtype), None, None
 
 
