@@ -228,6 +228,61 @@ def test_adamw_matches_torch():
     torch.testing.assert_close(p, ref_p.detach(), rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 8), (9, 256), (40, 512), (700, 1000), (5, 2048), (601, 4096), (3, 8192), (300, 8192)])
+def test_norm_with_residual_stream(rows, cols):
+    """x + delta and its norm in one kernel: forward bit for bit what addition and norm give, backward with the
+    residual's gradient added in fp32."""
+    from torchcomms_b200.ops import fused
+
+    w = (_bf(cols, seed=42, scale=0.1) + 1).detach().requires_grad_(True)
+    x, d = _bf(rows, cols, seed=40).requires_grad_(True), _bf(rows, cols, seed=41).requires_grad_(True)
+    s, y = fused.add_rms_norm(x, d, w, 1e-5)
+    assert torch.equal(s, (x + d).detach()) and torch.equal(y, fused.rms_norm((x + d).detach(), w, 1e-5))
+    gs, gy = _bf(rows, cols, seed=43), _bf(rows, cols, seed=44)
+    sd, wd = s.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    ref = sd * torch.rsqrt(sd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd
+    rs, rw = torch.autograd.grad(ref, (sd, wd), gy.double())
+    # Half a bf16 ulp (2^-9 relative) on top of fp32 sums of up to 8192 (ds) or `rows` (dw) terms of unit size.
+    for got, skip in ((torch.autograd.grad((s, y), (x, d, w), (gs, gy)), gs.double()),):
+        torch.testing.assert_close(got[0].double(), rs + skip, rtol=2**-8, atol=2e-5)
+        assert torch.equal(got[0], got[1])
+        torch.testing.assert_close(got[2].double(), rw, rtol=2**-8, atol=1e-6 * rows**0.5 + 2e-5)
+    x2 = s.detach().requires_grad_(True)
+    skip, y2 = fused.rms_norm_skip(x2, w, 1e-5)
+    assert torch.equal(skip, x2) and torch.equal(y2, y)
+    (dx,) = torch.autograd.grad((skip, y2), x2, (gs, gy), retain_graph=True)
+    assert torch.equal(dx, got[0])
+    (dx,) = torch.autograd.grad(y2, x2, gy)                        # a result nobody used counts as zero
+    torch.testing.assert_close(dx.double(), rs, rtol=2**-8, atol=2e-5)
+
+
+@pytest.mark.parametrize("tokens,heads,kv,hd", [(1, 1, 1, 8), (37, 6, 2, 96), (1000, 8, 8, 64), (513, 4, 1, 128)])
+@pytest.mark.parametrize("layout", ["contiguous", "transposed", "odd"])
+def test_split_rope_matches_split_and_rotate(tokens, heads, kv, hd, layout):
+    """Same bits as splitting the projection and rotating the pieces, in both directions, for gradients of any layout."""
+    from torchcomms_b200.ops import fused
+
+    cos_t, sin_t = fused.rope_tables(2048, hd, 10000.0, "cuda")
+    pos = torch.randint(0, 2048, (tokens,), dtype=torch.int32, device="cuda")
+    qkv = _bf(tokens, (heads + 2 * kv) * hd, seed=50).requires_grad_(True)
+    q, k, v = qkv.split([heads * hd, kv * hd, kv * hd], dim=-1)
+    want = (fused.apply_rope(q.reshape(tokens, heads, hd), pos, cos_t, sin_t),
+            fused.apply_rope(k.reshape(tokens, kv, hd), pos, cos_t, sin_t), v.reshape(tokens, kv, hd))
+    got = fused.split_rope(qkv, pos, cos_t, sin_t, heads, kv)
+    grads = []
+    for i, n in enumerate((heads, kv, kv)):
+        if layout == "contiguous":
+            grads.append(_bf(tokens, n, hd, seed=51 + i))
+        elif layout == "transposed":
+            grads.append(_bf(n, tokens, hd, seed=51 + i).transpose(0, 1))
+        else:
+            grads.append(_bf(tokens, n, hd + 1, seed=51 + i)[:, :, 1:])
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    (da,), (db,) = torch.autograd.grad(got, qkv, grads), torch.autograd.grad(want, qkv, grads)
+    assert torch.equal(da, db)
+
+
 @pytest.mark.parametrize("factor", [1.0, 0.37])
 def test_linear_cross_entropy_gradients_are_handed_out_once(factor):
     """The last backward gives its gradients away in place; retained graphs, hooks and later passes get copies."""

@@ -91,9 +91,12 @@ __device__ __forceinline__ float row_sum(float v, float (*scratch)[TPR / 32], in
 
 // Rows that fit the registers of TPR threads (VPT vectors of 8 each): one pass, all loads before the reduction.
 // Bound by memory; [4096, 4096]: 16.2 us when blocks of 256 walked rows in a fixed stride, 11.9 us (5.6 TB/s) now.
-template <int TPR, int VPT>
+// ADD: the row is x + delta, rounded to bf16 and also written to `sum` (the residual stream).
+template <int TPR, int VPT, bool ADD>
 __global__ void __launch_bounds__(TPR < 128 ? 128 : TPR) k_rmsnorm_fwd_reg(const __nv_bfloat16* __restrict__ x,
+                                                                            const __nv_bfloat16* __restrict__ delta,
                                                                             const __nv_bfloat16* __restrict__ w,
+                                                                            __nv_bfloat16* __restrict__ sum,
                                                                             __nv_bfloat16* __restrict__ y,
                                                                             float* __restrict__ rstd, int rows, int cols,
                                                                             float eps) {
@@ -110,10 +113,31 @@ __global__ void __launch_bounds__(TPR < 128 ? 128 : TPR) k_rmsnorm_fwd_reg(const
     const int v = lane + k * TPR;
     keep[k] = v < nvec ? xr[v] : make_uint4(0u, 0u, 0u, 0u);
   }
+  uint4 add[ADD ? VPT : 1];
+  if constexpr (ADD) {
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int v = lane + k * TPR;
+      add[k] = v < nvec ? reinterpret_cast<const uint4*>(delta + static_cast<size_t>(r) * cols)[v] : make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
     const int v = lane + k * TPR;
     if (v < nvec) wv[k] = reinterpret_cast<const uint4*>(w)[v];
+  }
+  if constexpr (ADD) {
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int v = lane + k * TPR;
+      float f[8], g[8];
+      unpack8(keep[k], f);
+      unpack8(add[k], g);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] += g[i];
+      keep[k] = pack8(f);
+      if (v < nvec) reinterpret_cast<uint4*>(sum + static_cast<size_t>(r) * cols)[v] = keep[k];
+    }
   }
   float ss = 0.0f;
 #pragma unroll
@@ -182,11 +206,13 @@ constexpr int norm_bwd_threads() { return TPR < kNormThreads ? kNormThreads : TP
 template <int TPR, int VPT>
 constexpr int norm_bwd_per_sm() { return TPR > 256 || (TPR == 32 && VPT == 4) ? 1 : 2; }
 
-template <int TPR, int VPT>
+// ADD: the row also fed something else, whose gradient `dskip` is added before the one rounding of dx.
+template <int TPR, int VPT, bool ADD>
 __global__ void __launch_bounds__(norm_bwd_threads<TPR>(), norm_bwd_per_sm<TPR, VPT>()) k_rmsnorm_bwd(const __nv_bfloat16* __restrict__ dy,
                                                                   const __nv_bfloat16* __restrict__ x,
                                                                   const __nv_bfloat16* __restrict__ w,
                                                                   const float* __restrict__ rstd,
+                                                                  const __nv_bfloat16* __restrict__ dskip,
                                                                   __nv_bfloat16* __restrict__ dx,
                                                                   float* __restrict__ dw_partial, int rows, int cols) {
   constexpr int kThreads = norm_bwd_threads<TPR>(), kRows = kThreads / TPR;
@@ -225,6 +251,14 @@ __global__ void __launch_bounds__(norm_bwd_threads<TPR>(), norm_bwd_per_sm<TPR, 
     }
     const float rs = nrs;
     if (r + step < rows) fetch(r + step);
+    uint4 skip[ADD ? VPT : 1];
+    if constexpr (ADD) {
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const int v = lane + k * TPR;
+        skip[k] = v < nvec ? reinterpret_cast<const uint4*>(dskip + static_cast<size_t>(r) * cols)[v] : zero;
+      }
+    }
     float dot = 0.0f;  // sum(dy * w * x)
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
@@ -251,6 +285,12 @@ __global__ void __launch_bounds__(norm_bwd_threads<TPR>(), norm_bwd_per_sm<TPR, 
           const float xhat = fx[i] * rs;
           o[i] = rs * (fd[i] * fw[i] - xhat * dot);
           dw[k][i] += fd[i] * xhat;
+        }
+        if constexpr (ADD) {
+          float fs[8];
+          unpack8(skip[k], fs);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] += fs[i];
         }
         dxr[v] = pack8(o);
       }
@@ -339,6 +379,18 @@ __device__ __forceinline__ uint32_t fast_div(uint32_t n, FastDiv f) {
   return f.d == 1 ? n : __umulhi(n, f.mul) >> f.shift;
 }
 
+// Rotates the four pairs of a vector. Spelled out, so that every kernel rounds alike.
+__device__ __forceinline__ void rotate8(float* f, float4 c4, float4 s4, float sign) {
+  const float* c = &c4.x;
+  const float* s = &s4.x;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float a = f[2 * j], b = f[2 * j + 1], sj = s[j] * sign;
+    f[2 * j] = __fmaf_rn(-b, sj, __fmul_rn(a, c[j]));
+    f[2 * j + 1] = __fmaf_rn(a, sj, __fmul_rn(b, c[j]));
+  }
+}
+
 // Bound by memory: every element is read and written once, so the source is read where the caller has it (a
 // slice of the fused projection's output) instead of being copied first and rotated in place, and the result is
 // the only write. Four vectors of 8 bf16 per thread, all loads before the first use. Queries and keys of 4093 tokens
@@ -371,16 +423,64 @@ __global__ void __launch_bounds__(256) k_rope(const __nv_bfloat16* x, __nv_bfloa
     if (i < total) {
       float f[8];
       unpack8(in[k], f);
-      const float* c = &cs[k].x;
-      const float* s = &sn[k].x;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float a = f[2 * j], b = f[2 * j + 1];
-        const float sj = s[j] * sign;
-        f[2 * j] = a * c[j] - b * sj;
-        f[2 * j + 1] = a * sj + b * c[j];
-      }
+      rotate8(f, cs[k], sn[k], sign);
       reinterpret_cast<uint4*>(y)[i] = pack8(f);
+    }
+  }
+}
+
+// Both directions of what sits between a fused QKV projection and attention. `packed` is the projection's output
+// (or its gradient), rows of (heads + 2 kv_heads) x head_dim; `part[0..2]` are queries, keys and values with their
+// own strides. Forward reads `packed`, rotates queries and keys and copies values; backward does the reverse, so
+// the gradient of the projection is written once, without rotating pieces first and joining them afterwards.
+struct QkvParts {
+  __nv_bfloat16* p[3];
+  int64_t stride_t[3], stride_h[3];
+};
+
+template <bool FWD>
+__global__ void __launch_bounds__(256) k_split_rope(__nv_bfloat16* packed, int64_t ld, QkvParts part, const int* __restrict__ pos,
+                                                    const float* __restrict__ cos_t, const float* __restrict__ sin_t, uint32_t total,
+                                                    FastDiv per_head, FastDiv all_heads, uint32_t heads, uint32_t kv_heads) {
+  const uint32_t base = blockIdx.x * (256u * kRopeVecs) + threadIdx.x;
+  uint4 in[kRopeVecs];
+  float4 cs[kRopeVecs], sn[kRopeVecs];
+  uint4* dst[kRopeVecs];
+  bool rotate[kRopeVecs];
+#pragma unroll
+  for (int k = 0; k < kRopeVecs; ++k) {
+    const uint32_t i = base + k * 256u;
+    dst[k] = nullptr;
+    if (i < total) {
+      const uint32_t th = fast_div(i, per_head), v = i - th * per_head.d;
+      const uint32_t t = fast_div(th, all_heads), h = th - t * all_heads.d;
+      const int which = h < heads ? 0 : h < heads + kv_heads ? 1 : 2;
+      const uint32_t hp = h - (which == 0 ? 0u : which == 1 ? heads : heads + kv_heads);
+      uint4* a = reinterpret_cast<uint4*>(packed + t * ld) + (h * per_head.d + v);
+      // selects instead of an indexed parameter, which would go through local memory
+      __nv_bfloat16* pp = which == 0 ? part.p[0] : which == 1 ? part.p[1] : part.p[2];
+      const int64_t st = which == 0 ? part.stride_t[0] : which == 1 ? part.stride_t[1] : part.stride_t[2];
+      const int64_t sh = which == 0 ? part.stride_h[0] : which == 1 ? part.stride_h[1] : part.stride_h[2];
+      uint4* b = reinterpret_cast<uint4*>(pp + t * st + hp * sh + v * 8);
+      in[k] = FWD ? *a : *b;
+      dst[k] = FWD ? b : a;
+      rotate[k] = which < 2;
+      if (rotate[k]) {
+        const size_t at = static_cast<size_t>(pos[t]) * per_head.d + v;
+        cs[k] = reinterpret_cast<const float4*>(cos_t)[at];
+        sn[k] = reinterpret_cast<const float4*>(sin_t)[at];
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kRopeVecs; ++k) {
+    if (dst[k] != nullptr && !rotate[k]) {
+      *dst[k] = in[k];  // values are copied bit by bit
+    } else if (dst[k] != nullptr) {
+      float f[8];
+      unpack8(in[k], f);
+      rotate8(f, cs[k], sn[k], FWD ? 1.0f : -1.0f);
+      *dst[k] = pack8(f);
     }
   }
 }
@@ -786,38 +886,61 @@ void note_kernel_launch(int n) { g_launches.fetch_add(static_cast<unsigned long 
 unsigned long long kernel_launch_count() { return g_launches.load(std::memory_order_relaxed); }
 unsigned long long fused_ops_launch_count() { return kernel_launch_count(); }
 
-cudaError_t launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y, float* rstd, int rows,
-                               int cols, float eps, cudaStream_t s) {
-  if (cols % 8 != 0 || rows <= 0) return cudaErrorInvalidValue;
+namespace {
+
+template <bool ADD>
+void rmsnorm_fwd_rows(const __nv_bfloat16* x, const __nv_bfloat16* delta, const __nv_bfloat16* w, __nv_bfloat16* sum,
+                      __nv_bfloat16* y, float* rstd, int rows, int cols, float eps, cudaStream_t s) {
   // Narrow rows: a warp each, four to a block. Above 1024 columns a block per row, wide enough for four vectors a
   // thread. Blocks are handed out as they finish, so no SM waits for a longer share of rows.
   const int quads = (rows + 3) / 4;
-  if (cols <= 256) k_rmsnorm_fwd_reg<32, 1><<<quads, 128, 0, s>>>(x, w, y, rstd, rows, cols, eps);
-  else if (cols <= 512) k_rmsnorm_fwd_reg<32, 2><<<quads, 128, 0, s>>>(x, w, y, rstd, rows, cols, eps);
-  else if (cols <= 1024) k_rmsnorm_fwd_reg<32, 4><<<quads, 128, 0, s>>>(x, w, y, rstd, rows, cols, eps);
-  else if (cols <= 2048) k_rmsnorm_fwd_reg<128, 2><<<rows, 128, 0, s>>>(x, w, y, rstd, rows, cols, eps);
-  else if (cols <= 4096) k_rmsnorm_fwd_reg<128, 4><<<rows, 128, 0, s>>>(x, w, y, rstd, rows, cols, eps);
-  else if (cols <= 8192) k_rmsnorm_fwd_reg<256, 4><<<rows, 256, 0, s>>>(x, w, y, rstd, rows, cols, eps);
-  else k_rmsnorm_fwd_wide<<<std::min(rows, kSms * 8), kNormThreads, 0, s>>>(x, w, y, rstd, rows, cols, eps);
+  if (cols <= 256) k_rmsnorm_fwd_reg<32, 1, ADD><<<quads, 128, 0, s>>>(x, delta, w, sum, y, rstd, rows, cols, eps);
+  else if (cols <= 512) k_rmsnorm_fwd_reg<32, 2, ADD><<<quads, 128, 0, s>>>(x, delta, w, sum, y, rstd, rows, cols, eps);
+  else if (cols <= 1024) k_rmsnorm_fwd_reg<32, 4, ADD><<<quads, 128, 0, s>>>(x, delta, w, sum, y, rstd, rows, cols, eps);
+  else if (cols <= 2048) k_rmsnorm_fwd_reg<128, 2, ADD><<<rows, 128, 0, s>>>(x, delta, w, sum, y, rstd, rows, cols, eps);
+  else if (cols <= 4096) k_rmsnorm_fwd_reg<128, 4, ADD><<<rows, 128, 0, s>>>(x, delta, w, sum, y, rstd, rows, cols, eps);
+  else k_rmsnorm_fwd_reg<256, 4, ADD><<<rows, 256, 0, s>>>(x, delta, w, sum, y, rstd, rows, cols, eps);
+}
+
+template <bool ADD>
+void rmsnorm_bwd_rows(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w, const float* rstd,
+                      const __nv_bfloat16* dskip, __nv_bfloat16* dx, float* part, int blocks, int rows, int cols, cudaStream_t s) {
+  if (cols <= 256) k_rmsnorm_bwd<32, 1, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
+  else if (cols <= 512) k_rmsnorm_bwd<32, 2, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
+  else if (cols <= 1024) k_rmsnorm_bwd<32, 4, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
+  else if (cols <= 2048) k_rmsnorm_bwd<256, 1, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
+  else if (cols <= 4096) k_rmsnorm_bwd<256, 2, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
+  else k_rmsnorm_bwd<512, 2, ADD><<<blocks, 512, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
+}
+
+} // namespace
+
+cudaError_t launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y, float* rstd, int rows,
+                               int cols, float eps, cudaStream_t s, const __nv_bfloat16* delta, __nv_bfloat16* sum) {
+  if (cols % 8 != 0 || rows <= 0) return cudaErrorInvalidValue;
+  if (delta != nullptr) {
+    if (cols > kNormThreads * kNormMaxVec * 8 || sum == nullptr) return cudaErrorInvalidValue;
+    rmsnorm_fwd_rows<true>(x, delta, w, sum, y, rstd, rows, cols, eps, s);
+  } else if (cols <= kNormThreads * kNormMaxVec * 8) {
+    rmsnorm_fwd_rows<false>(x, nullptr, w, nullptr, y, rstd, rows, cols, eps, s);
+  } else {
+    k_rmsnorm_fwd_wide<<<std::min(rows, kSms * 8), kNormThreads, 0, s>>>(x, w, y, rstd, rows, cols, eps);
+  }
   note_kernel_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
                                const float* rstd, __nv_bfloat16* dx, float* dw_partial, int* nblocks, int rows,
-                               int cols, cudaStream_t s) {
+                               int cols, cudaStream_t s, const __nv_bfloat16* dskip) {
   if (cols % 8 != 0 || rows <= 0 || cols > kNormThreads * kNormMaxVec * 8) return cudaErrorInvalidValue;
   const bool warp_rows = cols <= 1024;  // a warp per row, eight to a block
   const int per_sm = cols > 4096 ? norm_bwd_per_sm<512, 2>() : (cols > 512 && warp_rows) ? norm_bwd_per_sm<32, 4>() : 2;
   const int blocks = std::min(warp_rows ? (rows + 7) / 8 : rows, kSms * per_sm);
   if (nblocks) *nblocks = blocks;
   if (dw_partial == nullptr) return cudaSuccess;
-  if (cols <= 256) k_rmsnorm_bwd<32, 1><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dx, dw_partial, rows, cols);
-  else if (cols <= 512) k_rmsnorm_bwd<32, 2><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dx, dw_partial, rows, cols);
-  else if (cols <= 1024) k_rmsnorm_bwd<32, 4><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dx, dw_partial, rows, cols);
-  else if (cols <= 2048) k_rmsnorm_bwd<256, 1><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dx, dw_partial, rows, cols);
-  else if (cols <= 4096) k_rmsnorm_bwd<256, 2><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dx, dw_partial, rows, cols);
-  else k_rmsnorm_bwd<512, 2><<<blocks, 512, 0, s>>>(dy, x, w, rstd, dx, dw_partial, rows, cols);
+  if (dskip != nullptr) rmsnorm_bwd_rows<true>(dy, x, w, rstd, dskip, dx, dw_partial, blocks, rows, cols, s);
+  else rmsnorm_bwd_rows<false>(dy, x, w, rstd, nullptr, dx, dw_partial, blocks, rows, cols, s);
   note_kernel_launch();
   return cudaGetLastError();
 }
@@ -899,6 +1022,35 @@ cudaError_t for_row_slices(int rows, int per_row, Fn fn) {
 }
 
 } // namespace
+
+cudaError_t launch_split_rope(__nv_bfloat16* packed, int64_t ld, __nv_bfloat16* const* parts, const int64_t* stride_t,
+                              const int64_t* stride_h, const int* pos, const float* cos_t, const float* sin_t, int tokens,
+                              int heads, int kv_heads, int head_dim, bool backward, cudaStream_t s) {
+  if (head_dim <= 0 || head_dim % 8 != 0 || heads <= 0 || kv_heads <= 0 || ld % 8 != 0) return cudaErrorInvalidValue;
+  QkvParts q{};
+  uintptr_t bits = reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t);
+  for (int i = 0; i < 3; ++i) {
+    if (stride_t[i] % 8 != 0 || stride_h[i] % 8 != 0) return cudaErrorInvalidValue;
+    q.p[i] = parts[i];
+    q.stride_t[i] = stride_t[i];
+    q.stride_h[i] = stride_h[i];
+    bits |= reinterpret_cast<uintptr_t>(parts[i]);
+  }
+  if (bits & 15u) return cudaErrorMisalignedAddress;
+  const int all = heads + 2 * kv_heads, per_head = head_dim / 8;
+  return for_row_slices(tokens, all * per_head, [&](size_t t0, uint32_t total) {
+    QkvParts here = q;
+    for (int i = 0; i < 3; ++i) here.p[i] += static_cast<int64_t>(t0) * q.stride_t[i];
+    const int blocks = static_cast<int>((total + 256u * kRopeVecs - 1) / (256u * kRopeVecs));
+    if (backward) {
+      k_split_rope<false><<<blocks, 256, 0, s>>>(packed + static_cast<int64_t>(t0) * ld, ld, here, pos + t0, cos_t, sin_t, total,
+                                                 make_fast_div(per_head), make_fast_div(all), heads, kv_heads);
+    } else {
+      k_split_rope<true><<<blocks, 256, 0, s>>>(packed + static_cast<int64_t>(t0) * ld, ld, here, pos + t0, cos_t, sin_t, total,
+                                                make_fast_div(per_head), make_fast_div(all), heads, kv_heads);
+    }
+  });
+}
 
 cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, int rows, int ffn, cudaStream_t s) {
   if (ffn % 8 != 0) return cudaErrorInvalidValue;

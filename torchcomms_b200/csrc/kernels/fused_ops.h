@@ -11,15 +11,17 @@
 namespace b200c {
 
 // y = x * rsqrt(mean(x^2) + eps) * w ; rstd saved for the backward pass.
-// cols must be a multiple of 8.
+// cols must be a multiple of 8. With `delta` (cols <= 8192) the normalised row is sum = bf16(x + delta), which is
+// written as well.
 cudaError_t launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y, float* rstd,
-                               int rows, int cols, float eps, cudaStream_t s);
+                               int rows, int cols, float eps, cudaStream_t s, const __nv_bfloat16* delta = nullptr,
+                               __nv_bfloat16* sum = nullptr);
 // dx, and per-block partial weight gradients `dw_partial` [nblocks, cols]
 // (fp32), which `launch_colsum` folds into dw. Returns the number of blocks
-// it will use through *nblocks when dw_partial is null (sizing query).
+// it will use through *nblocks when dw_partial is null (sizing query). `dskip`, if given, is added to dx.
 cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
                                const float* rstd, __nv_bfloat16* dx, float* dw_partial, int* nblocks, int rows,
-                               int cols, cudaStream_t s);
+                               int cols, cudaStream_t s, const __nv_bfloat16* dskip = nullptr);
 // out[c] = sum_r in[r, c]  (fp32 in, 16-byte aligned, cols a multiple of 4; bf16 out)
 cudaError_t launch_colsum_bf16(const float* in, __nv_bfloat16* out, int rows, int cols, cudaStream_t s);
 
@@ -39,6 +41,14 @@ cudaError_t launch_quantize_rows(const __nv_bfloat16* x, int64_t ld, void* q, fl
 cudaError_t launch_rope(const __nv_bfloat16* x, int64_t stride_t, int64_t stride_h, __nv_bfloat16* y, const int* pos,
                         const float* cos_t, const float* sin_t, int tokens, int heads, int head_dim, bool inverse,
                         cudaStream_t s);
+
+// Queries, keys and values out of packed rows [tokens, (heads + 2 kv_heads) x head_dim] (row stride `ld`), queries
+// and keys rotated; `backward` goes the other way with the inverse rotation and writes every packed element.
+// parts / stride_t / stride_h: the three tensors [tokens, heads or kv_heads, head_dim] and their strides.
+// Strides are multiples of 8 elements, all pointers 16-byte aligned.
+cudaError_t launch_split_rope(__nv_bfloat16* packed, int64_t ld, __nv_bfloat16* const* parts, const int64_t* stride_t,
+                              const int64_t* stride_h, const int* pos, const float* cos_t, const float* sin_t, int tokens,
+                              int heads, int kv_heads, int head_dim, bool backward, cudaStream_t s);
 
 // h = silu(gate) * up where gate_up = [rows, 2*ffn] (gate first).
 cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, int rows, int ffn, cudaStream_t s);

@@ -150,6 +150,122 @@ struct RmsNormFn : torch::autograd::Function<RmsNormFn> {
   }
 };
 
+// The norm together with the residual stream it reads: (x, y) or, with a `delta` to add first, (x + delta, y). Both
+// results' gradients meet inside the backward kernel instead of in an addition of their own.
+bool norm_with_skip_applies(const at::Tensor& x, const at::Tensor& w) {
+  return plain_call(x, true) && plain_call(w, true) && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+      w.is_contiguous() && x.dim() >= 1 && x.size(-1) % 8 == 0 && x.size(-1) <= 8192 && x.numel() > 0 && w.numel() == x.size(-1) &&
+      x.device() == w.device();
+}
+
+variable_list norm_with_skip_backward(const variable_list& grads, const variable_list& saved, at::Tensor* dw) {
+  const at::Tensor &x = saved[0], &w = saved[1], &rstd = saved[2];
+  const at::Tensor dskip = grads[0].contiguous(), dy = grads[1].contiguous();
+  want(dskip, at::kBFloat16, "gradient of the residual");
+  want(dy, at::kBFloat16, "dy");
+  const int cols = static_cast<int>(x.size(-1)), rows = static_cast<int>(x.numel() / cols);
+  c10::cuda::CUDAGuard g(x.device());
+  int nblocks = 0;
+  B200C_CUDA_CHECK(launch_rmsnorm_bwd(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &nblocks, rows, cols, cur(x)));
+  at::Tensor dx = at::empty_like(x);
+  at::Tensor partial = at::empty({nblocks, cols}, x.options().dtype(at::kFloat));
+  *dw = at::empty_like(w);
+  B200C_CUDA_CHECK(launch_rmsnorm_bwd(bf(dy), bf(x), bf(w), rstd.data_ptr<float>(), bf_mut(dx), partial.data_ptr<float>(), &nblocks,
+                                      rows, cols, cur(x), bf(dskip)));
+  B200C_CUDA_CHECK(launch_colsum_bf16(partial.data_ptr<float>(), bf_mut(*dw), nblocks, cols, cur(x)));
+  return {dx};
+}
+
+struct SkipRmsNormFn : torch::autograd::Function<SkipRmsNormFn> {
+  static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& w, double eps) {
+    auto [y, rstd] = rmsnorm_fwd(x, w, eps);
+    ctx->save_for_backward({x, w, rstd});
+    return {x, y};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    at::Tensor dw;
+    const variable_list dx = norm_with_skip_backward(grads, ctx->get_saved_variables(), &dw);
+    return {dx[0], dw, at::Tensor()};
+  }
+};
+
+struct AddRmsNormFn : torch::autograd::Function<AddRmsNormFn> {
+  static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& delta, const at::Tensor& w, double eps) {
+    want(x, at::kBFloat16, "x");
+    want(delta, at::kBFloat16, "delta");
+    const int cols = static_cast<int>(x.size(-1)), rows = static_cast<int>(x.numel() / cols);
+    c10::cuda::CUDAGuard g(x.device());
+    at::Tensor sum = at::empty_like(x), y = at::empty_like(x);
+    at::Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
+    B200C_CUDA_CHECK(launch_rmsnorm_fwd(bf(x), bf(w), bf_mut(y), rstd.data_ptr<float>(), rows, cols, static_cast<float>(eps), cur(x),
+                                        bf(delta), bf_mut(sum)));
+    ctx->save_for_backward({sum, w, rstd});
+    return {sum, y};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    at::Tensor dw;
+    const variable_list dx = norm_with_skip_backward(grads, ctx->get_saved_variables(), &dw);
+    return {dx[0], dx[0], dw, at::Tensor()};
+  }
+};
+
+// Strides a split_rope launch can follow for [tokens, heads, head_dim].
+bool followable(const at::Tensor& t) {
+  return t.dim() == 3 && t.stride(2) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 &&
+      (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
+}
+
+struct SplitRopeFn : torch::autograd::Function<SplitRopeFn> {
+  static variable_list forward(AutogradContext* ctx, const at::Tensor& qkv, const at::Tensor& pos, const at::Tensor& cos_t,
+                               const at::Tensor& sin_t, int64_t heads, int64_t kv_heads) {
+    ctx->save_for_backward({pos, cos_t, sin_t});
+    const int64_t tokens = qkv.size(0), hd = qkv.size(1) / (heads + 2 * kv_heads);
+    c10::cuda::CUDAGuard g(qkv.device());
+    variable_list out{at::empty({tokens, heads, hd}, qkv.options()), at::empty({tokens, kv_heads, hd}, qkv.options()),
+                      at::empty({tokens, kv_heads, hd}, qkv.options())};
+    launch(qkv, out, pos, cos_t, sin_t, false);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    for (auto& t : grads) {
+      if (!followable(t)) t = t.clone(at::MemoryFormat::Contiguous);
+      TORCH_CHECK(t.scalar_type() == at::kBFloat16, "split_rope: bf16 gradients expected");
+    }
+    c10::cuda::CUDAGuard g(grads[0].device());
+    at::Tensor dqkv = at::empty({grads[0].size(0), (grads[0].size(1) + 2 * grads[1].size(1)) * grads[0].size(2)}, grads[0].options());
+    launch(dqkv, grads, saved[0], saved[1], saved[2], true);
+    return {dqkv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+  }
+  static void launch(const at::Tensor& packed, const variable_list& part, const at::Tensor& pos, const at::Tensor& cos_t,
+                     const at::Tensor& sin_t, bool backward) {
+    __nv_bfloat16* p[3];
+    int64_t st[3], sh[3];
+    for (int i = 0; i < 3; ++i) {
+      p[i] = reinterpret_cast<__nv_bfloat16*>(part[i].data_ptr());
+      st[i] = part[i].stride(0);
+      sh[i] = part[i].stride(1);
+    }
+    B200C_CUDA_CHECK(launch_split_rope(reinterpret_cast<__nv_bfloat16*>(packed.data_ptr()), packed.stride(0), p, st, sh,
+                                       pos.data_ptr<int>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(),
+                                       static_cast<int>(packed.size(0)), static_cast<int>(part[0].size(1)),
+                                       static_cast<int>(part[1].size(1)), static_cast<int>(part[0].size(2)), backward, cur(packed)));
+  }
+  static bool applies(const at::Tensor& qkv, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t, int64_t heads,
+                      int64_t kv_heads) {
+    if (!plain_call(qkv, true) || !plain_call(pos) || !plain_call(cos_t) || !plain_call(sin_t)) return false;
+    if (heads < 1 || kv_heads < 1 || qkv.dim() != 2 || qkv.numel() == 0 || qkv.size(1) % (8 * (heads + 2 * kv_heads)) != 0) return false;
+    const int64_t hd = qkv.size(1) / (heads + 2 * kv_heads);
+    auto table = [&](const at::Tensor& t) {
+      return t.scalar_type() == at::kFloat && t.is_contiguous() && t.dim() == 2 && t.size(1) == hd / 2 && t.device() == qkv.device() &&
+          (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
+    };
+    return qkv.scalar_type() == at::kBFloat16 && qkv.stride(1) == 1 && qkv.stride(0) % 8 == 0 &&
+        (reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 15u) == 0 && table(cos_t) && table(sin_t) && pos.scalar_type() == at::kInt &&
+        pos.is_contiguous() && pos.numel() == qkv.size(0) && pos.device() == qkv.device();
+  }
+};
+
 struct SwiGluFn : torch::autograd::Function<SwiGluFn> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& gate_up) {
     ctx->save_for_backward({gate_up});
@@ -215,6 +331,23 @@ void bind_ops(py::module_& m) {
   ops.def("rms_norm", [](const at::Tensor& x, const at::Tensor& w, double eps) -> std::optional<at::Tensor> {
     if (!plain_call(x, true) || !plain_call(w, true)) return std::nullopt;
     return RmsNormFn::apply(x.contiguous(), w, eps);
+  });
+  ops.def("rms_norm_skip", [](const at::Tensor& x, const at::Tensor& w, double eps) -> std::optional<std::vector<at::Tensor>> {
+    if (!norm_with_skip_applies(x, w)) return std::nullopt;
+    return SkipRmsNormFn::apply(x.contiguous(), w, eps);
+  });
+  ops.def("add_rms_norm", [](const at::Tensor& x, const at::Tensor& delta, const at::Tensor& w, double eps)
+              -> std::optional<std::vector<at::Tensor>> {
+    if (!norm_with_skip_applies(x, w) || !plain_call(delta, true) || delta.scalar_type() != at::kBFloat16 ||
+        delta.sizes() != x.sizes() || delta.device() != x.device()) {
+      return std::nullopt;
+    }
+    return AddRmsNormFn::apply(x.contiguous(), delta.contiguous(), w, eps);
+  });
+  ops.def("split_rope", [](const at::Tensor& qkv, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t,
+                           int64_t heads, int64_t kv_heads) -> std::optional<std::vector<at::Tensor>> {
+    if (!SplitRopeFn::applies(qkv, pos, cos_t, sin_t, heads, kv_heads)) return std::nullopt;
+    return SplitRopeFn::apply(qkv, pos, cos_t, sin_t, heads, kv_heads);
   });
   ops.def("swiglu", [](const at::Tensor& gate_up) -> std::optional<at::Tensor> {
     if (!plain_call(gate_up, true)) return std::nullopt;

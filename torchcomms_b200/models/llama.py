@@ -87,20 +87,16 @@ class Block(nn.Module):
         cfg = self.cfg
         b, s, d = x.shape
         hd, nh, nkv = cfg.head_dim, cfg.n_heads, cfg.n_kv_heads
-        h = fused.rms_norm(x.reshape(b * s, d), self.attn_norm, cfg.norm_eps)
-        qkv = F.linear(h, self.wqkv)
-        q, k, v = qkv.split([nh * hd, nkv * hd, nkv * hd], dim=-1)
-        q = fused.apply_rope(q.reshape(b * s, nh, hd), pos, cos_t, sin_t).view(b, s, nh, hd)
-        k = fused.apply_rope(k.reshape(b * s, nkv, hd), pos, cos_t, sin_t).view(b, s, nkv, hd)
-        v = v.reshape(b, s, nkv, hd)
+        x, h = fused.rms_norm_skip(x.reshape(b * s, d), self.attn_norm, cfg.norm_eps)
+        q, k, v = fused.split_rope(F.linear(h, self.wqkv), pos, cos_t, sin_t, nh, nkv)
+        q, k, v = q.view(b, s, nh, hd), k.view(b, s, nkv, hd), v.view(b, s, nkv, hd)
         o = F.scaled_dot_product_attention(
             q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True, enable_gqa=(nkv != nh)
         )
         o = o.transpose(1, 2).reshape(b * s, nh * hd)
-        x = x + F.linear(o, self.wo).view(b, s, d)
-        h = fused.rms_norm(x.reshape(b * s, d), self.ffn_norm, cfg.norm_eps)
+        x, h = fused.add_rms_norm(x, F.linear(o, self.wo), self.ffn_norm, cfg.norm_eps)
         h = fused.swiglu(F.linear(h, self.w13))
-        return x + F.linear(h, self.w2).view(b, s, d)
+        return (x + F.linear(h, self.w2)).view(b, s, d)
 
 
 class Head(nn.Module):

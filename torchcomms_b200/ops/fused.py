@@ -65,6 +65,18 @@ def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5) -> torch.Tenso
     return y.to(x.dtype)
 
 
+def rms_norm_skip(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5) -> tuple[torch.Tensor, torch.Tensor]:
+    """``(x, rms_norm(x, w))``: the residual stream and its norm, whose gradients meet in one kernel."""
+    out = _k.rms_norm_skip(x, w, eps) if x.is_cuda and _native(x, w) else None
+    return (x, rms_norm(x, w, eps)) if out is None else (out[0], out[1])
+
+
+def add_rms_norm(x: torch.Tensor, delta: torch.Tensor, w: torch.Tensor, eps: float = 1e-5) -> tuple[torch.Tensor, torch.Tensor]:
+    """``(s, rms_norm(s, w))`` for ``s = x + delta``."""
+    out = _k.add_rms_norm(x, delta, w, eps) if x.is_cuda and _native(x, delta, w) else None
+    return rms_norm_skip(x + delta, w, eps) if out is None else (out[0], out[1])
+
+
 # ------------------------------------------------------------------- SwiGLU
 
 
@@ -121,6 +133,20 @@ def apply_rope(x: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: t
     a, b = xf[..., 0], xf[..., 1]
     out = torch.stack((a * c - b * s, a * s + b * c), dim=-1)
     return out.reshape(x.shape).to(x.dtype)
+
+
+def split_rope(qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor, heads: int,
+               kv_heads: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """Rotated queries, rotated keys and values, each ``[tokens, heads or kv_heads, head_dim]``, out of the fused
+    projection ``qkv = [tokens, (heads + 2 * kv_heads) * head_dim]``."""
+    if qkv.is_cuda and _native(qkv, pos, cos_t, sin_t):
+        out = _k.split_rope(qkv, pos, cos_t, sin_t, heads, kv_heads)
+        if out is not None:
+            return out[0], out[1], out[2]
+    t, hd = qkv.shape[0], qkv.shape[1] // (heads + 2 * kv_heads)
+    q, k, v = qkv.split([heads * hd, kv_heads * hd, kv_heads * hd], dim=-1)
+    return (apply_rope(q.reshape(t, heads, hd), pos, cos_t, sin_t), apply_rope(k.reshape(t, kv_heads, hd), pos, cos_t, sin_t),
+            v.reshape(t, kv_heads, hd))
 
 
 # ------------------------------------------------- linear + cross entropy
