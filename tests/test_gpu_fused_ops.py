@@ -180,6 +180,26 @@ def test_cross_entropy_row_layouts(rows, vocab):
     torch.testing.assert_close(logits.double(), ref, rtol=2**-8, atol=1e-5)
 
 
+@pytest.mark.parametrize("rows,dim,vocab", [(1, 64, 9), (130, 128, 5001), (70, 256, 40002), (257, 64, 1000)])
+def test_linear_cross_entropy_any_vocabulary(rows, dim, vocab):
+    """Vocabularies off the 16-byte grid (padded logit rows) and on it, in one and in several chunks."""
+    from torchcomms_b200.ops import fused
+
+    x, w = _bf(rows, dim, seed=60).requires_grad_(True), _bf(vocab, dim, seed=61, scale=0.1).requires_grad_(True)
+    t = torch.randint(0, vocab, (rows,), device="cuda")
+    t[-1] = vocab - 1
+    xd, wd = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    ref = F.cross_entropy(xd @ wd.t(), t)
+    rx, rw = torch.autograd.grad(ref, (xd, wd))
+    for chunk in (4096, 100):
+        loss = fused.linear_cross_entropy(x, w, t, chunk)
+        dx, dw = torch.autograd.grad(loss, (x, w))
+        # bf16 logits of size up to 5 (2^-9 x 5 absolute) enter the loss, bf16 logit gradients the sums.
+        torch.testing.assert_close(loss.double(), ref.detach(), rtol=0, atol=1e-2)
+        assert float((dx.double() - rx).norm() / rx.norm()) < 1e-2
+        assert float((dw.double() - rw).norm() / rw.norm()) < 1e-2
+
+
 @pytest.mark.parametrize("numel", [1, 8, 4099, 3_000_001])
 def test_scale_by_matches_operators(numel):
     from torchcomms_b200 import _comms

@@ -570,13 +570,13 @@ constexpr int kCeMaxThreads = 512;
 // are no multiple of 8) peel up to 7 elements instead of giving up wide accesses. 4096 rows of 128256: 698 us with
 // 592 rows in work and a comparison per element, 512 us (4.1 TB/s) now.
 __global__ void __launch_bounds__(kCeMaxThreads, 2) k_cross_entropy(__nv_bfloat16* __restrict__ logits,
-                                                                    const int64_t* __restrict__ targets,
+                                                                    int64_t ld, const int64_t* __restrict__ targets,
                                                                     float* __restrict__ loss, int rows, int vocab,
                                                                     float grad_scale) {
   __shared__ float scratch[32];
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    __nv_bfloat16* row = logits + static_cast<size_t>(r) * vocab;
+    __nv_bfloat16* row = logits + static_cast<int64_t>(r) * ld;
     const int64_t tgt = targets[r];
     const int head = min(vocab, static_cast<int>((16u - (static_cast<uint32_t>(reinterpret_cast<uintptr_t>(row)) & 15u)) & 15u) / 2);
     const int nvec = (vocab - head) / 8, tail = head + nvec * 8;
@@ -1069,15 +1069,15 @@ cudaError_t launch_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate
   });
 }
 
-cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, const int64_t* targets, float* loss, int rows, int vocab,
-                                         float grad_scale, cudaStream_t s) {
-  if (rows <= 0 || vocab <= 0) return cudaErrorInvalidValue;
+cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, float* loss, int rows,
+                                         int vocab, float grad_scale, cudaStream_t s) {
+  if (rows <= 0 || vocab <= 0 || ld < vocab) return cudaErrorInvalidValue;
   // Rows in work at a time: 296 rows of a 128k vocabulary are 76 MB, which the 126 MB L2 keeps for the second
   // look; shorter rows take smaller blocks, more of them per SM, and stay below that. Every block has at least 128
   // threads: one for each element outside the vectors.
   const int threads = vocab <= 4096 ? 128 : vocab <= 16384 ? 256 : kCeMaxThreads;
   const int blocks = std::min(rows, kSms * 2 * (kCeMaxThreads / threads));
-  k_cross_entropy<<<blocks, threads, 0, s>>>(logits, targets, loss, rows, vocab, grad_scale);
+  k_cross_entropy<<<blocks, threads, 0, s>>>(logits, ld, targets, loss, rows, vocab, grad_scale);
   note_kernel_launch();
   return cudaGetLastError();
 }

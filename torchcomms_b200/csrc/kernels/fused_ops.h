@@ -55,9 +55,9 @@ cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, in
 cudaError_t launch_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate_up, __nv_bfloat16* dgate_up,
                               int rows, int ffn, cudaStream_t s);
 
-// Row-wise softmax cross-entropy: writes loss[r] and overwrites logits with
+// Row-wise softmax cross-entropy: writes loss[r] and overwrites logits (row stride `ld` elements) with
 // d(loss_sum * grad_scale)/dlogits. Rows whose target is < 0 are ignored.
-cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, const int64_t* targets, float* loss, int rows,
+cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, float* loss, int rows,
                                          int vocab, float grad_scale, cudaStream_t s);
 
 // out = in * bf16(*factor) on n bf16 values, the factor read from device memory; in and out 16-byte aligned.

@@ -360,14 +360,18 @@ void bind_ops(py::module_& m) {
   });
 
   ops.def("cross_entropy_fwd_bwd_", [](at::Tensor logits, const at::Tensor& targets, double grad_scale) {
-    want(logits, at::kBFloat16, "logits");
+    // Contiguous, or rows of a wider buffer.
+    const bool padded = logits.dim() == 2 && logits.stride(1) == 1 && logits.stride(0) >= logits.size(1);
+    TORCH_CHECK(logits.is_cuda() && (padded || logits.is_contiguous()), "logits: contiguous CUDA tensor expected");
+    TORCH_CHECK(logits.scalar_type() == at::kBFloat16, "logits: expected dtype ", at::kBFloat16, ", got ", logits.scalar_type());
     want(targets, at::kLong, "targets");
     const int vocab = static_cast<int>(logits.size(-1));
+    const int64_t ld = padded ? logits.stride(0) : vocab;
     const int rows = static_cast<int>(logits.numel() / vocab);
     TORCH_CHECK(targets.numel() == rows, "one target per row");
     c10::cuda::CUDAGuard g(logits.device());
     at::Tensor loss = at::empty({rows}, logits.options().dtype(at::kFloat));
-    B200C_CUDA_CHECK(launch_cross_entropy_fwd_bwd(bf_mut(logits), targets.data_ptr<int64_t>(), loss.data_ptr<float>(), rows,
+    B200C_CUDA_CHECK(launch_cross_entropy_fwd_bwd(bf_mut(logits), ld, targets.data_ptr<int64_t>(), loss.data_ptr<float>(), rows,
                                                   vocab, static_cast<float>(grad_scale), cur(logits)));
     return loss;
   });

@@ -172,7 +172,13 @@ class _LinearCrossEntropy(torch.autograd.Function):
         loss_sum = torch.zeros((), dtype=torch.float32, device=x.device)
         for r0 in range(0, rows, chunk_rows):
             r1 = min(rows, r0 + chunk_rows)
-            logits = x[r0:r1] @ weight.t()
+            if x.is_cuda and weight.shape[0] % 8 and x.dtype == weight.dtype == torch.bfloat16:
+                # Rows of such a vocabulary would start off 16-byte boundaries, which costs the three GEMMs their
+                # tiled loads; in a buffer of padded rows they do not.
+                logits = x.new_empty(r1 - r0, (weight.shape[0] + 63) // 64 * 64)[:, : weight.shape[0]]
+                torch.mm(x[r0:r1], weight.t(), out=logits)
+            else:
+                logits = x[r0:r1] @ weight.t()
             if x.is_cuda:
                 loss = _k.cross_entropy_fwd_bwd_(logits, targets[r0:r1].contiguous(), scale)
                 dlogits = logits
