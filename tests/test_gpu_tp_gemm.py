@@ -123,6 +123,22 @@ def test_quantize_rows_kernel_matches_operators(rows, cols, layout):
         assert _comms.ops.quantize_rows(x.t()) is None or cols == 1
 
 
+@pytest.mark.parametrize("exponent", [-30, -26, -3, 0, 40, 126])
+def test_quantize_rows_divides_exactly(exponent):
+    """Every significand of a row's maximum against every significand below it, 20 binades down, near both ends of the
+    range and at the smallest scale: the quotients are those of the division."""
+    from torchcomms_b200.ops.tp import quantize_rows
+
+    top = (1 + torch.arange(128, device="cuda", dtype=torch.float64) / 128) * 2.0**exponent
+    below = ((1 + torch.arange(128, dtype=torch.float64) / 128).unsqueeze(0) * 2.0 ** -torch.arange(20.0, dtype=torch.float64).unsqueeze(1)).reshape(-1)
+    x = torch.cat((top.unsqueeze(1), (below.cuda() * 2.0**exponent).expand(128, -1)), dim=1)
+    x = torch.where(x > top.unsqueeze(1), -x / 4, x).to(torch.bfloat16)  # nothing above the row's maximum
+    scale = x.float().abs().amax(dim=1).clamp_min(1e-8) / 448.0
+    q, s = quantize_rows(x)
+    assert torch.equal(s, scale)
+    assert torch.equal(q.view(torch.uint8), (x.float() / scale.unsqueeze(1)).to(torch.float8_e4m3fn).view(torch.uint8))
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 256, 128), (300, 264, 256), (1024, 1792, 2048), (128 * 9, 256 * 5, 1024)])
 def test_gemm_e4m3_rowwise_scales(m, n, k):
     from torchcomms_b200.ops.tp import gemm_e4m3_nt, quantize_rows

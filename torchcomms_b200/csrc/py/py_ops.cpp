@@ -32,6 +32,14 @@ cudaStream_t cur(const at::Tensor& t) {
   return at::cuda::getCurrentCUDAStream(t.device().index()).stream();
 }
 
+// Two status words; eight bytes are cleared by the copy engine's memset, without a kernel launch through the
+// tensor library.
+at::Tensor cleared_status(const at::Tensor& like) {
+  at::Tensor status = at::empty({2}, like.options().dtype(at::kInt));
+  B200C_CUDA_CHECK(cudaMemsetAsync(status.data_ptr(), 0, 8, cur(like)));
+  return status;
+}
+
 bool quantizable(const at::Tensor& x) {
   return plain_call(x) && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.numel() > 0 && x.stride(1) == 1 &&
       x.size(0) <= INT32_MAX && x.size(1) <= INT32_MAX;
@@ -431,7 +439,7 @@ void bind_ops(py::module_& m) {
     TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.size(1) == b.size(1), "a: [m, k], b: [n, k]");
     c10::cuda::CUDAGuard g(a.device());
     at::Tensor c = at::empty({a.size(0), b.size(0)}, a.options());
-    at::Tensor status = at::zeros({2}, a.options().dtype(at::kInt));
+    at::Tensor status = cleared_status(a);
     B200C_CUDA_CHECK(launch_gemm_bf16_nt(a.data_ptr(), b.data_ptr(), c.data_ptr(), static_cast<int>(a.size(0)),
                                          static_cast<int>(b.size(0)), static_cast<int>(a.size(1)),
                                          reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
@@ -448,7 +456,7 @@ void bind_ops(py::module_& m) {
     TORCH_CHECK(scale_a.numel() == a.size(0) && scale_b.numel() == b.size(0), "one scale per row of a and per row of b");
     c10::cuda::CUDAGuard g(a.device());
     at::Tensor c = at::empty({a.size(0), b.size(0)}, a.options().dtype(at::kBFloat16));
-    at::Tensor status = at::zeros({2}, a.options().dtype(at::kInt));
+    at::Tensor status = cleared_status(a);
     B200C_CUDA_CHECK(launch_gemm_e4m3_nt(a.data_ptr(), b.data_ptr(), c.data_ptr(), static_cast<int>(a.size(0)),
                                          static_cast<int>(b.size(0)), static_cast<int>(a.size(1)), scale_a.data_ptr<float>(),
                                          scale_b.data_ptr<float>(), reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
@@ -461,7 +469,7 @@ void bind_ops(py::module_& m) {
     TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.size(1) == b.size(1), "a: [m, k], b: [n, k]");
     c10::cuda::CUDAGuard g(a.device());
     at::Tensor c = at::empty({a.size(0), b.size(0)}, a.options());
-    at::Tensor status = at::zeros({2}, a.options().dtype(at::kInt));
+    at::Tensor status = cleared_status(a);
     B200C_CUDA_CHECK(launch_gemm_bf16_nt_pair(a.data_ptr(), b.data_ptr(), c.data_ptr(), static_cast<int>(a.size(0)),
                                               static_cast<int>(b.size(0)), static_cast<int>(a.size(1)),
                                               reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
