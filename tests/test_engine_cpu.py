@@ -43,3 +43,52 @@ def test_engine_trains_and_matches_across_world_sizes(tmp_path):
     # identical data on every rank: the averaged gradient equals the single-rank gradient
     for x, y in zip(a["losses"], b["losses"]):
         assert abs(x - y) < 5e-2, (a["losses"], b["losses"])
+
+
+def test_block_pieces_on_cpu_tensors():
+    """CPU tensors take the plain compositions of the fused block pieces, gradients included, and the kernels' entry
+    points decline them."""
+    import torch
+
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops import fused
+    from torchcomms_b200.ops.tp import quantize_rows
+
+    torch.manual_seed(3)
+    x, d, w = (torch.randn(6, 16, requires_grad=True) for _ in range(3))
+    w = w[0].detach().requires_grad_(True)
+    s, y = fused.add_rms_norm(x, d, w)
+    torch.testing.assert_close(s, x + d)
+    torch.testing.assert_close(y, fused.rms_norm(x + d, w))
+    skip, y2 = fused.rms_norm_skip(x, w)
+    assert skip is x
+    (g,) = torch.autograd.grad((skip, y2), x, (torch.ones_like(x), torch.ones_like(x)))
+    (ref,) = torch.autograd.grad(fused.rms_norm(x, w).sum() + x.sum(), x)
+    torch.testing.assert_close(g, ref)
+
+    cos_t, sin_t = fused.rope_tables(32, 8, 10000.0, "cpu")
+    pos = torch.arange(6, dtype=torch.int32)
+    qkv = torch.randn(6, (4 + 2 * 2) * 8, requires_grad=True)
+    q, k, v = fused.split_rope(qkv, pos, cos_t, sin_t, 4, 2)
+    parts = qkv.split([32, 16, 16], dim=-1)
+    torch.testing.assert_close(q, fused.apply_rope(parts[0].reshape(6, 4, 8), pos, cos_t, sin_t))
+    torch.testing.assert_close(k, fused.apply_rope(parts[1].reshape(6, 2, 8), pos, cos_t, sin_t))
+    torch.testing.assert_close(v, parts[2].reshape(6, 2, 8))
+    assert torch.autograd.grad(q.sum() + k.sum() + v.sum(), qkv)[0].shape == qkv.shape
+
+    b = torch.randn(3, 32).to(torch.bfloat16)
+    assert _comms.ops.quantize_rows(b) is None
+    assert _comms.ops.rms_norm(b, b[0], 1e-5) is None and _comms.ops.swiglu(b) is None
+    q8, scale = quantize_rows(b)
+    assert q8.dtype == torch.float8_e4m3fn
+    torch.testing.assert_close(scale, b.float().abs().amax(dim=1) / 448.0)
+    # A loss and its gradients twice over a retained graph give the same on the device without kernels.
+    xs, ws = torch.randn(5, 16, requires_grad=True), torch.randn(11, 16, requires_grad=True)
+    t = torch.randint(0, 11, (5,))
+    loss = fused.linear_cross_entropy(xs, ws, t, chunk_rows=2)
+    a = torch.autograd.grad(loss, (xs, ws), retain_graph=True)
+    c = torch.autograd.grad(loss, (xs, ws))
+    ref = torch.autograd.grad(torch.nn.functional.cross_entropy(xs @ ws.t(), t), (xs, ws))
+    for p, q_, r in zip(a, c, ref):
+        assert torch.equal(p, q_)
+        torch.testing.assert_close(p, r, rtol=1e-4, atol=1e-6)

@@ -144,11 +144,11 @@ def test_cross_entropy_loss_and_gradient(rows, vocab):
     torch.testing.assert_close(work.float(), lf.grad, rtol=3e-2, atol=2e-3)
 
 
-@pytest.mark.parametrize("vocab", [1, 7, 9, 16, 23, 4096, 4097, 16384, 16391, 40003])
-@pytest.mark.parametrize("rows", [1, 300, 1300])
+@pytest.mark.parametrize("rows,vocab", [(r, v) for r in (1, 300, 1300) for v in (1, 7, 9, 16, 23, 4096, 4097, 16384, 16391, 40003)]
+                         + [(r, v) for r in (1, 130) for v in (60007, 128256, 131071, 200001, 300007)])
 def test_cross_entropy_row_layouts(rows, vocab):
-    """Heads and tails of rows that start off a 16-byte boundary, every block size, targets at both ends, and rows
-    with masked (-inf, lowest finite) logits."""
+    """Heads and tails of rows that start off a 16-byte boundary, every block and cluster size, targets at both ends,
+    and rows with masked (-inf, lowest finite) logits."""
     from torchcomms_b200 import _comms
 
     logits = _bf(rows, vocab, seed=11, scale=3.0)
@@ -175,7 +175,7 @@ def test_cross_entropy_row_layouts(rows, vocab):
     if rows > 8 and vocab > 8:  # a row without any allowed token has no meaningful value, but stays finite
         assert torch.isfinite(loss[3]) and torch.isfinite(logits[3].float()).all()
         loss, ref_loss, logits, ref = (torch.cat((t[:3], t[4:])) for t in (loss, ref_loss, logits, ref))
-    # fp32 sums of up to 40003 exponentials; p - 1 at the target cancels to the sum's error; bf16 results (2^-9).
+    # fp32 sums of up to 300007 exponentials; p - 1 at the target cancels to the sum's error; bf16 results (2^-9).
     torch.testing.assert_close(loss.double(), ref_loss, rtol=2e-6, atol=1e-5)
     torch.testing.assert_close(logits.double(), ref, rtol=2**-8, atol=1e-5)
 
