@@ -329,3 +329,85 @@ def test_fused_training_and_link_ep_surface_multi_gpu(worker):
     if world < 2:
         pytest.skip("needs 2 GPUs")
     run_ranks(worker, world, timeout=150)
+
+
+def _solo_comm(name):
+    import torch.distributed as dist
+
+    import torchcomms_b200 as tc
+
+    os.environ.setdefault("RANK", "0")
+    os.environ.setdefault("WORLD_SIZE", "1")
+    return tc.new_comm("b200", torch.device("cuda", 0), name=name, store=dist.HashStore(), timeout=timedelta(seconds=60),
+                       abort_process_on_timeout_or_error=False)
+
+
+@pytest.mark.parametrize("fp8", [True, False])
+def test_single_rank_dispatch_and_combine(fp8):
+    """One rank's own kernels: token counts around the block size, rows that end inside a piece, unrouted tokens,
+    several calls on one buffer, kept handles."""
+    from torchcomms_b200.ops.moe_ep import Buffer
+
+    comm = _solo_comm(f"solo_ep_{int(fp8)}")
+    torch.manual_seed(5)
+    for hidden, experts, topk in ((512, 8, 1), (1536, 16, 4), (7168, 256, 8)):
+        buf = Buffer(comm, 130, hidden, experts, topk, fp8=fp8)
+        for tokens in (1, 3, 4, 5, 130, 2):
+            x = torch.randn(tokens, hidden, device="cuda").to(torch.bfloat16)
+            idx, w = _route(tokens, experts, topk, tokens)
+            idx[0, 0] = -1
+            if tokens > 4:
+                idx[4] = -1                                        # a token that goes nowhere
+            d = buf.dispatch(x, idx, w, keep_handle=True)
+            n = _check_dispatch(0, 1, experts, topk, 130, [x], [idx], [w], lambda r, what: buf._buf.view(0, what), fp8)
+            sent = (idx >= 0).any(dim=1)
+            assert n == int(sent.sum()) == int(d.num_tokens)
+            assert torch.equal(buf._buf.view(0, "send_slot")[:tokens, 0] >= 0, sent)
+            src = d.src[:n].long()
+            buf.combine_input[:n] = x[src] * 2
+            buf.combine_topk_weights[:n] = d.topk_weights[:n]
+            bias = torch.randn(tokens, hidden, device="cuda").to(torch.bfloat16)
+            wt, w_out = torch.rand(tokens, 1, device="cuda"), torch.empty(tokens, topk, device="cuda")
+            y = buf.combine(wt, bias, topk_weights_out=w_out)
+            ref = bias.double() + sent.unsqueeze(1) * wt.double() * 2 * x.double()
+            torch.testing.assert_close(y.double(), ref, rtol=2**-8, atol=1e-5)   # one rounding to bf16 of an fp32 sum
+            assert torch.equal(w_out, torch.where(idx >= 0, w, torch.zeros_like(w)) * sent.unsqueeze(1))
+            assert torch.equal(buf.combine(handle=d.handle), torch.where(sent.unsqueeze(1), x * 2, torch.zeros_like(x)))
+    comm.finalize()
+
+
+@pytest.mark.parametrize("fp8", [True, False])
+def test_single_rank_low_latency(fp8):
+    """One rank's own kernels: one to many tokens, unrouted pairs, counts and handles of several calls."""
+    from torchcomms_b200.ops.moe_ep import LowLatencyBuffer, per_token_cast_to_fp8
+
+    comm = _solo_comm(f"solo_ll_{int(fp8)}")
+    torch.manual_seed(6)
+    for hidden, experts, topk in ((512, 4, 1), (1536, 300, 4), (7168, 32, 8)):
+        ll = LowLatencyBuffer(comm, 64, hidden, experts, topk, fp8=fp8)
+        for tokens in (1, 2, 64, 7):
+            x = torch.randn(tokens, hidden, device="cuda").to(torch.bfloat16)
+            idx, w = _route(tokens, experts, topk, tokens)
+            idx[0, 0] = -1
+            r = ll.dispatch(x, idx)
+            counts = torch.bincount(idx[idx >= 0].long(), minlength=experts)
+            assert torch.equal(r.count.long(), counts) and torch.equal(r.layout_range[:, 0], counts)
+            assert torch.equal(r.send_slot >= 0, idx >= 0) and not r.begin.any()
+            q, s = per_token_cast_to_fp8(x)
+            for t in range(tokens):
+                for k in range(topk):
+                    e, i = int(idx[t, k]), int(r.send_slot[t, k])
+                    if e < 0:
+                        continue
+                    assert i < int(counts[e]) and int(r.src_info[e, i]) == t
+                    if fp8:
+                        torch.testing.assert_close(r.scales[e, i], s[t], rtol=1e-5, atol=1e-8)
+                        assert (r.x[e, i].view(torch.uint8) == q[t].view(torch.uint8)).float().mean() > 0.95  # but ties
+                    else:
+                        assert torch.equal(r.x[e, i], x[t])
+                    ll.expert_output[e, i] = x[t] * (e % 3 + 1)
+            y = ll.combine(idx, w, r)
+            coef = (w.double() * (idx % 3 + 1) * (idx >= 0)).sum(dim=1, keepdim=True)
+            # bf16 products, an fp32 sum of up to 8 of them, one rounding to bf16
+            torch.testing.assert_close(y.double(), coef * x.double(), rtol=2**-7, atol=1e-2)
+    comm.finalize()

@@ -38,6 +38,7 @@ struct EpDev {
   float* comb_topk_w[kMaxRanks];       // [rows, topk] fp32: expert-side per-expert weights (or their gradients) that combine returns
   // Local scratch.
   int* cnt;          // [nranks] tokens per destination; zero between calls
+  int* ticket;       // [1] blocks that have finished (single rank); zero between calls
   int* order;        // [max_tokens, nranks] number of the token among this rank's tokens for the destination, -1 = not sent
   long long* base;   // [nranks] first slot of this rank's rows in each destination
   int* recv_info;    // [1 + nranks]: total rows received, then rows per source

@@ -45,6 +45,7 @@ struct EpLlDev {
   // Local.
   int* cnt;                   // [2][num_experts] send counters, the idle parity is zeroed for the next call
   unsigned int* call;         // [1] calls so far
+  unsigned int* ticket;       // [1] blocks that have finished (single rank); zero between calls
   int* send_slot;             // [max_tokens][topk] row number within (expert, this source), -1 = not sent
   int* begin;                 // [num_experts] packed position of this rank's first row at each expert
 };

@@ -300,6 +300,7 @@ class EpBuffer {
       return p;
     };
     e.cnt = static_cast<int*>(local(sizeof(int) * kMaxRanks));
+    e.ticket = e.cnt + kMaxRanks - 1;  // a single rank uses cnt[0] only, others no ticket
     e.order = static_cast<int*>(local(sizeof(int) * static_cast<size_t>(max_tokens_) * nranks_));
     e.base = static_cast<long long*>(local(sizeof(long long) * kMaxRanks));
     e.recv_info = static_cast<int*>(local(sizeof(int) * (1 + kMaxRanks)));

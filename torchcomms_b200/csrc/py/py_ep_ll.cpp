@@ -260,7 +260,8 @@ class EpLlBuffer {
       return p;
     };
     e.cnt = static_cast<int*>(local(sizeof(int) * 2 * num_experts_));
-    e.call = static_cast<unsigned int*>(local(sizeof(unsigned int)));
+    e.call = static_cast<unsigned int*>(local(2 * sizeof(unsigned int)));
+    e.ticket = e.call + 1;
     e.send_slot = static_cast<int*>(local(sizeof(int) * static_cast<size_t>(max_tokens_) * topk_));
     e.begin = static_cast<int*>(local(sizeof(int) * num_experts_));
   }
