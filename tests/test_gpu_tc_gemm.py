@@ -20,6 +20,31 @@ def test_gemm_bf16_nt(m, n, k):
     torch.testing.assert_close(c.float(), ref, rtol=2e-2, atol=2e-2 * (k ** 0.5))
 
 
+@pytest.mark.parametrize("kind", ["e4m3", "bf16", "pairs"])
+@pytest.mark.parametrize("m,n,k", [(3332, 2160, 864), (2000, 4168, 432), (6500, 1032, 256)])
+def test_gemm_partial_last_column_tiles(m, n, k, kind):
+    """Column tiles of which only the first 64-column chunks exist, followed by further tiles of the same CTA: a chunk
+    that is not stored must not overwrite one that still is."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops.tp import quantize_rows
+
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = (torch.randn(m, k, generator=g, device="cuda") * 0.5).to(torch.bfloat16)
+    b = (torch.randn(n, k, generator=g, device="cuda") * 0.5).to(torch.bfloat16)
+    if kind == "e4m3":
+        (qa, sa), (qb, sb) = quantize_rows(a), quantize_rows(b)
+        ref = (qa.double() * sa.double().unsqueeze(1)) @ (qb.double() * sb.double().unsqueeze(1)).t()
+        run = lambda: _comms.ops.gemm_e4m3_nt(qa, qb, sa, sb)
+    else:
+        ref = a.double() @ b.double().t()
+        run = lambda: (_comms.ops.gemm_bf16_nt if kind == "bf16" else _comms.ops.gemm_bf16_nt_pair)(a, b)
+    for _ in range(5):
+        c, status = run()
+        assert int(status[0]) == 0
+        # Half a bf16 ulp (2^-9 relative), and k fp32 additions of terms of size 1/4 before it.
+        torch.testing.assert_close(c.double(), ref, rtol=2**-8, atol=1e-6 * k)
+
+
 @pytest.mark.parametrize("m", [1, 67, 128, 129, 300])
 @pytest.mark.parametrize("n,k", [(8, 8), (136, 72), (128, 256), (136, 264), (3584, 4096), (6144, 1928)])
 @pytest.mark.parametrize("fp8", [False, True])

@@ -514,8 +514,10 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
         }
         fence_proxy_async_smem();
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (issuer && ni * BN + j * kOutChunkCols < p.n) {  // chunks wholly past the last column are skipped
-          tma_store_2d(mo, buf, ni * BN + j * kOutChunkCols, out_row);
+        if (issuer) {
+          if (ni * BN + j * kOutChunkCols < p.n) tma_store_2d(mo, buf, ni * BN + j * kOutChunkCols, out_row);
+          // A chunk wholly past the last column stores nothing, but counts as a (then empty) group: the wait above
+          // reaches the buffer's last reader by counting groups.
           tma_store_commit();
         }
       }

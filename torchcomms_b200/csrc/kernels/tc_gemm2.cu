@@ -198,8 +198,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         fence_proxy_async_smem();
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (issuer && out_row < m && pn * kBN + j * kOutChunkCols < n) {
-          tma_store_2d(&maps.out, buf, pn * kBN + j * kOutChunkCols, out_row);
+        if (issuer) {
+          if (out_row < m && pn * kBN + j * kOutChunkCols < n) tma_store_2d(&maps.out, buf, pn * kBN + j * kOutChunkCols, out_row);
+          // Nothing to store outside the matrix, but an empty group all the same: the wait above counts groups.
           tma_store_commit();
         }
       }
