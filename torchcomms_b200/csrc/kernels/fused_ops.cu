@@ -654,28 +654,31 @@ __global__ void __launch_bounds__(kCeMaxThreads, 2) k_cross_entropy(__nv_bfloat1
 
 // out = in * bf16(*factor) for n bf16 values, the factor on the device. Both pointers 16-byte aligned; out may be
 // in, and then a factor of one (the gradient of a loss that is differentiated directly) leaves nothing to do.
-constexpr int kScaleVecs = 4;
-
+// Blocks stride over the data: with nothing to do, the 64 thousand blocks that cover a 1 GB gradient once take 45 us
+// to start and end, these 5.
 __global__ void __launch_bounds__(256) k_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* __restrict__ factor,
                                                      size_t n) {
   const float f = __bfloat162float(__float2bfloat16_rn(*factor));
   if (f == 1.0f && in == out) return;
-  const size_t nvec = n / 8, base = blockIdx.x * static_cast<size_t>(256 * kScaleVecs) + threadIdx.x;
-  uint4 q[kScaleVecs];
+  const size_t nvec = n / 8, stride = static_cast<size_t>(gridDim.x) * 256;
+  size_t v = blockIdx.x * static_cast<size_t>(256) + threadIdx.x;
+  auto one = [&](uint4 q) {
+    float x[8];
+    unpack8(q, x);
 #pragma unroll
-  for (int k = 0; k < kScaleVecs; ++k) {
-    if (base + k * 256 < nvec) q[k] = __ldcs(reinterpret_cast<const uint4*>(in) + base + k * 256);
+    for (int i = 0; i < 8; ++i) x[i] *= f;
+    return pack8(x);
+  };
+  const uint4* src = reinterpret_cast<const uint4*>(in);
+  uint4* dst = reinterpret_cast<uint4*>(out);
+  for (; v + 3 * stride < nvec; v += 4 * stride) {
+    uint4 q[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q[k] = __ldcs(src + v + k * stride);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dst[v + k * stride] = one(q[k]);
   }
-#pragma unroll
-  for (int k = 0; k < kScaleVecs; ++k) {
-    if (base + k * 256 < nvec) {
-      float x[8];
-      unpack8(q[k], x);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] *= f;
-      reinterpret_cast<uint4*>(out)[base + k * 256] = pack8(x);
-    }
-  }
+  for (; v < nvec; v += stride) dst[v] = one(src[v]);
   if (blockIdx.x == 0 && threadIdx.x < n % 8) {
     const size_t i = nvec * 8 + threadIdx.x;
     out[i] = __float2bfloat16_rn(__bfloat162float(in[i]) * f);
@@ -689,8 +692,8 @@ constexpr int kQuantKeep = 8;  // vectors of 8 a thread holds between the two lo
 // q[r, :] = e4m3(x[r, :] / scale[r]) with scale[r] = max(amax_r, 1e-8) / 448. A block per row, which stays in
 // registers between the maximum and the division (longer rows re-read the rest from L2): 2 bytes in and 1 byte
 // out per element is all that moves. The maximum is taken on the bit patterns, where NaN is above infinity and
-// so comes through. [4096, 4096] and [4096, 14336] together: 890 us operator by operator, 59 us (3.9 TB/s) here;
-// [67, 4096]: 27 us in eight launches, now 2.6. VEC: 16-byte loads (base, row stride and cols allow them).
+// so comes through. [4096, 4096] and [4096, 14336] together: 890 us operator by operator, 42 us (5.4 TB/s) here;
+// [67, 4096]: 27 us in eight launches, now 2.3. VEC: 16-byte loads (base, row stride and cols allow them).
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_quantize_rows(const __nv_bfloat16* __restrict__ x, int64_t ld,
                                                         uint8_t* __restrict__ q, float* __restrict__ scale, int cols) {
@@ -1101,7 +1104,7 @@ cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, int64_t ld, cons
 cudaError_t launch_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* factor, size_t n, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) return cudaErrorMisalignedAddress;
-  k_scale_bf16<<<covering_grid(n / 8, 256 * kScaleVecs), 256, 0, s>>>(in, out, factor, n);
+  k_scale_bf16<<<std::min<unsigned>(covering_grid(n / 8, 256 * 4), kSms * 8), 256, 0, s>>>(in, out, factor, n);
   note_kernel_launch();
   return cudaGetLastError();
 }
