@@ -170,18 +170,18 @@ class _LinearCrossEntropy(torch.autograd.Function):
         dx = torch.empty_like(x)
         dw = torch.empty_like(weight) if x.is_cuda and rows else torch.zeros_like(weight)
         loss_sum = torch.zeros((), dtype=torch.float32, device=x.device)
+        vocab = weight.shape[0]
+        # Rows of a vocabulary that is no multiple of 8 start off 16-byte boundaries, which costs the three GEMMs their
+        # tiled loads and stores. A copy of the weight with a few zero rows more puts logits and weight back on them:
+        # their logits are zero, stay zero, and add nothing. Below 24 M elements the copy costs as much as it saves.
+        pad = -vocab % 8 if x.is_cuda and x.dtype == weight.dtype == torch.bfloat16 and weight.numel() >= 24 << 20 else 0
+        wide = F.pad(weight, (0, 0, 0, pad)) if pad else weight
         for r0 in range(0, rows, chunk_rows):
             r1 = min(rows, r0 + chunk_rows)
-            if x.is_cuda and weight.shape[0] % 8 and x.dtype == weight.dtype == torch.bfloat16:
-                # Rows of such a vocabulary would start off 16-byte boundaries, which costs the three GEMMs their
-                # tiled loads; in a buffer of padded rows they do not.
-                logits = x.new_empty(r1 - r0, (weight.shape[0] + 63) // 64 * 64)[:, : weight.shape[0]]
-                torch.mm(x[r0:r1], weight.t(), out=logits)
-            else:
-                logits = x[r0:r1] @ weight.t()
+            logits = x[r0:r1] @ wide.t()
             if x.is_cuda:
-                loss = _k.cross_entropy_fwd_bwd_(logits, targets[r0:r1].contiguous(), scale)
-                dlogits = logits
+                dlogits = logits[:, :vocab] if pad else logits
+                loss = _k.cross_entropy_fwd_bwd_(dlogits, targets[r0:r1].contiguous(), scale)
             else:
                 lf = logits.float()
                 loss = F.cross_entropy(lf, targets[r0:r1], reduction="none", ignore_index=-1)
@@ -190,7 +190,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
                 dlogits = ((p - onehot) * (targets[r0:r1] >= 0).unsqueeze(-1) * scale).to(x.dtype)
             loss_sum += loss.sum()
             if x.is_cuda:
-                torch.mm(dlogits, weight, out=dx[r0:r1])
+                torch.mm(logits, wide, out=dx[r0:r1])  # the kernel left the gradient in the logits
             else:
                 dx[r0:r1] = dlogits @ weight
             if x.is_cuda and r0 == 0:
