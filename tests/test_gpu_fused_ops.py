@@ -276,6 +276,48 @@ def test_norm_with_residual_stream(rows, cols):
     torch.testing.assert_close(dx.double(), rs, rtol=2**-8, atol=2e-5)
 
 
+@pytest.mark.parametrize("offset", [1, 4, 7])
+def test_norm_and_swiglu_at_odd_offsets(offset):
+    """Contiguous views that start off a 16-byte boundary (a narrow of a flat buffer, a slice of a gradient) give the
+    bits that copies of them give, for every input and incoming gradient."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops import fused
+
+    def odd(*shape, seed):
+        n = 1
+        for d in shape:
+            n *= d
+        t = _bf(n + offset, seed=seed)[offset:].view(*shape)
+        assert t.is_contiguous() and t.data_ptr() % 16 != 0
+        return t
+
+    rows, cols = 37, 1032
+    x, d, w = odd(rows, cols, seed=70), odd(rows, cols, seed=71), odd(cols, seed=72)
+    gs, gy = odd(rows, cols, seed=73), odd(rows, cols, seed=74)
+    gu, dh = odd(rows, 2 * cols, seed=75), odd(rows, cols, seed=76)
+
+    def passes(*ts):
+        x, d, w, gs, gy, gu, dh = ts
+        x, d, w, gu = (t.detach().requires_grad_(True) for t in (x, d, w, gu))
+        s, y = fused.add_rms_norm(x, d, w)
+        out = [s, y, *torch.autograd.grad((s, y), (x, d, w), (gs, gy))]
+        s, y = fused.rms_norm_skip(x, w)
+        out += [s, y, *torch.autograd.grad((s, y), (x, w), (gs, gy))]
+        y = fused.rms_norm(x, w)
+        out += [y, *torch.autograd.grad(y, (x, w), gy)]
+        h = fused.swiglu(gu)
+        out += [h, *torch.autograd.grad(h, gu, dh)]
+        y, rstd = _comms.ops.rmsnorm_fwd(x, w, 1e-5)
+        out += [y, rstd, *_comms.ops.rmsnorm_bwd(gy, x, w, rstd), _comms.ops.swiglu_fwd(gu), _comms.ops.swiglu_bwd(dh, gu)]
+        return out
+
+    aligned = passes(*(t.clone() for t in (x, d, w, gs, gy, gu, dh)))
+    assert all(torch.equal(a, b) for a, b in zip(passes(x, d, w, gs, gy, gu, dh), aligned))
+    for i in range(7):                                             # one at a time
+        ts = [t if k == i else t.clone() for k, t in enumerate((x, d, w, gs, gy, gu, dh))]
+        assert all(torch.equal(a, b) for a, b in zip(passes(*ts), aligned)), i
+
+
 @pytest.mark.parametrize("tokens,heads,kv,hd", [(1, 1, 1, 8), (37, 6, 2, 96), (1000, 8, 8, 64), (513, 4, 1, 128)])
 @pytest.mark.parametrize("layout", ["contiguous", "transposed", "odd"])
 def test_split_rope_matches_split_and_rotate(tokens, heads, kv, hd, layout):

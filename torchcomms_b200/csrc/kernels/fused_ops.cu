@@ -907,6 +907,12 @@ unsigned long long fused_ops_launch_count() { return kernel_launch_count(); }
 
 namespace {
 
+// Vector accesses of 16 bytes (null pointers, as in a sizing query or for an absent operand, count as aligned).
+template <typename... P>
+bool misaligned16(const P*... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15u) != 0;
+}
+
 template <bool ADD>
 void rmsnorm_fwd_rows(const __nv_bfloat16* x, const __nv_bfloat16* delta, const __nv_bfloat16* w, __nv_bfloat16* sum,
                       __nv_bfloat16* y, float* rstd, int rows, int cols, float eps, cudaStream_t s) {
@@ -937,6 +943,7 @@ void rmsnorm_bwd_rows(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __n
 cudaError_t launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y, float* rstd, int rows,
                                int cols, float eps, cudaStream_t s, const __nv_bfloat16* delta, __nv_bfloat16* sum) {
   if (cols % 8 != 0 || rows <= 0) return cudaErrorInvalidValue;
+  if (misaligned16(x, w, y, delta, sum)) return cudaErrorMisalignedAddress;
   if (delta != nullptr) {
     if (cols > kNormThreads * kNormMaxVec * 8 || sum == nullptr) return cudaErrorInvalidValue;
     rmsnorm_fwd_rows<true>(x, delta, w, sum, y, rstd, rows, cols, eps, s);
@@ -958,6 +965,7 @@ cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, 
   const int blocks = std::min(warp_rows ? (rows + 7) / 8 : rows, kSms * per_sm);
   if (nblocks) *nblocks = blocks;
   if (dw_partial == nullptr) return cudaSuccess;
+  if (misaligned16(dy, x, w, dx, dskip, dw_partial)) return cudaErrorMisalignedAddress;
   if (dskip != nullptr) rmsnorm_bwd_rows<true>(dy, x, w, rstd, dskip, dx, dw_partial, blocks, rows, cols, s);
   else rmsnorm_bwd_rows<false>(dy, x, w, rstd, nullptr, dx, dw_partial, blocks, rows, cols, s);
   note_kernel_launch();
@@ -1073,6 +1081,7 @@ cudaError_t launch_split_rope(__nv_bfloat16* packed, int64_t ld, __nv_bfloat16* 
 
 cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, int rows, int ffn, cudaStream_t s) {
   if (ffn % 8 != 0) return cudaErrorInvalidValue;
+  if (misaligned16(gate_up, h)) return cudaErrorMisalignedAddress;
   return for_row_slices(rows, ffn / 8, [&](size_t r0, uint32_t total) {
     k_swiglu_fwd<<<(total + 256u * kSwigluVecs - 1) / (256u * kSwigluVecs), 256, 0, s>>>(gate_up + r0 * 2 * ffn, h + r0 * ffn, total,
                                                                                         make_fast_div(ffn / 8));
@@ -1082,6 +1091,7 @@ cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, in
 cudaError_t launch_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate_up, __nv_bfloat16* dgate_up, int rows,
                               int ffn, cudaStream_t s) {
   if (ffn % 8 != 0) return cudaErrorInvalidValue;
+  if (misaligned16(dh, gate_up, dgate_up)) return cudaErrorMisalignedAddress;
   return for_row_slices(rows, ffn / 8, [&](size_t r0, uint32_t total) {
     k_swiglu_bwd<<<(total + 256u * kSwigluVecs - 1) / (256u * kSwigluVecs), 256, 0, s>>>(
         dh + r0 * ffn, gate_up + r0 * 2 * ffn, dgate_up + r0 * 2 * ffn, total, make_fast_div(ffn / 8));

@@ -11,7 +11,8 @@
 namespace b200c {
 
 // y = x * rsqrt(mean(x^2) + eps) * w ; rstd saved for the backward pass.
-// cols must be a multiple of 8. With `delta` (cols <= 8192) the normalised row is sum = bf16(x + delta), which is
+// cols must be a multiple of 8; all bf16 pointers of the norm and SwiGLU launches are 16-byte aligned
+// (cudaErrorMisalignedAddress otherwise). With `delta` (cols <= 8192) the normalised row is sum = bf16(x + delta), which is
 // written as well.
 cudaError_t launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y, float* rstd,
                                int rows, int cols, float eps, cudaStream_t s, const __nv_bfloat16* delta = nullptr,

@@ -32,6 +32,11 @@ cudaStream_t cur(const at::Tensor& t) {
   return at::cuda::getCurrentCUDAStream(t.device().index()).stream();
 }
 
+bool on16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+// The kernels take vectors of 16 bytes. A contiguous view at an odd storage offset (a narrow of a flat buffer, a slice
+// of a gradient) does not start on such a boundary, and contiguous() leaves it where it is.
+at::Tensor vectorable(const at::Tensor& t) { return on16(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
+
 // Two status words; eight bytes are cleared by the copy engine's memset, without a kernel launch through the
 // tensor library.
 at::Tensor cleared_status(const at::Tensor& like) {
@@ -65,11 +70,10 @@ void rope_into(const at::Tensor& x, at::Tensor& y, const at::Tensor& pos, const 
   c10::cuda::CUDAGuard g(x.device());
   // A slice of a wider tensor (queries or keys of a fused projection) is read where it is; layouts that
   // 16-byte loads cannot follow are made contiguous first.
-  auto aligned = [](const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; };
-  const bool in_place = x.dim() == 3 && x.stride(2) == 1 && x.stride(0) % 8 == 0 && x.stride(1) % 8 == 0 && aligned(x);
+  const bool in_place = x.dim() == 3 && x.stride(2) == 1 && x.stride(0) % 8 == 0 && x.stride(1) % 8 == 0 && on16(x);
   const at::Tensor src = in_place || x.is_same(y) ? x : x.clone(at::MemoryFormat::Contiguous);
   const int64_t st = in_place ? src.stride(0) : per_token, sh = in_place ? src.stride(1) : head_dim;
-  const at::Tensor c = aligned(cos_t) ? cos_t : cos_t.clone(), sn = aligned(sin_t) ? sin_t : sin_t.clone();
+  const at::Tensor c = vectorable(cos_t), sn = vectorable(sin_t);
   B200C_CUDA_CHECK(launch_rope(bf(src), st, sh, bf_mut(y), pos.data_ptr<int>(), c.data_ptr<float>(), sn.data_ptr<float>(), tokens,
                                heads, head_dim, inverse, cur(x)));
 }
@@ -88,9 +92,10 @@ std::pair<at::Tensor, at::Tensor> rmsnorm_fwd(const at::Tensor& x, const at::Ten
   const int rows = static_cast<int>(x.numel() / cols);
   TORCH_CHECK(w.numel() == cols, "weight must have ", cols, " elements");
   c10::cuda::CUDAGuard g(x.device());
+  const at::Tensor xv = vectorable(x), wv = vectorable(w);
   at::Tensor y = at::empty_like(x);
   at::Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
-  B200C_CUDA_CHECK(launch_rmsnorm_fwd(bf(x), bf(w), bf_mut(y), rstd.data_ptr<float>(), rows, cols,
+  B200C_CUDA_CHECK(launch_rmsnorm_fwd(bf(xv), bf(wv), bf_mut(y), rstd.data_ptr<float>(), rows, cols,
                                       static_cast<float>(eps), cur(x)));
   return std::make_pair(y, rstd);
 }
@@ -106,10 +111,11 @@ std::pair<at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dy, const at::Te
   c10::cuda::CUDAGuard g(x.device());
   int nblocks = 0;
   B200C_CUDA_CHECK(launch_rmsnorm_bwd(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &nblocks, rows, cols, cur(x)));
+  const at::Tensor dyv = vectorable(dy), xv = vectorable(x), wv = vectorable(w);
   at::Tensor dx = at::empty_like(x);
   at::Tensor partial = at::empty({nblocks, cols}, x.options().dtype(at::kFloat));
   at::Tensor dw = at::empty_like(w);
-  B200C_CUDA_CHECK(launch_rmsnorm_bwd(bf(dy), bf(x), bf(w), rstd.data_ptr<float>(), bf_mut(dx),
+  B200C_CUDA_CHECK(launch_rmsnorm_bwd(bf(dyv), bf(xv), bf(wv), rstd.data_ptr<float>(), bf_mut(dx),
                                       partial.data_ptr<float>(), &nblocks, rows, cols, cur(x)));
   B200C_CUDA_CHECK(launch_colsum_bf16(partial.data_ptr<float>(), bf_mut(dw), nblocks, cols, cur(x)));
   return std::make_pair(dx, dw);
@@ -122,8 +128,9 @@ at::Tensor swiglu_fwd(const at::Tensor& gate_up) {
   c10::cuda::CUDAGuard g(gate_up.device());
   auto sizes = gate_up.sizes().vec();
   sizes.back() = ffn;
+  const at::Tensor guv = vectorable(gate_up);
   at::Tensor h = at::empty(sizes, gate_up.options());
-  B200C_CUDA_CHECK(launch_swiglu_fwd(bf(gate_up), bf_mut(h), rows, ffn, cur(gate_up)));
+  B200C_CUDA_CHECK(launch_swiglu_fwd(bf(guv), bf_mut(h), rows, ffn, cur(gate_up)));
   return h;
 }
 
@@ -133,8 +140,9 @@ at::Tensor swiglu_bwd(const at::Tensor& dh, const at::Tensor& gate_up) {
   const int ffn = static_cast<int>(gate_up.size(-1) / 2);
   const int rows = static_cast<int>(gate_up.numel() / (2 * static_cast<int64_t>(ffn)));
   c10::cuda::CUDAGuard g(gate_up.device());
+  const at::Tensor dhv = vectorable(dh), guv = vectorable(gate_up);
   at::Tensor d = at::empty_like(gate_up);
-  B200C_CUDA_CHECK(launch_swiglu_bwd(bf(dh), bf(gate_up), bf_mut(d), rows, ffn, cur(gate_up)));
+  B200C_CUDA_CHECK(launch_swiglu_bwd(bf(dhv), bf(guv), bf_mut(d), rows, ffn, cur(gate_up)));
   return d;
 }
 
@@ -175,11 +183,12 @@ variable_list norm_with_skip_backward(const variable_list& grads, const variable
   c10::cuda::CUDAGuard g(x.device());
   int nblocks = 0;
   B200C_CUDA_CHECK(launch_rmsnorm_bwd(nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &nblocks, rows, cols, cur(x)));
+  const at::Tensor dyv = vectorable(dy), xv = vectorable(x), wv = vectorable(w), skip = vectorable(dskip);
   at::Tensor dx = at::empty_like(x);
   at::Tensor partial = at::empty({nblocks, cols}, x.options().dtype(at::kFloat));
   *dw = at::empty_like(w);
-  B200C_CUDA_CHECK(launch_rmsnorm_bwd(bf(dy), bf(x), bf(w), rstd.data_ptr<float>(), bf_mut(dx), partial.data_ptr<float>(), &nblocks,
-                                      rows, cols, cur(x), bf(dskip)));
+  B200C_CUDA_CHECK(launch_rmsnorm_bwd(bf(dyv), bf(xv), bf(wv), rstd.data_ptr<float>(), bf_mut(dx), partial.data_ptr<float>(), &nblocks,
+                                      rows, cols, cur(x), bf(skip)));
   B200C_CUDA_CHECK(launch_colsum_bf16(partial.data_ptr<float>(), bf_mut(*dw), nblocks, cols, cur(x)));
   return {dx};
 }
@@ -203,10 +212,11 @@ struct AddRmsNormFn : torch::autograd::Function<AddRmsNormFn> {
     want(delta, at::kBFloat16, "delta");
     const int cols = static_cast<int>(x.size(-1)), rows = static_cast<int>(x.numel() / cols);
     c10::cuda::CUDAGuard g(x.device());
+    const at::Tensor xv = vectorable(x), dv = vectorable(delta), wv = vectorable(w);
     at::Tensor sum = at::empty_like(x), y = at::empty_like(x);
     at::Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
-    B200C_CUDA_CHECK(launch_rmsnorm_fwd(bf(x), bf(w), bf_mut(y), rstd.data_ptr<float>(), rows, cols, static_cast<float>(eps), cur(x),
-                                        bf(delta), bf_mut(sum)));
+    B200C_CUDA_CHECK(launch_rmsnorm_fwd(bf(xv), bf(wv), bf_mut(y), rstd.data_ptr<float>(), rows, cols, static_cast<float>(eps), cur(x),
+                                        bf(dv), bf_mut(sum)));
     ctx->save_for_backward({sum, w, rstd});
     return {sum, y};
   }
@@ -219,8 +229,7 @@ struct AddRmsNormFn : torch::autograd::Function<AddRmsNormFn> {
 
 // Strides a split_rope launch can follow for [tokens, heads, head_dim].
 bool followable(const at::Tensor& t) {
-  return t.dim() == 3 && t.stride(2) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 &&
-      (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
+  return t.dim() == 3 && t.stride(2) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && on16(t);
 }
 
 struct SplitRopeFn : torch::autograd::Function<SplitRopeFn> {
@@ -265,11 +274,9 @@ struct SplitRopeFn : torch::autograd::Function<SplitRopeFn> {
     if (heads < 1 || kv_heads < 1 || qkv.dim() != 2 || qkv.numel() == 0 || qkv.size(1) % (8 * (heads + 2 * kv_heads)) != 0) return false;
     const int64_t hd = qkv.size(1) / (heads + 2 * kv_heads);
     auto table = [&](const at::Tensor& t) {
-      return t.scalar_type() == at::kFloat && t.is_contiguous() && t.dim() == 2 && t.size(1) == hd / 2 && t.device() == qkv.device() &&
-          (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
+      return t.scalar_type() == at::kFloat && t.is_contiguous() && t.dim() == 2 && t.size(1) == hd / 2 && t.device() == qkv.device() && on16(t);
     };
-    return qkv.scalar_type() == at::kBFloat16 && qkv.stride(1) == 1 && qkv.stride(0) % 8 == 0 &&
-        (reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 15u) == 0 && table(cos_t) && table(sin_t) && pos.scalar_type() == at::kInt &&
+    return qkv.scalar_type() == at::kBFloat16 && qkv.stride(1) == 1 && qkv.stride(0) % 8 == 0 && on16(qkv) && table(cos_t) && table(sin_t) && pos.scalar_type() == at::kInt &&
         pos.is_contiguous() && pos.numel() == qkv.size(0) && pos.device() == qkv.device();
   }
 };
@@ -388,7 +395,7 @@ void bind_ops(py::module_& m) {
   // afterwards, so the product may take its place.
   ops.def("scale_by", [](const at::Tensor& t, const at::Tensor& factor, bool consume) {
     const bool direct = plain_call(t) && plain_call(factor) && t.scalar_type() == at::kBFloat16 &&
-        t.is_non_overlapping_and_dense() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0 && factor.dim() == 0 &&
+        t.is_non_overlapping_and_dense() && on16(t) && factor.dim() == 0 &&
         factor.scalar_type() == at::kFloat && factor.device() == t.device();
     if (!direct) return t * factor.to(t.scalar_type());
     c10::cuda::CUDAGuard g(t.device());
