@@ -248,6 +248,23 @@ def test_adamw_matches_torch():
     torch.testing.assert_close(p, ref_p.detach(), rtol=1e-4, atol=1e-5)
 
 
+def test_adamw_refuses_shards_off_the_vector_grid():
+    """Updated in place, so a shard at an odd offset cannot be copied: an error, and nothing is launched. Three elements
+    use no vectors and go anywhere."""
+    from torchcomms_b200.ops import fused
+
+    ts = [torch.zeros(65, device="cuda") for _ in range(4)]
+    for i in range(4):
+        with pytest.raises(RuntimeError):
+            fused.adamw_step_(*(t[1:] if k == i else t[:64] for k, t in enumerate(ts)), lr=0.1, step=1)
+    before = [t.clone() for t in ts]
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(before, ts))
+    ts[1].fill_(1.0)
+    fused.adamw_step_(*(t[1:4] for t in ts), lr=0.1, step=1)
+    assert bool((ts[0][1:4] < 0).all()) and not ts[0][0] and not ts[0][4:].any()
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 8), (9, 256), (40, 512), (700, 1000), (5, 2048), (601, 4096), (3, 8192), (300, 8192)])
 def test_norm_with_residual_stream(rows, cols):
     """x + delta and its norm in one kernel: forward bit for bit what addition and norm give, backward with the

@@ -1122,6 +1122,7 @@ cudaError_t launch_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const
 cudaError_t launch_adamw(float* p, const float* g, float* m, float* v, size_t n, float lr, float beta1, float beta2,
                          float eps, float weight_decay, int step, float grad_scale, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
+  if (n >= 4 && misaligned16(p, g, m, v)) return cudaErrorMisalignedAddress;  // fewer elements use no vectors
   const float bias1 = 1.0f - powf(beta1, static_cast<float>(step));
   const float bias2 = 1.0f - powf(beta2, static_cast<float>(step));
   k_adamw<<<covering_grid(n / 4, 256 * kAdamwVecs), 256, 0, s>>>(p, g, m, v, n, lr, beta1, beta2, eps, weight_decay, bias1, bias2,

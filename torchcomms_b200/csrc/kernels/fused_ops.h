@@ -64,7 +64,7 @@ cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, int64_t ld, cons
 // out = in * bf16(*factor) on n bf16 values, the factor read from device memory; in and out 16-byte aligned.
 cudaError_t launch_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* factor, size_t n, cudaStream_t s);
 
-// AdamW on flat fp32 tensors. `grad_scale` multiplies the gradient first
+// AdamW on flat fp32 tensors, 16-byte aligned from four elements on. `grad_scale` multiplies the gradient first
 // (loss scaling / averaging); `step` starts at 1.
 cudaError_t launch_adamw(float* p, const float* g, float* m, float* v, size_t n, float lr, float beta1, float beta2,
                          float eps, float weight_decay, int step, float grad_scale, cudaStream_t s);
