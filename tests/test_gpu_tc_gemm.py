@@ -70,6 +70,26 @@ def test_gemm_split_over_clusters(m, n, k, fp8):
     torch.testing.assert_close(c.double(), ref, rtol=2**-8, atol=1e-6 * k)
 
 
+@pytest.mark.parametrize("m,n,k", [(128, 3584, 4096), (128, 4096, 1792), (5, 4096, 4096), (100, 1032, 2056)])
+def test_gemm_split_repeats_and_rounds_no_worse(m, n, k):
+    """The same bits at every call; no more results away from the exact product's bf16 value than the kernel that adds
+    up K in one chain has (sums are closer, so the reverse holds by a wide margin), and each next to it."""
+    from torchcomms_b200 import _comms
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(n, k, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    c = _comms.ops.gemm_bf16_nt(a, b)[0]
+    for _ in range(20):
+        assert torch.equal(_comms.ops.gemm_bf16_nt(a, b)[0], c)
+    exact = a.double() @ b.double().t()
+    rounded = exact.to(torch.bfloat16)
+    chain = _comms.ops.gemm_bf16_nt_pair(a, b)[0]
+    assert int((c != rounded).sum()) <= int((chain != rounded).sum())
+    # Half a bf16 ulp (2^-9 relative), and k fp32 additions of terms of size 0.02 before it.
+    torch.testing.assert_close(c.double(), exact, rtol=2**-8, atol=2e-8 * k)
+
+
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (512, 512, 1024), (300, 264, 200), (1024, 7168, 2048), (4096, 4096, 4096),
                                    (8192, 1792, 512)])
 def test_gemm_bf16_nt_cta_pairs(m, n, k):
