@@ -238,19 +238,23 @@ cudaLaunchConfig_t split_config(int tiles, int splits, cudaStream_t stream, cuda
   return cfg;
 }
 
-// Clusters of each size that the GPU holds at once (they must fit one GPC, so not simply SMs / size).
+// Clusters of each size that the current GPU holds at once: they must fit one GPC, so not simply SMs / size, and GPUs
+// differ in how their SMs are spread over GPCs. The answer decides the order of summation, so it is kept per device,
+// and a query that failed is asked again at the next call.
 template <bool FP8>
-int resident_clusters(int splits) {
-  static std::atomic<int> known[kSplitMax + 1];
-  int n = known[splits].load(std::memory_order_relaxed);
+int resident_clusters(int device, int splits) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices][kSplitMax + 1];
+  std::atomic<int>* kept = device >= 0 && device < kDevices ? &known[device][splits] : nullptr;
+  int n = kept != nullptr ? kept->load(std::memory_order_relaxed) : 0;
   if (n == 0) {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = split_config(1, splits, nullptr, attr);
     if (cudaOccupancyMaxActiveClusters(&n, k_gemm_split<FP8>, &cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
-      n = -1;
+      return 0;
     }
-    known[splits].store(n, std::memory_order_relaxed);
+    if (kept != nullptr) kept->store(n, std::memory_order_relaxed);
   }
   return n;
 }
@@ -261,10 +265,11 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
   if (e != cudaSuccess) return e;
   // As many ways as leave every cluster resident and every CTA at least four K steps (below that the fixed cost of
   // filling the pipeline and meeting the cluster is larger than what another split saves).
-  int splits = 0;
+  int splits = 0, device = 0;
+  if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
   for (int s = 1; s <= kSplitMax; ++s) {
     if (s > 1 && p.k_iters < 4 * s) break;
-    if (resident_clusters<FP8>(s) >= tiles) splits = s;
+    if (resident_clusters<FP8>(device, s) >= tiles) splits = s;
   }
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
   cudaLaunchAttribute attr[1];
