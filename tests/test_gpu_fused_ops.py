@@ -51,6 +51,20 @@ def test_rmsnorm_row_layouts(rows, cols):
     torch.testing.assert_close(dw.double(), rdw, rtol=2**-8, atol=1e-6 * rows**0.5 + 2e-5)
 
 
+@pytest.mark.parametrize("cols", [8200, 10240, 10248, 16384, 40008])
+@pytest.mark.parametrize("rows", [1, 1300])
+def test_rmsnorm_forward_wide_rows(rows, cols):
+    """Rows that the registers do not hold, from one vector past them on, with fewer and more rows than blocks."""
+    from torchcomms_b200 import _comms
+
+    x, w = _bf(rows, cols, seed=77), _bf(cols, seed=78, scale=0.1) + 1
+    y, rstd = _comms.ops.rmsnorm_fwd(x, w, 1e-5)
+    ref = torch.rsqrt(x.double().pow(2).mean(-1) + 1e-5)
+    # fp32 sums of up to 40008 squares; half a bf16 ulp (2^-9 relative) on the result.
+    torch.testing.assert_close(rstd.double(), ref, rtol=5e-6, atol=0)
+    torch.testing.assert_close(y.double(), x.double() * ref.unsqueeze(1) * w.double(), rtol=2**-8, atol=1e-6)
+
+
 def test_swiglu_forward_backward():
     from torchcomms_b200.ops import fused
 

@@ -164,35 +164,46 @@ __global__ void __launch_bounds__(TPR < 128 ? 128 : TPR) k_rmsnorm_fwd_reg(const
   }
 }
 
-// Rows wider than the registers hold: the remainder is read twice (the second time from L2).
+// Rows wider than the registers hold: the first kNormMaxVec vectors of every thread stay there between the two looks,
+// the remainder is read twice (the second time from L2). Against reading the whole row twice: 41.3 us and 39.1 at 4096
+// x 12288, but 49.3 and 53.1 at 4096 x 16384, 53.4 and 62.6 at 2048 x 32768, 10.3 and 12.4 at 8 x 65536.
 __global__ void __launch_bounds__(kNormThreads) k_rmsnorm_fwd_wide(const __nv_bfloat16* __restrict__ x,
                                                                     const __nv_bfloat16* __restrict__ w,
                                                                     __nv_bfloat16* __restrict__ y,
                                                                     float* __restrict__ rstd, int rows, int cols,
                                                                     float eps) {
   __shared__ float scratch[32];
-  const int nvec = cols / 8;
+  const int nvec = cols / 8, tail = kNormMaxVec * kNormThreads + threadIdx.x;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(r) * cols);
     uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(r) * cols);
+    uint4 keep[kNormMaxVec];  // all there: this kernel's rows are wider than that
+#pragma unroll
+    for (int k = 0; k < kNormMaxVec; ++k) keep[k] = xr[threadIdx.x + k * kNormThreads];
     float ss = 0.0f;
-    for (int v = threadIdx.x; v < nvec; v += kNormThreads) {
+    auto square = [&](uint4 q) {
       float f[8];
-      unpack8(xr[v], f);
+      unpack8(q, f);
 #pragma unroll
       for (int i = 0; i < 8; ++i) ss += f[i] * f[i];
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < kNormMaxVec; ++k) square(keep[k]);
+    for (int v = tail; v < nvec; v += kNormThreads) square(xr[v]);
     ss = block_sum(ss, scratch);
     const float rs = rsqrtf(ss / static_cast<float>(cols) + eps);
     if (threadIdx.x == 0) rstd[r] = rs;
-    for (int v = threadIdx.x; v < nvec; v += kNormThreads) {
+    auto write = [&](uint4 q, int v) {
       float f[8], g[8];
-      unpack8(xr[v], f);
+      unpack8(q, f);
       unpack8(reinterpret_cast<const uint4*>(w)[v], g);
 #pragma unroll
       for (int i = 0; i < 8; ++i) f[i] = f[i] * rs * g[i];
       yr[v] = pack8(f);
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < kNormMaxVec; ++k) write(keep[k], threadIdx.x + k * kNormThreads);
+    for (int v = tail; v < nvec; v += kNormThreads) write(xr[v], v);
   }
 }
 
