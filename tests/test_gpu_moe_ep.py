@@ -234,6 +234,52 @@ def test_low_latency_emulated(nranks, fp8, topk):
             torch.testing.assert_close(ys[s].float(), coef * xs[s].float(), rtol=0.08, atol=0.05 * num_experts)
 
 
+@pytest.mark.parametrize("nranks,per_rank", [(1, 6), (3, 5), (4, 1030)])
+def test_low_latency_own_rows(nranks, per_rank):
+    """Rows for a rank's own experts stand behind the lower ranks' at every expert, also with more local experts than a
+    block keeps first rows for, and with every token at one expert."""
+    from torchcomms_b200 import _comms
+
+    tokens, hidden, topk, experts = 16, 512, 4, nranks * per_rank
+    buf = _comms.EpLlBuffer.emulated(nranks, tokens, hidden, experts, topk, False, 2000.0)
+    g = torch.Generator(device="cuda").manual_seed(per_rank)
+    for it in range(3):
+        xs = [torch.randn(tokens, hidden, generator=g, device="cuda").to(torch.bfloat16) for _ in range(nranks)]
+        idxs = [torch.rand(tokens, experts, generator=g, device="cuda").topk(topk, -1)[1].to(torch.int32) for _ in range(nranks)]
+        for r in range(nranks):
+            far = torch.randint(max(0, per_rank - 8), per_rank, (tokens,), generator=g, device="cuda").to(torch.int32)
+            idxs[r][:, 0] = far + per_rank * ((r + it) % nranks)      # the last experts of one rank
+            idxs[r][:, 1] = experts - 1                               # everybody
+            idxs[r][:, 0][far + per_rank * ((r + it) % nranks) == experts - 1] = -1
+            idxs[r][:, 2:][(idxs[r][:, 2:] == experts - 1) | (idxs[r][:, 2:] == idxs[r][:, :1])] = -1
+        outs = buf.dispatch(xs, idxs)
+        torch.cuda.synchronize()
+        assert buf.status()[0] == 0
+        for r in range(nranks):
+            px, _, src, count, rng = outs[r]
+            want = [[(ix == r * per_rank + le).any(dim=1).nonzero().flatten().tolist() for ix in idxs] for le in range(per_rank)]
+            for le in range(per_rank):
+                assert int(count[le]) == sum(len(t) for t in want[le])
+                if not int(count[le]):
+                    continue
+                at = 0
+                for s in range(nranks):
+                    assert rng[le, s].item() == (at << 32) | len(want[le][s])
+                    got = src[le, at : at + len(want[le][s])].tolist()
+                    assert sorted(got) == want[le][s]
+                    assert torch.equal(px[le, at : at + len(got)], xs[s][got])
+                    at += len(got)
+            buf.view(r, "out_x").copy_(px)
+        ys = [torch.empty(tokens, hidden, dtype=torch.bfloat16, device="cuda") for _ in range(nranks)]
+        ws = [torch.rand(tokens, topk, generator=g, device="cuda") for _ in range(nranks)]
+        buf.combine(ys, idxs, ws)
+        torch.cuda.synchronize()
+        assert buf.status()[0] == 0
+        for y, x, w, ix in zip(ys, xs, ws, idxs):
+            # an fp32 sum of up to 4 products, one rounding to bf16
+            torch.testing.assert_close(y.double(), (w.double() * (ix >= 0)).sum(1, keepdim=True) * x.double(), rtol=2**-8, atol=1e-5)
+
+
 def _ep_train_worker(rank, world):
     """The fused trainable layer against the all-to-all layer: same outputs, same gradients."""
     import copy
