@@ -457,3 +457,42 @@ def test_single_rank_low_latency(fp8):
             # bf16 products, an fp32 sum of up to 8 of them, one rounding to bf16
             torch.testing.assert_close(y.double(), coef * x.double(), rtol=2**-7, atol=1e-2)
     comm.finalize()
+
+
+def test_phase_trace_on_one_rank():
+    """Every traced kernel of a single rank stamps its phases in order, and grids with more blocks than the trace has
+    rows leave the rest alone."""
+    from torchcomms_b200.ops.moe_ep import Buffer, LowLatencyBuffer
+    from torchcomms_b200.ops.tp import AllGatherGemm, GemmReduceScatter
+
+    comm = _solo_comm("solo_trace")
+    impl = comm.get_backend_impl()
+    tokens, hidden, experts, topk = 4096, 512, 16, 4
+    x = torch.randn(tokens, hidden, device="cuda").to(torch.bfloat16)
+    idx, w = _route(tokens, experts, topk, 1)
+    buf = Buffer(comm, tokens, hidden, experts, topk, fp8=True)
+    ll = LowLatencyBuffer(comm, 64, hidden, experts, topk, fp8=True)
+    up, down = AllGatherGemm(comm, m_local=128, k=512), GemmReduceScatter(comm, m=128, n=512)
+    wt = torch.randn(1024, 512, device="cuda").to(torch.bfloat16)
+    recv = ll.dispatch(x[:64], idx[:64])
+    calls = {
+        "dispatch": (lambda: buf.dispatch(x, idx, w), (0, 1, 2, 3, 4), 640),
+        "combine": (lambda: buf.combine(), (0, 1, 2, 3), 256),
+        "ll dispatch": (lambda: ll.dispatch(x[:64], idx[:64]), (0, 1, 2, 3, 4, 5), 64),
+        "ll combine": (lambda: ll.combine(idx[:64], w[:64], recv), (0, 1, 2, 3), 16),
+        "gather -> gemm": (lambda: up(wt, x[:128]), (0, 1, 2, 3, 7), 8),
+        "gemm -> scatter": (lambda: down(x[:128], wt[:512]), (0, 1, 2, 3, 7), 4),
+    }
+    for name, (call, marks, blocks) in calls.items():
+        call()
+        trace = impl.enable_trace()
+        call()
+        torch.cuda.synchronize()
+        impl.disable_trace()
+        t = trace.cpu()
+        used = t[t[:, 0] > 0]
+        assert used.shape[0] >= blocks, (name, used.shape)
+        assert bool((used[:, list(marks)] > 0).all()), name
+        first_last = used[:, marks[-1]] - used[:, marks[0]]
+        assert bool((first_last >= 0).all()) and int(first_last.max()) < 1_000_000_000, name
+    comm.finalize()

@@ -347,19 +347,22 @@ __device__ __forceinline__ void post_flags(const CommDev& c, bool post_ready, ui
   }
 }
 
-// Stamps the device's nanosecond timer into slot `slot` of this block's trace row (thread 0 of the block).
-__device__ __forceinline__ void trace_mark(const CommDev& c, int slot) {
-  if (c.trace != nullptr && threadIdx.x == 0 && slot < kTraceSlots) {
-    c.trace[static_cast<size_t>(blockIdx.x) * kTraceSlots + slot] = static_cast<long long>(globaltimer_ns());
+// Stamps the device's nanosecond timer into slot `slot` of this block's row of `trace` (nullptr = off; grids of more
+// than kMaxBlocks blocks are traced as far as the rows go). Call from ONE thread (any thread: the fused GEMM kernels
+// stamp from the warp that owns the phase). Comparable across the SMs of one GPU, not across GPUs.
+__device__ __forceinline__ void trace_stamp_ns(long long* trace, int slot) {
+  if (trace != nullptr && slot < kTraceSlots && blockIdx.x < kMaxBlocks) {
+    trace[static_cast<size_t>(blockIdx.x) * kTraceSlots + slot] = static_cast<long long>(globaltimer_ns());
   }
 }
+__device__ __forceinline__ void trace_stamp_ns(const CommDev& c, int slot) { trace_stamp_ns(c.trace, slot); }
 
-// Stamps the device's nanosecond timer into slot `slot` of this block's trace row. Call from ONE thread
-// (any thread: the fused GEMM kernels stamp from the warp that owns the phase). Comparable across the SMs
-// of one GPU, not across GPUs.
-__device__ __forceinline__ void trace_stamp_ns(const CommDev& c, int slot) {
-  if (c.trace != nullptr && slot < kTraceSlots) {
-    c.trace[static_cast<size_t>(blockIdx.x) * kTraceSlots + slot] = static_cast<long long>(globaltimer_ns());
+// The same from thread 0 of the block. Kernels of a few microseconds are built twice, so that the untraced one does
+// not even ask (ON = false).
+template <bool ON = true>
+__device__ __forceinline__ void trace_mark(const CommDev& c, int slot) {
+  if constexpr (ON) {
+    if (threadIdx.x == 0) trace_stamp_ns(c.trace, slot);
   }
 }
 

@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_emu(const CommDev* c
 // 23.3 us there).
 constexpr int kEpSoloTokens = 4;
 
+template <bool TRACE>
 __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDev e, DispatchArgs a) {
   constexpr int kSteps = kEpChunkCols / 512;
   __shared__ int s_slot[kEpSoloTokens];
@@ -259,6 +260,7 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
   const int t0 = blockIdx.x * kEpSoloTokens, here = min(kEpSoloTokens, a.num_tokens - t0);
   const int groups = e.hidden / 128, nchunks = (e.hidden + kEpChunkCols - 1) / kEpChunkCols;
   const size_t row_bytes = e.fp8 ? static_cast<size_t>(e.hidden) : static_cast<size_t>(e.hidden) * 2;
+  trace_mark<TRACE>(c, 0);  // the marks of the general kernel
   uint4 v0[kSteps], v1[kSteps];
   auto load = [&](int item) {
     const int t = t0 + item / nchunks, col0 = (item % nchunks) * kEpChunkCols + lane * 16;
@@ -299,6 +301,8 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
     }
   }
   __syncthreads();
+  trace_mark<TRACE>(c, 1);
+  trace_mark<TRACE>(c, 2);  // no counts to exchange
   if (warp < here) {  // metadata
     const int slot = s_slot[warp];
     if (lane == 0) e.send_slot[t0 + warp] = slot;
@@ -333,6 +337,7 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
     item += kEpWarps;
     if (item < here * nchunks) load(item);
   }
+  trace_mark<TRACE>(c, 3);
   if (threadIdx.x == 0) {
     __threadfence();  // this block's numbers are counted before it reports
     if (atomicAdd(e.ticket, 1) == static_cast<int>(gridDim.x) - 1) {
@@ -344,6 +349,7 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
       *e.ticket = 0;
     }
   }
+  trace_mark<TRACE>(c, 4);
 }
 
 struct CombineArgs {
@@ -365,7 +371,7 @@ struct CombineArgs {
 // flight per lane. One rank (RANKS = 1) has one source per token, so it takes
 // four columns and works on pieces of rows, to the same number of loads
 // (4096 x 7168: 39.0 us before, now 17.0, 6.9 TB/s).
-template <int RANKS, int COLS>
+template <int RANKS, int COLS, bool TRACE>
 __device__ void ep_combine_body(const CommDev& c, const EpDev& e, const CombineArgs& a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * kEpWarps + warp, nwarps = gridDim.x * kEpWarps;
@@ -374,9 +380,9 @@ __device__ void ep_combine_body(const CommDev& c, const EpDev& e, const CombineA
   const int* send_slot = a.send_slot != nullptr ? a.send_slot : e.send_slot;
   BlockEpoch ep;
   if (RANKS > 1) ep.load(c, kFlagSetEp);
-  if (RANKS > 1) trace_mark(c, 0);
+  trace_mark<TRACE>(c, 0);
   bool ok = RANKS == 1 || block_barrier(c, kFlagSetEp, ep, 0x93);
-  if (RANKS > 1) trace_mark(c, 1);
+  trace_mark<TRACE>(c, 1);
   if (ok) {
     const int piece = RANKS == 1 ? COLS * 256 : e.hidden;  // columns of one work item
     const int pieces = (e.hidden + piece - 1) / piece;
@@ -466,22 +472,23 @@ __device__ void ep_combine_body(const CommDev& c, const EpDev& e, const CombineA
         }
       }
     }
-    if (RANKS > 1) trace_mark(c, 2);
+    trace_mark<TRACE>(c, 2);
     // Nobody overwrites its expert outputs while a peer still reads them.
     ok = RANKS == 1 || block_barrier(c, kFlagSetEp, ep, 0x94);
-    if (RANKS > 1) trace_mark(c, 3);
+    trace_mark<TRACE>(c, 3);
   }
   if (RANKS > 1) ep.store(c, kFlagSetEp);
 }
 
 __global__ void __launch_bounds__(kEpThreads) k_ep_combine(CommDev c, EpDev e, CombineArgs a) {
-  ep_combine_body<kMaxRanks, 2>(c, e, a);
+  ep_combine_body<kMaxRanks, 2, true>(c, e, a);
 }
+template <bool TRACE>
 __global__ void __launch_bounds__(kEpThreads) k_ep_combine_solo(CommDev c, EpDev e, CombineArgs a) {
-  ep_combine_body<1, 4>(c, e, a);
+  ep_combine_body<1, 4, TRACE>(c, e, a);
 }
 __global__ void __launch_bounds__(kEpThreads) k_ep_combine_emu(const CommDev* cs, const EpDev* es, const CombineArgs* as) {
-  ep_combine_body<kMaxRanks, 2>(cs[blockIdx.y], es[blockIdx.y], as[blockIdx.y]);
+  ep_combine_body<kMaxRanks, 2, true>(cs[blockIdx.y], es[blockIdx.y], as[blockIdx.y]);
 }
 
 struct PullArgs {
@@ -612,7 +619,8 @@ cudaError_t launch_ep_dispatch(const CommDev* comms, const EpDev* eps, int emu_r
   for (int i = 0; i < n; ++i) args[i] = {x[i], topk_idx[i], topk_w[i], num_tokens};
   if (emu_ranks <= 0 && e0.nranks == 1) {
     const int blocks = std::max(1, (num_tokens + kEpSoloTokens - 1) / kEpSoloTokens);
-    k_ep_dispatch_solo<<<blocks, kEpThreads, 0, stream>>>(comms[0], e0, args[0]);
+    (comms[0].trace != nullptr ? k_ep_dispatch_solo<true> : k_ep_dispatch_solo<false>)<<<blocks, kEpThreads, 0, stream>>>(
+        comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }
@@ -636,7 +644,8 @@ cudaError_t launch_ep_combine(const CommDev* comms, const EpDev* eps, int emu_ra
     // the pieces (16.9 us for 4096 x 7168) beat a grid that covers them once (18.3).
     const int64_t items = static_cast<int64_t>(num_tokens) * ((e0.hidden + 1023) / 1024);
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((items + kEpWarps - 1) / kEpWarps, 148 * 4));
-    k_ep_combine_solo<<<static_cast<unsigned>(blocks), kEpThreads, 0, stream>>>(comms[0], e0, args[0]);
+    (comms[0].trace != nullptr ? k_ep_combine_solo<true> : k_ep_combine_solo<false>)<<<static_cast<unsigned>(blocks), kEpThreads, 0,
+                                                                                       stream>>>(comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }

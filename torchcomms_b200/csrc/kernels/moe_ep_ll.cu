@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(kLlThreads)
 // A single rank: the number a row gets at its expert is its packed position, so a block numbers one token's rows and
 // sends them, and nobody waits for anybody; the last block to finish leaves the counts. An ordinary launch, where the
 // general kernel is a cooperative one with a grid-wide meeting (128 tokens of 7168, top-8: 13.3 us there).
+template <bool TRACE>
 __global__ void __launch_bounds__(kLlThreads) k_ep_ll_dispatch_solo(CommDev c, EpLlDev e, LlDispatchArgs a) {
   __shared__ long long s_row[32];
   __shared__ int s_last;
@@ -365,6 +366,7 @@ __global__ void __launch_bounds__(kLlThreads) k_ep_ll_dispatch_solo(CommDev c, E
   const int E = e.num_experts, M = e.max_tokens, groups = e.hidden / 128;
   const size_t row_bytes = e.fp8 ? static_cast<size_t>(e.hidden) : static_cast<size_t>(e.hidden) * 2;
   const int t = blockIdx.x;
+  trace_mark<TRACE>(c, 0);  // the marks of the general kernel; without peers 1 to 3 coincide
   if (t < a.num_tokens) {
     if (warp == 0) {
       long long row = -1;
@@ -389,6 +391,9 @@ __global__ void __launch_bounds__(kLlThreads) k_ep_ll_dispatch_solo(CommDev c, E
       s_row[lane] = row;
     }
     __syncthreads();
+    trace_mark<TRACE>(c, 1);
+    trace_mark<TRACE>(c, 2);
+    trace_mark<TRACE>(c, 3);
     const long long row = s_row[lane];
     const uint32_t live = __ballot_sync(0xffffffffu, row >= 0);
     for (int col_lo = warp * kLlChunkCols; live != 0 && col_lo < e.hidden; col_lo += kLlWarps * kLlChunkCols) {
@@ -408,13 +413,17 @@ __global__ void __launch_bounds__(kLlThreads) k_ep_ll_dispatch_solo(CommDev c, E
     }
   }
   __syncthreads();
+  trace_mark<TRACE>(c, 4);
   if (threadIdx.x == 0) {
     __threadfence();  // this block's rows are counted before it reports
     s_last = atomicAdd(e.ticket, 1u) == gridDim.x - 1 ? 1 : 0;
     __threadfence();
   }
   __syncthreads();
-  if (!s_last) return;
+  if (!s_last) {
+    trace_mark<TRACE>(c, 5);
+    return;
+  }
   for (int ex = threadIdx.x; ex < E; ex += kLlThreads) {
     const int n = __ldcg(e.cnt + ex);
     a.recv.packed_count[ex] = n <= M ? n : 0;
@@ -424,6 +433,7 @@ __global__ void __launch_bounds__(kLlThreads) k_ep_ll_dispatch_solo(CommDev c, E
     e.cnt[ex] = 0;
   }
   if (threadIdx.x == 0) *e.ticket = 0;
+  trace_mark<TRACE>(c, 5);
 }
 
 struct LlCombineArgs {
@@ -582,7 +592,8 @@ cudaError_t launch_ep_ll_dispatch(const CommDev* comms, const EpLlDev* eps, int 
   std::vector<LlDispatchArgs> args(n);
   for (int i = 0; i < n; ++i) args[i] = {x[i], topk_idx[i], recv[i], num_tokens};
   if (emu_ranks <= 0 && e0.nranks == 1) {
-    k_ep_ll_dispatch_solo<<<std::max(1, num_tokens), kLlThreads, 0, stream>>>(comms[0], e0, args[0]);
+    (comms[0].trace != nullptr ? k_ep_ll_dispatch_solo<true> : k_ep_ll_dispatch_solo<false>)<<<std::max(1, num_tokens), kLlThreads, 0,
+                                                                                               stream>>>(comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }

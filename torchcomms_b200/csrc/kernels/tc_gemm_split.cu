@@ -56,6 +56,7 @@ struct SplitParams {
   uint32_t* status;
   const float* scale_a;  // e4m3: per row of A, per row of B
   const float* scale_b;
+  long long* trace;
   int m, n, k_iters, tiles_m;
 };
 
@@ -76,7 +77,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   return v;
 }
 
-template <bool FP8>
+template <bool FP8, bool TRACE>
 __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_constant__ SplitMaps maps, SplitParams p) {
   constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(kBlockM, kSplitBN) : make_idesc_bf16(kBlockM, kSplitBN);
   extern __shared__ char smem_raw[];
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
         tma_load_2d(sa, &maps.a, &bars->full[s], kb * kBlockK, mi * kBlockM);
         tma_load_2d(sa + kSplitABytes, &maps.b, &bars->full[s], kb * kBlockK, ni * kSplitBN);
       }
+      if (TRACE) trace_stamp_ns(p.trace, 1);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -145,6 +148,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
         umma_commit(&bars->empty[s]);
       }
       umma_commit(&bars->acc_full);
+      if (TRACE) trace_stamp_ns(p.trace, 2);
     }
   } else {
     // The accumulator is complete, so every stage has been read: the partial tile may overwrite them.
@@ -218,9 +222,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
     for (int i = 0; i < 4; ++i) po[i] = pack_bf16(__float_as_uint(acc[2 * i]), __float_as_uint(acc[2 * i + 1]));
     *reinterpret_cast<uint4*>(p.c + static_cast<size_t>(grow) * p.n + gcol) = o;
   }
+  if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 3);
   if (threadIdx.x == 0 && bars->failed && p.status != nullptr) p.status[0] = p.status[0] | kStatusTimeout;
   __syncwarp();
   cluster_sync_all();  // a peer may still be reading this CTA's partial tile
+  if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 7);
 }
 
 cudaLaunchConfig_t split_config(int tiles, int splits, cudaStream_t stream, cudaLaunchAttribute* attr) {
@@ -250,7 +256,7 @@ int resident_clusters(int device, int splits) {
   if (n == 0) {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = split_config(1, splits, nullptr, attr);
-    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_split<FP8>, &cfg) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_split<FP8, false>, &cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       return 0;
     }
@@ -261,7 +267,12 @@ int resident_clusters(int device, int splits) {
 
 template <bool FP8>
 cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles, cudaStream_t stream, bool* done) {
-  cudaError_t e = cudaFuncSetAttribute(k_gemm_split<FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemBytes);
+  // The untraced kernel is the one that resident_clusters asks about: one CTA per SM, as the traced one.
+  const auto kernel = p.trace != nullptr ? k_gemm_split<FP8, true> : k_gemm_split<FP8, false>;
+  cudaError_t e = cudaFuncSetAttribute(k_gemm_split<FP8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemBytes);
+  if (e == cudaSuccess && p.trace != nullptr) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemBytes);
+  }
   if (e != cudaSuccess) return e;
   // As many ways as leave every cluster resident and every CTA at least four K steps (below that the fixed cost of
   // filling the pipeline and meeting the cluster is larger than what another split saves).
@@ -274,7 +285,7 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
-  e = cudaLaunchKernelEx(&cfg, k_gemm_split<FP8>, maps, p);
+  e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
   note_kernel_launch();
   *done = true;
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -283,7 +294,7 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
 } // namespace
 
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                                 const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done) {
+                                 const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done, long long* trace) {
   *done = false;
   const int64_t tiles_m = (static_cast<int64_t>(m) + kBlockM - 1) / kBlockM, tiles_n = (static_cast<int64_t>(n) + kSplitBN - 1) / kSplitBN;
   if (tiles_m * tiles_n > kSplitMaxTiles) return cudaSuccess;
@@ -292,6 +303,7 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   SplitParams p{};
   p.c = static_cast<__nv_bfloat16*>(c);
   p.status = status;
+  p.trace = trace;
   p.scale_a = scale_a;
   p.scale_b = scale_b;
   p.m = m;
