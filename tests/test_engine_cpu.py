@@ -92,3 +92,15 @@ def test_block_pieces_on_cpu_tensors():
     for p, q_, r in zip(a, c, ref):
         assert torch.equal(p, q_)
         torch.testing.assert_close(p, r, rtol=1e-4, atol=1e-6)
+
+
+def test_padded_head_follows_rows_and_weight():
+    """The choice between a padded copy of the weight and none looks at the rows as well as at the weight."""
+    from torchcomms_b200.ops.fused import _worth_padding
+
+    m = 1 << 20
+    assert _worth_padding(4096, 20 * m) and _worth_padding(4096, m) and _worth_padding(512, 25 * m)  # several times faster
+    assert _worth_padding(1, 250 * m) and _worth_padding(2, 25 * m)
+    # the GPU waits for the host either way: a copy only takes longer
+    assert not _worth_padding(64, 2 * m) and not _worth_padding(1500, m) and not _worth_padding(2, 20 * m)
+    assert not _worth_padding(0, 500 * m)

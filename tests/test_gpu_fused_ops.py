@@ -194,9 +194,11 @@ def test_cross_entropy_row_layouts(rows, vocab):
     torch.testing.assert_close(logits.double(), ref, rtol=2**-8, atol=1e-5)
 
 
-@pytest.mark.parametrize("rows,dim,vocab", [(1, 64, 9), (130, 128, 5001), (70, 256, 40002), (130, 640, 40001), (257, 64, 1000)])
+@pytest.mark.parametrize("rows,dim,vocab", [(1, 64, 9), (130, 128, 5001), (70, 256, 40002), (130, 640, 40001), (257, 64, 1000),
+                                            (2, 256, 98305), (512, 512, 13107), (512, 512, 13109), (3000, 256, 5365)])
 def test_linear_cross_entropy_any_vocabulary(rows, dim, vocab):
-    """Vocabularies off the 16-byte grid (large ones with a padded weight) and on it, in one and in several chunks."""
+    """Vocabularies off the 16-byte grid (from some sizes on with a padded weight, both sides of the line here) and on
+    it, in one and in several chunks."""
     from torchcomms_b200.ops import fused
 
     x, w = _bf(rows, dim, seed=60).requires_grad_(True), _bf(vocab, dim, seed=61, scale=0.1).requires_grad_(True)

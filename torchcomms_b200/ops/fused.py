@@ -152,6 +152,21 @@ def split_rope(qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t:
 # ------------------------------------------------- linear + cross entropy
 
 
+def _worth_padding(rows: int, weight: int) -> bool:
+    """Whether a head off the 16-byte grid works on a zero-padded copy of its weight (``weight`` elements).
+
+    The three products on two-element accesses take about 0.04 us longer per million weight elements and row, and as
+    long again for reading the weight as for 128 rows. The copy costs a read and a write of the weight, which they win
+    back, and 35 us of host time for its launches; a pass forward and backward has the GPU wait for the host (172 us)
+    until the products are that much longer. Such a pass without and with the copy, in us: at 3844 M (200 rows, 11.7 M
+    elements) 251 and 208, at 4097 M (128, 16 M) 236 and 205, at 4126 M (4096, 1 M) 304 and 206, at 4800 M (64, 25 M)
+    245 and 212; below, at 2500 M (512, 3.9 M) 175 and 206; above, at 16 G (512, 25 M) 663 and 214, at 64 G (1, 501 M)
+    1960 and 1485. From 24 M elements on, fewer rows take the copy as well (16 rows, 25 M: 189 and 208, even at 32
+    rows): their products are as accurate as the others' that way (error of dx 0.0017, without it 0.0034).
+    """
+    return rows > 0 and (weight >= 24 << 20 or weight * (rows + 128) >= 4 << 30)
+
+
 class _LinearCrossEntropy(torch.autograd.Function):
     """``mean(cross_entropy(x @ W^T, targets))`` without keeping the logits.
 
@@ -173,8 +188,8 @@ class _LinearCrossEntropy(torch.autograd.Function):
         vocab = weight.shape[0]
         # Rows of a vocabulary that is no multiple of 8 start off 16-byte boundaries, which costs the three GEMMs their
         # tiled loads and stores. A copy of the weight with a few zero rows more puts logits and weight back on them:
-        # their logits are zero, stay zero, and add nothing. Below 24 M elements the copy costs as much as it saves.
-        pad = -vocab % 8 if x.is_cuda and x.dtype == weight.dtype == torch.bfloat16 and weight.numel() >= 24 << 20 else 0
+        # their logits are zero, stay zero, and add nothing.
+        pad = -vocab % 8 if x.is_cuda and x.dtype == weight.dtype == torch.bfloat16 and _worth_padding(rows, weight.numel()) else 0
         wide = F.pad(weight, (0, 0, 0, pad)) if pad else weight
         for r0 in range(0, rows, chunk_rows):
             r1 = min(rows, r0 + chunk_rows)
@@ -214,7 +229,12 @@ class _LinearCrossEntropy(torch.autograd.Function):
 
 
 def linear_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor, chunk_rows: int = 4096) -> torch.Tensor:
-    """Mean token cross-entropy of the logits ``x @ weight.T`` (``x``: [rows, dim])."""
+    """Mean token cross-entropy of the logits ``x @ weight.T`` (``x``: [rows, dim]).
+
+    The forward pass holds the logits of ``chunk_rows`` rows and the gradient of the weight; for a bf16 vocabulary that is
+    no multiple of 8 also, from the sizes of ``_worth_padding`` on, a padded copy of the weight (1 GB at 128257 x 4096).
+    A vocabulary padded by the caller needs none.
+    """
     return _LinearCrossEntropy.apply(x.contiguous(), weight, targets, chunk_rows)
 
 
