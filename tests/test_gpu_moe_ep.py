@@ -60,7 +60,7 @@ def _check_dispatch(r, nranks, epr, topk, max_tokens, xs, idxs, ws, view, fp8):
     return n
 
 
-@pytest.mark.parametrize("nranks,fp8", [(2, True), (4, True), (8, True), (4, False)])
+@pytest.mark.parametrize("nranks,fp8", [(1, True), (2, True), (4, True), (8, True), (4, False)])
 def test_dispatch_combine_emulated(nranks, fp8):
     from torchcomms_b200 import _comms
 

@@ -75,8 +75,8 @@ constexpr int kEpChunkCols = 1024;  // columns of one work item of the send loop
 // Bound by memory (a bf16 row in, a quantised row out), so what counts is how many bytes are in flight and how
 // little happens before the rows move. Tokens are numbered per destination by a thread each: ballots inside a
 // warp, one atomic per block and destination. The send loop hands out pieces of rows, so that every warp has the
-// same share and issues its whole piece's loads at once. One rank, 4096 tokens of 7168 to e4m3: 49.6 us with a
-// warp per token and a meeting after every phase, 23.4 us (3.8 TB/s) now.
+// same share and issues its whole piece's loads at once. (4096 tokens of 7168 to e4m3 on one rank, when that ran
+// here: 49.6 us with a warp per token and more grid-wide meetings, 23.4 us in this form.)
 __device__ void ep_dispatch_body(const CommDev& c, const EpDev& e, const DispatchArgs& a) {
   cg::grid_group grid = cg::this_grid();
   __shared__ int s_first[kEpWarps][kMaxRanks];  // tokens of the block's earlier warps, per destination
@@ -130,7 +130,7 @@ __device__ void ep_dispatch_body(const CommDev& c, const EpDev& e, const Dispatc
   trace_mark(c, 1);
 
   // B. publish the counts to every rank, learn where this rank's rows start inside each destination's receive
-  //    buffer (rows are packed by source). A single rank's rows start at 0.
+  //    buffer (rows are packed by source).
   if (blockIdx.x == 0) {
     if (threadIdx.x < e.nranks) {
       const int d = threadIdx.x;
@@ -140,8 +140,7 @@ __device__ void ep_dispatch_body(const CommDev& c, const EpDev& e, const Dispatc
         e.count_matrix[p][e.rank * e.nranks + d] = n;
       }
     }
-    if (e.nranks > 1) ep_rank_barrier(c, 0x91);
-    else __syncthreads();
+    ep_rank_barrier(c, 0x91);
     const long long* m = e.count_matrix[e.rank];
     if (threadIdx.x < e.nranks) {
       const int d = threadIdx.x;
@@ -156,7 +155,7 @@ __device__ void ep_dispatch_body(const CommDev& c, const EpDev& e, const Dispatc
       e.recv_info[0] = static_cast<int>(total);
     }
   }
-  if (e.nranks > 1) grid.sync();
+  grid.sync();
   trace_mark(c, 2);
 
   // C. quantise and send; one work item = one token x kEpChunkCols columns
@@ -181,7 +180,7 @@ __device__ void ep_dispatch_body(const CommDev& c, const EpDev& e, const Dispatc
     if (lane < e.nranks) {
       const int n = e.order[static_cast<size_t>(t) * e.nranks + lane];
       if (n >= 0) {
-        slot = (e.nranks > 1 ? static_cast<int>(e.base[lane]) : 0) + n;
+        slot = static_cast<int>(e.base[lane]) + n;
         if (slot >= e.nranks * e.max_tokens) {  // cannot happen with consistent inputs; never write out of bounds
           c.status[0] = c.status[0] | kStatusBadArg;
           slot = -1;
@@ -229,13 +228,11 @@ __device__ void ep_dispatch_body(const CommDev& c, const EpDev& e, const Dispatc
     }
   }
   trace_mark(c, 3);
-  if (e.nranks > 1) {
-    grid.sync();
-    // D. every rank's rows have landed before anybody returns
-    if (blockIdx.x == 0) {
-      ep_rank_barrier(c, 0x92);
-      trace_mark(c, 4);
-    }
+  grid.sync();
+  // D. every rank's rows have landed before anybody returns
+  if (blockIdx.x == 0) {
+    ep_rank_barrier(c, 0x92);
+    trace_mark(c, 4);
   }
 }
 
@@ -248,8 +245,8 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_emu(const CommDev* c
 
 // A single rank: rows may stand in any order from 0, so a block numbers its own tokens with one atomic and sends them
 // at once, and nobody waits for anybody. The last block to finish leaves the count. An ordinary launch that covers
-// the tokens, where the general kernel is a cooperative one with a grid-wide meeting (4096 tokens of 7168 to e4m3:
-// 23.3 us there).
+// the tokens, where the general kernel is a cooperative one with grid-wide meetings (4096 tokens of 7168 to e4m3:
+// 23.3 us there, 22.0 us (4.0 TB/s) here).
 constexpr int kEpSoloTokens = 4;
 
 template <bool TRACE>

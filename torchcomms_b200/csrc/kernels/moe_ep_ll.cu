@@ -121,9 +121,8 @@ __device__ __forceinline__ void ll_send_piece(const EpLlDev& e, const __nv_bfloa
 
 // Rows for other ranks go into fixed slots there and are packed by the receiver as they arrive. Rows for this
 // rank's own experts need no slot: their packed position is this rank's first row at the expert plus the number
-// they were given, so they are quantised straight into the packed tensors. A single rank therefore moves every
-// row once and exchanges nothing: 128 tokens of 7168, top-8 of 256 experts, 36.9 us through slots and arrival flags,
-// now 13.2.
+// they were given, so they are quantised straight into the packed tensors. (128 tokens of 7168, top-8 of 256 experts on
+// one rank, when that ran here: 36.9 us with every row through slots and arrival flags, 13.2 us with none.)
 __device__ void ll_dispatch_body(const CommDev& c, const EpLlDev& e, const LlDispatchArgs& a) {
   cg::grid_group grid = cg::this_grid();
   __shared__ int s_cnt[kMaxRanks];
@@ -166,52 +165,50 @@ __device__ void ll_dispatch_body(const CommDev& c, const EpLlDev& e, const LlDis
   if (blockIdx.x == 0 && threadIdx.x == 0) *e.call = call;
 
   const int nchunks = (e.hidden + kLlChunkCols - 1) / kLlChunkCols;
-  if (N > 1) {
-    // B. the row counts are final: tagged with the call, they go to every peer ahead of the rows
-    for (int i = gtid; i < E * N; i += gthreads) {
-      const int ex = i / N, p = i - ex * N;
-      if (p == e.rank) continue;  // own counts are read where they are
-      const unsigned long long v = (static_cast<unsigned long long>(call) << 32) | static_cast<unsigned int>(cnt[ex]);
-      st_release_sys_u64(reinterpret_cast<uint64_t*>(e.counts[p] + (static_cast<size_t>(par) * E + ex) * N + e.rank), v);
-    }
-    trace_mark(c, 2);
+  // B. the row counts are final: tagged with the call, they go to every peer ahead of the rows
+  for (int i = gtid; i < E * N; i += gthreads) {
+    const int ex = i / N, p = i - ex * N;
+    if (p == e.rank) continue;  // own counts are read where they are
+    const unsigned long long v = (static_cast<unsigned long long>(call) << 32) | static_cast<unsigned int>(cnt[ex]);
+    st_release_sys_u64(reinterpret_cast<uint64_t*>(e.counts[p] + (static_cast<size_t>(par) * E + ex) * N + e.rank), v);
+  }
+  trace_mark(c, 2);
 
-    // A1. store the peers' rows into their fixed slots; one work item = one token x kLlChunkCols columns
-    for (int item = gwarp; item < a.num_tokens * nchunks; item += nwarps) {
-      const int t = item / nchunks;
-      const int col_lo = (item - t * nchunks) * kLlChunkCols;
-      const int col_hi = min(e.hidden, col_lo + kLlChunkCols);
-      int d = -1;
-      long long row = -1;
-      if (lane < e.topk) {
-        const int idx = a.topk_idx[static_cast<size_t>(t) * e.topk + lane];
-        const int i = e.send_slot[static_cast<size_t>(t) * e.topk + lane];
-        if (i >= 0 && idx / Le != e.rank) {
-          d = idx / Le;
-          row = static_cast<long long>(par_rows) + (static_cast<long long>(idx - d * Le) * N + e.rank) * M + i;
-        }
+  // A1. store the peers' rows into their fixed slots; one work item = one token x kLlChunkCols columns
+  for (int item = gwarp; item < a.num_tokens * nchunks; item += nwarps) {
+    const int t = item / nchunks;
+    const int col_lo = (item - t * nchunks) * kLlChunkCols;
+    const int col_hi = min(e.hidden, col_lo + kLlChunkCols);
+    int d = -1;
+    long long row = -1;
+    if (lane < e.topk) {
+      const int idx = a.topk_idx[static_cast<size_t>(t) * e.topk + lane];
+      const int i = e.send_slot[static_cast<size_t>(t) * e.topk + lane];
+      if (i >= 0 && idx / Le != e.rank) {
+        d = idx / Le;
+        row = static_cast<long long>(par_rows) + (static_cast<long long>(idx - d * Le) * N + e.rank) * M + i;
       }
-      const uint32_t live = __ballot_sync(0xffffffffu, d >= 0);
-      if (live == 0) continue;
-      ll_send_piece(
-          e, static_cast<const __nv_bfloat16*>(a.x) + static_cast<size_t>(t) * e.hidden, col_lo, col_hi, live,
-          [&](int k, int e0, uint4 v0, uint4 v1) {
-            const int dk = __shfl_sync(0xffffffffu, d, k);
-            const long long rk = __shfl_sync(0xffffffffu, row, k);
-            char* dst = e.slot_x[dk] + static_cast<size_t>(rk) * row_bytes + static_cast<size_t>(e0) * 2;
-            st16(dst, v0);
-            st16(dst + 16, v1);
-          },
-          [&](int k, int e0, uint4 packed, float scale) {
-            const int dk = __shfl_sync(0xffffffffu, d, k);
-            const long long rk = __shfl_sync(0xffffffffu, row, k);
-            st16(e.slot_x[dk] + static_cast<size_t>(rk) * row_bytes + e0, packed);
-            if ((lane & 7) == 0) e.slot_scales[dk][static_cast<size_t>(rk) * groups + e0 / 128] = scale;
-          });
-      // This piece of every row is stored: tell the receivers (release-ordered, after the whole warp's stores).
-      __syncwarp();
-      if (d >= 0) red_add_release_sys_u32(e.slot_arrived[d] + row, 1u);
     }
+    const uint32_t live = __ballot_sync(0xffffffffu, d >= 0);
+    if (live == 0) continue;
+    ll_send_piece(
+        e, static_cast<const __nv_bfloat16*>(a.x) + static_cast<size_t>(t) * e.hidden, col_lo, col_hi, live,
+        [&](int k, int e0, uint4 v0, uint4 v1) {
+          const int dk = __shfl_sync(0xffffffffu, d, k);
+          const long long rk = __shfl_sync(0xffffffffu, row, k);
+          char* dst = e.slot_x[dk] + static_cast<size_t>(rk) * row_bytes + static_cast<size_t>(e0) * 2;
+          st16(dst, v0);
+          st16(dst + 16, v1);
+        },
+        [&](int k, int e0, uint4 packed, float scale) {
+          const int dk = __shfl_sync(0xffffffffu, d, k);
+          const long long rk = __shfl_sync(0xffffffffu, row, k);
+          st16(e.slot_x[dk] + static_cast<size_t>(rk) * row_bytes + e0, packed);
+          if ((lane & 7) == 0) e.slot_scales[dk][static_cast<size_t>(rk) * groups + e0 / 128] = scale;
+        });
+    // This piece of every row is stored: tell the receivers (release-ordered, after the whole warp's stores).
+    __syncwarp();
+    if (d >= 0) red_add_release_sys_u32(e.slot_arrived[d] + row, 1u);
   }
   trace_mark(c, 3);
 
@@ -279,14 +276,6 @@ __device__ void ll_dispatch_body(const CommDev& c, const EpLlDev& e, const LlDis
   }
   trace_mark(c, 4);
 
-  if (N == 1) {  // every row is in place; only the counts are left
-    for (int le = gtid; le < Le; le += gthreads) {
-      const int n = cnt[le] <= M ? cnt[le] : 0;
-      a.recv.packed_count[le] = n;
-      a.recv.layout_range[le] = static_cast<long long>(n);
-    }
-    return;
-  }
   // C2. pack the peers' rows of each local expert, sources in rank order
   const int nsub = max(1, static_cast<int>(gridDim.x) / Le);
   for (int item = blockIdx.x; item < Le * nsub; item += gridDim.x) {
@@ -357,7 +346,7 @@ __global__ void __launch_bounds__(kLlThreads)
 
 // A single rank: the number a row gets at its expert is its packed position, so a block numbers one token's rows and
 // sends them, and nobody waits for anybody; the last block to finish leaves the counts. An ordinary launch, where the
-// general kernel is a cooperative one with a grid-wide meeting (128 tokens of 7168, top-8: 13.3 us there).
+// general kernel is a cooperative one with a grid-wide meeting (128 tokens of 7168, top-8: 13.3 us there, 6.0 here).
 template <bool TRACE>
 __global__ void __launch_bounds__(kLlThreads) k_ep_ll_dispatch_solo(CommDev c, EpLlDev e, LlDispatchArgs a) {
   __shared__ long long s_row[32];
