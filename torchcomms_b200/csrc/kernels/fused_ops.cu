@@ -409,7 +409,7 @@ __device__ __forceinline__ void rotate8(float* f, float4 c4, float4 s4, float si
 // (4.6 TB/s) without.
 constexpr int kRopeVecs = 4;
 
-__global__ void __launch_bounds__(256) k_rope(const __nv_bfloat16* x, __nv_bfloat16* y,
+__global__ void __launch_bounds__(256) k_rope(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                               const int* __restrict__ pos, const float* __restrict__ cos_t,
                                               const float* __restrict__ sin_t, uint32_t total, FastDiv per_head,
                                               FastDiv heads, int64_t stride_t, int64_t stride_h, float sign) {

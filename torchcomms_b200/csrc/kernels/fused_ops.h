@@ -38,7 +38,7 @@ cudaError_t launch_quantize_rows(const __nv_bfloat16* x, int64_t ld, void* q, fl
 // contiguous y; pos[t] indexes the cos/sin tables [max_pos, head_dim/2]. `inverse`
 // rotates by the negative angle (the backward pass). x may be a slice of a wider
 // tensor: element strides of its token and head dimensions, multiples of 8 like
-// head_dim; x, y and the tables 16-byte aligned. y may be x itself if that is contiguous.
+// head_dim; x, y and the tables 16-byte aligned.
 cudaError_t launch_rope(const __nv_bfloat16* x, int64_t stride_t, int64_t stride_h, __nv_bfloat16* y, const int* pos,
                         const float* cos_t, const float* sin_t, int tokens, int heads, int head_dim, bool inverse,
                         cudaStream_t s);

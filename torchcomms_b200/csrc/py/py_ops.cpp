@@ -54,9 +54,9 @@ void quantize_into(const at::Tensor& x, at::Tensor& q, at::Tensor& scale) {
                                         static_cast<int>(x.size(1)), cur(x)));
 }
 
-// y = x rotated; y contiguous, possibly x itself.
-void rope_into(const at::Tensor& x, at::Tensor& y, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t,
-               bool inverse) {
+// x rotated, contiguous.
+at::Tensor rope(const at::Tensor& x, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t, bool inverse) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16, "x: bf16 CUDA tensor expected");
   want(pos, at::kInt, "pos");
   want(cos_t, at::kFloat, "cos");
   want(sin_t, at::kFloat, "sin");
@@ -68,20 +68,15 @@ void rope_into(const at::Tensor& x, at::Tensor& y, const at::Tensor& pos, const 
   TORCH_CHECK(pos.numel() == tokens, "pos must have one entry per token");
   TORCH_CHECK(cos_t.size(-1) == head_dim / 2 && sin_t.size(-1) == head_dim / 2, "cos/sin tables: [max_pos, head_dim/2]");
   c10::cuda::CUDAGuard g(x.device());
+  at::Tensor y = at::empty_like(x, at::MemoryFormat::Contiguous);
   // A slice of a wider tensor (queries or keys of a fused projection) is read where it is; layouts that
   // 16-byte loads cannot follow are made contiguous first.
   const bool in_place = x.dim() == 3 && x.stride(2) == 1 && x.stride(0) % 8 == 0 && x.stride(1) % 8 == 0 && on16(x);
-  const at::Tensor src = in_place || x.is_same(y) ? x : x.clone(at::MemoryFormat::Contiguous);
+  const at::Tensor src = in_place ? x : x.clone(at::MemoryFormat::Contiguous);
   const int64_t st = in_place ? src.stride(0) : per_token, sh = in_place ? src.stride(1) : head_dim;
   const at::Tensor c = vectorable(cos_t), sn = vectorable(sin_t);
   B200C_CUDA_CHECK(launch_rope(bf(src), st, sh, bf_mut(y), pos.data_ptr<int>(), c.data_ptr<float>(), sn.data_ptr<float>(), tokens,
                                heads, head_dim, inverse, cur(x)));
-}
-
-at::Tensor rope(const at::Tensor& x, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t, bool inverse) {
-  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16, "x: bf16 CUDA tensor expected");
-  at::Tensor y = at::empty_like(x, at::MemoryFormat::Contiguous);
-  rope_into(x, y, pos, cos_t, sin_t, inverse);
   return y;
 }
 
@@ -329,12 +324,7 @@ void bind_ops(py::module_& m) {
   ops.def("rmsnorm_fwd", &rmsnorm_fwd);
   ops.def("rmsnorm_bwd", &rmsnorm_bwd);
 
-  ops.def("rope_", [](at::Tensor x, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t, bool inverse) {
-    want(x, at::kBFloat16, "x");
-    rope_into(x, x, pos, cos_t, sin_t, inverse);
-    return x;
-  });
-  // Out of place: x [..., tokens, heads, head_dim] of any strides -> contiguous.
+  // x [..., tokens, heads, head_dim] of any strides -> contiguous.
   ops.def("rope", &rope);
 
   ops.def("swiglu_fwd", &swiglu_fwd);
