@@ -124,6 +124,40 @@ def test_dispatch_combine_emulated(nranks, fp8):
             assert not pulled[r][counts[r]:].any()
 
 
+@pytest.mark.parametrize("nranks,tokens", [(2, 1111), (3, 530)])
+def test_dispatch_emulated_numbers_tokens_over_several_blocks(nranks, tokens):
+    """More tokens than a block numbers, no multiple of a block's or a warp's, some of them routed nowhere, two calls."""
+    from torchcomms_b200 import _comms
+
+    max_tokens, hidden, topk, epr = 1200, 512, 2, 4
+    buf = _comms.EpBuffer.emulated(nranks, max_tokens, hidden, nranks * epr, topk, False, 2000.0)
+    torch.manual_seed(tokens)
+    for it in range(2):
+        xs = [torch.randn(tokens, hidden, device="cuda").to(torch.bfloat16) for _ in range(nranks)]
+        routes = [_route(tokens, nranks * epr, topk, 10 * it + r) for r in range(nranks)]
+        idxs, ws = [a for a, _ in routes], [b for _, b in routes]
+        for r in range(nranks):
+            idxs[r][r :: 7] = -1                                      # tokens that go nowhere
+            idxs[r][256:290, 1] = -1
+        buf.dispatch(xs, idxs, ws)
+        torch.cuda.synchronize()
+        assert buf.status()[0] == 0
+        counts = [_check_dispatch(r, nranks, epr, topk, max_tokens, xs, idxs, ws, buf.view, False) for r in range(nranks)]
+        for r in range(nranks):
+            src = buf.view(r, "recv_src")[: counts[r]].long()
+            rows = torch.stack(xs)[src // max_tokens, src % max_tokens]
+            assert torch.equal(buf.view(r, "recv_x")[: counts[r]], rows)        # every row, not a sample
+            buf.view(r, "combine_x")[: counts[r]] = rows * (r + 1)
+        outs = [torch.empty(tokens, hidden, dtype=torch.bfloat16, device="cuda") for _ in range(nranks)]
+        buf.combine(outs, [], [])
+        torch.cuda.synchronize()
+        assert buf.status()[0] == 0
+        for s in range(nranks):
+            hit = torch.stack([((idxs[s] // epr == d) & (idxs[s] >= 0)).any(dim=1) * (d + 1) for d in range(nranks)]).sum(0)
+            # bf16 products by up to 3 (2^-9), an fp32 sum, one rounding to bf16
+            torch.testing.assert_close(outs[s].double(), hit.unsqueeze(1) * xs[s].double(), rtol=2**-7, atol=1e-6)
+
+
 def test_layout_kernel():
     from torchcomms_b200.ops.moe_ep import get_dispatch_layout
 
