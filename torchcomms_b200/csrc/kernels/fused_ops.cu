@@ -578,8 +578,9 @@ constexpr int kCeMaxThreads = 512;
 // work at a time than L2 holds (see the launcher), and the exponentials come next: two per element on the
 // special-function unit. The rest is kept off the issue slots: one maximum and one comparison per 8 elements,
 // and the target's column is looked for per vector. Rows that start off a 16-byte boundary (vocabularies that
-// are no multiple of 8) peel up to 7 elements instead of giving up wide accesses. 4096 rows of 128256: 698 us with
-// 592 rows in work and a comparison per element, 512 us (4.1 TB/s) now.
+// are no multiple of 8) peel up to 7 elements instead of giving up wide accesses. 4096 rows of 128256
+// between a head's GEMMs: 698 us with 592 rows in work and a comparison per element, 480 to 570 us now, by the clock
+// that the power cap leaves.
 __global__ void __launch_bounds__(kCeMaxThreads, 2) k_cross_entropy(__nv_bfloat16* __restrict__ logits,
                                                                     int64_t ld, const int64_t* __restrict__ targets,
                                                                     float* __restrict__ loss, int rows, int vocab,
