@@ -90,6 +90,26 @@ def test_gemm_split_repeats_and_rounds_no_worse(m, n, k):
     torch.testing.assert_close(c.double(), exact, rtol=2**-8, atol=2e-8 * k)
 
 
+@pytest.mark.parametrize("m,n,k", [(5, 1024, 2048), (700, 4096, 256)])
+def test_gemm_in_a_graph_clears_its_status(m, n, k):
+    from torchcomms_b200 import _comms
+
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(n, k, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    want, status = _comms.ops.gemm_bf16_nt(a, b)
+    assert not status.any()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        c, status = _comms.ops.gemm_bf16_nt(a, b)
+    for _ in range(2):
+        status.fill_(7)
+        c.zero_()
+        graph.replay()
+        assert torch.equal(c, want) and not status.any()
+
+
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (512, 512, 1024), (300, 264, 200), (1024, 7168, 2048), (4096, 4096, 4096),
                                    (8192, 1792, 512)])
 def test_gemm_bf16_nt_cta_pairs(m, n, k):

@@ -26,6 +26,9 @@ cudaError_t launch_gemm_e4m3_nt(const void* a, const void* b, void* c, int m, in
 cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                            const float* scale_b, uint32_t* status, cudaStream_t stream);
 
+// Clears the two status words that a product reports into, ahead of it on the same stream.
+cudaError_t launch_clear_status(uint32_t* status, cudaStream_t stream);
+
 // The same product where 128 x 128 tiles are too few to fill the GPU: clusters of CTAs split K and sum in
 // distributed shared memory. Sets *done when it launched; otherwise (more than kSplitMaxTiles tiles) nothing
 // happened and the persistent kernels are the ones to call. Argument rules checked by launch_gemm_nt. `trace`: the

@@ -229,6 +229,10 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 7);
 }
 
+__global__ void k_clear_status(uint32_t* status) {
+  if (threadIdx.x < 2) status[threadIdx.x] = 0u;
+}
+
 cudaLaunchConfig_t split_config(int tiles, int splits, cudaStream_t stream, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
@@ -292,6 +296,12 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
 }
 
 } // namespace
+
+cudaError_t launch_clear_status(uint32_t* status, cudaStream_t stream) {
+  k_clear_status<<<1, 32, 0, stream>>>(status);
+  note_kernel_launch();
+  return cudaGetLastError();
+}
 
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                  const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done, long long* trace) {
