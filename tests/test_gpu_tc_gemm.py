@@ -45,11 +45,13 @@ def test_gemm_partial_last_column_tiles(m, n, k, kind):
         torch.testing.assert_close(c.double(), ref, rtol=2**-8, atol=1e-6 * k)
 
 
-@pytest.mark.parametrize("m", [1, 67, 128, 129, 300])
-@pytest.mark.parametrize("n,k", [(8, 8), (136, 72), (128, 256), (136, 264), (3584, 4096), (6144, 1928)])
+@pytest.mark.parametrize("m", [1, 32, 33, 67, 128, 129, 300])
+@pytest.mark.parametrize("n,k", [(8, 8), (136, 72), (128, 256), (136, 264), (520, 704), (520, 712), (264, 896), (264, 904),
+                                 (3584, 4096), (6144, 1928), (10248, 1032)])
 @pytest.mark.parametrize("fp8", [False, True])
 def test_gemm_split_over_clusters(m, n, k, fp8):
-    """Products of fewer tiles than SMs: every number of K shares, ragged edges in all three sizes."""
+    """Products of fewer tiles than SMs: every number of K shares, ragged edges in all three sizes, both sides of the
+    lines below which the persistent kernel takes them."""
     from torchcomms_b200 import _comms
     from torchcomms_b200.ops.tp import quantize_rows
 

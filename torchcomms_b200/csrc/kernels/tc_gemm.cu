@@ -1329,7 +1329,7 @@ cudaError_t launch_allgather_gemm(const CommDev& comm, const AgGemmArgs& a, cuda
   if (comm.nranks == 1) {  // nothing to gather: the plain product, where that fills the GPU better
     bool done = false;
     e = launch_gemm_nt_split(a.x_shards[0], a.w, a.y, a.m_local, a.n, p.k, a.fp8 ? a.scale_x_shards[0] : nullptr, a.scale_w,
-                             const_cast<uint32_t*>(comm.status), stream, &done, comm.trace);
+                             const_cast<uint32_t*>(comm.status), stream, &done, &comm);
     if (e != cudaSuccess || done) return e;
   }
   if (pairs) return tp_launch_pair<TpMode::AG_GEMM>(0, maps, comm, p, stream);
@@ -1347,7 +1347,7 @@ cudaError_t launch_gemm_reduce_scatter(const CommDev& comm, const GemmRsArgs& a,
   if (comm.nranks == 1) {  // nothing to scatter
     bool done = false;
     e = launch_gemm_nt_split(a.h, a.w, a.out, a.m, a.n, p.k, a.fp8 ? a.scale_h : nullptr, a.scale_w,
-                             const_cast<uint32_t*>(comm.status), stream, &done, comm.trace);
+                             const_cast<uint32_t*>(comm.status), stream, &done, &comm);
     if (e != cudaSuccess || done) return e;
   }
   const int tiles = (a.m / kBlockM) * (a.n / kTpBN);

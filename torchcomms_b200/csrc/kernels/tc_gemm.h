@@ -30,14 +30,15 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
 cudaError_t launch_clear_status(uint32_t* status, cudaStream_t stream);
 
 // The same product where 128 x 128 tiles are too few to fill the GPU: clusters of CTAs split K and sum in
-// distributed shared memory. Sets *done when it launched; otherwise (more than kSplitMaxTiles tiles) nothing
-// happened and the persistent kernels are the ones to call. Argument rules checked by launch_gemm_nt. `trace`: the
-// communicator's phase trace, stamped like the fused layers' kernels (start, loads issued, MMAs committed, tile
-// stored, CTA done).
+// distributed shared memory. Sets *done when it launched; otherwise (more than kSplitMaxTiles tiles, or a plain product
+// that the persistent kernel is faster at) nothing happened and the persistent kernels are the ones to call. Argument
+// rules checked by launch_gemm_nt. `layer`: the communicator of a fused layer on one rank, whose own kernel is slower
+// at every such size (13 to 70 us against 6 to 59 over 128..4096 rows, 256..18432 columns and K of 128..8192); its
+// phase trace is stamped like that kernel's (start, loads issued, MMAs committed, tile stored, CTA done).
 constexpr int kSplitMaxTiles = 148;
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                  const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done,
-                                 long long* trace = nullptr);
+                                 const CommDev* layer = nullptr);
 
 // The same product on CTA pairs (clusters of two CTAs, tcgen05 cta_group::2):
 // each pair owns a 256 x 256 tile and reads every B element once. Same

@@ -269,8 +269,26 @@ int resident_clusters(int device, int splits) {
   return n;
 }
 
+// Whether the split kernel beats the persistent one (tiles of 128 x 256) on a plain product. Meeting the cluster and
+// adding up the shares costs it 1 us more than the direct stores of a full tile, nothing where the tile has few rows;
+// a K step is 0.28 us of the persistent kernel's time and 0.2 us of this one's, over the CTAs that share K. Replayed from
+// a graph, persistent / split in us (bf16 unless e4m3 is said):
+//   few rows: 1 x 2048 x 512 7.4 / 6.1, 32 x 2048 x 512 7.5 / 6.9
+//   K shared, line at 12 steps of 64, in e4m3 at 8 of 128: 128 x 2048 x 512 7.7 / 8.4, x 768 8.9 / 8.8, x 1536
+//   12.2 / 11.3; e4m3 128 x 2048 x 768 8.6 / 10.1, x 1024 9.2 / 8.9
+//   K not shared: half the tile on twice the SMs pays later, the more row tiles read the same weights again:
+//   128 x 14336 x 768 9.6 / 10.7, x 1024 12.1 / 12.5, x 2048 20.4 / 18.3; 256 x 9216 x 2560 22.1 / 19.7;
+//   2048 x 1024 x 3072 18.8 / 22.6, x 4096 23.7 / 26.3, x 6144 38.3 / 35.6
+// Of 3830 shapes (rows 1..8192, columns 256..18432, K 64..24576) some 50 are then up to 9 % slower than the persistent
+// kernel would be, where they were 1700 and up to 43 % with every product of few tiles here.
+bool split_pays(int m, int tiles_m, int k_iters, bool fp8, bool shares_k) {
+  if (m <= 32) return true;
+  if (shares_k) return k_iters >= (fp8 ? 8 : 12);
+  return k_iters >= (tiles_m == 1 ? 16 : tiles_m == 2 ? 40 : tiles_m <= 8 ? 64 : 80);
+}
+
 template <bool FP8>
-cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles, cudaStream_t stream, bool* done) {
+cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles, bool plain, cudaStream_t stream, bool* done) {
   // The untraced kernel is the one that resident_clusters asks about: one CTA per SM, as the traced one.
   const auto kernel = p.trace != nullptr ? k_gemm_split<FP8, true> : k_gemm_split<FP8, false>;
   cudaError_t e = cudaFuncSetAttribute(k_gemm_split<FP8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemBytes);
@@ -287,6 +305,7 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
     if (resident_clusters<FP8>(device, s) >= tiles) splits = s;
   }
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
+  if (plain && !split_pays(p.m, p.tiles_m, p.k_iters, FP8, splits > 1)) return cudaSuccess;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
   e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
@@ -304,7 +323,7 @@ cudaError_t launch_clear_status(uint32_t* status, cudaStream_t stream) {
 }
 
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                                 const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done, long long* trace) {
+                                 const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done, const CommDev* layer) {
   *done = false;
   const int64_t tiles_m = (static_cast<int64_t>(m) + kBlockM - 1) / kBlockM, tiles_n = (static_cast<int64_t>(n) + kSplitBN - 1) / kSplitBN;
   if (tiles_m * tiles_n > kSplitMaxTiles) return cudaSuccess;
@@ -313,7 +332,7 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   SplitParams p{};
   p.c = static_cast<__nv_bfloat16*>(c);
   p.status = status;
-  p.trace = trace;
+  p.trace = layer != nullptr ? layer->trace : nullptr;
   p.scale_a = scale_a;
   p.scale_b = scale_b;
   p.m = m;
@@ -321,7 +340,9 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   p.k_iters = (k + kBlockK - 1) / kBlockK;
   p.tiles_m = static_cast<int>(tiles_m);
   const int tiles = static_cast<int>(tiles_m * tiles_n);
-  return scale_a != nullptr ? launch_split<true>(maps, p, tiles, stream, done) : launch_split<false>(maps, p, tiles, stream, done);
+  const bool plain = layer == nullptr;
+  return scale_a != nullptr ? launch_split<true>(maps, p, tiles, plain, stream, done)
+                            : launch_split<false>(maps, p, tiles, plain, stream, done);
 }
 
 } // namespace b200c
