@@ -80,9 +80,9 @@ def test_swiglu_forward_backward():
     torch.testing.assert_close(gu.grad.float(), guf.grad, rtol=3e-2, atol=3e-2)
 
 
-@pytest.mark.parametrize("rows,ffn", [(1, 8), (3, 264), (511, 8), (1025, 520), (7, 14336)])
+@pytest.mark.parametrize("rows,ffn", [(1, 8), (3, 264), (511, 8), (1025, 520), (7, 14336), (592, 4096), (593, 4096), (2500, 1000)])
 def test_swiglu_every_vector(rows, ffn):
-    """Row lengths that end anywhere in a block's span of vectors."""
+    """Row lengths that end anywhere in a block's span of vectors, one and two vectors per thread."""
     from torchcomms_b200 import _comms
 
     gu, dh = _bf(rows, 2 * ffn, seed=4, scale=3.0), _bf(rows, ffn, seed=5)

@@ -498,19 +498,22 @@ __global__ void __launch_bounds__(256) k_split_rope(__nv_bfloat16* packed, int64
 
 // -------------------------------------------------------------- SwiGLU ------
 
-// Both directions stream their operands once and are bound by memory: every thread takes kSwigluVecs vectors of
-// each operand, all loads before the first use, and finds its row with a multiply instead of a 64-bit division.
-// [4096, 2 x 14336]: forward 60.8 us, now 53.8 (6.5 TB/s); backward 101.2 us, now 83.5 (7.0 TB/s).
-constexpr int kSwigluVecs = 2;
-
+// Both directions stream their operands once and are bound by memory: every thread takes VECS vectors of each
+// operand, all loads before the first use, and finds its row with a multiply instead of a 64-bit division.
+// [4096, 2 x 14336]: forward 60.8 us, now 53.8 (6.5 TB/s); backward 101.2 us, now 83.5 (7.0 TB/s). Two vectors per
+// thread once every vector cannot have a resident thread of its own (148 x 2048 threads); below that a pass is one
+// chain of latencies, which a second vector's arithmetic makes longer: forward / backward of [100, 2 x 8192] 2.9 / 3.5 us
+// with two, 2.3 / 2.8 with one, of [1, 2 x 4096] 2.6 / 3.0 and 2.0 / 2.3; of [700, 2 x 4096] (358 thousand vectors)
+// 4.2 / 5.0 with two.
 __device__ __forceinline__ float sigmoid_of(float g) { return 1.0f / (1.0f + __expf(-g)); }
 
+template <int VECS>
 __global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* __restrict__ gate_up, __nv_bfloat16* __restrict__ h,
                                                     uint32_t total, FastDiv per_row) {
-  const uint32_t base = blockIdx.x * (256u * kSwigluVecs) + threadIdx.x;
-  uint4 gv[kSwigluVecs], uv[kSwigluVecs];
+  const uint32_t base = blockIdx.x * (256u * VECS) + threadIdx.x;
+  uint4 gv[VECS], uv[VECS];
 #pragma unroll
-  for (int k = 0; k < kSwigluVecs; ++k) {
+  for (int k = 0; k < VECS; ++k) {
     const uint32_t i = base + k * 256u;
     if (i < total) {
       // row r holds 2 x per_row vectors: gate, then up
@@ -520,7 +523,7 @@ __global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* __restr
     }
   }
 #pragma unroll
-  for (int k = 0; k < kSwigluVecs; ++k) {
+  for (int k = 0; k < VECS; ++k) {
     const uint32_t i = base + k * 256u;
     if (i < total) {
       float g[8], u[8], o[8];
@@ -533,12 +536,13 @@ __global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* __restr
   }
 }
 
+template <int VECS>
 __global__ void __launch_bounds__(256) k_swiglu_bwd(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gate_up,
                                                     __nv_bfloat16* __restrict__ dgate_up, uint32_t total, FastDiv per_row) {
-  const uint32_t base = blockIdx.x * (256u * kSwigluVecs) + threadIdx.x;
-  uint4 gv[kSwigluVecs], uv[kSwigluVecs], dv[kSwigluVecs];
+  const uint32_t base = blockIdx.x * (256u * VECS) + threadIdx.x;
+  uint4 gv[VECS], uv[VECS], dv[VECS];
 #pragma unroll
-  for (int k = 0; k < kSwigluVecs; ++k) {
+  for (int k = 0; k < VECS; ++k) {
     const uint32_t i = base + k * 256u;
     if (i < total) {
       const size_t at = static_cast<size_t>(i) + static_cast<size_t>(fast_div(i, per_row)) * per_row.d;
@@ -548,7 +552,7 @@ __global__ void __launch_bounds__(256) k_swiglu_bwd(const __nv_bfloat16* __restr
     }
   }
 #pragma unroll
-  for (int k = 0; k < kSwigluVecs; ++k) {
+  for (int k = 0; k < VECS; ++k) {
     const uint32_t i = base + k * 256u;
     if (i < total) {
       const size_t at = static_cast<size_t>(i) + static_cast<size_t>(fast_div(i, per_row)) * per_row.d;
@@ -1060,6 +1064,9 @@ cudaError_t for_row_slices(int rows, int per_row, Fn fn) {
   return cudaGetLastError();
 }
 
+// Vectors per thread of the SwiGLU kernels (see there).
+unsigned swiglu_vecs(uint32_t total) { return total <= static_cast<uint32_t>(kSms) * 2048u ? 1u : 2u; }
+
 } // namespace
 
 cudaError_t launch_split_rope(__nv_bfloat16* packed, int64_t ld, __nv_bfloat16* const* parts, const int64_t* stride_t,
@@ -1095,8 +1102,9 @@ cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, in
   if (ffn % 8 != 0) return cudaErrorInvalidValue;
   if (misaligned16(gate_up, h)) return cudaErrorMisalignedAddress;
   return for_row_slices(rows, ffn / 8, [&](size_t r0, uint32_t total) {
-    k_swiglu_fwd<<<(total + 256u * kSwigluVecs - 1) / (256u * kSwigluVecs), 256, 0, s>>>(gate_up + r0 * 2 * ffn, h + r0 * ffn, total,
-                                                                                        make_fast_div(ffn / 8));
+    const unsigned vecs = swiglu_vecs(total);
+    (vecs == 1 ? k_swiglu_fwd<1> : k_swiglu_fwd<2>)<<<covering_grid(total, 256 * vecs), 256, 0, s>>>(
+        gate_up + r0 * 2 * ffn, h + r0 * ffn, total, make_fast_div(ffn / 8));
   });
 }
 
@@ -1105,7 +1113,8 @@ cudaError_t launch_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate
   if (ffn % 8 != 0) return cudaErrorInvalidValue;
   if (misaligned16(dh, gate_up, dgate_up)) return cudaErrorMisalignedAddress;
   return for_row_slices(rows, ffn / 8, [&](size_t r0, uint32_t total) {
-    k_swiglu_bwd<<<(total + 256u * kSwigluVecs - 1) / (256u * kSwigluVecs), 256, 0, s>>>(
+    const unsigned vecs = swiglu_vecs(total);
+    (vecs == 1 ? k_swiglu_bwd<1> : k_swiglu_bwd<2>)<<<covering_grid(total, 256 * vecs), 256, 0, s>>>(
         dh + r0 * ffn, gate_up + r0 * 2 * ffn, dgate_up + r0 * 2 * ffn, total, make_fast_div(ffn / 8));
   });
 }
