@@ -34,7 +34,7 @@ def test_rmsnorm_forward_backward(rows, cols):
 
 
 @pytest.mark.parametrize("cols", [8, 256, 264, 512, 1000, 1024, 1032, 2048, 2056, 4096, 4104, 8192])
-@pytest.mark.parametrize("rows", [1, 9, 1200, 2377])
+@pytest.mark.parametrize("rows", [1, 4, 9, 74, 75, 148, 149, 1200, 2377])
 def test_rmsnorm_row_layouts(rows, cols):
     """Every split of a row over threads, at its edges, with fewer and more rows than row groups on the GPU."""
     from torchcomms_b200 import _comms
@@ -287,7 +287,7 @@ def test_adamw_refuses_shards_off_the_vector_grid():
     assert bool((ts[0][1:4] < 0).all()) and not ts[0][0] and not ts[0][4:].any()
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 8), (9, 256), (40, 512), (700, 1000), (5, 2048), (601, 4096), (3, 8192), (300, 8192)])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (9, 256), (40, 512), (80, 512), (140, 776), (700, 1000), (5, 2048), (601, 4096), (3, 8192), (300, 8192)])
 def test_norm_with_residual_stream(rows, cols):
     """x + delta and its norm in one kernel: forward bit for bit what addition and norm give, backward with the
     residual's gradient added in fp32."""

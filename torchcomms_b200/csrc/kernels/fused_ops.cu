@@ -943,13 +943,23 @@ void rmsnorm_fwd_rows(const __nv_bfloat16* x, const __nv_bfloat16* delta, const 
   else k_rmsnorm_fwd_reg<256, 4, ADD><<<rows, 256, 0, s>>>(x, delta, w, sum, y, rstd, rows, cols, eps);
 }
 
+// Rows of the backward as a warp each, eight to a block, or as a block each (every row that needs more than 1024
+// columns). A warp holds up to 32 elements of its row and the block then adds up eight shares of the weight gradient;
+// with few rows that is a longer chain than a block per row, whose many partial rows cost more from some rows on.
+// Warp / block, in us with the column sum: 1 x 776 5.0 / 3.5, 64 x 776 5.4 / 4.1, 148 x 1024 5.4 / 4.5, 200 x 1024
+// 5.5 / 5.5, 296 x 1024 5.7 / 6.0; 16 x 512 4.3 / 3.7, 64 x 512 4.5 / 4.2, 148 x 512 4.5 / 4.5, 200 x 512 4.5 / 5.0;
+// 1 x 256 3.8 / 3.5.
+bool bwd_warp_rows(int rows, int cols) {
+  return cols <= 1024 && rows > (cols > 512 ? kSms : cols > 256 ? kSms / 2 : 4);
+}
+
 template <bool ADD>
 void rmsnorm_bwd_rows(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w, const float* rstd,
                       const __nv_bfloat16* dskip, __nv_bfloat16* dx, float* part, int blocks, int rows, int cols, cudaStream_t s) {
-  if (cols <= 256) k_rmsnorm_bwd<32, 1, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
+  if (cols <= 2048 && !bwd_warp_rows(rows, cols)) k_rmsnorm_bwd<256, 1, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
+  else if (cols <= 256) k_rmsnorm_bwd<32, 1, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
   else if (cols <= 512) k_rmsnorm_bwd<32, 2, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
   else if (cols <= 1024) k_rmsnorm_bwd<32, 4, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
-  else if (cols <= 2048) k_rmsnorm_bwd<256, 1, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
   else if (cols <= 4096) k_rmsnorm_bwd<256, 2, ADD><<<blocks, kNormThreads, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
   else k_rmsnorm_bwd<512, 2, ADD><<<blocks, 512, 0, s>>>(dy, x, w, rstd, dskip, dx, part, rows, cols);
 }
@@ -976,7 +986,7 @@ cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, 
                                const float* rstd, __nv_bfloat16* dx, float* dw_partial, int* nblocks, int rows,
                                int cols, cudaStream_t s, const __nv_bfloat16* dskip) {
   if (cols % 8 != 0 || rows <= 0 || cols > kNormThreads * kNormMaxVec * 8) return cudaErrorInvalidValue;
-  const bool warp_rows = cols <= 1024;  // a warp per row, eight to a block
+  const bool warp_rows = bwd_warp_rows(rows, cols);
   const int per_sm = cols > 4096 ? norm_bwd_per_sm<512, 2>() : (cols > 512 && warp_rows) ? norm_bwd_per_sm<32, 4>() : 2;
   const int blocks = std::min(warp_rows ? (rows + 7) / 8 : rows, kSms * per_sm);
   if (nblocks) *nblocks = blocks;
