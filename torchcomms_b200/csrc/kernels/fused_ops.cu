@@ -866,18 +866,19 @@ __device__ __forceinline__ float adamw_one(float p, float g, float& m, float& v,
 
 // Seven streams, each touched once: bound by memory. A block takes a contiguous span, two vectors per thread, and the
 // grid covers the tensors once; with blocks that stride through them the streams reach memory in a less even order
-// (218112000 elements: 1013 us striding over 1184 blocks, 890 us, 6.9 TB/s, so).
-constexpr int kAdamwVecs = 2;
-
+// (218112000 elements: 1013 us striding over 1184 blocks, 890 us, 6.9 TB/s, so). Small tensors are one chain of
+// latencies, which a second vector makes longer, and take one vector per thread up to three blocks per SM: 50000
+// elements 2.3 us with two and 2.1 with one, 400000 2.8 and 2.6, but 800000 3.5 and 3.7.
+template <int VECS>
 __global__ void __launch_bounds__(256) k_adamw(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                                                float* __restrict__ v, size_t n, float lr, float beta1, float beta2,
                                                float eps, float weight_decay, float bias1, float bias2, float grad_scale) {
   const size_t nvec = n / 4;
   const float inv_bias1 = 1.0f / bias1, inv_bias2 = 1.0f / bias2, decay = 1.0f - lr * weight_decay;
-  const size_t base = blockIdx.x * static_cast<size_t>(256 * kAdamwVecs) + threadIdx.x;
-  float4 pp[kAdamwVecs], gg[kAdamwVecs], mm[kAdamwVecs], vv[kAdamwVecs];
+  const size_t base = blockIdx.x * static_cast<size_t>(256 * VECS) + threadIdx.x;
+  float4 pp[VECS], gg[VECS], mm[VECS], vv[VECS];
 #pragma unroll
-  for (int u = 0; u < kAdamwVecs; ++u) {
+  for (int u = 0; u < VECS; ++u) {
     const size_t j = base + u * 256;
     if (j < nvec) {
       pp[u] = reinterpret_cast<float4*>(p)[j];
@@ -887,7 +888,7 @@ __global__ void __launch_bounds__(256) k_adamw(float* __restrict__ p, const floa
     }
   }
 #pragma unroll
-  for (int u = 0; u < kAdamwVecs; ++u) {
+  for (int u = 0; u < VECS; ++u) {
     const size_t j = base + u * 256;
     if (j < nvec) {
       float* pa = &pp[u].x;
@@ -1156,8 +1157,9 @@ cudaError_t launch_adamw(float* p, const float* g, float* m, float* v, size_t n,
   if (n >= 4 && misaligned16(p, g, m, v)) return cudaErrorMisalignedAddress;  // fewer elements use no vectors
   const float bias1 = 1.0f - powf(beta1, static_cast<float>(step));
   const float bias2 = 1.0f - powf(beta2, static_cast<float>(step));
-  k_adamw<<<covering_grid(n / 4, 256 * kAdamwVecs), 256, 0, s>>>(p, g, m, v, n, lr, beta1, beta2, eps, weight_decay, bias1, bias2,
-                                                    grad_scale);
+  const unsigned vecs = n / 4 <= static_cast<size_t>(kSms) * 3 * 256 ? 1u : 2u;
+  (vecs == 1 ? k_adamw<1> : k_adamw<2>)<<<covering_grid(n / 4, 256 * vecs), 256, 0, s>>>(p, g, m, v, n, lr, beta1, beta2, eps,
+                                                                                         weight_decay, bias1, bias2, grad_scale);
   note_kernel_launch();
   return cudaGetLastError();
 }
