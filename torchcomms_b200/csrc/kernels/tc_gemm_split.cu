@@ -57,7 +57,7 @@ struct SplitParams {
   const float* scale_a;  // e4m3: per row of A, per row of B
   const float* scale_b;
   long long* trace;
-  int m, n, k_iters, tiles_m;
+  int m, n, k, k_iters, tiles_m;  // k in 16-bit units
 };
 
 __device__ __forceinline__ uint32_t cluster_nctarank() {
@@ -269,22 +269,25 @@ int resident_clusters(int device, int splits) {
   return n;
 }
 
-// Whether the split kernel beats the persistent one (tiles of 128 x 256) on a plain product. Meeting the cluster and
-// adding up the shares costs it 1 us more than the direct stores of a full tile, nothing where the tile has few rows;
-// a K step is 0.28 us of the persistent kernel's time and 0.2 us of this one's, over the CTAs that share K. Replayed from
-// a graph, persistent / split in us (bf16 unless e4m3 is said):
-//   few rows: 1 x 2048 x 512 7.4 / 6.1, 32 x 2048 x 512 7.5 / 6.9
-//   K shared, line at 12 steps of 64, in e4m3 at 8 of 128: 128 x 2048 x 512 7.7 / 8.4, x 768 8.9 / 8.8, x 1536
-//   12.2 / 11.3; e4m3 128 x 2048 x 768 8.6 / 10.1, x 1024 9.2 / 8.9
+// Whether the split kernel beats the persistent one (tiles of 128 x 256) on a plain product; `k` in 16-bit units. Meeting
+// the cluster and adding up the shares costs it 1 us more than the direct stores of a full tile, less where the tile has
+// few rows; a K step is 0.28 us of the persistent kernel's time and 0.2 us of this one's, over the CTAs that share K.
+// Rows that do not start on 128-byte lines make every step longer, most where few CTAs load. Replayed from a graph,
+// persistent / split in us (bf16 unless e4m3 is said):
+//   few rows, up to 32 or, in e4m3, 64: 1 x 2048 x 512 7.4 / 6.1, 32 x 2048 x 512 7.5 / 6.9; e4m3 48 x 2048 x 256
+//   7.7 / 6.8, 64 x 2048 x 256 7.8 / 7.4
+//   K shared, line at 12 steps of 64, in e4m3 (of 128) or off the lines at 8: 128 x 2048 x 512 7.7 / 8.4, x 768
+//   8.9 / 8.8, x 1536 12.2 / 11.3; e4m3 128 x 2048 x 768 8.6 / 10.1, x 1024 9.2 / 8.9
 //   K not shared: half the tile on twice the SMs pays later, the more row tiles read the same weights again:
 //   128 x 14336 x 768 9.6 / 10.7, x 1024 12.1 / 12.5, x 2048 20.4 / 18.3; 256 x 9216 x 2560 22.1 / 19.7;
-//   2048 x 1024 x 3072 18.8 / 22.6, x 4096 23.7 / 26.3, x 6144 38.3 / 35.6
-// Of 3830 shapes (rows 1..8192, columns 256..18432, K 64..24576) some 50 are then up to 9 % slower than the persistent
-// kernel would be, where they were 1700 and up to 43 % with every product of few tiles here.
-bool split_pays(int m, int tiles_m, int k_iters, bool fp8, bool shares_k) {
-  if (m <= 32) return true;
-  if (shares_k) return k_iters >= (fp8 ? 8 : 12);
-  return k_iters >= (tiles_m == 1 ? 16 : tiles_m == 2 ? 40 : tiles_m <= 8 ? 64 : 80);
+//   2048 x 1024 x 3072 18.8 / 22.6, x 4096 23.7 / 26.3, x 6144 38.3 / 35.6; off the lines from 12 steps on, 0.9 to 1.1
+//   times as fast at 10..15, 1.0 to 1.3 from 29 on
+bool split_pays(int m, int tiles_m, int k, bool fp8, bool shares_k) {
+  if (m <= (fp8 ? 64 : 32)) return true;
+  const bool on_lines = k % kBlockK == 0;
+  const int k_iters = (k + kBlockK - 1) / kBlockK;
+  if (shares_k) return k_iters >= (fp8 || !on_lines ? 8 : 12);
+  return k_iters >= (!on_lines ? 12 : tiles_m == 1 ? 16 : tiles_m == 2 ? 40 : tiles_m <= 8 ? 64 : 80);
 }
 
 template <bool FP8>
@@ -305,7 +308,7 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
     if (resident_clusters<FP8>(device, s) >= tiles) splits = s;
   }
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
-  if (plain && !split_pays(p.m, p.tiles_m, p.k_iters, FP8, splits > 1)) return cudaSuccess;
+  if (plain && !split_pays(p.m, p.tiles_m, p.k, FP8, splits > 1)) return cudaSuccess;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
   e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
@@ -337,6 +340,7 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   p.scale_b = scale_b;
   p.m = m;
   p.n = n;
+  p.k = k;
   p.k_iters = (k + kBlockK - 1) / kBlockK;
   p.tiles_m = static_cast<int>(tiles_m);
   const int tiles = static_cast<int>(tiles_m * tiles_n);
