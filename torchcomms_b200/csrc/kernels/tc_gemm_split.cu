@@ -248,12 +248,13 @@ cudaLaunchConfig_t split_config(int tiles, int splits, cudaStream_t stream, cuda
   return cfg;
 }
 
+constexpr int kDevices = 64;  // whose answers are kept
+
 // Clusters of each size that the current GPU holds at once: they must fit one GPC, so not simply SMs / size, and GPUs
 // differ in how their SMs are spread over GPCs. The answer decides the order of summation, so it is kept per device,
 // and a query that failed is asked again at the next call.
 template <bool FP8>
 int resident_clusters(int device, int splits) {
-  constexpr int kDevices = 64;
   static std::atomic<int> known[kDevices][kSplitMax + 1];
   std::atomic<int>* kept = device >= 0 && device < kDevices ? &known[device][splits] : nullptr;
   int n = kept != nullptr ? kept->load(std::memory_order_relaxed) : 0;
@@ -292,17 +293,23 @@ bool split_pays(int m, int tiles_m, int k, bool fp8, bool shares_k) {
 
 template <bool FP8>
 cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles, bool plain, cudaStream_t stream, bool* done) {
-  // The untraced kernel is the one that resident_clusters asks about: one CTA per SM, as the traced one.
+  // The untraced kernel is the one that resident_clusters asks about: one CTA per SM, as the traced one. Its attribute
+  // stays with the device and is set once.
+  static std::atomic<bool> ready[kDevices];
   const auto kernel = p.trace != nullptr ? k_gemm_split<FP8, true> : k_gemm_split<FP8, false>;
-  cudaError_t e = cudaFuncSetAttribute(k_gemm_split<FP8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemBytes);
+  int splits = 0, device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  const bool kept = device >= 0 && device < kDevices;
+  if (e == cudaSuccess && !(kept && ready[device].load(std::memory_order_acquire))) {
+    e = cudaFuncSetAttribute(k_gemm_split<FP8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemBytes);
+    if (e == cudaSuccess && kept) ready[device].store(true, std::memory_order_release);
+  }
   if (e == cudaSuccess && p.trace != nullptr) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmemBytes);
   }
   if (e != cudaSuccess) return e;
   // As many ways as leave every cluster resident and every CTA at least four K steps (below that the fixed cost of
   // filling the pipeline and meeting the cluster is larger than what another split saves).
-  int splits = 0, device = 0;
-  if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
   for (int s = 1; s <= kSplitMax; ++s) {
     if (s > 1 && p.k_iters < 4 * s) break;
     if (resident_clusters<FP8>(device, s) >= tiles) splits = s;
