@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "early_launch.cuh"
 #include "launch_count.h"
 
 namespace b200c {
@@ -508,9 +509,10 @@ __global__ void __launch_bounds__(256) k_split_rope(__nv_bfloat16* packed, int64
 __device__ __forceinline__ float sigmoid_of(float g) { return 1.0f / (1.0f + __expf(-g)); }
 
 template <int VECS>
-__global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* __restrict__ gate_up, __nv_bfloat16* __restrict__ h,
-                                                    uint32_t total, FastDiv per_row) {
+__global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, uint32_t total, FastDiv per_row) {
   const uint32_t base = blockIdx.x * (256u * VECS) + threadIdx.x;
+  grid_release();
+  grid_wait();
   uint4 gv[VECS], uv[VECS];
 #pragma unroll
   for (int k = 0; k < VECS; ++k) {
@@ -711,9 +713,10 @@ constexpr int kQuantKeep = 8;  // vectors of 8 a thread holds between the two lo
 // so comes through. [4096, 4096] and [4096, 14336] together: 890 us operator by operator, 42 us (5.4 TB/s) here;
 // [67, 4096]: 27 us in eight launches, now 2.3. VEC: 16-byte loads (base, row stride and cols allow them).
 template <bool VEC>
-__global__ void __launch_bounds__(256) k_quantize_rows(const __nv_bfloat16* __restrict__ x, int64_t ld,
-                                                        uint8_t* __restrict__ q, float* __restrict__ scale, int cols) {
+__global__ void __launch_bounds__(256) k_quantize_rows(const __nv_bfloat16* x, int64_t ld, uint8_t* q, float* scale, int cols) {
   __shared__ uint32_t part[8];
+  grid_release();
+  grid_wait();
   const int tid = threadIdx.x, nt = blockDim.x;
   const __nv_bfloat16* row = x + static_cast<int64_t>(blockIdx.x) * ld;
   uint8_t* out = q + static_cast<size_t>(blockIdx.x) * cols;
@@ -1021,8 +1024,8 @@ cudaError_t launch_quantize_rows(const __nv_bfloat16* x, int64_t ld, void* q, fl
   // Enough threads that a row of up to 8 vectors each stays in registers; with few rows on the GPU more threads
   // shorten the row instead.
   const int threads = cols <= 1024 ? 32 : (cols <= 4096 && rows > kSms * 4) ? 128 : 256;
-  if (vec) k_quantize_rows<true><<<rows, threads, 0, s>>>(x, ld, static_cast<uint8_t*>(q), scale, cols);
-  else k_quantize_rows<false><<<rows, threads, 0, s>>>(x, ld, static_cast<uint8_t*>(q), scale, cols);
+  launch_early(vec ? k_quantize_rows<true> : k_quantize_rows<false>, static_cast<unsigned>(rows), static_cast<unsigned>(threads), s, x, ld,
+               static_cast<uint8_t*>(q), scale, cols);
   note_kernel_launch();
   return cudaGetLastError();
 }
@@ -1114,8 +1117,8 @@ cudaError_t launch_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, in
   if (misaligned16(gate_up, h)) return cudaErrorMisalignedAddress;
   return for_row_slices(rows, ffn / 8, [&](size_t r0, uint32_t total) {
     const unsigned vecs = swiglu_vecs(total);
-    (vecs == 1 ? k_swiglu_fwd<1> : k_swiglu_fwd<2>)<<<covering_grid(total, 256 * vecs), 256, 0, s>>>(
-        gate_up + r0 * 2 * ffn, h + r0 * ffn, total, make_fast_div(ffn / 8));
+    launch_early(vecs == 1 ? k_swiglu_fwd<1> : k_swiglu_fwd<2>, covering_grid(total, 256 * vecs), 256, s, gate_up + r0 * 2 * ffn,
+                 h + r0 * ffn, total, make_fast_div(ffn / 8));
   });
 }
 

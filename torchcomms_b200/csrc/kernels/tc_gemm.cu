@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <string>
 
+#include "early_launch.cuh"
 #include "launch_count.h"
 #include "tc_gemm.cuh"
 
@@ -361,6 +362,10 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  if (!kFused) {
+    grid_release();
+    grid_wait();
+  }
   const uint32_t epoch = bars->epoch;  // calls completed before this one
   if (kFused && threadIdx.x == 0) trace_stamp_ns(c, 0);
 
@@ -1104,9 +1109,19 @@ cudaError_t tp_launch_t(int grid, const TpMaps& maps, const CommDev& c, const Tp
   // Per device, so not cached in a process-wide flag.
   cudaError_t e = cudaFuncSetAttribute(k_tp_gemm<MODE, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTpSmemBytes);
   if (e != cudaSuccess) return e;
-  k_tp_gemm<MODE, FP8><<<grid, tp_threads<MODE>(), kTpSmemBytes, stream>>>(maps, c, p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(tp_threads<MODE>());
+  cfg.dynamicSmemBytes = kTpSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = MODE == TpMode::PLAIN ? 1 : 0;  // the fused modes meet other GPUs and start when their stream does
+  e = cudaLaunchKernelEx(&cfg, k_tp_gemm<MODE, FP8>, maps, c, p);
   note_kernel_launch();
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // The operand type (p.fp8) picks the instantiation: the bf16 kernels carry no trace of the fp8 path.

@@ -315,11 +315,12 @@ __host__ __device__ constexpr uint32_t make_idesc_e4m3(int m, int n) {
       | (static_cast<uint32_t>(m >> 4) << 24);  // M / 16
 }
 
-// Epilogue of the fp8 products: acc[i] *= row_scale * col_scale[col0 + i] (columns past `n` give zero).
-__device__ __forceinline__ void scale_acc32(uint32_t (&r)[32], float row_scale, const float* __restrict__ col_scale, int col0, int n) {
+// Epilogue of the fp8 products: acc[i] *= row_scale * col_scale[col0 + i] (columns past `n` give zero). Ordinary loads:
+// the scales may have been written while this kernel's blocks were already resident.
+__device__ __forceinline__ void scale_acc32(uint32_t (&r)[32], float row_scale, const float* col_scale, int col0, int n) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    const float b = col0 + i < n ? __ldg(col_scale + col0 + i) : 0.0f;
+    const float b = col0 + i < n ? col_scale[col0 + i] : 0.0f;
     r[i] = __float_as_uint(__uint_as_float(r[i]) * (row_scale * b));
   }
 }

@@ -11,13 +11,16 @@
 // some results round differently and fewer of them away from the exact product's bf16 value (0.07 % of 128 x 3584 x
 // 4096, there 0.24 %). m x n x k = 128 x 3584 x 4096 and 128 x 4096 x 1792 in bf16: 31.8 and
 // 28.3 us with one 128 x 256 tile on each of 14 and 16 CTAs, 25.1 us for both here
-// (28 x 4 and 32 x 4 CTAs); 67 x 6144 x 4096 in e4m3: 15.3 us, now 11.0.
+// (28 x 4 and 32 x 4 CTAs); 67 x 6144 x 4096 in e4m3: 15.3 us, now 11.0. Behind another kernel the set-up (barriers,
+// tensor memory) overlaps with that one's end: bf16 rows quantised and multiplied, 67 x 6144 x 4096, take 13.8 us a pass,
+// 18.4 when every launch and the clearing of the status words waited for the one in front.
 //   warp 0, one lane : TMA producer
 //   warp 1           : allocates tensor memory; one lane issues tcgen05.mma
 //   warps 2..5       : accumulator -> shared memory; then all warps reduce
 #include <algorithm>
 #include <atomic>
 
+#include "early_launch.cuh"
 #include "launch_count.h"
 #include "tc_gemm.cuh"
 #include "tc_gemm.h"
@@ -107,6 +110,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  grid_release();
+  grid_wait();
   if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 0);
 
   if (warp == 0) {
@@ -214,7 +219,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
     if (FP8) {
       const float ra = p.scale_a[grow];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] *= ra * __ldg(p.scale_b + gcol + i);
+      for (int i = 0; i < 8; ++i) acc[i] *= ra * p.scale_b[gcol + i];
     }
     uint4 o;
     uint32_t* po = &o.x;
@@ -243,8 +248,10 @@ cudaLaunchConfig_t split_config(int tiles, int splits, cudaStream_t stream, cuda
   attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cfg;
 }
 
@@ -259,8 +266,9 @@ int resident_clusters(int device, int splits) {
   std::atomic<int>* kept = device >= 0 && device < kDevices ? &known[device][splits] : nullptr;
   int n = kept != nullptr ? kept->load(std::memory_order_relaxed) : 0;
   if (n == 0) {
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = split_config(1, splits, nullptr, attr);
+    cfg.numAttrs = 1;  // the cluster size
     if (cudaOccupancyMaxActiveClusters(&n, k_gemm_split<FP8, false>, &cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       return 0;
@@ -316,7 +324,7 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
   }
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
   if (plain && !split_pays(p.m, p.tiles_m, p.k, FP8, splits > 1)) return cudaSuccess;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
   e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
   note_kernel_launch();

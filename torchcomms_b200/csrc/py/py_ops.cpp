@@ -3,6 +3,7 @@
 
 #include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/InferenceMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
 
@@ -37,19 +38,38 @@ bool on16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr(
 // of a gradient) does not start on such a boundary, and contiguous() leaves it where it is.
 at::Tensor vectorable(const at::Tensor& t) { return on16(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
 
-// Two cleared status words, without a launch through the tensor library. On a stream eight bytes are cleared as fast by
-// a memset as by a kernel; in a graph a memset node holds the product behind it up (m x n x k = 128 x 256 x 64 in bf16:
-// 10.1 us a replay, with a kernel node 6.9; 128 x 6144 x 4096 in e4m3 16.2 and 12.8).
+// Two cleared status words for one product. A memset per call costs a launch, and keeps the product from starting while
+// the kernel in front of it drains. So words are cut from a block that was cleared in one go on the same stream, each
+// handed out once; the last block of a thread stays with it (one: a call on another stream starts a new one). A graph
+// replays its launches on the same words, so a captured call clears its own, by a kernel node: a memset node holds the
+// product behind it up (m x n x k = 128 x 256 x 64 in bf16: 10.1 us a replay, with a kernel node 6.9; 128 x 6144 x 4096
+// in e4m3 16.2 and 12.8).
 at::Tensor cleared_status(const at::Tensor& like) {
-  at::Tensor status = at::empty({2}, like.options().dtype(at::kInt));
+  const cudaStream_t stream = cur(like);
+  const auto opts = like.options().dtype(at::kInt);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  B200C_CUDA_CHECK(cudaStreamIsCapturing(cur(like), &capture));
-  if (capture == cudaStreamCaptureStatusNone) {
-    B200C_CUDA_CHECK(cudaMemsetAsync(status.data_ptr(), 0, 8, cur(like)));
-  } else {
-    B200C_CUDA_CHECK(launch_clear_status(reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(like)));
+  B200C_CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone) {
+    at::Tensor status = at::empty({2}, opts);
+    B200C_CUDA_CHECK(launch_clear_status(reinterpret_cast<uint32_t*>(status.data_ptr<int>()), stream));
+    return status;
   }
-  return status;
+  constexpr int64_t kCalls = 1024;
+  struct Block {
+    at::Tensor words;  // [kCalls, 2]
+    unsigned long long stream_id = 0;
+    int64_t next = 0;
+  };
+  thread_local Block block;
+  unsigned long long id = 0;  // unlike the handle, never given to another stream
+  B200C_CUDA_CHECK(cudaStreamGetId(stream, &id));
+  if (!block.words.defined() || block.next == kCalls || block.stream_id != id || block.words.device() != like.device() ||
+      block.words.is_inference() != c10::InferenceMode::is_enabled()) {
+    at::Tensor words = at::empty({kCalls, 2}, opts);
+    B200C_CUDA_CHECK(cudaMemsetAsync(words.data_ptr(), 0, words.nbytes(), stream));
+    block = Block{std::move(words), id, 0};
+  }
+  return block.words.select(0, block.next++);
 }
 
 bool quantizable(const at::Tensor& x) {
