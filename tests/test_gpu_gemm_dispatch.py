@@ -1,0 +1,58 @@
+"""Every kernel that a plain product can take, at the edges of the rule that picks it, against a 64-bit product."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# Narrow pair tiles at most one wave, more than one; short sums on single CTAs, and one step more; rows off the 128-byte
+# lines; row and column remainders of every tile.
+@pytest.mark.parametrize("m,n,k", [(256, 9472, 256), (257, 9480, 256), (129, 136, 1024), (700, 6144, 1024), (700, 6144, 1088), (700, 6152, 1032),
+                                   (4096, 2304, 128), (4096, 2320, 1040), (1000, 6144, 2048), (385, 264, 8)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_plain_product(m, n, k, fp8):
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops.tp import quantize_rows
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    k = 2 * k if fp8 else k  # the rule counts bytes
+    a = (torch.randn(m, k, generator=g, device="cuda") * 0.5).to(torch.bfloat16)
+    b = (torch.randn(n, k, generator=g, device="cuda") * 0.5).to(torch.bfloat16)
+    if fp8:
+        (qa, sa), (qb, sb) = quantize_rows(a), quantize_rows(b)
+        ref = (qa.double() * sa.double().unsqueeze(1)) @ (qb.double() * sb.double().unsqueeze(1)).t()
+        run = lambda: _comms.ops.gemm_e4m3_nt(qa, qb, sa, sb)
+    else:
+        ref = a.double() @ b.double().t()
+        run = lambda: _comms.ops.gemm_bf16_nt(a, b)
+    first = None
+    for _ in range(3):
+        c, status = run()
+        assert int(status[0]) == 0
+        # Half a bf16 ulp (2^-9 relative), and k fp32 additions of terms of size 1/4 before it.
+        torch.testing.assert_close(c.double(), ref, rtol=2**-8, atol=1e-6 * k)
+        assert first is None or torch.equal(c, first)
+        first = c
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 256, 64), (128, 3584, 4096), (384, 512, 704), (512, 5120, 512)])
+def test_gather_layer_leaves_its_input_behind(m, n, k):
+    """A single rank's layer reads the activations where they are; its input buffer holds them afterwards all the same."""
+    from torchcomms_b200.ops.tp import AllGatherGemm
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(n, k, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    layer = AllGatherGemm(None, m_local=m, k=k)
+    layer.input.zero_()
+    y = layer(w, x)
+    assert torch.equal(layer.input, x) and torch.equal(layer(w), y)
+    torch.testing.assert_close(y.double(), x.double() @ w.double().t(), rtol=2**-8, atol=2e-7 * k)
+    # What cannot be read in place is copied first: other layouts and types, and the buffer itself.
+    wide = torch.zeros(m, k + 8, device="cuda", dtype=torch.bfloat16)
+    wide[:, :k] = x
+    off = torch.zeros(m * k + 1, device="cuda", dtype=torch.bfloat16)[1:].view(m, k).copy_(x)
+    for other in (wide[:, :k], off, x.t().contiguous().t(), x.float(), layer.input):
+        if other is not layer.input and other.data_ptr() != layer.input.data_ptr():
+            layer.input.zero_()
+        assert torch.equal(layer(w, other), y) and torch.equal(layer.input, x)

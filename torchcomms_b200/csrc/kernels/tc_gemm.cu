@@ -367,7 +367,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
     grid_wait();
   }
   const uint32_t epoch = bars->epoch;  // calls completed before this one
-  if (kFused && threadIdx.x == 0) trace_stamp_ns(c, 0);
+  if (threadIdx.x == 0) trace_stamp_ns(c, 0);
 
   // m-tile ordinal -> real m-tile. All-gather: own rows first, then the
   // sources in ring order (the order in which the copy warps fetch them).
@@ -419,7 +419,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
           tma_load_2d(sa + Cfg::kABytes, &maps.b, &bars->full[s], kb * kBlockK, ni * BN);
         }
       }
-      if (kFused) trace_stamp_ns(c, 1);
+      trace_stamp_ns(c, 1);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer
@@ -456,7 +456,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
         }
         umma_commit(&bars->acc_full[as]);  // accumulator complete
       }
-      if (kFused) trace_stamp_ns(c, 2);
+      trace_stamp_ns(c, 2);
     }
   } else if (warp < 6) {
     // ---------------- epilogue: TMEM -> bf16 -> swizzled staging -> TMA store
@@ -668,6 +668,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
   }
   if (!kFused) {
     if (threadIdx.x == 0 && bars->failed && p.status != nullptr) p.status[0] = p.status[0] | kStatusTimeout;
+    if (threadIdx.x == 0) trace_stamp_ns(c, 7);
     return;
   }
   if (threadIdx.x == 0) {
@@ -1188,14 +1189,30 @@ cudaError_t launch_gemm_e4m3_nt(const void* a, const void* b, void* c, int m, in
 
 // k in 16-bit units; scales non-null = e4m3 operands.
 cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                           const float* scale_b, uint32_t* status, cudaStream_t stream) {
+                           const float* scale_b, uint32_t* status, cudaStream_t stream, const CommDev* layer, void* a_copy) {
   if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || n % 8 != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) {
     return cudaErrorInvalidValue;
   }
   bool done = false;
-  const cudaError_t split = launch_gemm_nt_split(a, b, c, m, n, k, scale_a, scale_b, status, stream, &done);
-  if (split != cudaSuccess || done) return split;
+  cudaError_t e = launch_gemm_nt_split(a, b, c, m, n, k, scale_a, scale_b, status, stream, &done, layer, a_copy);
+  if (e != cudaSuccess || done) return e;
+  if (a_copy != nullptr) {
+    e = cudaMemcpyAsync(a_copy, a, static_cast<size_t>(m) * k * 2, cudaMemcpyDeviceToDevice, stream);
+    if (e != cudaSuccess) return e;
+  }
+  // Pairs beat single CTAs wherever the tensor cores decide (a K step is 0.27 us of either, and a pair's covers twice the
+  // tile), and tiles of 128 columns the ones of 256 as long as no pair gets a second one. Single CTAs are left with short
+  // sums whose 128 x 256 tiles fill the GPU once, where pairs would not; rows that do not start on 128-byte lines cost
+  // them more than pairs. In us, replayed from a graph, single / pairs of 256 / pairs of 128 columns, e4m3: 256 x 6144 x
+  // 4096 19.1 / 17.0 / 15.7; 1000 x 6144 x 4096 34.1 / 29.0 / 36.6, x 4112 45.7 / 34.7 / 37.4; 2048 x 8192 x 2048 34.8 /
+  // 32.2 / 43.3; 768 x 6144 x 256 6.9 / 7.8 / 7.9; bf16: 1000 x 4096 x 1024 9.3 / 10.2 / 14.1, x
+  // 2048 17.2 / 15.7 / 24.0.
+  const int tiles_m = (m + kBlockM - 1) / kBlockM, tiles_n = (n + kTpBN - 1) / kTpBN;
+  if (pair_tiles_fit(m, n, scale_a != nullptr)) return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, true, layer);
+  if (k > 16 * kBlockK || k % kBlockK != 0 || static_cast<int64_t>(tiles_m) * tiles_n > sm_count()) {
+    return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, false, layer);
+  }
   TpMaps maps;
   if (!make_map(&maps.a_local, a, m, k, kBlockM) || !make_map(&maps.b, b, n, k, kTpBN) ||
       !make_map(&maps.out[0], c, m, n, kBlockM)) {
@@ -1206,6 +1223,7 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   for (int r = 1; r < kMaxRanks; ++r) maps.out[r] = maps.out[0];
   CommDev none{};
   none.nranks = 1;
+  none.trace = layer != nullptr ? layer->trace : nullptr;
   TpParams p{};
   p.status = status;
   p.m_total = m;
@@ -1215,7 +1233,6 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   p.fp8 = scale_a != nullptr ? 1 : 0;
   p.scale_a = scale_a;
   p.scale_b = scale_b;
-  const int tiles_m = (m + kBlockM - 1) / kBlockM, tiles_n = (n + kTpBN - 1) / kTpBN;
   p.gm = pick_group(tiles_m, kBlockM, k, 16);
   return tp_launch<TpMode::PLAIN>(std::min(sm_count(), tiles_m * tiles_n), maps, none, p, stream);
 }
@@ -1333,20 +1350,30 @@ cudaError_t tp_launch_emu(const TpEmu& e, int nranks, cudaStream_t stream) {
   return e.p[0].fp8 ? tp_launch_emu_t<MODE, true>(e, nranks, stream) : tp_launch_emu_t<MODE, false>(e, nranks, stream);
 }
 
+// A fused layer's product on a single rank; k in elements. `a_copy`: the layer's input buffer, where A comes from elsewhere.
+cudaError_t layer_product(const CommDev& comm, const void* a, const void* w, void* y, int m, int n, int k, int fp8,
+                          const float* scale_a, const float* scale_w, void* a_copy, cudaStream_t stream) {
+  if (n <= 0 || n % kTpBN != 0 || k <= 0 || k % (fp8 ? 2 * kBlockK : kBlockK) != 0) return cudaErrorInvalidValue;
+  if (fp8 && (scale_a == nullptr || scale_w == nullptr)) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15u) return cudaErrorInvalidValue;
+  const int k16 = fp8 ? k / 2 : k;
+  return launch_gemm_nt(a, w, y, m, n, k16, fp8 ? scale_a : nullptr, scale_w, const_cast<uint32_t*>(comm.status), stream, &comm, a_copy);
+}
+
 } // namespace
 
 cudaError_t launch_allgather_gemm(const CommDev& comm, const AgGemmArgs& a, cudaStream_t stream) {
+  if (comm.nranks == 1) {  // nothing to gather
+    if (a.m_local <= 0 || a.m_local % kBlockM != 0) return cudaErrorInvalidValue;
+    return layer_product(comm, a.x_src != nullptr ? a.x_src : a.x_shards[0], a.w, a.y, a.m_local, a.n, a.k, a.fp8, a.scale_x_shards[0],
+                         a.scale_w, a.x_src != nullptr ? const_cast<void*>(a.x_shards[0]) : nullptr, stream);
+  }
+  if (a.x_src != nullptr) return cudaErrorInvalidValue;  // peers read the shard where it is
   TpMaps maps;
   TpParams p;
   const bool pairs = a.m_local > 0 && use_pairs(a.m_local);
   cudaError_t e = build_ag(comm, a, pairs, maps, p);
   if (e != cudaSuccess) return e;
-  if (comm.nranks == 1) {  // nothing to gather: the plain product, where that fills the GPU better
-    bool done = false;
-    e = launch_gemm_nt_split(a.x_shards[0], a.w, a.y, a.m_local, a.n, p.k, a.fp8 ? a.scale_x_shards[0] : nullptr, a.scale_w,
-                             const_cast<uint32_t*>(comm.status), stream, &done, &comm);
-    if (e != cudaSuccess || done) return e;
-  }
   if (pairs) return tp_launch_pair<TpMode::AG_GEMM>(0, maps, comm, p, stream);
   // All CTAs take part in the copy, so the grid is the whole GPU even when
   // there are fewer tiles than SMs.
@@ -1354,17 +1381,15 @@ cudaError_t launch_allgather_gemm(const CommDev& comm, const AgGemmArgs& a, cuda
 }
 
 cudaError_t launch_gemm_reduce_scatter(const CommDev& comm, const GemmRsArgs& a, cudaStream_t stream) {
+  if (comm.nranks == 1) {  // nothing to scatter, and nothing to add up: the tiles are the result
+    if (a.m <= 0 || a.m % kBlockM != 0) return cudaErrorInvalidValue;
+    return layer_product(comm, a.h, a.w, a.out, a.m, a.n, a.k_local, a.fp8, a.scale_h, a.scale_w, nullptr, stream);
+  }
   TpMaps maps;
   TpParams p;
   const bool pairs = a.m > 0 && comm.nranks > 0 && use_pairs(a.m / comm.nranks);
   cudaError_t e = build_rs(comm, a, pairs, maps, p);
   if (e != cudaSuccess) return e;
-  if (comm.nranks == 1) {  // nothing to scatter
-    bool done = false;
-    e = launch_gemm_nt_split(a.h, a.w, a.out, a.m, a.n, p.k, a.fp8 ? a.scale_h : nullptr, a.scale_w,
-                             const_cast<uint32_t*>(comm.status), stream, &done, &comm);
-    if (e != cudaSuccess || done) return e;
-  }
   const int tiles = (a.m / kBlockM) * (a.n / kTpBN);
   if (pairs) return tp_launch_pair<TpMode::GEMM_RS>(tiles / 2, maps, comm, p, stream);
   return tp_launch<TpMode::GEMM_RS>(std::min(sm_count(), tiles), maps, comm, p, stream);

@@ -22,29 +22,34 @@ cudaError_t launch_gemm_bf16_nt(const void* a, const void* b, void* c, int m, in
 // tiles, tensor maps and pipeline are those of the bf16 kernel; only the tcgen05.mma kind differs.
 cudaError_t launch_gemm_e4m3_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                 const float* scale_b, uint32_t* status, cudaStream_t stream);
-// Common entry of the two above (k in 16-bit units, scales null = bf16).
+// Common entry of the two above (k in 16-bit units, scales null = bf16), which picks the kernel. `layer`: the
+// communicator of a fused layer on one rank, whose phase trace is stamped (start, loads issued, MMAs committed, tiles
+// stored, CTA done). `a_copy`: a second [m, k] buffer (16-byte aligned, not overlapping `a`) that receives a copy of A.
 cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                           const float* scale_b, uint32_t* status, cudaStream_t stream);
+                           const float* scale_b, uint32_t* status, cudaStream_t stream, const CommDev* layer = nullptr,
+                           void* a_copy = nullptr);
 
 // Clears the two status words that a product reports into, ahead of it on the same stream.
 cudaError_t launch_clear_status(uint32_t* status, cudaStream_t stream);
 
 // The same product where 128 x 128 tiles are too few to fill the GPU: clusters of CTAs split K and sum in
-// distributed shared memory. Sets *done when it launched; otherwise (more than kSplitMaxTiles tiles, or a plain product
-// that the persistent kernel is faster at) nothing happened and the persistent kernels are the ones to call. Argument
-// rules checked by launch_gemm_nt. `layer`: the communicator of a fused layer on one rank, whose own kernel is slower
-// at every such size (13 to 70 us against 6 to 59 over 128..4096 rows, 256..18432 columns and K of 128..8192); its
-// phase trace is stamped like that kernel's (start, loads issued, MMAs committed, tile stored, CTA done).
+// distributed shared memory. Sets *done when it launched; otherwise (more than kSplitMaxTiles tiles, or a product that
+// another kernel is faster at) nothing happened. Argument rules checked by launch_gemm_nt. `layer`, `a_copy`: as above;
+// with a copy to make this kernel is taken wherever it fits, since it passes the copy on by the way.
 constexpr int kSplitMaxTiles = 148;
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                  const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done,
-                                 const CommDev* layer = nullptr);
+                                 const CommDev* layer = nullptr, void* a_copy = nullptr);
 
 // The same product on CTA pairs (clusters of two CTAs, tcgen05 cta_group::2):
-// each pair owns a 256 x 256 tile and reads every B element once. Same
-// argument rules; any m, n % 8 == 0, k % 8 == 0.
-cudaError_t launch_gemm_bf16_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, uint32_t* status,
-                                     cudaStream_t stream);
+// each pair owns a tile of 256 rows and 256 (`narrow`: 128) columns and reads every
+// B element once. Any m, n % 8 == 0, k % 8 == 0 (in 16-bit units); scales
+// non-null = e4m3 operands. `layer`: as above.
+cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
+                                const float* scale_b, uint32_t* status, cudaStream_t stream, bool narrow = false,
+                                const CommDev* layer = nullptr);
+// Whether the narrow tiles of an m x n product are at most as many as the GPU holds pairs.
+bool pair_tiles_fit(int m, int n, bool fp8);
 
 // Column-parallel layer fused with the all-gather of its input.
 // x_shards[r] is rank r's [m_local, k] bf16 activation shard in symmetric
@@ -60,6 +65,8 @@ cudaError_t launch_gemm_bf16_nt_pair(const void* a, const void* b, void* c, int 
 // complete before it is read, and no rank returns while its shard is in use.
 struct AgGemmArgs {
   const void* x_shards[kMaxRanks];
+  // Single rank only: the activations where the caller has them, read instead of x_shards[0], which receives a copy.
+  const void* x_src;
   void* x_full;
   const void* w;
   void* y;

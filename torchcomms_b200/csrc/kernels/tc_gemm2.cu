@@ -1,10 +1,14 @@
-// bf16 GEMM on CTA pairs (tcgen05 cta_group::2). See tc_gemm.h.
+// GEMM on CTA pairs (tcgen05 cta_group::2), bf16 or e4m3. See tc_gemm.h.
 //
 // A cluster of two CTAs owns a 256 x 256 output tile. Each CTA loads its own
 // 128 rows of A and HALF of the B tile (128 of the 256 rows of B) per k-step,
 // so the pair reads every B element once instead of twice; the leader CTA
 // issues one 256 x 256 x 16 MMA for both, accumulating into the tensor memory
 // of both. The smaller per-CTA stage (32 KB) also buys a 6-deep TMA ring.
+// Tensor cores bound it: 4096 x 28672 x 4096 in e4m3 341 us (2.8 PFLOP/s before
+// the power cap sets in; tiles of 128 x 256 on single CTAs 365), 4096 x 14336 x
+// 4096 in bf16 317 (337). Tiles of 128 columns are for products whose tiles all
+// find a pair at once; a K step takes them as long, so a second wave does not pay.
 //
 // Roles per CTA (192 threads): warp 0 lane 0 TMA producer (both CTAs), warp 1
 // tensor-memory allocation (both CTAs) and MMA issue (leader only), warps 2-5
@@ -17,7 +21,9 @@
 #include "tc_gemm.h"
 
 #include <algorithm>
+#include <atomic>
 
+#include "early_launch.cuh"
 #include "launch_count.h"
 #include "tc_gemm.cuh"
 
@@ -27,15 +33,22 @@ namespace {
 
 using namespace tc;
 
-constexpr int kBN = 256;
-constexpr int kStages = 6;
-constexpr int kABytes = kBlockM * kBlockK * 2;        // 16 KB: this CTA's 128 rows of A
-constexpr int kBHalfBytes = (kBN / 2) * kBlockK * 2;  // 16 KB: this CTA's half of the B tile
-constexpr int kStageBytes = kABytes + kBHalfBytes;
+constexpr int kABytes = kBlockM * kBlockK * 2;  // 16 KB: this CTA's 128 rows of A
 constexpr int kOutChunkCols = 64;
 constexpr int kOutChunkBytes = kBlockM * kOutChunkCols * 2;
-constexpr int kSmemBytes = kStages * kStageBytes + 2 * kOutChunkBytes + 1024 + 256;
 constexpr int kThreads = 192;
+constexpr int kAccCols = 256;  // tensor-memory columns of one accumulator
+
+constexpr int kStages = 6;
+
+// Shared memory for tiles of BN columns: each CTA holds half of the B tile. (Eight stages, which tiles of 128 columns
+// leave room for, gain nothing: 512 x 4096 x 4096 in e4m3 15.1 us either way.)
+template <int BN>
+struct PairTile {
+  static constexpr int kBHalfBytes = (BN / 2) * kBlockK * 2;
+  static constexpr int kStageBytes = kABytes + kBHalfBytes;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 2 * kOutChunkBytes + 1024 + 256;
+};
 
 struct PairBarriers {
   uint64_t full[8];
@@ -48,8 +61,16 @@ struct PairBarriers {
 
 struct PairMaps {
   CUtensorMap a;    // box 128 rows x 64 columns
-  CUtensorMap b;    // box 128 rows x 64 columns (half of the 256-row B tile)
+  CUtensorMap b;    // box BN / 2 rows x 64 columns (half of the B tile)
   CUtensorMap out;  // box 128 rows x 64 columns
+};
+
+struct PairParams {
+  uint32_t* status;
+  const float* scale_a;  // e4m3: per row of A, per row of B
+  const float* scale_b;
+  long long* trace;
+  int m, n, k, gm;  // k in 16-bit units
 };
 
 // Pair-tile `t` of the schedule: groups of `gm` 256-row tiles, n-major inside a group.
@@ -63,9 +84,10 @@ __device__ __forceinline__ void pair_tile_at(int t, int tiles_m, int tiles_n, in
   *pn = rem / gsz;
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
-    k_gemm_pair(const __grid_constant__ PairMaps maps, int m, int n, int k, int gm, uint32_t* status) {
-  constexpr uint32_t idesc = make_idesc_bf16(2 * kBlockM, kBN);
+template <bool FP8, int BN>
+__global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant__ PairMaps maps, PairParams p) {
+  constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(2 * kBlockM, BN) : make_idesc_bf16(2 * kBlockM, BN);
+  constexpr int kStageBytes = PairTile<BN>::kStageBytes;
   extern __shared__ char smem_raw[];
   // The carve-up must be identical in both CTAs (the MMA addresses both with one descriptor).
   char* stages = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -75,9 +97,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t cta = cluster_ctarank();  // 0 leads
   const bool leader = cta == 0;
   const int cluster_id = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
-  const int tiles_m = (m + 2 * kBlockM - 1) / (2 * kBlockM), tiles_n = (n + kBN - 1) / kBN;
+  const int tiles_m = (p.m + 2 * kBlockM - 1) / (2 * kBlockM), tiles_n = (p.n + BN - 1) / BN;
   const int total_tiles = tiles_m * tiles_n;
-  const int k_iters = (k + kBlockK - 1) / kBlockK;
+  const int k_iters = (p.k + kBlockK - 1) / kBlockK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -92,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc_pair(&bars->tmem_base, 2 * kBN);
+    tmem_alloc_pair(&bars->tmem_base, 2 * kAccCols);
     tmem_relinquish_pair();
   }
   tc_fence_before_sync();
@@ -100,6 +122,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   cluster_sync_all();  // both CTAs' barriers exist before anybody signals across
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  grid_release();
+  grid_wait();  // everything above may run while the kernel in front still does
+  if (threadIdx.x == 0) trace_stamp_ns(p.trace, 0);
 
   if (warp == 0) {
     // ---------------- TMA producer (each CTA loads its own A rows and its half of B)
@@ -107,9 +132,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t it = 0;
       for (int t = cluster_id; t < total_tiles && !bars->failed; t += nclusters) {
         int pm, pn;
-        pair_tile_at(t, tiles_m, tiles_n, gm, &pm, &pn);
+        pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
         const int a_row = (pm * 2 + static_cast<int>(cta)) * kBlockM;
-        const int b_row = pn * kBN + static_cast<int>(cta) * (kBN / 2);
+        const int b_row = pn * BN + static_cast<int>(cta) * (BN / 2);
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
@@ -124,6 +149,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           tma_load_2d_pair(sa + kABytes, &maps.b, &bars->full[s], kb * kBlockK, b_row);
         }
       }
+      trace_stamp_ns(p.trace, 1);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only)
@@ -136,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         tc_fence_after_sync();
-        const uint32_t tmem_acc = tmem_base + as * kBN;
+        const uint32_t tmem_acc = tmem_base + as * kAccCols;
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
@@ -149,13 +175,19 @@ __global__ void __launch_bounds__(kThreads, 1)
           const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + kABytes);
 #pragma unroll
           for (int kk = 0; kk < kBlockK / kUmmaK; ++kk) {
-            umma_bf16_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), idesc, (kb | kk) != 0);
+            // 16 bf16 (or 32 e4m3) = 32 bytes further along K inside the swizzled row
+            if (FP8) {
+              umma_f8_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), idesc, (kb | kk) != 0);
+            } else {
+              umma_bf16_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), idesc, (kb | kk) != 0);
+            }
           }
           umma_commit_pair(&bars->empty[s], 3);  // both CTAs may refill the stage
         }
         umma_commit_pair(&bars->acc_full[as], 3);  // both CTAs' epilogues may read
       }
     }
+    if (lane == 0) trace_stamp_ns(p.trace, 2);
   } else {
     // ---------------- epilogue (both CTAs, own 128 rows)
     const int q = warp & 3;
@@ -165,24 +197,26 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int t = cluster_id; t < total_tiles; t += nclusters, ++tile_iter) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
       int pm, pn;
-      pair_tile_at(t, tiles_m, tiles_n, gm, &pm, &pn);
+      pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
       if (!mbar_wait(&bars->acc_full[as], aph)) {
         bars->failed = 1;
         break;
       }
       tc_fence_after_sync();
       const int out_row = (pm * 2 + static_cast<int>(cta)) * kBlockM;
-      for (int j = 0; j < kBN / kOutChunkCols; ++j, ++chunk_iter) {
+      const float row_scale = FP8 && out_row + row_in_tile < p.m ? p.scale_a[out_row + row_in_tile] : 0.0f;
+      for (int j = 0; j < BN / kOutChunkCols; ++j, ++chunk_iter) {
         char* buf = obuf + (chunk_iter & 1u) * kOutChunkBytes;
         if (issuer) tma_store_wait_read<1>();
         asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           uint32_t r[32];
-          tmem_ld_32x32(tmem_base + as * kBN + (static_cast<uint32_t>(q * 32) << 16) +
+          tmem_ld_32x32(tmem_base + as * kAccCols + (static_cast<uint32_t>(q * 32) << 16) +
                             static_cast<uint32_t>(j * kOutChunkCols + half * 32),
                         r);
           tmem_ld_wait();
+          if (FP8) scale_acc32(r, row_scale, p.scale_b, pn * BN + j * kOutChunkCols + half * 32, p.n);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             const int chunk16 = half * 4 + v;
@@ -191,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                               pack_bf16(r[8 * v + 4], r[8 * v + 5]), pack_bf16(r[8 * v + 6], r[8 * v + 7]));
           }
         }
-        if (j == kBN / kOutChunkCols - 1) {
+        if (j == BN / kOutChunkCols - 1) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive_leader(&bars->acc_empty[as]);
@@ -199,62 +233,114 @@ __global__ void __launch_bounds__(kThreads, 1)
         fence_proxy_async_smem();
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (issuer) {
-          if (out_row < m && pn * kBN + j * kOutChunkCols < n) tma_store_2d(&maps.out, buf, pn * kBN + j * kOutChunkCols, out_row);
+          if (out_row < p.m && pn * BN + j * kOutChunkCols < p.n) tma_store_2d(&maps.out, buf, pn * BN + j * kOutChunkCols, out_row);
           // Nothing to store outside the matrix, but an empty group all the same: the wait above counts groups.
           tma_store_commit();
         }
       }
     }
-    if (issuer) tma_store_wait_all<0>();
+    if (issuer) {
+      tma_store_wait_all<0>();
+      trace_stamp_ns(p.trace, 3);
+    }
   }
 
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();  // the peer may still be reading this CTA's shared memory / signalling its barriers
   if (warp == 1) {
-    tmem_dealloc_pair(tmem_base, 2 * kBN);
+    tmem_dealloc_pair(tmem_base, 2 * kAccCols);
   }
-  if (threadIdx.x == 0 && bars->failed && status != nullptr) status[0] = status[0] | kStatusTimeout;
+  if (threadIdx.x == 0 && bars->failed && p.status != nullptr) p.status[0] = p.status[0] | kStatusTimeout;
+  if (threadIdx.x == 0) trace_stamp_ns(p.trace, 7);
 }
 
-} // namespace
+constexpr int kDevices = 64;  // whose answers are kept
 
-cudaError_t launch_gemm_bf16_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, uint32_t* status,
-                                     cudaStream_t stream) {
-  if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || n % 8 != 0) return cudaErrorInvalidValue;
-  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) {
-    return cudaErrorInvalidValue;
-  }
-  PairMaps maps;
-  if (!make_map(&maps.a, a, m, k, kBlockM) || !make_map(&maps.b, b, n, k, kBlockM) || !make_map(&maps.out, c, m, n, kBlockM)) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-  if (e != cudaSuccess) return e;
-  const int tiles_m = (m + 2 * kBlockM - 1) / (2 * kBlockM), tiles_n = (n + kBN - 1) / kBN;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = stream;
+// Pairs that the current GPU holds at once (each CTA fills an SM), or 0 after an error. Kept per device; a query that
+// failed is asked again at the next call.
+template <bool FP8, int BN>
+int resident_pairs() {
+  static std::atomic<int> known[kDevices];
+  int device = 0, n = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return 0;
+  std::atomic<int>* kept = device >= 0 && device < kDevices ? &known[device] : nullptr;
+  if (kept != nullptr) n = kept->load(std::memory_order_acquire);
+  if (n > 0) return n;
+  if (cudaFuncSetAttribute(k_gemm_pair<FP8, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairTile<BN>::kSmemBytes) != cudaSuccess) return 0;
   cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = PairTile<BN>::kSmemBytes;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  // As many pairs as the device can hold at once (each CTA fills an SM).
-  int max_clusters = 0;
-  cfg.gridDim = dim3(2);
-  e = cudaOccupancyMaxActiveClusters(&max_clusters, k_gemm_pair, &cfg);
-  if (e != cudaSuccess) return e;
-  if (max_clusters < 1) return cudaErrorInvalidConfiguration;
-  const int clusters = std::min(max_clusters, tiles_m * tiles_n);
-  cfg.gridDim = dim3(2 * clusters);
+  if (cudaOccupancyMaxActiveClusters(&n, k_gemm_pair<FP8, BN>, &cfg) != cudaSuccess || n < 1) return 0;
+  if (kept != nullptr) kept->store(n, std::memory_order_release);
+  return n;
+}
+
+template <bool FP8, int BN>
+cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cudaStream_t stream) {
+  const int pairs = resident_pairs<FP8, BN>();
+  if (pairs < 1) {
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+  }
+  PairMaps maps;
+  if (!make_map(&maps.a, a, p.m, p.k, kBlockM) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.out, c, p.m, p.n, kBlockM)) {
+    return cudaErrorInvalidValue;
+  }
+  const int tiles_m = (p.m + 2 * kBlockM - 1) / (2 * kBlockM), tiles_n = (p.n + BN - 1) / BN;
   // A rows of a group stay in L2 while the pairs sweep over n: at most 8 pair-tiles and ~40 MB.
-  const size_t a_tile_bytes = static_cast<size_t>(2 * kBlockM) * k * 2;
-  const int gm = std::max(1, std::min({8, tiles_m, static_cast<int>((40u << 20) / std::max<size_t>(a_tile_bytes, 1))}));
-  e = cudaLaunchKernelEx(&cfg, k_gemm_pair, maps, m, n, k, gm, status);
+  const size_t a_tile_bytes = static_cast<size_t>(2 * kBlockM) * p.k * 2;
+  p.gm = std::max(1, std::min({8, tiles_m, static_cast<int>((40u << 20) / std::max<size_t>(a_tile_bytes, 1))}));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(pairs, static_cast<int64_t>(tiles_m) * tiles_n)));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = PairTile<BN>::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gemm_pair<FP8, BN>, maps, p);
   note_kernel_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+} // namespace
+
+bool pair_tiles_fit(int m, int n, bool fp8) {
+  const int pairs = fp8 ? resident_pairs<true, 128>() : resident_pairs<false, 128>();
+  return static_cast<int64_t>((m + 2 * kBlockM - 1) / (2 * kBlockM)) * ((n + 127) / 128) <= pairs;
+}
+
+cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
+                                const float* scale_b, uint32_t* status, cudaStream_t stream, bool narrow, const CommDev* layer) {
+  if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || n % 8 != 0) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) {
+    return cudaErrorInvalidValue;
+  }
+  PairParams p{};
+  p.status = status;
+  p.scale_a = scale_a;
+  p.scale_b = scale_b;
+  p.trace = layer != nullptr ? layer->trace : nullptr;
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  if (narrow) return scale_a != nullptr ? launch_pair<true, 128>(a, b, c, p, stream) : launch_pair<false, 128>(a, b, c, p, stream);
+  return scale_a != nullptr ? launch_pair<true, 256>(a, b, c, p, stream) : launch_pair<false, 256>(a, b, c, p, stream);
 }
 
 } // namespace b200c

@@ -52,6 +52,7 @@ struct SplitBarriers {
 
 struct SplitMaps {
   CUtensorMap a, b;
+  CUtensorMap a_copy;  // where the operand A is also wanted (p.copy_a), laid out as A
 };
 
 struct SplitParams {
@@ -61,6 +62,7 @@ struct SplitParams {
   const float* scale_b;
   long long* trace;
   int m, n, k, k_iters, tiles_m;  // k in 16-bit units
+  int copy_a;
 };
 
 __device__ __forceinline__ uint32_t cluster_nctarank() {
@@ -93,10 +95,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   const int kb0 = static_cast<int>(static_cast<int64_t>(p.k_iters) * part / splits);
   const int kb1 = static_cast<int>(static_cast<int64_t>(p.k_iters) * (part + 1) / splits);
 
+  // The first column of tiles passes its stages of A on (see warp 2 below).
+  const bool copies = p.copy_a != 0 && ni == 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kSplitStages; ++s) {
       mbar_init(&bars->full[s], 1);
-      mbar_init(&bars->empty[s], 1);
+      mbar_init(&bars->empty[s], copies ? 2 : 1);
     }
     mbar_init(&bars->acc_full, 1);
     bars->failed = 0;
@@ -158,6 +162,21 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   } else {
     // The accumulator is complete, so every stage has been read: the partial tile may overwrite them.
     const int q = warp & 3, row = q * 32 + lane;
+    if (copies && warp == 2 && lane == 0) {
+      for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
+        const int s = it % kSplitStages;
+        if (!mbar_wait(&bars->full[s], (it / kSplitStages) & 1u)) {
+          bars->failed = 1;
+          break;
+        }
+        tma_store_2d(&maps.a_copy, stages + s * kSplitStageBytes, kb * kBlockK, mi * kBlockM);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(&bars->empty[s]);
+      }
+      tma_store_wait_all<0>();
+    }
+    __syncwarp();
     float* mine = reinterpret_cast<float*>(stages) + row * kSplitPitch;
     if (mbar_wait(&bars->acc_full, 0)) {
       tc_fence_after_sync();
@@ -278,29 +297,25 @@ int resident_clusters(int device, int splits) {
   return n;
 }
 
-// Whether the split kernel beats the persistent one (tiles of 128 x 256) on a plain product; `k` in 16-bit units. Meeting
-// the cluster and adding up the shares costs it 1 us more than the direct stores of a full tile, less where the tile has
-// few rows; a K step is 0.28 us of the persistent kernel's time and 0.2 us of this one's, over the CTAs that share K.
-// Rows that do not start on 128-byte lines make every step longer, most where few CTAs load. Replayed from a graph,
-// persistent / split in us (bf16 unless e4m3 is said):
-//   few rows, up to 32 or, in e4m3, 64: 1 x 2048 x 512 7.4 / 6.1, 32 x 2048 x 512 7.5 / 6.9; e4m3 48 x 2048 x 256
-//   7.7 / 6.8, 64 x 2048 x 256 7.8 / 7.4
-//   K shared, line at 12 steps of 64, in e4m3 (of 128) or off the lines at 8: 128 x 2048 x 512 7.7 / 8.4, x 768
-//   8.9 / 8.8, x 1536 12.2 / 11.3; e4m3 128 x 2048 x 768 8.6 / 10.1, x 1024 9.2 / 8.9
-//   K not shared: half the tile on twice the SMs pays later, the more row tiles read the same weights again:
-//   128 x 14336 x 768 9.6 / 10.7, x 1024 12.1 / 12.5, x 2048 20.4 / 18.3; 256 x 9216 x 2560 22.1 / 19.7;
-//   2048 x 1024 x 3072 18.8 / 22.6, x 4096 23.7 / 26.3, x 6144 38.3 / 35.6; off the lines from 12 steps on, 0.9 to 1.1
-//   times as fast at 10..15, 1.0 to 1.3 from 29 on
-bool split_pays(int m, int tiles_m, int k, bool fp8, bool shares_k) {
-  if (m <= (fp8 ? 64 : 32)) return true;
-  const bool on_lines = k % kBlockK == 0;
-  const int k_iters = (k + kBlockK - 1) / kBlockK;
-  if (shares_k) return k_iters >= (fp8 || !on_lines ? 8 : 12);
-  return k_iters >= (!on_lines ? 12 : tiles_m == 1 ? 16 : tiles_m == 2 ? 40 : tiles_m <= 8 ? 64 : 80);
+// Whether the split kernel beats the others (tc_gemm.cu has their rule); `k` in 16-bit units. Meeting the cluster and
+// adding up the shares costs it 2 us more than the direct stores of a full tile, less where the tile has few rows; a K
+// step of 64 units is 0.27 us of the others' time and 0.2 us of this one's, over the CTAs that share K.
+// Replayed from a graph, best of the others / split in us (bf16 unless e4m3 is said):
+//   few rows: 1 x 256 x 256 4.2 / 3.8, 32 x 2560 x 256 4.5 / 4.5, e4m3 1 x 14336 x 256 6.6 / 4.4; up to 64, line at 6
+//   steps: 64 x 6144 x 256 5.0 / 5.2, 64 x 2560 x 1024 8.1 / 6.6, e4m3 64 x 2560 x 256 5.0 / 5.4, 64 x 1024 x 1024 6.7 / 5.8
+//   K shared, line at 10 steps: e4m3 128 x 4096 x 1024 (8) 6.9 / 7.2, x 2048 (16) 9.3 / 8.5; 384 x 1024 x 1024 (16)
+//   8.2 / 8.4, 512 x 1024 x 2048 (32) 12.8 / 10.1; e4m3 1536 x 256 x 8192 (64) 23.0 / 12.0
+//   K not shared: half the tile on twice the SMs is worth it only where narrow pair tiles would need a second wave, from
+//   20 steps on: e4m3 128 x 14336 x 4096 (32) 19.9 / 18.7; 192 x 8192 x 4096, one wave of pairs, 15.9 / 17.6
+bool split_pays(int m, int n, int k_iters, bool fp8, bool shares_k) {
+  if (m <= 32) return true;
+  if (m <= 64) return k_iters >= 6;
+  if (shares_k) return k_iters >= 10;
+  return k_iters >= 20 && !pair_tiles_fit(m, n, fp8);
 }
 
 template <bool FP8>
-cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles, bool plain, cudaStream_t stream, bool* done) {
+cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles, cudaStream_t stream, bool* done) {
   // The untraced kernel is the one that resident_clusters asks about: one CTA per SM, as the traced one. Its attribute
   // stays with the device and is set once.
   static std::atomic<bool> ready[kDevices];
@@ -323,7 +338,7 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
     if (resident_clusters<FP8>(device, s) >= tiles) splits = s;
   }
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
-  if (plain && !split_pays(p.m, p.tiles_m, p.k, FP8, splits > 1)) return cudaSuccess;
+  if (p.copy_a == 0 && !split_pays(p.m, p.n, p.k_iters, FP8, splits > 1)) return cudaSuccess;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
   e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
@@ -341,13 +356,17 @@ cudaError_t launch_clear_status(uint32_t* status, cudaStream_t stream) {
 }
 
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                                 const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done, const CommDev* layer) {
+                                 const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done, const CommDev* layer,
+                                 void* a_copy) {
   *done = false;
   const int64_t tiles_m = (static_cast<int64_t>(m) + kBlockM - 1) / kBlockM, tiles_n = (static_cast<int64_t>(n) + kSplitBN - 1) / kSplitBN;
   if (tiles_m * tiles_n > kSplitMaxTiles) return cudaSuccess;
   SplitMaps maps;
   if (!make_map(&maps.a, a, m, k, kBlockM) || !make_map(&maps.b, b, n, k, kSplitBN)) return cudaErrorInvalidValue;
+  maps.a_copy = maps.a;
+  if (a_copy != nullptr && !make_map(&maps.a_copy, a_copy, m, k, kBlockM)) return cudaErrorInvalidValue;
   SplitParams p{};
+  p.copy_a = a_copy != nullptr ? 1 : 0;
   p.c = static_cast<__nv_bfloat16*>(c);
   p.status = status;
   p.trace = layer != nullptr ? layer->trace : nullptr;
@@ -359,9 +378,7 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   p.k_iters = (k + kBlockK - 1) / kBlockK;
   p.tiles_m = static_cast<int>(tiles_m);
   const int tiles = static_cast<int>(tiles_m * tiles_n);
-  const bool plain = layer == nullptr;
-  return scale_a != nullptr ? launch_split<true>(maps, p, tiles, plain, stream, done)
-                            : launch_split<false>(maps, p, tiles, plain, stream, done);
+  return scale_a != nullptr ? launch_split<true>(maps, p, tiles, stream, done) : launch_split<false>(maps, p, tiles, stream, done);
 }
 
 } // namespace b200c

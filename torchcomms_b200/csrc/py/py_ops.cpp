@@ -494,9 +494,9 @@ void bind_ops(py::module_& m) {
     c10::cuda::CUDAGuard g(a.device());
     at::Tensor c = at::empty({a.size(0), b.size(0)}, a.options());
     at::Tensor status = cleared_status(a);
-    B200C_CUDA_CHECK(launch_gemm_bf16_nt_pair(a.data_ptr(), b.data_ptr(), c.data_ptr(), static_cast<int>(a.size(0)),
-                                              static_cast<int>(b.size(0)), static_cast<int>(a.size(1)),
-                                              reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
+    B200C_CUDA_CHECK(launch_gemm_nt_pair(a.data_ptr(), b.data_ptr(), c.data_ptr(), static_cast<int>(a.size(0)),
+                                         static_cast<int>(b.size(0)), static_cast<int>(a.size(1)), nullptr, nullptr,
+                                         reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
     return std::make_pair(c, status);
   });
 
