@@ -10,6 +10,7 @@
 #include "../backends/cuda_backend.hpp"
 #include "../cuda/driver_api.hpp"
 #include "../kernels/tc_gemm.h"
+#include "plain_call.hpp"
 
 namespace b200c {
 
@@ -130,8 +131,15 @@ class TpLayer {
     return at::from_blob(bases_[rank_] + data_bytes_, {rows_}, opts);
   }
 
-  // ag_gemm: y[nranks*m_local, n] = all_gather(input()) @ w[n, k]^T
-  at::Tensor ag_gemm(const at::Tensor& w, const c10::optional<at::Tensor>& scale_w) {
+  // Whether ag_gemm() takes `x` from where it is: a single rank's kernel reads it there and leaves the copy in input().
+  bool reads_in_place(const at::Tensor& x) const {
+    return nranks_ == 1 && ag_ && !fp8_ && plain_call(x, true) && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() == 2 &&
+        x.size(0) == rows_ && x.size(1) == cols_ && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0 &&
+        x.data_ptr() != static_cast<void*>(bases_[rank_]);
+  }
+
+  // ag_gemm: y[nranks*m_local, n] = all_gather(input()) @ w[n, k]^T; `x`: goes to input() first.
+  at::Tensor ag_gemm(const at::Tensor& w, const c10::optional<at::Tensor>& scale_w, const c10::optional<at::Tensor>& x) {
     TORCH_CHECK(ag_, "not an ag_gemm layer");
     TORCH_CHECK(w.is_cuda() && w.is_contiguous() && w.scalar_type() == (fp8_ ? at::kFloat8_e4m3fn : at::kBFloat16) &&
                     w.dim() == 2 && w.size(1) == cols_,
@@ -141,8 +149,11 @@ class TpLayer {
                           scale_w->is_contiguous() && scale_w->numel() == w.size(0)),
                 "fp8: scale_w must be contiguous fp32 [n]");
     c10::cuda::CUDAGuard g(w.device());
+    const bool in_place = x.has_value() && reads_in_place(*x) && x->device() == w.device();
+    if (x.has_value() && !in_place) input().copy_(*x);
     at::Tensor y = at::empty({static_cast<int64_t>(rows_) * nranks_, w.size(0)}, w.options().dtype(at::kBFloat16));
     AgGemmArgs a{};
+    if (in_place) a.x_src = x->data_ptr();
     if (fp8_) {
       a.fp8 = 1;
       for (int p = 0; p < nranks_; ++p) a.scale_x_shards[p] = reinterpret_cast<const float*>(bases_[p] + data_bytes_);
@@ -159,6 +170,7 @@ class TpLayer {
     a.ctrl = ctrl_;
     std::vector<at::Tensor> keep{w, y};
     if (fp8_) keep.push_back(*scale_w);
+    if (in_place) keep.push_back(*x);
     launch([&](const CommDev& c, cudaStream_t s) { B200C_CUDA_CHECK(launch_allgather_gemm(c, a, s)); },
            fp8_ ? "ag_gemm_fp8/kernel" : "ag_gemm/kernel", keep);
     return y;
@@ -432,7 +444,8 @@ void bind_tp(py::module_& m) {
            py::arg("fp8") = false)
       .def("input", &TpLayer::input)
       .def("input_scales", &TpLayer::input_scales)
-      .def("ag_gemm", &TpLayer::ag_gemm, py::arg("w"), py::arg("scale_w") = py::none(), py::call_guard<py::gil_scoped_release>())
+      .def("ag_gemm", &TpLayer::ag_gemm, py::arg("w"), py::arg("scale_w") = py::none(), py::arg("x") = py::none(),
+           py::call_guard<py::gil_scoped_release>())
       .def("gemm_rs", &TpLayer::gemm_rs, py::arg("h"), py::arg("w"), py::arg("scale_h") = py::none(),
            py::arg("scale_w") = py::none(), py::call_guard<py::gil_scoped_release>())
       .def("status", &TpLayer::status);

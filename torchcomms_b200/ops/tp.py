@@ -84,6 +84,8 @@ class AllGatherGemm:
     def __call__(self, w: torch.Tensor, x_shard: Optional[torch.Tensor] = None, scale_w: Optional[torch.Tensor] = None,
                  scale_x: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``fp8``: ``w`` e4m3 with ``scale_w [n]``; ``x_shard`` e4m3 with ``scale_x [m_local]``, or bf16 (quantised here)."""
+        if x_shard is not None and not self.fp8 and type(x_shard) is torch.Tensor:
+            return self._layer.ag_gemm(w, scale_w, x_shard)  # goes to ``input`` on the way
         if x_shard is not None:
             quantise = self.fp8 and x_shard.dtype != torch.float8_e4m3fn
             # bf16 rows are quantised straight into the peer-readable buffers where the kernel takes them.
