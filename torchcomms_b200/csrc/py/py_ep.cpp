@@ -22,6 +22,7 @@ class EpBuffer {
   // Real: one rank per process, memory from the communicator's symmetric allocator.
   EpBuffer(std::shared_ptr<CudaBackend> backend, int max_tokens, int hidden, int num_experts, int topk, bool fp8)
       : backend_(std::move(backend)), n_local_(1) {
+    device_ = backend_->device().index();
     setup_dims(backend_->size(), max_tokens, hidden, num_experts, topk, fp8);
     c10::cuda::CUDAGuard g(backend_->device());
     seg_ = backend_->symm().allocate(total_, false);
@@ -34,6 +35,7 @@ class EpBuffer {
   // Emulation: `nranks` virtual ranks on the current device (kernel tests).
   EpBuffer(int nranks, int max_tokens, int hidden, int num_experts, int topk, bool fp8, double wait_ms)
       : n_local_(nranks) {
+    device_ = at::cuda::current_device();
     setup_dims(nranks, max_tokens, hidden, num_experts, topk, fp8);
     const size_t flag_bytes = static_cast<size_t>(kFlagSets) * kMaxBlocks * kMaxRanks * sizeof(uint32_t);
     std::vector<char*> bases(nranks);
@@ -221,28 +223,41 @@ class EpBuffer {
     TORCH_CHECK(i >= 0 && i < n_local_, "bad local rank");
     const EpDev& e = eps_[i];
     const int r = e.rank;
-    auto opts = at::TensorOptions().device(at::kCUDA, at::cuda::current_device());
     const int64_t R = rows();
-    if (what == "recv_x") {
-      return fp8_ ? at::from_blob(e.recv_x[r], {R, hidden_}, opts.dtype(at::kFloat8_e4m3fn))
-                  : at::from_blob(e.recv_x[r], {R, hidden_}, opts.dtype(at::kBFloat16));
-    }
-    if (what == "recv_scales") return at::from_blob(e.recv_scales[r], {R, hidden_ / 128}, opts.dtype(at::kFloat));
-    if (what == "recv_src") return at::from_blob(e.recv_src[r], {R}, opts.dtype(at::kInt));
-    if (what == "recv_topk_idx") return at::from_blob(e.recv_topk_idx[r], {R, topk_}, opts.dtype(at::kInt));
-    if (what == "recv_topk_weights") return at::from_blob(e.recv_topk_w[r], {R, topk_}, opts.dtype(at::kFloat));
-    if (what == "combine_x") return at::from_blob(e.combine_x[r], {R, hidden_}, opts.dtype(at::kBFloat16));
-    if (what == "stage_x") return at::from_blob(e.stage_x[r], {max_tokens_, hidden_}, opts.dtype(at::kBFloat16));
-    if (what == "combine_topk_weights") return at::from_blob(e.comb_topk_w[r], {R, topk_}, opts.dtype(at::kFloat));
-    if (what == "recv_info") return at::from_blob(e.recv_info, {1 + nranks_}, opts.dtype(at::kInt));
-    if (what == "send_slot") return at::from_blob(e.send_slot, {max_tokens_, nranks_}, opts.dtype(at::kInt));
+    if (what == "recv_x") return over(e.recv_x[r], {R, hidden_}, fp8_ ? at::kFloat8_e4m3fn : at::kBFloat16);
+    if (what == "recv_scales") return over(e.recv_scales[r], {R, hidden_ / 128}, at::kFloat);
+    if (what == "recv_src") return over(e.recv_src[r], {R}, at::kInt);
+    if (what == "recv_topk_idx") return over(e.recv_topk_idx[r], {R, topk_}, at::kInt);
+    if (what == "recv_topk_weights") return over(e.recv_topk_w[r], {R, topk_}, at::kFloat);
+    if (what == "combine_x") return over(e.combine_x[r], {R, hidden_}, at::kBFloat16);
+    if (what == "stage_x") return over(e.stage_x[r], {max_tokens_, hidden_}, at::kBFloat16);
+    if (what == "combine_topk_weights") return over(e.comb_topk_w[r], {R, topk_}, at::kFloat);
+    if (what == "recv_info") return over(e.recv_info, {1 + nranks_}, at::kInt);
+    if (what == "send_slot") return over(e.send_slot, {max_tokens_, nranks_}, at::kInt);
     TORCH_CHECK(false, "unknown view '", what, "'");
+  }
+  // What a dispatch leaves at its receiver, in one call: rows, their scales (e4m3 only), expert ids and weights, sources,
+  // the number of rows (0-d) and the rows per source rank.
+  std::tuple<at::Tensor, std::optional<at::Tensor>, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor> received() {
+    const EpDev& e = eps_[0];
+    const int r = e.rank;
+    const int64_t R = rows();
+    std::optional<at::Tensor> scales;
+    if (fp8_) scales = over(e.recv_scales[r], {R, hidden_ / 128}, at::kFloat);
+    return {over(e.recv_x[r], {R, hidden_}, fp8_ ? at::kFloat8_e4m3fn : at::kBFloat16), std::move(scales),
+            over(e.recv_topk_idx[r], {R, topk_}, at::kInt), over(e.recv_topk_w[r], {R, topk_}, at::kFloat), over(e.recv_src[r], {R}, at::kInt),
+            over(e.recv_info, {}, at::kInt), over(e.recv_info + 1, {nranks_}, at::kInt)};
   }
   std::vector<uint32_t> status() const {
     return status_host_ ? std::vector<uint32_t>(status_host_, status_host_ + 5) : std::vector<uint32_t>{};
   }
 
  private:
+  // The device is known: left to find it out, the tensor library asks the driver about every pointer.
+  at::Tensor over(void* p, at::IntArrayRef sizes, at::ScalarType type) const {
+    const at::Device dev(at::kCUDA, device_);
+    return at::for_blob(p, sizes).options(at::TensorOptions().device(dev).dtype(type)).target_device(dev).make_tensor();
+  }
   void setup_dims(int nranks, int max_tokens, int hidden, int num_experts, int topk, bool fp8) {
     TORCH_CHECK(hidden % 512 == 0, "hidden must be a multiple of 512");
     TORCH_CHECK(num_experts % nranks == 0, "num_experts must divide by the number of ranks");
@@ -315,6 +330,7 @@ class EpBuffer {
   std::shared_ptr<CudaBackend> backend_;
   std::shared_ptr<SymmSegment> seg_;
   int n_local_;
+  c10::DeviceIndex device_ = 0;
   int nranks_ = 1, max_tokens_ = 0, hidden_ = 0, num_experts_ = 0, topk_ = 0;
   bool fp8_ = true;
   size_t off_x_ = 0, off_scales_ = 0, off_src_ = 0, off_idx_ = 0, off_w_ = 0, off_count_ = 0, off_combine_ = 0, off_stage_ = 0, off_comb_w_ = 0, total_ = 0;
@@ -348,6 +364,7 @@ void bind_ep(py::module_& m) {
       .def("pull", &EpBuffer::pull, py::arg("out"), py::arg("recv_src") = std::vector<at::Tensor>{},
            py::arg("num_rows") = std::vector<at::Tensor>{})
       .def("view", &EpBuffer::view, py::arg("local_rank"), py::arg("what"))
+      .def("received", &EpBuffer::received)
       .def("rows", &EpBuffer::rows)
       .def("status", &EpBuffer::status);
 

@@ -22,6 +22,7 @@ class EpLlBuffer {
  public:
   EpLlBuffer(std::shared_ptr<CudaBackend> backend, int max_tokens, int hidden, int num_experts, int topk, bool fp8)
       : backend_(std::move(backend)), n_local_(1) {
+    device_ = backend_->device().index();
     setup_dims(backend_->size(), max_tokens, hidden, num_experts, topk, fp8);
     c10::cuda::CUDAGuard g(backend_->device());
     // Zero-filled on every rank before anybody returns: the count tables read "no call yet".
@@ -35,6 +36,7 @@ class EpLlBuffer {
   // Emulation: `nranks` virtual ranks on the current device (kernel tests).
   EpLlBuffer(int nranks, int max_tokens, int hidden, int num_experts, int topk, bool fp8, double wait_ms)
       : n_local_(nranks) {
+    device_ = at::cuda::current_device();
     setup_dims(nranks, max_tokens, hidden, num_experts, topk, fp8);
     const size_t flag_bytes = static_cast<size_t>(kFlagSets) * kMaxBlocks * kMaxRanks * sizeof(uint32_t);
     std::vector<char*> bases(nranks);
@@ -109,14 +111,24 @@ class EpLlBuffer {
       auto opts = x[i].options();
       at::Tensor px = at::empty({Le, R, hidden_}, opts.dtype(fp8_ ? at::kFloat8_e4m3fn : at::kBFloat16));
       at::Tensor ps = fp8_ ? at::empty({Le, R, hidden_ / 128}, opts.dtype(at::kFloat)) : at::Tensor();
-      at::Tensor src = at::empty({Le, R}, opts.dtype(at::kInt));
-      at::Tensor count = at::empty({Le}, opts.dtype(at::kInt));
-      at::Tensor range = at::empty({Le, nranks_}, opts.dtype(at::kLong));
+      // The small outputs come out of one allocation: each costs as much host time as the dispatch kernel runs for.
+      int64_t bytes = 0;
+      auto take = [&bytes](int64_t n) {
+        const int64_t at = bytes;
+        bytes += static_cast<int64_t>(align256(static_cast<size_t>(n)));
+        return at;
+      };
+      const int64_t at_src = take(Le * R * 4), at_count = take(Le * 4), at_range = take(Le * nranks_ * 8);
+      const int64_t at_slot = take(handles ? static_cast<int64_t>(T) * topk_ * 4 : 0), at_begin = take(handles ? num_experts_ * 4 : 0);
+      const at::Tensor block = at::empty({bytes}, opts.dtype(at::kByte));
+      at::Tensor src = piece(block, at_src, {Le, R}, at::kInt);
+      at::Tensor count = piece(block, at_count, {Le}, at::kInt);
+      at::Tensor range = piece(block, at_range, {Le, nranks_}, at::kLong);
       recv[i] = {px.data_ptr(), fp8_ ? ps.data_ptr<float>() : nullptr, src.data_ptr<int>(), count.data_ptr<int>(),
                  reinterpret_cast<long long*>(range.data_ptr<int64_t>()), nullptr, nullptr};
       outs[i] = {px, ps, src, count, range};
       if (handles) {
-        at::Tensor slot = at::empty({T, topk_}, opts.dtype(at::kInt)), begin = at::empty({num_experts_}, opts.dtype(at::kInt));
+        at::Tensor slot = piece(block, at_slot, {T, topk_}, at::kInt), begin = piece(block, at_begin, {num_experts_}, at::kInt);
         recv[i].send_slot = slot.data_ptr<int>();
         recv[i].begin = begin.data_ptr<int>();
         outs[i].insert(outs[i].end(), {slot, begin});
@@ -193,12 +205,9 @@ class EpLlBuffer {
   at::Tensor view(int i, const std::string& what) {
     TORCH_CHECK(i >= 0 && i < n_local_, "bad local rank");
     const EpLlDev& e = eps_[i];
-    auto opts = at::TensorOptions().device(at::kCUDA, at::cuda::current_device());
-    if (what == "out_x") {
-      return at::from_blob(e.out_x[e.rank], {local_experts(), rows_per_expert(), hidden_}, opts.dtype(at::kBFloat16));
-    }
-    if (what == "send_slot") return at::from_blob(e.send_slot, {max_tokens_, topk_}, opts.dtype(at::kInt));
-    if (what == "begin") return at::from_blob(e.begin, {num_experts_}, opts.dtype(at::kInt));
+    if (what == "out_x") return over(e.out_x[e.rank], {local_experts(), rows_per_expert(), hidden_}, at::kBFloat16);
+    if (what == "send_slot") return over(e.send_slot, {max_tokens_, topk_}, at::kInt);
+    if (what == "begin") return over(e.begin, {num_experts_}, at::kInt);
     TORCH_CHECK(false, "unknown view '", what, "'");
   }
   std::vector<uint32_t> status() const {
@@ -207,6 +216,18 @@ class EpLlBuffer {
   size_t symmetric_bytes() const { return total_; }
 
  private:
+  // The device is known: left to find it out, the tensor library asks the driver about every pointer.
+  at::Tensor over(void* p, at::IntArrayRef sizes, at::ScalarType type) const {
+    const at::Device dev(at::kCUDA, device_);
+    return at::for_blob(p, sizes).options(at::TensorOptions().device(dev).dtype(type)).target_device(dev).make_tensor();
+  }
+  // A tensor of its own over a piece of `block`, whose memory lives as long as one of its pieces.
+  static at::Tensor piece(const at::Tensor& block, int64_t byte, at::IntArrayRef sizes, at::ScalarType type) {
+    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(block.storage()), block.key_set(), c10::scalarTypeToTypeMeta(type));
+    t.unsafeGetTensorImpl()->set_storage_offset(byte / static_cast<int64_t>(c10::elementSize(type)));
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    return t;
+  }
   void setup_dims(int nranks, int max_tokens, int hidden, int num_experts, int topk, bool fp8) {
     TORCH_CHECK(hidden % 512 == 0, "hidden must be a multiple of 512");
     TORCH_CHECK(num_experts % nranks == 0, "num_experts must divide by the number of ranks");
@@ -269,6 +290,7 @@ class EpLlBuffer {
   std::shared_ptr<CudaBackend> backend_;
   std::shared_ptr<SymmSegment> seg_;
   int n_local_;
+  c10::DeviceIndex device_ = 0;
   int nranks_ = 1, max_tokens_ = 0, hidden_ = 0, num_experts_ = 0, topk_ = 0;
   bool fp8_ = true;
   size_t off_x_ = 0, off_scales_ = 0, off_src_ = 0, off_arrived_ = 0, off_counts_ = 0, off_out_ = 0, counts_bytes_ = 0, total_ = 0;

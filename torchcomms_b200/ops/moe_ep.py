@@ -105,18 +105,9 @@ class Buffer:
         """``keep_handle``: copy the layout out of the buffer so that it survives later dispatches."""
         self._num_tokens = x.shape[0]
         self._buf.dispatch([x.contiguous()], [topk_idx.to(torch.int32).contiguous()], [topk_weights.float().contiguous()])
-        info = self._buf.view(0, "recv_info")
-        out = Dispatched(
-            x=self._buf.view(0, "recv_x"),
-            scales=self._buf.view(0, "recv_scales") if self.fp8 else None,
-            topk_idx=self._buf.view(0, "recv_topk_idx"),
-            topk_weights=self._buf.view(0, "recv_topk_weights"),
-            src=self._buf.view(0, "recv_src"),
-            num_tokens=info[0],
-            tokens_per_src=info[1:],
-        )
+        out = Dispatched(*self._buf.received())
         if keep_handle:
-            out.handle = Handle(self._buf.view(0, "send_slot")[: x.shape[0]].clone(), out.src.clone(), info[0].clone(),
+            out.handle = Handle(self._buf.view(0, "send_slot")[: x.shape[0]].clone(), out.src.clone(), out.num_tokens.clone(),
                                 x.shape[0])
         return out
 
