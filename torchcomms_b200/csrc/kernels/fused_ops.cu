@@ -705,36 +705,57 @@ __global__ void __launch_bounds__(256) k_scale_bf16(const __nv_bfloat16* in, __n
 
 // ------------------------------------------------- row quantisation (e4m3) ---
 
-constexpr int kQuantKeep = 8;  // vectors of 8 a thread holds between the two looks at its row
+// 32 bytes of global memory in one access; the address on a 32-byte boundary.
+__device__ __forceinline__ void ld32(const void* p, uint4* v) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w)
+               : "l"(p)
+               : "memory");
+}
 
 // q[r, :] = e4m3(x[r, :] / scale[r]) with scale[r] = max(amax_r, 1e-8) / 448. A block per row, which stays in
 // registers between the maximum and the division (longer rows re-read the rest from L2): 2 bytes in and 1 byte
 // out per element is all that moves. The maximum is taken on the bit patterns, where NaN is above infinity and
-// so comes through. [4096, 4096] and [4096, 14336] together: 890 us operator by operator, 42 us (5.4 TB/s) here;
-// [67, 4096]: 27 us in eight launches, now 2.3. VEC: 16-byte loads (base, row stride and cols allow them).
-template <bool VEC>
+// so comes through. VEC elements per access: 16 where base, row stride and cols allow 32-byte loads and 16-byte stores, 8
+// where they allow half of that, 1 otherwise; KEEP accesses of a thread stay in registers. In us with 8 and 16: [4096,
+// 4096] 10.7 and 8.9 (5.7 TB/s), [4096, 8192] 19.9 and 15.9, [4096, 14336] 27.2 and 26.8 (6.6 TB/s), [67, 4096] 1.9 and 1.4;
+// the first and third operator by operator: 890 us.
+template <int VEC, int KEEP>
 __global__ void __launch_bounds__(256) k_quantize_rows(const __nv_bfloat16* x, int64_t ld, uint8_t* q, float* scale, int cols) {
+  constexpr int kQuads = VEC >= 8 ? VEC / 8 : 1;  // 16-byte pieces of an access
   __shared__ uint32_t part[8];
   grid_release();
   grid_wait();
   const int tid = threadIdx.x, nt = blockDim.x;
   const __nv_bfloat16* row = x + static_cast<int64_t>(blockIdx.x) * ld;
   uint8_t* out = q + static_cast<size_t>(blockIdx.x) * cols;
-  const int nvec = VEC ? cols / 8 : 0;
-  uint4 keep[kQuantKeep];
+  const int nvec = VEC > 1 ? cols / VEC : 0;
+  uint4 keep[KEEP][kQuads];
   uint32_t mx = 0;  // two 16-bit lanes
-  auto look = [&](uint4 v) {
-    mx = __vmaxu2(mx, __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu)));
+  auto fetch = [&](int v, uint4* to) {
+    if constexpr (VEC == 16) ld32(row + static_cast<int64_t>(v) * 16, to);
+    else to[0] = reinterpret_cast<const uint4*>(row)[v];
   };
-  if constexpr (VEC) {
+  auto look = [&](const uint4* v) {
 #pragma unroll
-    for (int k = 0; k < kQuantKeep; ++k) {
-      const int v = tid + k * nt;
-      keep[k] = v < nvec ? reinterpret_cast<const uint4*>(row)[v] : make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i < kQuads; ++i) {
+      mx = __vmaxu2(mx, __vmaxu2(__vmaxu2(v[i].x & 0x7fff7fffu, v[i].y & 0x7fff7fffu), __vmaxu2(v[i].z & 0x7fff7fffu, v[i].w & 0x7fff7fffu)));
+    }
+  };
+  if constexpr (VEC > 1) {
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+#pragma unroll
+      for (int i = 0; i < kQuads; ++i) keep[k][i] = make_uint4(0u, 0u, 0u, 0u);
+      if (tid + k * nt < nvec) fetch(tid + k * nt, keep[k]);
     }
 #pragma unroll
-    for (int k = 0; k < kQuantKeep; ++k) look(keep[k]);
-    for (int v = tid + kQuantKeep * nt; v < nvec; v += nt) look(reinterpret_cast<const uint4*>(row)[v]);
+    for (int k = 0; k < KEEP; ++k) look(keep[k]);
+    for (int v = tid + KEEP * nt; v < nvec; v += nt) {
+      uint4 w[kQuads];
+      fetch(v, w);
+      look(w);
+    }
   } else {
     for (int c = tid; c < cols; c += nt) mx = __vmaxu2(mx, reinterpret_cast<const uint16_t*>(row)[c] & 0x7fffu);
   }
@@ -759,28 +780,31 @@ __global__ void __launch_bounds__(256) k_quantize_rows(const __nv_bfloat16* x, i
     const float q0 = v * rc;
     return __fmaf_rn(__fmaf_rn(-q0, sc, v), rc, q0);
   };
-  auto convert = [&](uint4 v, int at, auto quotient) {
-    float f[8];
-    unpack8(v, f);
-    uint32_t o[2];
+  auto convert = [&](const uint4* v, int at, auto quotient) {
+    uint32_t o[2 * kQuads];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const __nv_fp8x2_storage_t lo =
-          __nv_cvt_float2_to_fp8x2(make_float2(quotient(f[4 * i]), quotient(f[4 * i + 1])), __NV_SATFINITE, __NV_E4M3);
-      const __nv_fp8x2_storage_t hi =
-          __nv_cvt_float2_to_fp8x2(make_float2(quotient(f[4 * i + 2]), quotient(f[4 * i + 3])), __NV_SATFINITE, __NV_E4M3);
+    for (int i = 0; i < 2 * kQuads; ++i) {
+      const uint4 w = v[i / 2];
+      const float2 a = bf2_to_f2(i % 2 == 0 ? w.x : w.z), b = bf2_to_f2(i % 2 == 0 ? w.y : w.w);
+      const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(quotient(a.x), quotient(a.y)), __NV_SATFINITE, __NV_E4M3);
+      const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(quotient(b.x), quotient(b.y)), __NV_SATFINITE, __NV_E4M3);
       o[i] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
     }
-    reinterpret_cast<uint2*>(out)[at] = make_uint2(o[0], o[1]);
+    if constexpr (VEC == 16) reinterpret_cast<uint4*>(out)[at] = make_uint4(o[0], o[1], o[2], o[3]);
+    else reinterpret_cast<uint2*>(out)[at] = make_uint2(o[0], o[1]);
   };
   auto write_row = [&](auto quotient) {
-    if constexpr (VEC) {
+    if constexpr (VEC > 1) {
 #pragma unroll
-      for (int k = 0; k < kQuantKeep; ++k) {
+      for (int k = 0; k < KEEP; ++k) {
         const int v = tid + k * nt;
         if (v < nvec) convert(keep[k], v, quotient);
       }
-      for (int v = tid + kQuantKeep * nt; v < nvec; v += nt) convert(reinterpret_cast<const uint4*>(row)[v], v, quotient);
+      for (int v = tid + KEEP * nt; v < nvec; v += nt) {
+        uint4 w[kQuads];
+        fetch(v, w);
+        convert(w, v, quotient);
+      }
     } else {
       for (int c = tid; c < cols; c += nt) {
         out[c] = __nv_cvt_float_to_fp8(quotient(__bfloat162float(row[c])), __NV_SATFINITE, __NV_E4M3);
@@ -1020,12 +1044,14 @@ cudaError_t launch_cast_scale(const void* in, int in_kind, void* out, int out_ki
 
 cudaError_t launch_quantize_rows(const __nv_bfloat16* x, int64_t ld, void* q, float* scale, int rows, int cols, cudaStream_t s) {
   if (rows <= 0 || cols <= 0) return cudaErrorInvalidValue;
-  const bool vec = cols % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q) & 7u) == 0;
-  // Enough threads that a row of up to 8 vectors each stays in registers; with few rows on the GPU more threads
+  const uintptr_t xa = reinterpret_cast<uintptr_t>(x), qa = reinterpret_cast<uintptr_t>(q);
+  const bool wide = cols % 16 == 0 && ld % 16 == 0 && xa % 32 == 0 && qa % 16 == 0;
+  const bool vec = cols % 8 == 0 && ld % 8 == 0 && xa % 16 == 0 && qa % 8 == 0;
+  // Enough threads that a row of up to KEEP accesses each stays in registers; with few rows on the GPU more threads
   // shorten the row instead.
-  const int threads = cols <= 1024 ? 32 : (cols <= 4096 && rows > kSms * 4) ? 128 : 256;
-  launch_early(vec ? k_quantize_rows<true> : k_quantize_rows<false>, static_cast<unsigned>(rows), static_cast<unsigned>(threads), s, x, ld,
-               static_cast<uint8_t*>(q), scale, cols);
+  const unsigned threads = cols <= 1024 ? 32 : cols <= 4096 && (wide || rows > kSms * 4) ? 128 : 256;
+  const auto kernel = !wide ? (vec ? k_quantize_rows<8, 8> : k_quantize_rows<1, 1>) : cols > 8192 ? k_quantize_rows<16, 4> : k_quantize_rows<16, 2>;
+  launch_early(kernel, static_cast<unsigned>(rows), threads, s, x, ld, static_cast<uint8_t*>(q), scale, cols);
   note_kernel_launch();
   return cudaGetLastError();
 }
