@@ -20,6 +20,7 @@
 // (comms/common/algorithms/all_reduce/all_reduce_dda.cuh:20-112).
 #include "coll_common.cuh"
 #include "collectives.h"
+#include "early_launch.cuh"
 
 namespace b200c {
 
@@ -129,6 +130,8 @@ __global__ void __launch_bounds__(kArNormMaxHidden / 8) k_add_rmsnorm(ArNormArgs
   using P = Pack<__nv_bfloat16>;
   constexpr int N = P::N;
   __shared__ float s_part[kArNormMaxHidden / 8 / 32];
+  grid_release();
+  grid_wait();
   const int v = static_cast<int>(threadIdx.x);
   const bool live = v < a.hidden / N;
   const size_t at = static_cast<size_t>(blockIdx.x) * a.hidden + static_cast<size_t>(v) * N;
@@ -188,7 +191,7 @@ cudaError_t launch_all_reduce_rmsnorm(const CommDev* comms, int emu_ranks, const
   }
   if (emu_ranks <= 0 && comms[0].nranks == 1) {
     const int threads = (args[0].hidden / 8 + 31) / 32 * 32;
-    coll::k_add_rmsnorm<<<args[0].rows, threads, 0, stream>>>(args[0]);
+    launch_early(coll::k_add_rmsnorm, static_cast<unsigned>(args[0].rows), static_cast<unsigned>(threads), stream, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }

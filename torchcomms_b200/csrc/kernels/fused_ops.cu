@@ -539,9 +539,11 @@ __global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* gate_up
 }
 
 template <int VECS>
-__global__ void __launch_bounds__(256) k_swiglu_bwd(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gate_up,
-                                                    __nv_bfloat16* __restrict__ dgate_up, uint32_t total, FastDiv per_row) {
+__global__ void __launch_bounds__(256) k_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate_up, __nv_bfloat16* dgate_up,
+                                                    uint32_t total, FastDiv per_row) {
   const uint32_t base = blockIdx.x * (256u * VECS) + threadIdx.x;
+  grid_release();
+  grid_wait();
   uint4 gv[VECS], uv[VECS], dv[VECS];
 #pragma unroll
   for (int k = 0; k < VECS; ++k) {
@@ -1154,8 +1156,8 @@ cudaError_t launch_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate
   if (misaligned16(dh, gate_up, dgate_up)) return cudaErrorMisalignedAddress;
   return for_row_slices(rows, ffn / 8, [&](size_t r0, uint32_t total) {
     const unsigned vecs = swiglu_vecs(total);
-    (vecs == 1 ? k_swiglu_bwd<1> : k_swiglu_bwd<2>)<<<covering_grid(total, 256 * vecs), 256, 0, s>>>(
-        dh + r0 * ffn, gate_up + r0 * 2 * ffn, dgate_up + r0 * 2 * ffn, total, make_fast_div(ffn / 8));
+    launch_early(vecs == 1 ? k_swiglu_bwd<1> : k_swiglu_bwd<2>, covering_grid(total, 256 * vecs), 256, s, dh + r0 * ffn,
+                 gate_up + r0 * 2 * ffn, dgate_up + r0 * 2 * ffn, total, make_fast_div(ffn / 8));
   });
 }
 

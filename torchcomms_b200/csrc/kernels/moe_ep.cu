@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "early_launch.cuh"
 #include "launch_count.h"
 
 namespace cg = cooperative_groups;
@@ -257,6 +258,8 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
   const int t0 = blockIdx.x * kEpSoloTokens, here = min(kEpSoloTokens, a.num_tokens - t0);
   const int groups = e.hidden / 128, nchunks = (e.hidden + kEpChunkCols - 1) / kEpChunkCols;
   const size_t row_bytes = e.fp8 ? static_cast<size_t>(e.hidden) : static_cast<size_t>(e.hidden) * 2;
+  grid_release();
+  grid_wait();
   trace_mark<TRACE>(c, 0);  // the marks of the general kernel
   uint4 v0[kSteps], v1[kSteps];
   auto load = [&](int item) {
@@ -482,6 +485,8 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_combine(CommDev c, EpDev e, C
 }
 template <bool TRACE>
 __global__ void __launch_bounds__(kEpThreads) k_ep_combine_solo(CommDev c, EpDev e, CombineArgs a) {
+  grid_release();
+  grid_wait();
   ep_combine_body<1, 4, TRACE>(c, e, a);
 }
 __global__ void __launch_bounds__(kEpThreads) k_ep_combine_emu(const CommDev* cs, const EpDev* es, const CombineArgs* as) {
@@ -616,8 +621,8 @@ cudaError_t launch_ep_dispatch(const CommDev* comms, const EpDev* eps, int emu_r
   for (int i = 0; i < n; ++i) args[i] = {x[i], topk_idx[i], topk_w[i], num_tokens};
   if (emu_ranks <= 0 && e0.nranks == 1) {
     const int blocks = std::max(1, (num_tokens + kEpSoloTokens - 1) / kEpSoloTokens);
-    (comms[0].trace != nullptr ? k_ep_dispatch_solo<true> : k_ep_dispatch_solo<false>)<<<blocks, kEpThreads, 0, stream>>>(
-        comms[0], e0, args[0]);
+    launch_early(comms[0].trace != nullptr ? k_ep_dispatch_solo<true> : k_ep_dispatch_solo<false>, static_cast<unsigned>(blocks), kEpThreads,
+                 stream, comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }
@@ -641,8 +646,8 @@ cudaError_t launch_ep_combine(const CommDev* comms, const EpDev* eps, int emu_ra
     // the pieces (16.9 us for 4096 x 7168) beat a grid that covers them once (18.3).
     const int64_t items = static_cast<int64_t>(num_tokens) * ((e0.hidden + 1023) / 1024);
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((items + kEpWarps - 1) / kEpWarps, 148 * 4));
-    (comms[0].trace != nullptr ? k_ep_combine_solo<true> : k_ep_combine_solo<false>)<<<static_cast<unsigned>(blocks), kEpThreads, 0,
-                                                                                       stream>>>(comms[0], e0, args[0]);
+    launch_early(comms[0].trace != nullptr ? k_ep_combine_solo<true> : k_ep_combine_solo<false>, static_cast<unsigned>(blocks), kEpThreads,
+                 stream, comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }

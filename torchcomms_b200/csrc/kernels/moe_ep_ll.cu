@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "early_launch.cuh"
 #include "launch_count.h"
 
 namespace cg = cooperative_groups;
@@ -355,6 +356,8 @@ __global__ void __launch_bounds__(kLlThreads) k_ep_ll_dispatch_solo(CommDev c, E
   const int E = e.num_experts, M = e.max_tokens, groups = e.hidden / 128;
   const size_t row_bytes = e.fp8 ? static_cast<size_t>(e.hidden) : static_cast<size_t>(e.hidden) * 2;
   const int t = blockIdx.x;
+  grid_release();
+  grid_wait();
   trace_mark<TRACE>(c, 0);  // the marks of the general kernel; without peers 1 to 3 coincide
   if (t < a.num_tokens) {
     if (warp == 0) {
@@ -525,6 +528,8 @@ __global__ void __launch_bounds__(kLlThreads) k_ep_ll_combine(CommDev c, EpLlDev
   ll_combine_body<false>(c, e, a);
 }
 __global__ void __launch_bounds__(kLlThreads) k_ep_ll_combine_solo(CommDev c, EpLlDev e, LlCombineArgs a) {
+  grid_release();
+  grid_wait();
   ll_combine_body<true>(c, e, a);
 }
 __global__ void __launch_bounds__(kLlThreads)
@@ -581,8 +586,8 @@ cudaError_t launch_ep_ll_dispatch(const CommDev* comms, const EpLlDev* eps, int 
   std::vector<LlDispatchArgs> args(n);
   for (int i = 0; i < n; ++i) args[i] = {x[i], topk_idx[i], recv[i], num_tokens};
   if (emu_ranks <= 0 && e0.nranks == 1) {
-    (comms[0].trace != nullptr ? k_ep_ll_dispatch_solo<true> : k_ep_ll_dispatch_solo<false>)<<<std::max(1, num_tokens), kLlThreads, 0,
-                                                                                               stream>>>(comms[0], e0, args[0]);
+    launch_early(comms[0].trace != nullptr ? k_ep_ll_dispatch_solo<true> : k_ep_ll_dispatch_solo<false>,
+                 static_cast<unsigned>(std::max(1, num_tokens)), kLlThreads, stream, comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }
@@ -604,7 +609,7 @@ cudaError_t launch_ep_ll_combine(const CommDev* comms, const EpLlDev* eps, int e
     // No block waits for another one: an ordinary launch with a warp per piece.
     const int64_t items = static_cast<int64_t>(num_tokens) * ((e0.hidden + 255) / 256);
     const int blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((items + kLlWarps - 1) / kLlWarps, 148 * 4)));
-    k_ep_ll_combine_solo<<<blocks, kLlThreads, 0, stream>>>(comms[0], e0, args[0]);
+    launch_early(k_ep_ll_combine_solo, static_cast<unsigned>(blocks), kLlThreads, stream, comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }
