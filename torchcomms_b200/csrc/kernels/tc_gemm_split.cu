@@ -4,19 +4,21 @@
 //
 // What bounds them is how fast the weights reach the SMs, and one tile per SM
 // would leave most SMs without work. So a cluster of S CTAs takes one tile, each
-// CTA a share of K: its TMA -> tcgen05.mma pipeline runs over that share alone,
-// the fp32 accumulators meet in distributed shared memory, and every CTA sums,
-// scales and stores 1/S of the tile. No workspace, no atomics, a fixed order of
-// summation: the same bits at every call. Shares of K make shorter fp32 chains than the persistent kernels', so
-// some results round differently and fewer of them away from the exact product's bf16 value (0.07 % of 128 x 3584 x
-// 4096, there 0.24 %). m x n x k = 128 x 3584 x 4096 and 128 x 4096 x 1792 in bf16: 31.8 and
-// 28.3 us with one 128 x 256 tile on each of 14 and 16 CTAs, 25.1 us for both here
-// (28 x 4 and 32 x 4 CTAs); 67 x 6144 x 4096 in e4m3: 15.3 us, now 11.0. Behind another kernel the set-up (barriers,
-// tensor memory) overlaps with that one's end: bf16 rows quantised and multiplied, 67 x 6144 x 4096, take 13.8 us a pass,
-// 18.4 when every launch and the clearing of the status words waited for the one in front.
+// CTA a share of K: its TMA -> tcgen05.mma pipeline runs over that share alone.
+// Every CTA then owns 1/S of the tile's columns, sums, scales and stores them: the
+// others send their fp32 accumulators of these columns from registers into its
+// shared memory (st.async), where one barrier counts the bytes, so nobody meets
+// the whole cluster and the sums start as the last share arrives. No workspace, no
+// atomics, a fixed order of summation: the same bits at every call. Shares of K
+// make shorter fp32 chains than the other kernels', so some results round
+// differently and fewer of them away from the exact product's bf16 value (0.07 % of
+// 128 x 3584 x 4096, there 0.24 %). 128 x 3584 x 4096 in bf16, operands in L2, in us from the start: loads issued 4.5,
+// accumulators complete 5.9, shares sent 7.5 and received 8.6, done 9.7; when the cluster met, read one another's
+// accumulators and met again, 11.4. In e4m3 128 x 6144 x 4096 8.8, before 13. Behind another kernel the set-up
+// (barriers, tensor memory) overlaps with that one's end.
 //   warp 0, one lane : TMA producer
 //   warp 1           : allocates tensor memory; one lane issues tcgen05.mma
-//   warps 2..5       : accumulator -> shared memory; then all warps reduce
+//   warps 2..5       : accumulators -> their owners, then the own columns
 #include <algorithm>
 #include <atomic>
 
@@ -32,23 +34,47 @@ namespace {
 using namespace tc;
 
 constexpr int kSplitBN = 128;
-constexpr int kSplitStages = 6;
+constexpr int kSplitStages = 5;
 constexpr int kSplitABytes = kBlockM * kBlockK * 2;
 constexpr int kSplitBBytes = kSplitBN * kBlockK * 2;
 constexpr int kSplitStageBytes = kSplitABytes + kSplitBBytes;
 constexpr int kSplitThreads = 192;
-constexpr int kSplitPitch = kSplitBN + 4;  // floats per row of the partial tile: 16-byte rows, no bank conflicts
-constexpr int kSplitMax = 8;               // portable cluster size
-constexpr int kSplitSmemBytes = kSplitStages * kSplitStageBytes + 1024 + 256;
-static_assert(kBlockM * kSplitPitch * 4 <= kSplitStages * kSplitStageBytes, "the partial tile reuses the pipeline stages");
+constexpr int kSplitMax = 8;                // portable cluster size
+constexpr int kSplitPrefetch = 16;          // K steps whose weights a CTA asks into L2 ahead of time
+constexpr int kSplitGroups = kSplitBN / 8;  // a tile's columns are shared out among the cluster in groups of eight
+// The first group of CTA `o`; `per_split` = groups per CTA, rounded up to 1/65536. The last CTA may own fewer.
+__host__ __device__ constexpr int first_group(int o, int per_split) {
+  const int g = (o * per_split + 65535) >> 16;
+  return g < kSplitGroups ? g : kSplitGroups;
+}
+constexpr int groups_per_split(int splits) { return (kSplitGroups * 65536 + splits - 1) / splits; }
+// Clusters of six and seven would need more room than the others for what a CTA receives.
+constexpr bool split_allowed(int splits) { return splits != 6 && splits != 7; }
+// What a CTA receives: for its groups, 128 rows of eight fp32 from every other CTA.
+constexpr int most_share_bytes() {
+  int most = 0;
+  for (int s = 1; s <= kSplitMax; ++s) {
+    for (int o = 0; o < s && split_allowed(s); ++o) {
+      const int own = first_group(o + 1, groups_per_split(s)) - first_group(o, groups_per_split(s));
+      const int bytes = (s - 1) * own * kBlockM * 32;
+      most = bytes > most ? bytes : most;
+    }
+  }
+  return most;
+}
+constexpr int kSplitSmemBytes = kSplitStages * kSplitStageBytes + most_share_bytes() + 1024 + 768;
+static_assert(kSplitSmemBytes <= 227 * 1024, "shared memory of one CTA");
 
 struct SplitBarriers {
+  alignas(16) float scale_b[kSplitBN];  // e4m3: of the tile's columns
   uint64_t full[kSplitStages];
   uint64_t empty[kSplitStages];
   uint64_t acc_full;
+  uint64_t shares;  // the other CTAs' shares have arrived
   uint32_t tmem_base;
   uint32_t failed;
 };
+static_assert(sizeof(SplitBarriers) <= 768, "kSplitSmemBytes");
 
 struct SplitMaps {
   CUtensorMap a, b;
@@ -62,7 +88,7 @@ struct SplitParams {
   const float* scale_b;
   long long* trace;
   int m, n, k, k_iters, tiles_m;  // k in 16-bit units
-  int copy_a;
+  int copy_a, per_split;
 };
 
 __device__ __forceinline__ uint32_t cluster_nctarank() {
@@ -76,35 +102,64 @@ __device__ __forceinline__ uint32_t map_shared(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
+// Four values into another CTA's shared memory; their 16 bytes count on that CTA's barrier.
+__device__ __forceinline__ void st_async_f4(uint32_t addr, const uint32_t* r, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(bar)
+               : "memory");
+}
+// 32 bytes to global memory in one access; the address on a 32-byte boundary.
+__device__ __forceinline__ void st_global_32(void* p, const uint32_t* r) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]),
+               "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// 32 lanes x 16 columns of fp32.
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Asks for a tile to be in L2; moves nothing that anybody sees.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
 }
 
 template <bool FP8, bool TRACE>
 __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_constant__ SplitMaps maps, SplitParams p) {
   constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(kBlockM, kSplitBN) : make_idesc_bf16(kBlockM, kSplitBN);
   extern __shared__ char smem_raw[];
+  // The same place in every CTA of the cluster: shares are written across.
   char* stages = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  SplitBarriers* bars = reinterpret_cast<SplitBarriers*>(stages + kSplitStages * kSplitStageBytes);
+  char* received = stages + kSplitStages * kSplitStageBytes;
+  SplitBarriers* bars = reinterpret_cast<SplitBarriers*>(received + most_share_bytes());
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = static_cast<int>(cluster_nctarank()), part = static_cast<int>(cluster_ctarank());
   const int tile = blockIdx.x / splits;
   const int mi = tile % p.tiles_m, ni = tile / p.tiles_m;
   const int kb0 = static_cast<int>(static_cast<int64_t>(p.k_iters) * part / splits);
   const int kb1 = static_cast<int>(static_cast<int64_t>(p.k_iters) * (part + 1) / splits);
+  const int rows = min(kBlockM, p.m - mi * kBlockM);
+  const int groups = min(kSplitGroups, (p.n - ni * kSplitBN) / 8);  // n is a multiple of 8
+  const int own_lo = first_group(part, p.per_split), own_hi = min(first_group(part + 1, p.per_split), groups);
 
-  // The first column of tiles passes its stages of A on (see warp 2 below).
-  const bool copies = p.copy_a != 0 && ni == 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kSplitStages; ++s) {
       mbar_init(&bars->full[s], 1);
-      mbar_init(&bars->empty[s], copies ? 2 : 1);
+      mbar_init(&bars->empty[s], p.copy_a != 0 ? 2 : 1);  // see warp 2
     }
     mbar_init(&bars->acc_full, 1);
+    mbar_init(&bars->shares, 1);
     bars->failed = 0;
     fence_barrier_init();
+    mbar_expect_tx(&bars->shares, static_cast<uint32_t>((splits - 1) * max(own_hi - own_lo, 0) * rows * 32));
+    // The weights' way into L2 does not depend on the kernel in front. No more of them than L2 has room for.
+    for (int kb = kb0; kb < min(kb1, kb0 + kSplitPrefetch); ++kb) tma_prefetch_2d(&maps.b, kb * kBlockK, ni * kSplitBN);
   }
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, kSplitBN);
@@ -113,6 +168,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  cluster_arrive();  // this CTA's barriers exist
   const uint32_t tmem_base = bars->tmem_base;
   grid_release();
   grid_wait();
@@ -160,96 +216,128 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
       if (TRACE) trace_stamp_ns(p.trace, 2);
     }
   } else {
-    // The accumulator is complete, so every stage has been read: the partial tile may overwrite them.
-    const int q = warp & 3, row = q * 32 + lane;
-    if (copies && warp == 2 && lane == 0) {
+    if (p.copy_a != 0 && warp == 2 && lane == 0) {
+      // Every column of tiles has all of A pass by; each passes the steps on whose turn it is.
+      const int tiles_n = static_cast<int>(gridDim.x) / splits / p.tiles_m;
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const int s = it % kSplitStages;
         if (!mbar_wait(&bars->full[s], (it / kSplitStages) & 1u)) {
           bars->failed = 1;
           break;
         }
-        tma_store_2d(&maps.a_copy, stages + s * kSplitStageBytes, kb * kBlockK, mi * kBlockM);
-        tma_store_commit();
-        tma_store_wait_read<0>();
+        if (kb % tiles_n == ni) {
+          tma_store_2d(&maps.a_copy, stages + s * kSplitStageBytes, kb * kBlockK, mi * kBlockM);
+          tma_store_commit();
+          tma_store_wait_read<0>();
+        }
         mbar_arrive(&bars->empty[s]);
       }
       tma_store_wait_all<0>();
     }
     __syncwarp();
-    float* mine = reinterpret_cast<float*>(stages) + row * kSplitPitch;
-    if (mbar_wait(&bars->acc_full, 0)) {
-      tc_fence_after_sync();
-#pragma unroll
-      for (int j = 0; j < kSplitBN / 32; ++j) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(j * 32), r);
+    const int q = warp & 3, row = q * 32 + lane;
+    const uint32_t acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    float ra = 0.0f;
+    if (FP8) {  // the scales come in while the product runs
+      if (row < rows) ra = p.scale_a[mi * kBlockM + row];
+      bars->scale_b[row] = ni * kSplitBN + row < p.n ? p.scale_b[ni * kSplitBN + row] : 0.0f;
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    }
+    // After a failed wait the shares still go out and come in, so that no CTA leaves while another one writes to it.
+    if (!mbar_wait(&bars->acc_full, 0)) bars->failed = 1;
+    tc_fence_after_sync();
+    cluster_wait();  // the peers' barriers exist
+    if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 4);
+    // Every CTA runs this part once: a chain of latencies, and some 25 bytes per ns between the CTAs' shared memories. (From
+    // there to there by bulk copies: 2.4 us for what takes 1.6 straight from the registers.) Two groups of columns at a
+    // time, from `at` on; the last two where one remains. Warps without rows have nothing to do.
+    const bool live = q * 32 < rows;
+    uint32_t r[16];
+#pragma unroll 1
+    for (int o = 0; o < splits && live; ++o) {
+      if (o == part) continue;
+      const int lo = first_group(o, p.per_split), next = first_group(o + 1, p.per_split), hi = min(next, groups);
+      const int slot = part < o ? part : part - 1;
+      const uint32_t to = map_shared(smem_u32(received) + static_cast<uint32_t>((slot * (next - lo) * 2 * kBlockM + row) * 16), static_cast<uint32_t>(o));
+      const uint32_t bar = map_shared(smem_u32(&bars->shares), static_cast<uint32_t>(o));
+#pragma unroll 1
+      for (int g = lo; g < hi; g += 2) {
+        const int at = min(g, kSplitGroups - 2);
+        tmem_ld_32x16(acc + static_cast<uint32_t>(at * 8), r);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          *reinterpret_cast<uint4*>(mine + j * 32 + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+        for (int v = 0; v < 4; ++v) {
+          const int here = at + v / 2;
+          if (row < rows && here >= g && here < hi) st_async_f4(to + static_cast<uint32_t>(((here - lo) * 2 + v % 2) * kBlockM * 16), r + 4 * v, bar);
+        }
+        __syncwarp();
+      }
+    }
+    if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 5);
+    if (splits > 1) {
+      if (!mbar_wait(&bars->shares, 0) && !mbar_wait(&bars->shares, 0)) bars->failed = 1;  // longer than a peer's own waits
+      asm volatile("fence.acq_rel.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 6);
+    // This CTA's columns: the sum over the cluster in its order, scaled, rounded once.
+    const int step = (first_group(part + 1, p.per_split) - own_lo) * 2 * kBlockM;  // from one CTA's share to the next
+    const float4* in = reinterpret_cast<const float4*>(received) + row;
+    __nv_bfloat16* out = p.c + static_cast<size_t>(mi * kBlockM + row) * p.n + ni * kSplitBN;
+    const bool wide = p.n % 16 == 0 && (reinterpret_cast<uintptr_t>(p.c) & 31u) == 0;
+#pragma unroll 1
+    for (int g = own_lo; g < own_hi && live; g += 2) {
+      const int at = min(g, kSplitGroups - 2);
+      tmem_ld_32x16(acc + static_cast<uint32_t>(at * 8), r);
+      tmem_ld_wait();
+      const float4* from = in + (at - own_lo) * 2 * kBlockM;
+      const bool first = at >= g, second = at + 1 < own_hi;  // which of the two are wanted
+      float sum[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sum[i] = 0.0f;
+#pragma unroll 1
+      for (int s = 0; s < splits; ++s) {
+        if (s == part) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) sum[i] += __uint_as_float(r[i]);
+          continue;
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const float4 f = (v < 2 ? first : second) ? from[v * kBlockM] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          sum[4 * v] += f.x;
+          sum[4 * v + 1] += f.y;
+          sum[4 * v + 2] += f.z;
+          sum[4 * v + 3] += f.w;
+        }
+        from += step;
+      }
+      if (FP8) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum[i] *= ra * bars->scale_b[at * 8 + i];
+      }
+      uint32_t o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] = pack_bf16(__float_as_uint(sum[2 * i]), __float_as_uint(sum[2 * i + 1]));
+      if (row < rows) {
+        if (first && second && wide && at % 2 == 0) {
+          st_global_32(out + at * 8, o);
+        } else {
+          if (first) *reinterpret_cast<uint4*>(out + at * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+          if (second) *reinterpret_cast<uint4*>(out + at * 8 + 8) = make_uint4(o[4], o[5], o[6], o[7]);
         }
       }
-    } else {
-      bars->failed = 1;
+      __syncwarp();
     }
+    if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 3);
   }
 
   __syncwarp();
+  if (warp < 2) cluster_wait();
   tc_fence_before_sync();
-  cluster_sync_all();  // every CTA's partial tile is in its shared memory
-  tc_fence_after_sync();
+  __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, kSplitBN);
-
-  // This CTA's share of the tile's 16-byte output vectors: sum over the cluster, scale, round once.
-  constexpr int kVecsPerRow = kSplitBN / 8;
-  const uint32_t base = smem_u32(stages);
-  const int rows_here = min(kBlockM, p.m - mi * kBlockM);
-  const int vecs = rows_here * kVecsPerRow;
-  for (int v = part * kSplitThreads + static_cast<int>(threadIdx.x); v < vecs; v += splits * kSplitThreads) {
-    const int row = v / kVecsPerRow, col = (v % kVecsPerRow) * 8;
-    const int gcol = ni * kSplitBN + col;
-    if (gcol >= p.n) continue;
-    const uint32_t at = base + static_cast<uint32_t>(row * kSplitPitch + col) * 4u;
-    float4 lo[kSplitMax], hi[kSplitMax];
-#pragma unroll
-    for (int s = 0; s < kSplitMax; ++s) {
-      if (s < splits) {
-        const uint32_t from = map_shared(at, static_cast<uint32_t>(s));
-        lo[s] = ld_cluster_f4(from);
-        hi[s] = ld_cluster_f4(from + 16u);
-      }
-    }
-    float acc[8] = {lo[0].x, lo[0].y, lo[0].z, lo[0].w, hi[0].x, hi[0].y, hi[0].z, hi[0].w};
-#pragma unroll
-    for (int s = 1; s < kSplitMax; ++s) {
-      if (s < splits) {
-        acc[0] += lo[s].x;
-        acc[1] += lo[s].y;
-        acc[2] += lo[s].z;
-        acc[3] += lo[s].w;
-        acc[4] += hi[s].x;
-        acc[5] += hi[s].y;
-        acc[6] += hi[s].z;
-        acc[7] += hi[s].w;
-      }
-    }
-    const int grow = mi * kBlockM + row;
-    if (FP8) {
-      const float ra = p.scale_a[grow];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] *= ra * p.scale_b[gcol + i];
-    }
-    uint4 o;
-    uint32_t* po = &o.x;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) po[i] = pack_bf16(__float_as_uint(acc[2 * i]), __float_as_uint(acc[2 * i + 1]));
-    *reinterpret_cast<uint4*>(p.c + static_cast<size_t>(grow) * p.n + gcol) = o;
-  }
-  if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 3);
   if (threadIdx.x == 0 && bars->failed && p.status != nullptr) p.status[0] = p.status[0] | kStatusTimeout;
-  __syncwarp();
-  cluster_sync_all();  // a peer may still be reading this CTA's partial tile
   if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 7);
 }
 
@@ -297,21 +385,18 @@ int resident_clusters(int device, int splits) {
   return n;
 }
 
-// Whether the split kernel beats the others (tc_gemm.cu has their rule); `k` in 16-bit units. Meeting the cluster and
-// adding up the shares costs it 2 us more than the direct stores of a full tile, less where the tile has few rows; a K
-// step of 64 units is 0.27 us of the others' time and 0.2 us of this one's, over the CTAs that share K.
-// Replayed from a graph, best of the others / split in us (bf16 unless e4m3 is said):
-//   few rows: 1 x 256 x 256 4.2 / 3.8, 32 x 2560 x 256 4.5 / 4.5, e4m3 1 x 14336 x 256 6.6 / 4.4; up to 64, line at 6
-//   steps: 64 x 6144 x 256 5.0 / 5.2, 64 x 2560 x 1024 8.1 / 6.6, e4m3 64 x 2560 x 256 5.0 / 5.4, 64 x 1024 x 1024 6.7 / 5.8
-//   K shared, line at 10 steps: e4m3 128 x 4096 x 1024 (8) 6.9 / 7.2, x 2048 (16) 9.3 / 8.5; 384 x 1024 x 1024 (16)
-//   8.2 / 8.4, 512 x 1024 x 2048 (32) 12.8 / 10.1; e4m3 1536 x 256 x 8192 (64) 23.0 / 12.0
-//   K not shared: half the tile on twice the SMs is worth it only where narrow pair tiles would need a second wave, from
-//   20 steps on: e4m3 128 x 14336 x 4096 (32) 19.9 / 18.7; 192 x 8192 x 4096, one wave of pairs, 15.9 / 17.6
+// Whether the split kernel beats the others (tc_gemm.cu has their rule). Sending shares to their owners costs it 2 us
+// more than a kernel that has its tile to itself; a K step of 64 units (16 bits) is 0.27 us of the others' time and 0.2 us
+// of this one's, over the CTAs that share K. Replayed from a graph, best of the others / split in us:
+//   K shared (from 8 steps on): e4m3 128 x 4096 x 1024 (8 steps) 7.0 / 6.2, x 4112 (33) 14.1 / 11.5; bf16 64 x 1024 x 512 (8)
+//   5.6 / 5.2, 128 x 1024 x 512 5.8 / 5.7, 384 x 2560 x 512 6.1 / 6.6, 128 x 6144 x 1024 (16) 8.7 / 8.0, 128 x 1024 x 4096
+//   (64) 21.7 / 9.0, 4096 x 256 x 8192 41.5 / 26.1
+//   not shared: in e4m3 where narrow pair tiles would need a second wave, 128 x 14336 x 512 7.4 / 5.7, x 4096 19.7 / 16.3,
+//   and up to 8 steps, 128 x 6144 x 256 5.5 / 4.2, but 192 x 8192 x 2048 10.1 / 10.3; in bf16 up to 4 steps, 32 x 2560 x 256
+//   4.50 / 4.46, but 32 x 14336 x 1024 10.5 / 11.4 and 192 x 8192 x 1024 9.0 / 9.9
 bool split_pays(int m, int n, int k_iters, bool fp8, bool shares_k) {
-  if (m <= 32) return true;
-  if (m <= 64) return k_iters >= 6;
-  if (shares_k) return k_iters >= 10;
-  return k_iters >= 20 && !pair_tiles_fit(m, n, fp8);
+  if (shares_k) return fp8 || m <= 64 || k_iters >= 10;
+  return fp8 ? k_iters <= 8 || !pair_tiles_fit(m, n, fp8) : k_iters <= 4 && pair_tiles_fit(m, n, fp8);
 }
 
 template <bool FP8>
@@ -335,13 +420,16 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
   // filling the pipeline and meeting the cluster is larger than what another split saves).
   for (int s = 1; s <= kSplitMax; ++s) {
     if (s > 1 && p.k_iters < 4 * s) break;
+    if (!split_allowed(s)) continue;
     if (resident_clusters<FP8>(device, s) >= tiles) splits = s;
   }
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
   if (p.copy_a == 0 && !split_pays(p.m, p.n, p.k_iters, FP8, splits > 1)) return cudaSuccess;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
-  e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
+  SplitParams q = p;
+  q.per_split = groups_per_split(splits);
+  e = cudaLaunchKernelEx(&cfg, kernel, maps, q);
   note_kernel_launch();
   *done = true;
   return e != cudaSuccess ? e : cudaGetLastError();
