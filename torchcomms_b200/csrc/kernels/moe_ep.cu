@@ -37,6 +37,7 @@ struct DispatchArgs {
   const int* topk_idx;    // [num_tokens, topk]
   const float* topk_w;    // [num_tokens, topk]
   int num_tokens;
+  int per_block;          // single rank: tokens of a block, at most kEpWarps
 };
 
 // 16 bf16 of a lane to e4m3, with one scale per 128 elements (8 neighbouring lanes). Returns the scale.
@@ -247,15 +248,17 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_emu(const CommDev* c
 // A single rank: rows may stand in any order from 0, so a block numbers its own tokens with one atomic and sends them
 // at once, and nobody waits for anybody. The last block to finish leaves the count. An ordinary launch that covers
 // the tokens, where the general kernel is a cooperative one with grid-wide meetings (4096 tokens of 7168 to e4m3:
-// 23.3 us there, 22.0 us (4.0 TB/s) here).
-constexpr int kEpSoloTokens = 4;
+// 23.3 us there, 21.1 us (4.2 TB/s) here; as they are 22.6 (5.2 TB/s), and 24.9 with two accesses of 16 bytes for a lane's
+// 32). A block takes 2, 4 or 8 tokens (which share its start and its atomic, and
+// divide over its warps) as long as 640 blocks are left: in us with 2, 4 and 8 tokens, 64 x 7168 to e4m3 4.9 / 6.7 / 9.6,
+// 512 x 7168 6.8 / 7.9 / 9.9, 4096 x 7168 22.9 / 21.1 / 20.2, 8192 x 1024 21.6 / 12.9 / 10.3, 8192 x 7168 40.5 / 37.6 / 35.9.
 
-template <bool TRACE>
+template <bool WIDE, bool TRACE>
 __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDev e, DispatchArgs a) {
   constexpr int kSteps = kEpChunkCols / 512;
-  __shared__ int s_slot[kEpSoloTokens];
+  __shared__ int s_slot[kEpWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t0 = blockIdx.x * kEpSoloTokens, here = min(kEpSoloTokens, a.num_tokens - t0);
+  const int t0 = blockIdx.x * a.per_block, here = min(a.per_block, a.num_tokens - t0);
   const int groups = e.hidden / 128, nchunks = (e.hidden + kEpChunkCols - 1) / kEpChunkCols;
   const size_t row_bytes = e.fp8 ? static_cast<size_t>(e.hidden) : static_cast<size_t>(e.hidden) * 2;
   grid_release();
@@ -268,8 +271,12 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
 #pragma unroll
     for (int i = 0; i < kSteps; ++i) {
       if (col0 + i * 512 < e.hidden) {
-        v0[i] = ld16_stream(xr + col0 + i * 512);
-        v1[i] = ld16_stream(xr + col0 + i * 512 + 8);
+        if constexpr (WIDE) {
+          ld32_stream(xr + col0 + i * 512, v0[i], v1[i]);
+        } else {
+          v0[i] = ld16_stream(xr + col0 + i * 512);
+          v1[i] = ld16_stream(xr + col0 + i * 512 + 8);
+        }
       }
     }
   };
@@ -328,9 +335,7 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
           st16(e.recv_x[0] + static_cast<size_t>(slot) * row_bytes + e0, packed);
           if ((lane & 7) == 0) e.recv_scales[0][static_cast<size_t>(slot) * groups + e0 / 128] = scale;
         } else {
-          char* dst = e.recv_x[0] + static_cast<size_t>(slot) * row_bytes + static_cast<size_t>(e0) * 2;
-          st16(dst, v0[i]);
-          st16(dst + 16, v1[i]);
+          st32(e.recv_x[0] + static_cast<size_t>(slot) * row_bytes + static_cast<size_t>(e0) * 2, v0[i], v1[i]);
         }
       }
     }
@@ -618,11 +623,16 @@ cudaError_t launch_ep_dispatch(const CommDev* comms, const EpDev* eps, int emu_r
   }
   const int n = emu_ranks > 0 ? emu_ranks : 1;
   std::vector<DispatchArgs> args(n);
-  for (int i = 0; i < n; ++i) args[i] = {x[i], topk_idx[i], topk_w[i], num_tokens};
+  for (int i = 0; i < n; ++i) args[i] = {x[i], topk_idx[i], topk_w[i], num_tokens, 0};
   if (emu_ranks <= 0 && e0.nranks == 1) {
-    const int blocks = std::max(1, (num_tokens + kEpSoloTokens - 1) / kEpSoloTokens);
-    launch_early(comms[0].trace != nullptr ? k_ep_dispatch_solo<true> : k_ep_dispatch_solo<false>, static_cast<unsigned>(blocks), kEpThreads,
-                 stream, comms[0], e0, args[0]);
+    const int per_block = num_tokens >= 640 * 8 ? 8 : num_tokens >= 640 * 4 ? 4 : 2;
+    static_assert(kEpWarps >= 8, "a warp for every token of a block");
+    args[0].per_block = per_block;
+    const int blocks = std::max(1, (num_tokens + per_block - 1) / per_block);
+    const bool wide = reinterpret_cast<uintptr_t>(x[0]) % 32 == 0;  // rows are multiples of 1024 bytes
+    const auto kernel = comms[0].trace != nullptr ? (wide ? k_ep_dispatch_solo<true, true> : k_ep_dispatch_solo<false, true>)
+                                                  : (wide ? k_ep_dispatch_solo<true, false> : k_ep_dispatch_solo<false, false>);
+    launch_early(kernel, static_cast<unsigned>(blocks), kEpThreads, stream, comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }

@@ -68,10 +68,13 @@ __device__ __forceinline__ void ll_send_piece(const EpLlDev& e, const __nv_bfloa
   const int lane = threadIdx.x & 31;
   constexpr int kSteps = kLlChunkCols / 512;
   uint4 v0[kSteps], v1[kSteps];
+  const bool wide = (reinterpret_cast<uintptr_t>(xr) & 31u) == 0;  // rows are multiples of 1024 bytes, so the same for all
 #pragma unroll
   for (int i = 0; i < kSteps; ++i) {  // the whole piece is in flight before the first use
     const int e0 = col_lo + lane * 16 + i * 512;
-    if (e0 < col_hi) {
+    if (e0 < col_hi && wide) {
+      ld32_stream(xr + e0, v0[i], v1[i]);
+    } else if (e0 < col_hi) {
       v0[i] = ld16(xr + e0);
       v1[i] = ld16(xr + e0 + 8);
     }
@@ -266,8 +269,7 @@ __device__ void ll_dispatch_body(const CommDev& c, const EpLlDev& e, const LlDis
         [&](int k, int e0, uint4 v0, uint4 v1) {
           const long long rk = __shfl_sync(0xffffffffu, row, k);
           char* dst = static_cast<char*>(a.recv.packed_x) + static_cast<size_t>(rk) * row_bytes + static_cast<size_t>(e0) * 2;
-          st16(dst, v0);
-          st16(dst + 16, v1);
+          st32(dst, v0, v1);
         },
         [&](int k, int e0, uint4 packed, float scale) {
           const long long rk = __shfl_sync(0xffffffffu, row, k);
@@ -394,8 +396,7 @@ __global__ void __launch_bounds__(kLlThreads) k_ep_ll_dispatch_solo(CommDev c, E
           min(e.hidden, col_lo + kLlChunkCols), live,
           [&](int k, int e0, uint4 v0, uint4 v1) {
             char* dst = static_cast<char*>(a.recv.packed_x) + static_cast<size_t>(s_row[k]) * row_bytes + static_cast<size_t>(e0) * 2;
-            st16(dst, v0);
-            st16(dst + 16, v1);
+            st32(dst, v0, v1);
           },
           [&](int k, int e0, uint4 packed, float scale) {
             const size_t rk = static_cast<size_t>(s_row[k]);

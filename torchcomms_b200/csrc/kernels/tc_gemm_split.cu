@@ -388,12 +388,12 @@ int resident_clusters(int device, int splits) {
 // Whether the split kernel beats the others (tc_gemm.cu has their rule). Sending shares to their owners costs it 2 us
 // more than a kernel that has its tile to itself; a K step of 64 units (16 bits) is 0.27 us of the others' time and 0.2 us
 // of this one's, over the CTAs that share K. Replayed from a graph, best of the others / split in us:
-//   K shared (from 8 steps on): e4m3 128 x 4096 x 1024 (8 steps) 7.0 / 6.2, x 4112 (33) 14.1 / 11.5; bf16 64 x 1024 x 512 (8)
-//   5.6 / 5.2, 128 x 1024 x 512 5.8 / 5.7, 384 x 2560 x 512 6.1 / 6.6, 128 x 6144 x 1024 (16) 8.7 / 8.0, 128 x 1024 x 4096
+//   K shared (from 8 steps on): e4m3 128 x 4096 x 1024 (8 steps) 7.0 / 6.2, x 4112 (33) 14.7 / 10.8; bf16 64 x 1024 x 512 (8)
+//   5.6 / 5.2, 128 x 1024 x 512 5.8 / 5.7, 384 x 2560 x 512 6.2 / 7.0, 128 x 6144 x 1024 (16) 8.7 / 8.0, 128 x 1024 x 4096
 //   (64) 21.7 / 9.0, 4096 x 256 x 8192 41.5 / 26.1
 //   not shared: in e4m3 where narrow pair tiles would need a second wave, 128 x 14336 x 512 7.4 / 5.7, x 4096 19.7 / 16.3,
 //   and up to 8 steps, 128 x 6144 x 256 5.5 / 4.2, but 192 x 8192 x 2048 10.1 / 10.3; in bf16 up to 4 steps, 32 x 2560 x 256
-//   4.50 / 4.46, but 32 x 14336 x 1024 10.5 / 11.4 and 192 x 8192 x 1024 9.0 / 9.9
+//   4.50 / 4.46, but 32 x 14336 x 1024 10.5 / 11.4 and 192 x 8192 x 1024 9.0 / 10.1
 bool split_pays(int m, int n, int k_iters, bool fp8, bool shares_k) {
   if (shares_k) return fp8 || m <= 64 || k_iters >= 10;
   return fp8 ? k_iters <= 8 || !pair_tiles_fit(m, n, fp8) : k_iters <= 4 && pair_tiles_fit(m, n, fp8);
