@@ -19,6 +19,7 @@
 //   warp 0, one lane : TMA producer
 //   warp 1           : allocates tensor memory; one lane issues tcgen05.mma
 //   warps 2..5       : accumulators -> their owners, then the own columns
+// The phase trace has, besides the marks of the other kernels, 4: accumulators complete, 5: shares sent, 6: received.
 #include <algorithm>
 #include <atomic>
 
