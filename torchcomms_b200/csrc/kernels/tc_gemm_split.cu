@@ -246,6 +246,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
     }
     // After a failed wait the shares still go out and come in, so that no CTA leaves while another one writes to it.
     if (!mbar_wait(&bars->acc_full, 0)) bars->failed = 1;
+    __syncwarp();  // every lane leaves the wait by itself; the cluster barrier and the loads below want them together
     tc_fence_after_sync();
     cluster_wait();  // the peers' barriers exist
     if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 4);
