@@ -63,3 +63,37 @@ def test_status_words_are_each_call_s_own():
     assert len({s.data_ptr() for s in seen}) == len(seen) and all(s.shape == (2,) for s in seen)
     seen[0].fill_(7)
     assert not torch.stack(seen[1:]).any()
+
+
+def test_taking_turns_between_streams_allocates_results_only():
+    from torchcomms_b200 import _comms
+
+    a = torch.ones(8, 64, device="cuda", dtype=torch.bfloat16)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+
+    def turns(n):
+        for i in range(n):
+            with torch.cuda.stream(streams[i % 3]):
+                seen.append(_comms.ops.gemm_bf16_nt(a, a))
+
+    seen = []
+    turns(6)
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    turns(300)
+    # One result per call; at most one new block of words per stream.
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] - before <= 300 + 3
+    torch.cuda.synchronize()
+    assert len({s.data_ptr() for _, s in seen}) == len(seen) and not torch.stack([s for _, s in seen]).any()
+
+
+def test_status_words_have_versions_of_their_own():
+    from torchcomms_b200 import _comms
+
+    a = torch.ones(8, 64, device="cuda", dtype=torch.bfloat16)
+    first, second = (_comms.ops.gemm_bf16_nt(a, a)[1] for _ in range(2))
+    first.fill_(7)
+    assert second._version == 0 and not second.any()
+    with torch.inference_mode():
+        third = _comms.ops.gemm_bf16_nt(a, a)[1]
+    assert third.is_inference() and not first.is_inference() and not third.any()

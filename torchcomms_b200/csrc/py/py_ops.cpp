@@ -3,14 +3,17 @@
 
 #include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/CUDAContext.h>
-#include <c10/core/InferenceMode.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
+
+#include <array>
 
 #include "../cuda/driver_api.hpp"
 #include "../kernels/fused_ops.h"
 #include "../kernels/launch_count.h"
 #include "../kernels/tc_gemm.h"
+#include "piece.hpp"
 #include "plain_call.hpp"
 
 namespace b200c {
@@ -40,36 +43,48 @@ at::Tensor vectorable(const at::Tensor& t) { return on16(t) ? t : t.clone(at::Me
 
 // Two cleared status words for one product. A memset per call costs a launch, and keeps the product from starting while
 // the kernel in front of it drains. So words are cut from a block that was cleared in one go on the same stream, each
-// handed out once; the last block of a thread stays with it (one: a call on another stream starts a new one). A graph
-// replays its launches on the same words, so a captured call clears its own, by a kernel node: a memset node holds the
-// product behind it up (m x n x k = 128 x 256 x 64 in bf16: 10.1 us a replay, with a kernel node 6.9; 128 x 6144 x 4096
-// in e4m3 16.2 and 12.8).
+// handed out once. A thread keeps the blocks of the four streams that it used last (8 KB each), so that one that takes
+// turns between streams does not start a block at every call. A graph replays its launches on the same words, so a
+// captured call clears its own, by a kernel node: a memset node holds the product behind it up (m x n x k = 128 x 256 x
+// 64 in bf16: 10.1 us a replay, with a kernel node 6.9; 128 x 6144 x 4096 in e4m3 16.2 and 12.8).
 at::Tensor cleared_status(const at::Tensor& like) {
   const cudaStream_t stream = cur(like);
-  const auto opts = like.options().dtype(at::kInt);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   B200C_CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
   if (capture != cudaStreamCaptureStatusNone) {
-    at::Tensor status = at::empty({2}, opts);
+    at::Tensor status = at::empty({2}, like.options().dtype(at::kInt));
     B200C_CUDA_CHECK(launch_clear_status(reinterpret_cast<uint32_t*>(status.data_ptr<int>()), stream));
     return status;
   }
-  constexpr int64_t kCalls = 1024;
+  constexpr int64_t kCalls = 1024, kBytes = 8;
   struct Block {
-    at::Tensor words;  // [kCalls, 2]
+    c10::Storage words;
+    c10::DeviceIndex device = -1;
     unsigned long long stream_id = 0;
-    int64_t next = 0;
+    int64_t next = kCalls;
+    uint64_t last_used = 0;
   };
-  thread_local Block block;
-  unsigned long long id = 0;  // unlike the handle, never given to another stream
+  thread_local std::array<Block, 4> blocks;
+  thread_local uint64_t calls = 0;
+  unsigned long long id = 0;  // unlike the handle, never given to another stream of the device
   B200C_CUDA_CHECK(cudaStreamGetId(stream, &id));
-  if (!block.words.defined() || block.next == kCalls || block.stream_id != id || block.words.device() != like.device() ||
-      block.words.is_inference() != c10::InferenceMode::is_enabled()) {
-    at::Tensor words = at::empty({kCalls, 2}, opts);
-    B200C_CUDA_CHECK(cudaMemsetAsync(words.data_ptr(), 0, words.nbytes(), stream));
-    block = Block{std::move(words), id, 0};
+  const c10::DeviceIndex device = like.device().index();
+  Block* block = &blocks[0];
+  for (Block& b : blocks) {
+    if (b.device == device && b.stream_id == id) {
+      block = &b;
+      break;
+    }
+    if (b.last_used < block->last_used) block = &b;
   }
-  return block.words.select(0, block.next++);
+  if (block->device != device || block->stream_id != id || block->next == kCalls) {
+    c10::Allocator* memory = c10::cuda::CUDACachingAllocator::get();
+    c10::Storage words(c10::Storage::use_byte_size_t(), kCalls * kBytes, memory->allocate(kCalls * kBytes), memory, /*resizable=*/true);
+    B200C_CUDA_CHECK(cudaMemsetAsync(words.mutable_data(), 0, kCalls * kBytes, stream));
+    *block = Block{std::move(words), device, id, 0, 0};
+  }
+  block->last_used = ++calls;
+  return piece(block->words, kBytes * block->next++, {2}, at::kInt);
 }
 
 bool quantizable(const at::Tensor& x) {
