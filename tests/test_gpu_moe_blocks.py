@@ -38,3 +38,28 @@ def test_dispatch(tokens, hidden, fp8, offset, monkeypatch):
         else:
             assert torch.equal(d.x[:n], x[src])
     comm.finalize()
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+def test_low_latency_outputs_can_be_saved_together(fp8, tmp_path, monkeypatch):
+    """torch.save refuses tensors of different types over one storage; outputs that share an allocation are of one type."""
+    import torchcomms_b200 as tc
+    from torchcomms_b200.ops.moe_ep import LowLatencyBuffer
+
+    for name, value in (("RANK", "0"), ("WORLD_SIZE", "1"), ("LOCAL_RANK", "0")):
+        monkeypatch.setenv(name, value)
+    comm = tc.new_comm("b200", torch.device("cuda", 0), name=f"ll_saved{fp8}", store=dist.HashStore())
+    buf = LowLatencyBuffer(comm, 16, 512, 8, 2, fp8=fp8)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(13, 512, generator=g, device="cuda").to(torch.bfloat16)
+    r = buf.dispatch(x, torch.randint(0, 8, (13, 2), generator=g, device="cuda", dtype=torch.int32))
+    outputs = {k: v for k, v in vars(r).items() if v is not None}
+    small = ("count", "src_info", "layout_range", "send_slot", "begin")
+    torch.save(outputs, tmp_path / "outputs.pt")
+    back = torch.load(tmp_path / "outputs.pt")
+    assert set(back) == set(outputs) and int(back["count"].sum()) == 26
+    assert all(torch.equal(back[k], outputs[k]) for k in small)
+    # Each keeps a version counter of its own.
+    r.count.zero_()
+    assert all(getattr(r, k)._version == 0 for k in small if k != "count")
+    comm.finalize()

@@ -11,6 +11,7 @@
 
 #include "../backends/cuda_backend.hpp"
 #include "../kernels/moe_ep_ll.h"
+#include "piece.hpp"
 
 namespace b200c {
 
@@ -111,24 +112,25 @@ class EpLlBuffer {
       auto opts = x[i].options();
       at::Tensor px = at::empty({Le, R, hidden_}, opts.dtype(fp8_ ? at::kFloat8_e4m3fn : at::kBFloat16));
       at::Tensor ps = fp8_ ? at::empty({Le, R, hidden_ / 128}, opts.dtype(at::kFloat)) : at::Tensor();
-      // The small outputs come out of one allocation: each costs as much host time as the dispatch kernel runs for.
+      at::Tensor range = at::empty({Le, nranks_}, opts.dtype(at::kLong));
+      // The int32 outputs come out of one allocation: each costs as much host time as the dispatch kernel runs for.
       int64_t bytes = 0;
       auto take = [&bytes](int64_t n) {
         const int64_t at = bytes;
-        bytes += static_cast<int64_t>(align256(static_cast<size_t>(n)));
+        bytes += static_cast<int64_t>(align256(static_cast<size_t>(n) * 4));
         return at;
       };
-      const int64_t at_src = take(Le * R * 4), at_count = take(Le * 4), at_range = take(Le * nranks_ * 8);
-      const int64_t at_slot = take(handles ? static_cast<int64_t>(T) * topk_ * 4 : 0), at_begin = take(handles ? num_experts_ * 4 : 0);
-      const at::Tensor block = at::empty({bytes}, opts.dtype(at::kByte));
-      at::Tensor src = piece(block, at_src, {Le, R}, at::kInt);
-      at::Tensor count = piece(block, at_count, {Le}, at::kInt);
-      at::Tensor range = piece(block, at_range, {Le, nranks_}, at::kLong);
+      const int64_t at_src = take(Le * R), at_count = take(Le);
+      const int64_t at_slot = take(handles ? static_cast<int64_t>(T) * topk_ : 0), at_begin = take(handles ? num_experts_ : 0);
+      const at::Tensor block = at::empty({bytes / 4}, opts.dtype(at::kInt));
+      at::Tensor src = piece(block.storage(), at_src, {Le, R}, at::kInt);
+      at::Tensor count = piece(block.storage(), at_count, {Le}, at::kInt);
       recv[i] = {px.data_ptr(), fp8_ ? ps.data_ptr<float>() : nullptr, src.data_ptr<int>(), count.data_ptr<int>(),
                  reinterpret_cast<long long*>(range.data_ptr<int64_t>()), nullptr, nullptr};
       outs[i] = {px, ps, src, count, range};
       if (handles) {
-        at::Tensor slot = piece(block, at_slot, {T, topk_}, at::kInt), begin = piece(block, at_begin, {num_experts_}, at::kInt);
+        at::Tensor slot = piece(block.storage(), at_slot, {T, topk_}, at::kInt);
+        at::Tensor begin = piece(block.storage(), at_begin, {num_experts_}, at::kInt);
         recv[i].send_slot = slot.data_ptr<int>();
         recv[i].begin = begin.data_ptr<int>();
         outs[i].insert(outs[i].end(), {slot, begin});
@@ -220,13 +222,6 @@ class EpLlBuffer {
   at::Tensor over(void* p, at::IntArrayRef sizes, at::ScalarType type) const {
     const at::Device dev(at::kCUDA, device_);
     return at::for_blob(p, sizes).options(at::TensorOptions().device(dev).dtype(type)).target_device(dev).make_tensor();
-  }
-  // A tensor of its own over a piece of `block`, whose memory lives as long as one of its pieces.
-  static at::Tensor piece(const at::Tensor& block, int64_t byte, at::IntArrayRef sizes, at::ScalarType type) {
-    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(block.storage()), block.key_set(), c10::scalarTypeToTypeMeta(type));
-    t.unsafeGetTensorImpl()->set_storage_offset(byte / static_cast<int64_t>(c10::elementSize(type)));
-    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
-    return t;
   }
   void setup_dims(int nranks, int max_tokens, int hidden, int num_experts, int topk, bool fp8) {
     TORCH_CHECK(hidden % 512 == 0, "hidden must be a multiple of 512");
