@@ -726,7 +726,7 @@ constexpr int kPairStageBytes = kBlockM * kBlockK * 2 + (kTpBN / 2) * kBlockK * 
 constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + 2 * kOutChunkBytes + 1024 + 256;
 
 template <TpMode MODE, bool FP8>
-__global__ void __launch_bounds__(tp_threads<MODE>(), 1) k_tp_gemm_pair(const __grid_constant__ TpMaps maps, CommDev c, TpParams p) {
+__device__ __forceinline__ void tp_gemm_pair_body(const TpMaps& maps, const CommDev& c, const TpParams& p) {
   constexpr int BN = kTpBN;
   constexpr int kAB = kBlockM * kBlockK * 2;
   constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(2 * kBlockM, BN) : make_idesc_bf16(2 * kBlockM, BN);
@@ -1081,6 +1081,17 @@ __global__ void __launch_bounds__(tp_threads<MODE>(), 1) k_tp_gemm_pair(const __
   }
 }
 
+template <TpMode MODE, bool FP8>
+__global__ void __launch_bounds__(tp_threads<MODE>(), 1) k_tp_gemm_pair(const __grid_constant__ TpMaps maps, CommDev c, TpParams p) {
+  tp_gemm_pair_body<MODE, FP8>(maps, c, p);
+}
+
+// Several ranks in one cooperative launch (tests), as k_tp_gemm_emu: blockIdx.y is the rank.
+template <TpMode MODE, bool FP8>
+__global__ void __launch_bounds__(tp_threads<MODE>(), 1) k_tp_gemm_pair_emu(const __grid_constant__ TpEmu e) {
+  tp_gemm_pair_body<MODE, FP8>(e.maps[blockIdx.y], e.c[blockIdx.y], e.p[blockIdx.y]);
+}
+
 // ------------------------------------------------------------ launchers ----
 
 int sm_count() {
@@ -1345,8 +1356,39 @@ cudaError_t tp_launch_emu_t(const TpEmu& e, int nranks, cudaStream_t stream) {
                                      dim3(tp_threads<MODE>()), params, kTpSmemBytes, stream);
 }
 
+// The same on CTA pairs: every rank gets its share of the pairs that the GPU holds at once.
+template <TpMode MODE, bool FP8>
+cudaError_t tp_launch_pair_emu_t(const TpEmu& e, int nranks, cudaStream_t stream) {
+  cudaError_t err = cudaFuncSetAttribute(k_tp_gemm_pair_emu<MODE, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+  if (err != cudaSuccess) return err;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(tp_threads<MODE>());
+  cfg.dynamicSmemBytes = kPairSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeCooperative;
+  attr[1].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int pairs = 0;
+  err = cudaOccupancyMaxActiveClusters(&pairs, k_tp_gemm_pair_emu<MODE, FP8>, &cfg);
+  if (err != cudaSuccess) return err;
+  if (pairs < nranks) return cudaErrorInvalidConfiguration;
+  cfg.gridDim = dim3(2 * static_cast<unsigned>(pairs / nranks), static_cast<unsigned>(nranks));
+  cfg.numAttrs = 2;
+  err = cudaLaunchKernelEx(&cfg, k_tp_gemm_pair_emu<MODE, FP8>, e);
+  note_kernel_launch();
+  return err;
+}
+
 template <TpMode MODE>
-cudaError_t tp_launch_emu(const TpEmu& e, int nranks, cudaStream_t stream) {
+cudaError_t tp_launch_emu(const TpEmu& e, int nranks, bool pairs, cudaStream_t stream) {
+  if (pairs) return e.p[0].fp8 ? tp_launch_pair_emu_t<MODE, true>(e, nranks, stream) : tp_launch_pair_emu_t<MODE, false>(e, nranks, stream);
   return e.p[0].fp8 ? tp_launch_emu_t<MODE, true>(e, nranks, stream) : tp_launch_emu_t<MODE, false>(e, nranks, stream);
 }
 
@@ -1395,26 +1437,28 @@ cudaError_t launch_gemm_reduce_scatter(const CommDev& comm, const GemmRsArgs& a,
   return tp_launch<TpMode::GEMM_RS>(std::min(sm_count(), tiles), maps, comm, p, stream);
 }
 
-cudaError_t launch_allgather_gemm_emu(const CommDev* comms, const AgGemmArgs* args, int nranks, cudaStream_t stream) {
+cudaError_t launch_allgather_gemm_emu(const CommDev* comms, const AgGemmArgs* args, int nranks, bool pairs, cudaStream_t stream) {
   if (nranks < 1 || nranks > kTpEmuRanks) return cudaErrorInvalidValue;
   TpEmu e{};
   for (int r = 0; r < nranks; ++r) {
     e.c[r] = comms[r];
-    cudaError_t err = build_ag(comms[r], args[r], false, e.maps[r], e.p[r]);
+    cudaError_t err = build_ag(comms[r], args[r], pairs, e.maps[r], e.p[r]);
     if (err != cudaSuccess) return err;
+    if (pairs && e.p[r].m_local % (2 * kBlockM) != 0) return cudaErrorInvalidValue;
   }
-  return tp_launch_emu<TpMode::AG_GEMM>(e, nranks, stream);
+  return tp_launch_emu<TpMode::AG_GEMM>(e, nranks, pairs, stream);
 }
 
-cudaError_t launch_gemm_reduce_scatter_emu(const CommDev* comms, const GemmRsArgs* args, int nranks, cudaStream_t stream) {
+cudaError_t launch_gemm_reduce_scatter_emu(const CommDev* comms, const GemmRsArgs* args, int nranks, bool pairs, cudaStream_t stream) {
   if (nranks < 1 || nranks > kTpEmuRanks) return cudaErrorInvalidValue;
   TpEmu e{};
   for (int r = 0; r < nranks; ++r) {
     e.c[r] = comms[r];
-    cudaError_t err = build_rs(comms[r], args[r], false, e.maps[r], e.p[r]);
+    cudaError_t err = build_rs(comms[r], args[r], pairs, e.maps[r], e.p[r]);
     if (err != cudaSuccess) return err;
+    if (pairs && e.p[r].m_local % (2 * kBlockM) != 0) return cudaErrorInvalidValue;
   }
-  return tp_launch_emu<TpMode::GEMM_RS>(e, nranks, stream);
+  return tp_launch_emu<TpMode::GEMM_RS>(e, nranks, pairs, stream);
 }
 
 } // namespace b200c

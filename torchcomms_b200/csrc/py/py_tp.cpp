@@ -252,11 +252,12 @@ class TpLayer {
 // Up to four ranks of one layer shape on ONE device (kernel tests): every
 // rank's buffers are ordinary device memory of this GPU, the kernels of all
 // ranks run as one cooperative launch and talk through the same flags and
-// staging areas as separate GPUs would.
+// staging areas as separate GPUs would. `pairs`: the kernels on CTA pairs (shards
+// of a multiple of 256 rows).
 class TpEmuWorld {
  public:
-  TpEmuWorld(int nranks, const std::string& kind, int rows, int cols, double wait_ms, bool fp8)
-      : ag_(kind == "ag_gemm"), fp8_(fp8), nranks_(nranks), rows_(rows), cols_(cols) {
+  TpEmuWorld(int nranks, const std::string& kind, int rows, int cols, double wait_ms, bool fp8, bool pairs)
+      : ag_(kind == "ag_gemm"), fp8_(fp8), pairs_(pairs), nranks_(nranks), rows_(rows), cols_(cols) {
     TORCH_CHECK(kind == "ag_gemm" || kind == "gemm_rs", "kind must be 'ag_gemm' or 'gemm_rs'");
     TORCH_CHECK(nranks >= 1 && nranks <= 4, "1 to 4 emulated ranks");
     if (ag_) {
@@ -353,7 +354,7 @@ class TpEmuWorld {
       a.ctrl = ctrl_[r];
     }
     cudaStream_t s = at::cuda::getCurrentCUDAStream().stream();
-    B200C_CUDA_CHECK(launch_allgather_gemm_emu(comms_.data(), args.data(), nranks_, s));
+    B200C_CUDA_CHECK(launch_allgather_gemm_emu(comms_.data(), args.data(), nranks_, pairs_, s));
     return ys;
   }
 
@@ -402,14 +403,14 @@ class TpEmuWorld {
       a.ctrl = ctrl_[r];
     }
     cudaStream_t s = at::cuda::getCurrentCUDAStream().stream();
-    B200C_CUDA_CHECK(launch_gemm_reduce_scatter_emu(comms_.data(), args.data(), nranks_, s));
+    B200C_CUDA_CHECK(launch_gemm_reduce_scatter_emu(comms_.data(), args.data(), nranks_, pairs_, s));
     return outs;
   }
 
   std::vector<uint32_t> status() const { return std::vector<uint32_t>(status_host_, status_host_ + 5); }
 
  private:
-  bool ag_, fp8_;
+  bool ag_, fp8_, pairs_;
   int nranks_, rows_, cols_;
   size_t data_bytes_ = 0, flag_bytes_ = 0;
   std::vector<char*> bases_;
@@ -426,8 +427,8 @@ class TpEmuWorld {
 
 void bind_tp(py::module_& m) {
   py::class_<TpEmuWorld>(m, "TpEmuWorld")
-      .def(py::init<int, const std::string&, int, int, double, bool>(), py::arg("nranks"), py::arg("kind"), py::arg("rows"),
-           py::arg("cols"), py::arg("wait_ms") = 2000.0, py::arg("fp8") = false)
+      .def(py::init<int, const std::string&, int, int, double, bool, bool>(), py::arg("nranks"), py::arg("kind"), py::arg("rows"),
+           py::arg("cols"), py::arg("wait_ms") = 2000.0, py::arg("fp8") = false, py::arg("pairs") = false)
       .def("input", &TpEmuWorld::input)
       .def("input_scales", &TpEmuWorld::input_scales)
       .def("ag_gemm", &TpEmuWorld::ag_gemm, py::arg("ws"), py::arg("scale_ws") = std::vector<at::Tensor>{})
