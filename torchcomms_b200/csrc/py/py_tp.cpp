@@ -45,26 +45,20 @@ class TpLayer {
       data_bytes_ = align256(static_cast<size_t>(rows) * cols * 2);  // [nranks, m/nranks, n]
       flag_bytes_ = align256(static_cast<size_t>(rows / nranks_ / 128) * (cols / 256) * nranks_ * 4);
     }
-    const size_t total = data_bytes_ + flag_bytes_;
-    if (backend_) {
+    // A single rank's layers are plain products: only the gather's input is a buffer of the layer.
+    const size_t total = ag_ || nranks_ > 1 ? data_bytes_ + flag_bytes_ : 0;
+    if (backend_ && total > 0) {
       c10::cuda::CUDAGuard g(backend_->device());
       seg_ = backend_->symm().allocate(total, false);
       for (int p = 0; p < nranks_; ++p) bases_.push_back(seg_->peer_ptrs[p]);
-    } else {
+    } else if (total > 0) {
       void* p = nullptr;
       B200C_CUDA_CHECK(cudaMalloc(&p, total));
       B200C_CUDA_CHECK(cudaMemset(p, 0, total));
       local_.push_back(p);
       bases_.push_back(static_cast<char*>(p));
-      const size_t fb = static_cast<size_t>(kFlagSets) * kMaxBlocks * kMaxRanks * sizeof(uint32_t);
-      void* f = nullptr;
-      B200C_CUDA_CHECK(cudaMalloc(&f, fb));
-      B200C_CUDA_CHECK(cudaMemset(f, 0, fb));
-      local_.push_back(f);
-      void* ep = nullptr;
-      B200C_CUDA_CHECK(cudaMalloc(&ep, kFlagSets * kMaxBlocks * sizeof(uint32_t)));
-      B200C_CUDA_CHECK(cudaMemset(ep, 0, kFlagSets * kMaxBlocks * sizeof(uint32_t)));
-      local_.push_back(ep);
+    }
+    if (!backend_) {
       B200C_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&status_host_), 64, cudaHostAllocMapped));
       std::memset(status_host_, 0, 64);
       uint32_t* sdev = nullptr;
@@ -72,17 +66,17 @@ class TpLayer {
       std::memset(&solo_, 0, sizeof(solo_));
       solo_.rank = 0;
       solo_.nranks = 1;
-      solo_.flags[0] = static_cast<uint32_t*>(f);
-      solo_.epochs = static_cast<uint32_t*>(ep);
       solo_.status = sdev;
       solo_.timeout_ns = static_cast<unsigned long long>(wait_ms * 1e6);
     }
-    const size_t ctrl_bytes = tp_ctrl_words(ag_ ? rows * nranks_ : 0) * sizeof(uint32_t);
-    void* ctrl = nullptr;
-    B200C_CUDA_CHECK(cudaMalloc(&ctrl, ctrl_bytes));
-    B200C_CUDA_CHECK(cudaMemset(ctrl, 0, ctrl_bytes));
-    local_.push_back(ctrl);
-    ctrl_ = static_cast<uint32_t*>(ctrl);
+    if (nranks_ > 1) {
+      const size_t ctrl_bytes = tp_ctrl_words(ag_ ? rows * nranks_ : 0) * sizeof(uint32_t);
+      void* ctrl = nullptr;
+      B200C_CUDA_CHECK(cudaMalloc(&ctrl, ctrl_bytes));
+      B200C_CUDA_CHECK(cudaMemset(ctrl, 0, ctrl_bytes));
+      local_.push_back(ctrl);
+      ctrl_ = static_cast<uint32_t*>(ctrl);
+    }
     if (ag_ && nranks_ > 1) {
       void* full = nullptr;
       B200C_CUDA_CHECK(cudaMalloc(&full, static_cast<size_t>(rows) * nranks_ * cols * (fp8 ? 1 : 2)));
@@ -96,7 +90,7 @@ class TpLayer {
       local_.push_back(st);
       send_stage_ = st;
     }
-    if (ag_ && fp8) {
+    if (ag_ && fp8 && nranks_ > 1) {
       void* sf = nullptr;
       B200C_CUDA_CHECK(cudaMalloc(&sf, static_cast<size_t>(rows) * nranks_ * 4));
       B200C_CUDA_CHECK(cudaMemset(sf, 0, static_cast<size_t>(rows) * nranks_ * 4));
@@ -161,7 +155,7 @@ class TpLayer {
       a.scale_w = scale_w->data_ptr<float>();
     }
     for (int p = 0; p < nranks_; ++p) a.x_shards[p] = bases_[p];
-    a.x_full = x_full_ ? x_full_ : bases_[rank_];  // single rank: never read
+    a.x_full = x_full_;
     a.w = w.data_ptr();
     a.y = y.data_ptr();
     a.m_local = rows_;
@@ -201,7 +195,7 @@ class TpLayer {
     }
     a.h = h.data_ptr();
     a.w = w.data_ptr();
-    for (int p = 0; p < nranks_; ++p) {
+    for (int p = 0; p < nranks_ && nranks_ > 1; ++p) {
       a.partials[p] = bases_[p];
       a.arrived[p] = reinterpret_cast<uint32_t*>(bases_[p] + data_bytes_);
     }
