@@ -56,3 +56,25 @@ def test_gather_layer_leaves_its_input_behind(m, n, k):
         if other is not layer.input and other.data_ptr() != layer.input.data_ptr():
             layer.input.zero_()
         assert torch.equal(layer(w, other), y) and torch.equal(layer.input, x)
+
+
+# The kernel copies the activations on its way; a copy in front of it does.
+@pytest.mark.parametrize("m,n,k", [(128, 3584, 1024), (512, 5120, 512)])
+def test_gather_layer_in_a_graph(m, n, k):
+    from torchcomms_b200.ops.tp import AllGatherGemm
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    xs = [torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16) for _ in range(3)]
+    w = (torch.randn(n, k, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    layer = AllGatherGemm(None, m_local=m, k=k)
+    want = [layer(w, x) for x in xs]
+    src, graph = xs[0].clone(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        y = layer(w, src)
+    for x, ref in zip(xs, want):
+        src.copy_(x)
+        layer.input.zero_()
+        y.zero_()
+        graph.replay()
+        assert torch.equal(y, ref) and torch.equal(layer.input, x) and layer.status()[0] == 0

@@ -93,6 +93,7 @@ struct TpParams {
   // common
   uint32_t* ctrl;
   uint32_t* status;   // plain mode: where a failed wait is recorded (may be null)
+  int clear;          // plain mode: the status words are this call's own
   int m_total, m_local, n, k, gm;   // k in 16-bit units: K for bf16, K / 2 for e4m3
   // e4m3 operands: C = (row_scale[m] * col_scale[n]) * (A_q x B_q^T)
   int fp8;
@@ -365,6 +366,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
   if (!kFused) {
     grid_release();
     grid_wait();
+    if (p.clear != 0) clear_status(p.status);
   }
   const uint32_t epoch = bars->epoch;  // calls completed before this one
   if (threadIdx.x == 0) trace_stamp_ns(c, 0);
@@ -1237,6 +1239,7 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   none.trace = layer != nullptr ? layer->trace : nullptr;
   TpParams p{};
   p.status = status;
+  p.clear = layer == nullptr && status != nullptr ? 1 : 0;
   p.m_total = m;
   p.m_local = m;
   p.n = n;

@@ -22,15 +22,13 @@ cudaError_t launch_gemm_bf16_nt(const void* a, const void* b, void* c, int m, in
 // tiles, tensor maps and pipeline are those of the bf16 kernel; only the tcgen05.mma kind differs.
 cudaError_t launch_gemm_e4m3_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                 const float* scale_b, uint32_t* status, cudaStream_t stream);
-// Common entry of the two above (k in 16-bit units, scales null = bf16), which picks the kernel. `layer`: the
-// communicator of a fused layer on one rank, whose phase trace is stamped (start, loads issued, MMAs committed, tiles
+// Common entry of the two above (k in 16-bit units, scales null = bf16), which picks the kernel. `status`: two words, which
+// the kernel clears before it reports into them. `layer`: the communicator of a fused layer on one rank, whose status
+// words are not the call's own and keep what they hold, and whose phase trace is stamped (start, loads issued, MMAs committed, tiles
 // stored, CTA done). `a_copy`: a second [m, k] buffer (16-byte aligned, not overlapping `a`) that receives a copy of A.
 cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                            const float* scale_b, uint32_t* status, cudaStream_t stream, const CommDev* layer = nullptr,
                            void* a_copy = nullptr);
-
-// Clears the two status words that a product reports into, ahead of it on the same stream.
-cudaError_t launch_clear_status(uint32_t* status, cudaStream_t stream);
 
 // The same product where 128 x 128 tiles are too few to fill the GPU: clusters of CTAs split K and sum in
 // distributed shared memory. Sets *done when it launched; otherwise (more than kSplitMaxTiles tiles, or a product that

@@ -71,6 +71,7 @@ struct PairParams {
   const float* scale_b;
   long long* trace;
   int m, n, k, gm;  // k in 16-bit units
+  int clear;        // the status words are this call's own
 };
 
 // Pair-tile `t` of the schedule: groups of `gm` 256-row tiles, n-major inside a group.
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
   const uint32_t tmem_base = bars->tmem_base;
   grid_release();
   grid_wait();  // everything above may run while the kernel in front still does
+  if (p.clear != 0) clear_status(p.status);
   if (threadIdx.x == 0) trace_stamp_ns(p.trace, 0);
 
   if (warp == 0) {
@@ -337,6 +339,7 @@ cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, in
   }
   PairParams p{};
   p.status = status;
+  p.clear = layer == nullptr && status != nullptr ? 1 : 0;
   p.scale_a = scale_a;
   p.scale_b = scale_b;
   p.trace = layer != nullptr ? layer->trace : nullptr;

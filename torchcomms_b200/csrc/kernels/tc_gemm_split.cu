@@ -90,6 +90,7 @@ struct SplitParams {
   long long* trace;
   int m, n, k, k_iters, tiles_m;  // k in 16-bit units
   int copy_a, per_split;
+  int clear;  // the status words are this call's own
 };
 
 __device__ __forceinline__ uint32_t cluster_nctarank() {
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   const uint32_t tmem_base = bars->tmem_base;
   grid_release();
   grid_wait();
+  if (p.clear != 0) clear_status(p.status);
   if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 0);
 
   if (warp == 0) {
@@ -343,10 +345,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 7);
 }
 
-__global__ void k_clear_status(uint32_t* status) {
-  if (threadIdx.x < 2) status[threadIdx.x] = 0u;
-}
-
 cudaLaunchConfig_t split_config(int tiles, int splits, cudaStream_t stream, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
@@ -439,12 +437,6 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
 
 } // namespace
 
-cudaError_t launch_clear_status(uint32_t* status, cudaStream_t stream) {
-  k_clear_status<<<1, 32, 0, stream>>>(status);
-  note_kernel_launch();
-  return cudaGetLastError();
-}
-
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                  const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done, const CommDev* layer,
                                  void* a_copy) {
@@ -459,6 +451,7 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   p.copy_a = a_copy != nullptr ? 1 : 0;
   p.c = static_cast<__nv_bfloat16*>(c);
   p.status = status;
+  p.clear = layer == nullptr && status != nullptr ? 1 : 0;
   p.trace = layer != nullptr ? layer->trace : nullptr;
   p.scale_a = scale_a;
   p.scale_b = scale_b;

@@ -3,17 +3,13 @@
 
 #include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
-
-#include <array>
 
 #include "../cuda/driver_api.hpp"
 #include "../kernels/fused_ops.h"
 #include "../kernels/launch_count.h"
 #include "../kernels/tc_gemm.h"
-#include "piece.hpp"
 #include "plain_call.hpp"
 
 namespace b200c {
@@ -41,51 +37,8 @@ bool on16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr(
 // of a gradient) does not start on such a boundary, and contiguous() leaves it where it is.
 at::Tensor vectorable(const at::Tensor& t) { return on16(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
 
-// Two cleared status words for one product. A memset per call costs a launch, and keeps the product from starting while
-// the kernel in front of it drains. So words are cut from a block that was cleared in one go on the same stream, each
-// handed out once. A thread keeps the blocks of the four streams that it used last (8 KB each), so that one that takes
-// turns between streams does not start a block at every call. A graph replays its launches on the same words, so a
-// captured call clears its own, by a kernel node: a memset node holds the product behind it up (m x n x k = 128 x 256 x
-// 64 in bf16: 10.1 us a replay, with a kernel node 6.9; 128 x 6144 x 4096 in e4m3 16.2 and 12.8).
-at::Tensor cleared_status(const at::Tensor& like) {
-  const cudaStream_t stream = cur(like);
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  B200C_CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
-  if (capture != cudaStreamCaptureStatusNone) {
-    at::Tensor status = at::empty({2}, like.options().dtype(at::kInt));
-    B200C_CUDA_CHECK(launch_clear_status(reinterpret_cast<uint32_t*>(status.data_ptr<int>()), stream));
-    return status;
-  }
-  constexpr int64_t kCalls = 1024, kBytes = 8;
-  struct Block {
-    c10::Storage words;
-    c10::DeviceIndex device = -1;
-    unsigned long long stream_id = 0;
-    int64_t next = kCalls;
-    uint64_t last_used = 0;
-  };
-  thread_local std::array<Block, 4> blocks;
-  thread_local uint64_t calls = 0;
-  unsigned long long id = 0;  // unlike the handle, never given to another stream of the device
-  B200C_CUDA_CHECK(cudaStreamGetId(stream, &id));
-  const c10::DeviceIndex device = like.device().index();
-  Block* block = &blocks[0];
-  for (Block& b : blocks) {
-    if (b.device == device && b.stream_id == id) {
-      block = &b;
-      break;
-    }
-    if (b.last_used < block->last_used) block = &b;
-  }
-  if (block->device != device || block->stream_id != id || block->next == kCalls) {
-    c10::Allocator* memory = c10::cuda::CUDACachingAllocator::get();
-    c10::Storage words(c10::Storage::use_byte_size_t(), kCalls * kBytes, memory->allocate(kCalls * kBytes), memory, /*resizable=*/true);
-    B200C_CUDA_CHECK(cudaMemsetAsync(words.mutable_data(), 0, kCalls * kBytes, stream));
-    *block = Block{std::move(words), device, id, 0, 0};
-  }
-  block->last_used = ++calls;
-  return piece(block->words, kBytes * block->next++, {2}, at::kInt);
-}
+// The two status words of one product, which its kernel clears.
+at::Tensor status_words(const at::Tensor& like) { return at::empty({2}, like.options().dtype(at::kInt)); }
 
 bool quantizable(const at::Tensor& x) {
   return plain_call(x) && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.numel() > 0 && x.stride(1) == 1 &&
@@ -478,7 +431,7 @@ void bind_ops(py::module_& m) {
     TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.size(1) == b.size(1), "a: [m, k], b: [n, k]");
     c10::cuda::CUDAGuard g(a.device());
     at::Tensor c = at::empty({a.size(0), b.size(0)}, a.options());
-    at::Tensor status = cleared_status(a);
+    at::Tensor status = status_words(a);
     B200C_CUDA_CHECK(launch_gemm_bf16_nt(a.data_ptr(), b.data_ptr(), c.data_ptr(), static_cast<int>(a.size(0)),
                                          static_cast<int>(b.size(0)), static_cast<int>(a.size(1)),
                                          reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
@@ -495,7 +448,7 @@ void bind_ops(py::module_& m) {
     TORCH_CHECK(scale_a.numel() == a.size(0) && scale_b.numel() == b.size(0), "one scale per row of a and per row of b");
     c10::cuda::CUDAGuard g(a.device());
     at::Tensor c = at::empty({a.size(0), b.size(0)}, a.options().dtype(at::kBFloat16));
-    at::Tensor status = cleared_status(a);
+    at::Tensor status = status_words(a);
     B200C_CUDA_CHECK(launch_gemm_e4m3_nt(a.data_ptr(), b.data_ptr(), c.data_ptr(), static_cast<int>(a.size(0)),
                                          static_cast<int>(b.size(0)), static_cast<int>(a.size(1)), scale_a.data_ptr<float>(),
                                          scale_b.data_ptr<float>(), reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
@@ -508,7 +461,7 @@ void bind_ops(py::module_& m) {
     TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.size(1) == b.size(1), "a: [m, k], b: [n, k]");
     c10::cuda::CUDAGuard g(a.device());
     at::Tensor c = at::empty({a.size(0), b.size(0)}, a.options());
-    at::Tensor status = cleared_status(a);
+    at::Tensor status = status_words(a);
     B200C_CUDA_CHECK(launch_gemm_nt_pair(a.data_ptr(), b.data_ptr(), c.data_ptr(), static_cast<int>(a.size(0)),
                                          static_cast<int>(b.size(0)), static_cast<int>(a.size(1)), nullptr, nullptr,
                                          reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
