@@ -49,7 +49,7 @@ constexpr int kGemmThreads = 192;
 constexpr int kCtrlTiles = 4;
 constexpr int kOutChunkCols = 64;                                  // one 128-byte swizzle row of bf16
 constexpr int kOutChunkBytes = kBlockM * kOutChunkCols * 2;        // 16 KB
-constexpr int kTpSmemBytes = TileCfg<kTpBN>::kStages * TileCfg<kTpBN>::kStageBytes + 2 * kOutChunkBytes + 1024 + 256;
+constexpr int kTpSmemBytes = TileCfg<kTpBN>::kStages * TileCfg<kTpBN>::kStageBytes + 2 * kOutChunkBytes + 1024 + 256 + kTpBN * 4;
 
 enum class TpMode : int { PLAIN = 0, AG_GEMM = 1, GEMM_RS = 2 };
 
@@ -70,6 +70,7 @@ struct TpBarriers {
   int reduce_ok;
   uint32_t fwd_ready;   // reduce-scatter: tiles for other ranks that the epilogue has put into the send staging
 };
+static_assert(sizeof(TpBarriers) <= 256, "the column scales lie behind them");
 
 struct TpMaps {
   CUtensorMap a_local;          // A rows that are in this rank's own buffer
@@ -333,6 +334,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
   char* stages = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   char* obuf = stages + Cfg::kStages * Cfg::kStageBytes;
   TpBarriers* bars = reinterpret_cast<TpBarriers*>(obuf + 2 * kOutChunkBytes);
+  float* col_scales = reinterpret_cast<float*>(obuf + 2 * kOutChunkBytes + 256);  // e4m3: of the tile in the epilogue
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = gridDim.x;
   const int tiles_m = (p.m_total + kBlockM - 1) / kBlockM, tiles_n = (p.n + BN - 1) / BN;
@@ -465,12 +467,19 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
     const int q = warp & 3;
     const int row_in_tile = q * 32 + lane;
     const bool issuer = warp == 2 && lane == 0;
+    const int et = static_cast<int>(threadIdx.x) - 64;
+    ColScales<BN> fetched;
+    if (FP8 && static_cast<int>(blockIdx.x) < total_tiles) fetched.fetch(p.scale_b, tile_at(blockIdx.x, tiles_m, tiles_n, p.gm).ni * BN, p.n, et);
     uint32_t tile_iter = 0, chunk_iter = 0;
     for (int t = blockIdx.x; t < total_tiles; t += G, ++tile_iter) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
       const TileCoord tc_ = tile_at(t, tiles_m, tiles_n, p.gm);
       const int ni = tc_.ni;
       const int mi = mtile_of(tc_.ord);
+      if (FP8) {
+        fetched.put(col_scales, et);
+        if (t + G < total_tiles) fetched.fetch(p.scale_b, tile_at(t + G, tiles_m, tiles_n, p.gm).ni * BN, p.n, et);
+      }
       if (!mbar_wait(&bars->acc_full[as], aph)) {
         bars->failed = 1;
         break;
@@ -504,7 +513,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
                             static_cast<uint32_t>(j * kOutChunkCols + half * 32),
                         r);
           tmem_ld_wait();
-          if (FP8) scale_acc32(r, row_scale, p.scale_b, ni * BN + j * kOutChunkCols + half * 32, p.n);
+          if (FP8) scale_acc32(r, row_scale, col_scales + j * kOutChunkCols + half * 32);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             const int chunk16 = half * 4 + v;
@@ -725,7 +734,7 @@ __global__ void __launch_bounds__(tp_threads<MODE>(), 1) k_tp_gemm_emu(const __g
 
 constexpr int kPairStages = 6;
 constexpr int kPairStageBytes = kBlockM * kBlockK * 2 + (kTpBN / 2) * kBlockK * 2;  // 16 KB of A + 16 KB of B
-constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + 2 * kOutChunkBytes + 1024 + 256;
+constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + 2 * kOutChunkBytes + 1024 + 256 + kTpBN * 4;
 
 template <TpMode MODE, bool FP8>
 __device__ __forceinline__ void tp_gemm_pair_body(const TpMaps& maps, const CommDev& c, const TpParams& p) {
@@ -736,6 +745,7 @@ __device__ __forceinline__ void tp_gemm_pair_body(const TpMaps& maps, const Comm
   char* stages = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   char* obuf = stages + kPairStages * kPairStageBytes;
   TpBarriers* bars = reinterpret_cast<TpBarriers*>(obuf + 2 * kOutChunkBytes);
+  float* col_scales = reinterpret_cast<float*>(obuf + 2 * kOutChunkBytes + 256);  // e4m3: of the tile in the epilogue
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cta = static_cast<int>(cluster_ctarank());  // 0 leads
   const bool leader = cta == 0;
@@ -869,12 +879,19 @@ __device__ __forceinline__ void tp_gemm_pair_body(const TpMaps& maps, const Comm
     const int q = warp & 3;
     const int row_in_tile = q * 32 + lane;
     const bool issuer = warp == 2 && lane == 0;
+    const int et = static_cast<int>(threadIdx.x) - 64;
+    ColScales<BN> fetched;
+    if (FP8 && cluster_id < total_tiles) fetched.fetch(p.scale_b, tile_at(cluster_id, pair_tiles_m, tiles_n, p.gm).ni * BN, p.n, et);
     uint32_t tile_iter = 0, chunk_iter = 0;
     for (int t = cluster_id; t < total_tiles; t += nclusters, ++tile_iter) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
       int ord, ni;
       my_tile(t, &ord, &ni);
       const int mi = mtile_of(ord);
+      if (FP8) {
+        fetched.put(col_scales, et);
+        if (t + nclusters < total_tiles) fetched.fetch(p.scale_b, tile_at(t + nclusters, pair_tiles_m, tiles_n, p.gm).ni * BN, p.n, et);
+      }
       if (!mbar_wait(&bars->acc_full[as], aph)) {
         bars->failed = 1;
         break;
@@ -904,7 +921,7 @@ __device__ __forceinline__ void tp_gemm_pair_body(const TpMaps& maps, const Comm
                             static_cast<uint32_t>(j * kOutChunkCols + half * 32),
                         r);
           tmem_ld_wait();
-          if (FP8) scale_acc32(r, row_scale, p.scale_b, ni * BN + j * kOutChunkCols + half * 32, p.n);
+          if (FP8) scale_acc32(r, row_scale, col_scales + j * kOutChunkCols + half * 32);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             const int chunk16 = half * 4 + v;

@@ -47,7 +47,7 @@ template <int BN>
 struct PairTile {
   static constexpr int kBHalfBytes = (BN / 2) * kBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBHalfBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 2 * kOutChunkBytes + 1024 + 256;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 2 * kOutChunkBytes + 1024 + 256 + BN * 4;
 };
 
 struct PairBarriers {
@@ -58,6 +58,7 @@ struct PairBarriers {
   uint32_t tmem_base;
   uint32_t failed;
 };
+static_assert(sizeof(PairBarriers) <= 256, "the column scales lie behind them");
 
 struct PairMaps {
   CUtensorMap a;    // box 128 rows x 64 columns
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
   char* stages = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   char* obuf = stages + kStages * kStageBytes;
   PairBarriers* bars = reinterpret_cast<PairBarriers*>(obuf + 2 * kOutChunkBytes);
+  float* col_scales = reinterpret_cast<float*>(obuf + 2 * kOutChunkBytes + 256);  // e4m3: of the tile in the epilogue
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();  // 0 leads
   const bool leader = cta == 0;
@@ -195,11 +197,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
     const int q = warp & 3;
     const int row_in_tile = q * 32 + lane;
     const bool issuer = warp == 2 && lane == 0;
+    const int et = static_cast<int>(threadIdx.x) - 64;
+    const auto first_col = [&](int t) {
+      int pm, pn;
+      pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
+      return pn * BN;
+    };
+    ColScales<BN> fetched;
+    if (FP8 && cluster_id < total_tiles) fetched.fetch(p.scale_b, first_col(cluster_id), p.n, et);
     uint32_t tile_iter = 0, chunk_iter = 0;
     for (int t = cluster_id; t < total_tiles; t += nclusters, ++tile_iter) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
       int pm, pn;
       pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
+      if (FP8) {
+        fetched.put(col_scales, et);
+        if (t + nclusters < total_tiles) fetched.fetch(p.scale_b, first_col(t + nclusters), p.n, et);
+      }
       if (!mbar_wait(&bars->acc_full[as], aph)) {
         bars->failed = 1;
         break;
@@ -218,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
                             static_cast<uint32_t>(j * kOutChunkCols + half * 32),
                         r);
           tmem_ld_wait();
-          if (FP8) scale_acc32(r, row_scale, p.scale_b, pn * BN + j * kOutChunkCols + half * 32, p.n);
+          if (FP8) scale_acc32(r, row_scale, col_scales + j * kOutChunkCols + half * 32);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             const int chunk16 = half * 4 + v;
