@@ -4,8 +4,7 @@
 // kernel then sets up barriers, tensor memory and descriptors before it touches data. A kernel launched with
 // launch_early() does that part early; grid_wait() holds it until every grid in front of it is complete and its writes
 // are visible. The rules that keep this as safe as an ordinary launch:
-//   - nothing is read from or written to global memory before grid_wait(), in any thread (asking for lines to be in L2
-//     is neither: L2 is where the kernel in front writes to as well);
+//   - nothing is read from or written to global memory before grid_wait(), in any thread;
 //   - every block passes grid_wait(), so that a kernel is complete only after the ones in front of it are;
 //   - what a kernel reads may have been written while its blocks were already resident, so it is read with ordinary
 //     loads or TMA, never through the read-only path (no __ldg, no const __restrict__ pointers).

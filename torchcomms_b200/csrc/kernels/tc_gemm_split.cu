@@ -41,7 +41,6 @@ constexpr int kSplitBBytes = kSplitBN * kBlockK * 2;
 constexpr int kSplitStageBytes = kSplitABytes + kSplitBBytes;
 constexpr int kSplitThreads = 192;
 constexpr int kSplitMax = 8;                // portable cluster size
-constexpr int kSplitPrefetch = 16;          // K steps whose weights a CTA asks into L2 ahead of time
 constexpr int kSplitGroups = kSplitBN / 8;  // a tile's columns are shared out among the cluster in groups of eight
 // The first group of CTA `o`; `per_split` = groups per CTA, rounded up to 1/65536. The last CTA may own fewer.
 __host__ __device__ constexpr int first_group(int o, int per_split) {
@@ -127,10 +126,6 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-// Asks for a tile to be in L2; moves nothing that anybody sees.
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
-}
 
 template <bool FP8, bool TRACE>
 __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_constant__ SplitMaps maps, SplitParams p) {
@@ -160,8 +155,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
     bars->failed = 0;
     fence_barrier_init();
     mbar_expect_tx(&bars->shares, static_cast<uint32_t>((splits - 1) * max(own_hi - own_lo, 0) * rows * 32));
-    // The weights' way into L2 does not depend on the kernel in front. No more of them than L2 has room for.
-    for (int kb = kb0; kb < min(kb1, kb0 + kSplitPrefetch); ++kb) tma_prefetch_2d(&maps.b, kb * kBlockK, ni * kSplitBN);
   }
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, kSplitBN);
