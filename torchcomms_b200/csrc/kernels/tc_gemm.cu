@@ -95,6 +95,7 @@ struct TpParams {
   uint32_t* ctrl;
   uint32_t* status;   // plain mode: where a failed wait is recorded (may be null)
   int clear;          // plain mode: the status words are this call's own
+  int stage_bytes;    // plain mode: of one K step's loads
   int m_total, m_local, n, k, gm;   // k in 16-bit units: K for bf16, K / 2 for e4m3
   // e4m3 operands: C = (row_scale[m] * col_scale[n]) * (A_q x B_q^T)
   int fp8;
@@ -417,7 +418,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
             bars->failed = 1;
             break;
           }
-          mbar_expect_tx(&bars->full[s], Cfg::kStageBytes);
+          mbar_expect_tx(&bars->full[s], kFused ? Cfg::kStageBytes : static_cast<uint32_t>(p.stage_bytes));
           char* sa = stages + s * Cfg::kStageBytes;
           tma_load_2d(sa, ma, &bars->full[s], kb * kBlockK, a_row);
           tma_load_2d(sa + Cfg::kABytes, &maps.b, &bars->full[s], kb * kBlockK, ni * BN);
@@ -1244,7 +1245,7 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
     return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, false, layer);
   }
   TpMaps maps;
-  if (!make_map(&maps.a_local, a, m, k, kBlockM) || !make_map(&maps.b, b, n, k, kTpBN) ||
+  if (!make_map(&maps.a_local, a, m, k, a_box_rows(m)) || !make_map(&maps.b, b, n, k, kTpBN) ||
       !make_map(&maps.out[0], c, m, n, kBlockM)) {
     return cudaErrorInvalidValue;
   }
@@ -1257,6 +1258,7 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   TpParams p{};
   p.status = status;
   p.clear = layer == nullptr && status != nullptr ? 1 : 0;
+  p.stage_bytes = a_box_rows(m) * kBlockK * 2 + TileCfg<kTpBN>::kBBytes;
   p.m_total = m;
   p.m_local = m;
   p.n = n;

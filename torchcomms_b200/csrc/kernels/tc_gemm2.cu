@@ -73,6 +73,7 @@ struct PairParams {
   long long* trace;
   int m, n, k, gm;  // k in 16-bit units
   int clear;        // the status words are this call's own
+  int stage_bytes;  // of one K step's loads, both CTAs together
 };
 
 // Pair-tile `t` of the schedule: groups of `gm` 256-row tiles, n-major inside a group.
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
             break;
           }
           // The leader's barrier counts all four loads of the stage.
-          if (leader) mbar_expect_tx(&bars->full[s], 2 * kStageBytes);
+          if (leader) mbar_expect_tx(&bars->full[s], static_cast<uint32_t>(p.stage_bytes));
           char* sa = stages + s * kStageBytes;
           tma_load_2d_pair(sa, &maps.a, &bars->full[s], kb * kBlockK, a_row);
           tma_load_2d_pair(sa + kABytes, &maps.b, &bars->full[s], kb * kBlockK, b_row);
@@ -308,9 +309,10 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
     return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
   }
   PairMaps maps;
-  if (!make_map(&maps.a, a, p.m, p.k, kBlockM) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.out, c, p.m, p.n, kBlockM)) {
+  if (!make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m)) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.out, c, p.m, p.n, kBlockM)) {
     return cudaErrorInvalidValue;
   }
+  p.stage_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN>::kBHalfBytes);
   const int tiles_m = (p.m + 2 * kBlockM - 1) / (2 * kBlockM), tiles_n = (p.n + BN - 1) / BN;
   // A rows of a group stay in L2 while the pairs sweep over n: at most 8 pair-tiles and ~40 MB. Every group reads B again,
   // so where L2 does not keep that either (above 48 MB) groups are of up to 16 pair-tiles and 32 MB. In us under the power

@@ -89,7 +89,8 @@ struct SplitParams {
   long long* trace;
   int m, n, k, k_iters, tiles_m;  // k in 16-bit units
   int copy_a, per_split;
-  int clear;  // the status words are this call's own
+  int clear;        // the status words are this call's own
+  int stage_bytes;  // of one K step's loads
 };
 
 __device__ __forceinline__ uint32_t cluster_nctarank() {
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
           bars->failed = 1;
           break;
         }
-        mbar_expect_tx(&bars->full[s], kSplitStageBytes);
+        mbar_expect_tx(&bars->full[s], static_cast<uint32_t>(p.stage_bytes));
         char* sa = stages + s * kSplitStageBytes;
         tma_load_2d(sa, &maps.a, &bars->full[s], kb * kBlockK, mi * kBlockM);
         tma_load_2d(sa + kSplitABytes, &maps.b, &bars->full[s], kb * kBlockK, ni * kSplitBN);
@@ -437,9 +438,9 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   const int64_t tiles_m = (static_cast<int64_t>(m) + kBlockM - 1) / kBlockM, tiles_n = (static_cast<int64_t>(n) + kSplitBN - 1) / kSplitBN;
   if (tiles_m * tiles_n > kSplitMaxTiles) return cudaSuccess;
   SplitMaps maps;
-  if (!make_map(&maps.a, a, m, k, kBlockM) || !make_map(&maps.b, b, n, k, kSplitBN)) return cudaErrorInvalidValue;
+  if (!make_map(&maps.a, a, m, k, a_box_rows(m)) || !make_map(&maps.b, b, n, k, kSplitBN)) return cudaErrorInvalidValue;
   maps.a_copy = maps.a;
-  if (a_copy != nullptr && !make_map(&maps.a_copy, a_copy, m, k, kBlockM)) return cudaErrorInvalidValue;
+  if (a_copy != nullptr && !make_map(&maps.a_copy, a_copy, m, k, a_box_rows(m))) return cudaErrorInvalidValue;
   SplitParams p{};
   p.copy_a = a_copy != nullptr ? 1 : 0;
   p.c = static_cast<__nv_bfloat16*>(c);
@@ -451,6 +452,7 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   p.m = m;
   p.n = n;
   p.k = k;
+  p.stage_bytes = a_box_rows(m) * kBlockK * 2 + kSplitBBytes;
   p.k_iters = (k + kBlockK - 1) / kBlockK;
   p.tiles_m = static_cast<int>(tiles_m);
   const int tiles = static_cast<int>(tiles_m * tiles_n);
