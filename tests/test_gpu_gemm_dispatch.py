@@ -35,6 +35,15 @@ def test_plain_product(m, n, k, fp8):
         first = c
 
 
+# A wave less on single CTAs than on pairs: one wave, with rows off the lines and a long sum, and three; as many waves; more
+# tiles than SMs for the split kernel, and fewer with unshared sums on and off the lines; boxes of 1, 5, 67 and all rows of A.
+@pytest.mark.parametrize("m,n,k", [(1, 28672, 256), (67, 28672, 576), (128, 22016, 1096), (640, 7168, 1152), (300, 10240, 1032), (384, 28672, 128),
+                                   (384, 28672, 136), (5, 14336, 1088), (100, 14336, 1096), (128, 14336, 1032), (256, 9472, 2112), (5, 9472, 1032)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_plain_product_by_waves(m, n, k, fp8):
+    test_plain_product(m, n, k, fp8)
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 256, 64), (128, 3584, 4096), (384, 512, 704), (512, 5120, 512)])
 def test_gather_layer_leaves_its_input_behind(m, n, k):
     """A single rank's layer reads the activations where they are; its input buffer holds them afterwards all the same."""

@@ -96,6 +96,7 @@ struct TpParams {
   uint32_t* status;   // plain mode: where a failed wait is recorded (may be null)
   int clear;          // plain mode: the status words are this call's own
   int stage_bytes;    // plain mode: of one K step's loads
+  int late;           // plain mode: not launched early
   int m_total, m_local, n, k, gm;   // k in 16-bit units: K for bf16, K / 2 for e4m3
   // e4m3 operands: C = (row_scale[m] * col_scale[n]) * (A_q x B_q^T)
   int fp8;
@@ -338,7 +339,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
   float* col_scales = reinterpret_cast<float*>(obuf + 2 * kOutChunkBytes + 256);  // e4m3: of the tile in the epilogue
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = gridDim.x;
-  const int tiles_m = (p.m_total + kBlockM - 1) / kBlockM, tiles_n = (p.n + BN - 1) / BN;
+  const int tiles_m = (p.m_total - 1) / kBlockM + 1, tiles_n = (p.n - 1) / BN + 1;
   const int tiles_per_src = kFused ? p.m_local / kBlockM : tiles_m;
   const int total_tiles = tiles_m * tiles_n;
   const int k_iters = (p.k + kBlockK - 1) / kBlockK;
@@ -1150,7 +1151,7 @@ cudaError_t tp_launch_t(int grid, const TpMaps& maps, const CommDev& c, const Tp
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = MODE == TpMode::PLAIN ? 1 : 0;  // the fused modes meet other GPUs and start when their stream does
+  cfg.numAttrs = MODE == TpMode::PLAIN && p.late == 0 ? 1 : 0;  // the fused modes meet other GPUs and start when their stream does
   e = cudaLaunchKernelEx(&cfg, k_tp_gemm<MODE, FP8>, maps, c, p);
   note_kernel_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -1232,18 +1233,23 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
     e = cudaMemcpyAsync(a_copy, a, static_cast<size_t>(m) * k * 2, cudaMemcpyDeviceToDevice, stream);
     if (e != cudaSuccess) return e;
   }
-  // Pairs beat single CTAs wherever the tensor cores decide (a K step is 0.27 us of either, and a pair's covers twice the
-  // tile), and tiles of 128 columns the ones of 256 as long as no pair gets a second one. Single CTAs are left with short
-  // sums whose 128 x 256 tiles fill the GPU once, where pairs would not; rows that do not start on 128-byte lines cost
-  // them more than pairs. In us, replayed from a graph, single / pairs of 256 / pairs of 128 columns, e4m3: 256 x 6144 x
-  // 4096 19.1 / 17.0 / 15.7; 1000 x 6144 x 4096 34.1 / 29.0 / 36.6, x 4112 45.7 / 34.7 / 37.4; 2048 x 8192 x 2048 34.8 /
-  // 32.2 / 43.3; 768 x 6144 x 256 6.9 / 7.8 / 7.9; bf16: 1000 x 4096 x 1024 9.3 / 10.2 / 14.1, x
-  // 2048 17.2 / 15.7 / 24.0.
-  const int tiles_m = (m + kBlockM - 1) / kBlockM, tiles_n = (n + kTpBN - 1) / kTpBN;
-  if (pair_tiles_fit(m, n, scale_a != nullptr)) return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, true, layer);
-  if (k > 16 * kBlockK || k % kBlockK != 0 || static_cast<int64_t>(tiles_m) * tiles_n > sm_count()) {
-    return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, false, layer);
-  }
+  // A K step is 0.27 us of either, and a pair's covers twice the tile: so pairs, of 128 columns as long as each finds a pair
+  // at once, or else of 256. But pairs work in units of 256 rows, and where half of the last one is empty they may need a
+  // wave more than single CTAs; those are left with these products, as long as a wave counts (up to four; off the 128-byte
+  // lines, where they load more slowly, two), and with short sums whose tiles fill the GPU once. In us, replayed from a graph, single /
+  // pairs of 256 / pairs of 128 columns: e4m3 256 x 6144 x 8192 24.5 / 24.2 / 24.0; 1000 x 6144 x 8192 51.1 / 44.7 / 61.6, x
+  // 8208 79.3 / 56.7 / 63.3; 768 x 6144 x 512 6.7 / 7.6 / 7.8; bf16 1000 x 4096 x 1024 9.7 / 10.4 / 14.4, x 2048 14.8 /
+  // 15.4 / 24.1. With a wave less: bf16 128 x 28672 x 4096 45.4 / 52.7 / 79.6, 640 x 7168 x 4096 29.9 / 43.2 / 60.7, 300 x 28672
+  // x 4096 86.2 / 89.4 / 136.2 (three waves and four), 384 x 28672 x 4104 128.3 / 110.4 / 139.7, 796 x 9496 x 2144 30.4 /
+  // 36.4 / 54.4 (two and three), 3874 x 11928 x 1920 138.4 / 129.4 / 240.
+  const bool fp8 = scale_a != nullptr, on_lines = k % kBlockK == 0;
+  if (pair_tiles_fit(m, n, fp8)) return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, true, layer);
+  const int64_t tiles_n = (n - 1) / kTpBN + 1, singles = ((m - 1) / kBlockM + 1) * tiles_n, pairs = ((m - 1) / (2 * kBlockM) + 1) * tiles_n;
+  const int64_t sms = sm_count(), at_once = std::max(1, pairs_at_once(fp8));
+  const int64_t waves = (singles - 1) / sms + 1;
+  const bool wave_less = waves < (pairs - 1) / at_once + 1 && waves <= (on_lines ? 4 : 2);
+  const bool short_sum = k <= 16 * kBlockK && on_lines && waves == 1;
+  if (!wave_less && !short_sum) return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, false, layer);
   TpMaps maps;
   if (!make_map(&maps.a_local, a, m, k, a_box_rows(m)) || !make_map(&maps.b, b, n, k, kTpBN) ||
       !make_map(&maps.out[0], c, m, n, kBlockM)) {
@@ -1266,8 +1272,12 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   p.fp8 = scale_a != nullptr ? 1 : 0;
   p.scale_a = scale_a;
   p.scale_b = scale_b;
-  p.gm = pick_group(tiles_m, kBlockM, k, 16);
-  return tp_launch<TpMode::PLAIN>(std::min(sm_count(), tiles_m * tiles_n), maps, none, p, stream);
+  p.gm = pick_group((m - 1) / kBlockM + 1, kBlockM, k, 16);
+  // Blocks that start early take the SMs that the kernel in front leaves, and not one of each neighbouring two as those of a
+  // grid smaller than the GPU do on their own. Where rows off the lines keep the loads of an SM busy, that costs long sums
+  // more than an early start gives: 128 x 28672 x 4104 in bf16 55.3 us, 48.6 started late, but x 264 8.1 and 9.0.
+  p.late = !on_lines && singles < sms && k > 16 * kBlockK ? 1 : 0;
+  return tp_launch<TpMode::PLAIN>(static_cast<int>(std::min(sms, singles)), maps, none, p, stream);
 }
 
 size_t tp_ctrl_words(int m_total) {

@@ -62,8 +62,8 @@ inline bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
 
 // Rows of the boxes that bring A where it has `m` rows: those of its only tile, in groups of eight (the period of the
 // swizzle). A box row past the matrix takes as long as one in it, and longer where few rows are left; what a stage holds
-// below the box gives rows of the accumulator that nobody reads. In us with boxes of 128 rows and so: 1 x 6144 x 4096 in e4m3
-// 17.7 and 14.2, 8 x 6144 x 4096 17.2 and 14.0, 1 x 14336 x 4096 in bf16 39.5 and 26.0, 32 x 6144 x 8192 25.0 and 24.9.
+// below the box gives rows of the accumulator that nobody reads. In us with boxes of 128 rows and so: 1 x 6144 x 8192 in e4m3
+// 17.7 and 14.2; in bf16 8 x 6144 x 4096 17.2 and 14.0, 1 x 14336 x 4096 39.5 and 26.0, 32 x 6144 x 8192 25.0 and 24.9.
 constexpr int a_box_rows(int m) { return m >= kBlockM ? kBlockM : (m + 7) / 8 * 8; }
 
 #ifdef __CUDACC__

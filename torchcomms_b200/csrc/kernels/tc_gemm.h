@@ -46,7 +46,8 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
 cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                 const float* scale_b, uint32_t* status, cudaStream_t stream, bool narrow = false,
                                 const CommDev* layer = nullptr);
-// Whether the narrow tiles of an m x n product are at most as many as the GPU holds pairs.
+// Pairs that the GPU holds at once (0 after an error), and whether the narrow tiles of an m x n product are at most as many.
+int pairs_at_once(bool fp8);
 bool pair_tiles_fit(int m, int n, bool fp8);
 
 // Column-parallel layer fused with the all-gather of its input.

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
   const uint32_t cta = cluster_ctarank();  // 0 leads
   const bool leader = cta == 0;
   const int cluster_id = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
-  const int tiles_m = (p.m + 2 * kBlockM - 1) / (2 * kBlockM), tiles_n = (p.n + BN - 1) / BN;
+  const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / BN + 1;
   const int total_tiles = tiles_m * tiles_n;
   const int k_iters = (p.k + kBlockK - 1) / kBlockK;
 
@@ -313,7 +313,7 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
     return cudaErrorInvalidValue;
   }
   p.stage_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN>::kBHalfBytes);
-  const int tiles_m = (p.m + 2 * kBlockM - 1) / (2 * kBlockM), tiles_n = (p.n + BN - 1) / BN;
+  const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / BN + 1;
   // A rows of a group stay in L2 while the pairs sweep over n: at most 8 pair-tiles and ~40 MB. Every group reads B again,
   // so where L2 does not keep that either (above 48 MB) groups are of up to 16 pair-tiles and 32 MB. In us under the power
   // cap with 8 and 16: 4096 x 28672 x 4096 in e4m3 (B of 117 MB) 397 and 390, 8192 x 14336 x 4096 (59 MB) 400 and 392; 4096 x
@@ -342,9 +342,11 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
 
 } // namespace
 
+int pairs_at_once(bool fp8) { return fp8 ? resident_pairs<true, 256>() : resident_pairs<false, 256>(); }
+
 bool pair_tiles_fit(int m, int n, bool fp8) {
   const int pairs = fp8 ? resident_pairs<true, 128>() : resident_pairs<false, 128>();
-  return static_cast<int64_t>((m + 2 * kBlockM - 1) / (2 * kBlockM)) * ((n + 127) / 128) <= pairs;
+  return static_cast<int64_t>((m - 1) / (2 * kBlockM) + 1) * ((n - 1) / 128 + 1) <= pairs;
 }
 
 cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,

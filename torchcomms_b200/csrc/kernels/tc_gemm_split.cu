@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
     tc_fence_after_sync();
     cluster_wait();  // the peers' barriers exist
     if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 4);
-    // Every CTA runs this part once: a chain of latencies, and some 25 bytes per ns between the CTAs' shared memories. (From
+    // Every CTA runs this part once: a chain of latencies, and some 30 bytes per ns between the CTAs' shared memories. (From
     // there to there by bulk copies: 2.4 us for what takes 1.6 straight from the registers.) Two groups of columns at a
     // time, from `at` on; the last two where one remains. Warps without rows have nothing to do.
     const bool live = q * 32 < rows;
@@ -382,15 +382,18 @@ int resident_clusters(int device, int splits) {
 // Whether the split kernel beats the others (tc_gemm.cu has their rule). Sending shares to their owners costs it 2 us
 // more than a kernel that has its tile to itself; a K step of 64 units (16 bits) is 0.27 us of the others' time and 0.2 us
 // of this one's, over the CTAs that share K. Replayed from a graph, best of the others / split in us:
-//   K shared (from 8 steps on): e4m3 128 x 4096 x 1024 (8 steps) 7.0 / 6.2, x 4112 (33) 14.7 / 10.8; bf16 64 x 1024 x 512 (8)
-//   5.6 / 5.2, 128 x 1024 x 512 5.8 / 5.7, 384 x 2560 x 512 6.2 / 7.0, 128 x 6144 x 1024 (16) 8.7 / 8.0, 128 x 1024 x 4096
-//   (64) 21.7 / 9.0, 4096 x 256 x 8192 41.5 / 26.1
-//   not shared: in e4m3 where narrow pair tiles would need a second wave, 128 x 14336 x 512 7.4 / 5.7, x 4096 19.7 / 16.3,
-//   and up to 8 steps, 128 x 6144 x 256 5.5 / 4.2, but 192 x 8192 x 2048 10.1 / 10.3; in bf16 up to 4 steps, 32 x 2560 x 256
-//   4.50 / 4.46, but 32 x 14336 x 1024 10.5 / 11.4 and 192 x 8192 x 1024 9.0 / 10.1
-bool split_pays(int m, int n, int k_iters, bool fp8, bool shares_k) {
+//   K shared (from 8 steps on): e4m3 128 x 4096 x 2048 (16 steps) 8.9 / 7.9, x 8192 (64) 23.1 / 11.8; bf16 64 x 1024 x 512 (8)
+//   5.7 / 5.2, 128 x 1024 x 512 5.9 / 5.8, 384 x 2560 x 512 6.4 / 6.7, 128 x 6144 x 1024 (16) 8.9 / 7.8, 128 x 1024 x 4096
+//   (64) 21.9 / 9.2
+//   not shared, more tiles than pairs: bf16 128 x 14336 x 1024 9.4 / 9.1, x 2048 15.2 / 14.0, x 4096 27.8 / 26.9, x 8192 50.6 /
+//   48.5; off the 128-byte lines x 1032 (17 steps) 12.0 / 11.4, x 2056 18.2 / 19.5, x 4104 31.7 / 38.2
+//   not shared, at most as many: bf16 256 x 9472 x 2048 (32) 14.0 / 14.4, x 8192 43.5 / 45.2; over such sizes split takes
+//   0.96 to 1.0 of the others' time up to 32 steps, 1.0 at 64 and 1.02 at 128; off the lines 1.02 at 5 steps, 1.1 at 17
+bool split_pays(int m, int n, int k, int k_iters, bool fp8, bool shares_k) {
   if (shares_k) return fp8 || m <= 64 || k_iters >= 10;
-  return fp8 ? k_iters <= 8 || !pair_tiles_fit(m, n, fp8) : k_iters <= 4 && pair_tiles_fit(m, n, fp8);
+  const bool fit = pair_tiles_fit(m, n, fp8);
+  if (k % kBlockK == 0) return !fit || k_iters <= 32;
+  return k_iters <= (fit ? 8 : 17);
 }
 
 template <bool FP8>
@@ -411,14 +414,14 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
   }
   if (e != cudaSuccess) return e;
   // As many ways as leave every cluster resident and every CTA at least four K steps (below that the fixed cost of
-  // filling the pipeline and meeting the cluster is larger than what another split saves).
+  // filling the pipeline and exchanging the shares is larger than what another split saves).
   for (int s = 1; s <= kSplitMax; ++s) {
     if (s > 1 && p.k_iters < 4 * s) break;
     if (!split_allowed(s)) continue;
     if (resident_clusters<FP8>(device, s) >= tiles) splits = s;
   }
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
-  if (p.copy_a == 0 && !split_pays(p.m, p.n, p.k_iters, FP8, splits > 1)) return cudaSuccess;
+  if (p.copy_a == 0 && !split_pays(p.m, p.n, p.k, p.k_iters, FP8, splits > 1)) return cudaSuccess;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
   SplitParams q = p;
