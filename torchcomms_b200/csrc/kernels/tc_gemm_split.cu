@@ -424,6 +424,11 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
   if (p.copy_a == 0 && !split_pays(p.m, p.n, p.k, p.k_iters, FP8, splits > 1)) return cudaSuccess;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
+  // Clusters of three and five do not pack into the SMs as the kernel in front leaves them, so that fewer are resident than
+  // on an empty GPU, and a second wave follows. Where room for less than ten more CTAs is left, they start late instead. In
+  // us, early / late, 128 rows x 4096, tiles of 45 in clusters of three: 40 12.9 / 13.9, 42 15.6 / 14.2, 45 18.9 / 14.1; of
+  // 26 in clusters of five: 25 11.8 / 12.1, 26 13.4 / 11.8. Even sizes pack: 33 in clusters of four 11.8 / 12.8, 74 in two 15.9 / 17.2.
+  if (splits % 2 == 1 && splits > 1 && (resident_clusters<FP8>(device, splits) - tiles) * splits < 10) cfg.numAttrs = 1;
   SplitParams q = p;
   q.per_split = groups_per_split(splits);
   e = cudaLaunchKernelEx(&cfg, kernel, maps, q);
