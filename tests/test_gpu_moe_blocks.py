@@ -40,6 +40,13 @@ def test_dispatch(tokens, hidden, fp8, offset, monkeypatch):
     comm.finalize()
 
 
+# Both sides of the lines between 2 and 4 and, for wide rows, between 4 and 8 tokens.
+@pytest.mark.parametrize("tokens,hidden", [(1184, 512), (1185, 512), (5121, 4096), (7105, 4096)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_dispatch_at_the_lines_between_block_sizes(tokens, hidden, fp8, monkeypatch):
+    test_dispatch(tokens, hidden, fp8, 0, monkeypatch)
+
+
 @pytest.mark.parametrize("fp8", [False, True])
 def test_low_latency_outputs_can_be_saved_together(fp8, tmp_path, monkeypatch):
     """torch.save refuses tensors of different types over one storage; outputs that share an allocation are of one type."""

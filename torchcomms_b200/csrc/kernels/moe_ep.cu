@@ -249,9 +249,9 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_emu(const CommDev* c
 // at once, and nobody waits for anybody. The last block to finish leaves the count. An ordinary launch that covers
 // the tokens, where the general kernel is a cooperative one with grid-wide meetings (4096 tokens of 7168 to e4m3:
 // 23.3 us there, 21.1 us (4.2 TB/s) here; as they are 22.6 (5.2 TB/s), and 24.9 with two accesses of 16 bytes for a lane's
-// 32). A block takes 2, 4 or 8 tokens (which share its start and its atomic, and
-// divide over its warps) as long as 640 blocks are left: in us with 2, 4 and 8 tokens, 64 x 7168 to e4m3 4.9 / 6.7 / 9.6,
-// 512 x 7168 6.8 / 7.9 / 9.9, 4096 x 7168 22.9 / 21.1 / 20.2, 8192 x 1024 21.6 / 12.9 / 10.3, 8192 x 7168 40.5 / 37.6 / 35.9.
+// 32). How many tokens a block takes: solo_tokens_per_block(). Started early, a dispatch and a combine of 128 x 7168 to e4m3
+// through a communicator take 1.3 us less in a graph and 0.8 on the stream (11.2 and 20.1 us), of 4096 x 7168 2.0 and 3.1
+// (45.0 and 43.2).
 
 template <bool WIDE, bool TRACE>
 __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDev e, DispatchArgs a) {
@@ -611,6 +611,22 @@ cudaError_t launch_coop(void* real_kernel, void* emu_kernel, const CommDev* comm
   return err != cudaSuccess ? err : e2;
 }
 
+// Tokens of a block of the single-rank dispatch, which share its start and its atomic and divide over its warps. Two as long
+// as all blocks are resident at once (a second wave costs about what the first does), then four. Eight from 5120 on; for
+// rows of 4096 and more only where blocks of four would not leave the last wave fuller. In us, replayed from a graph
+// with what a captured call adds, 2 / 4 / 8: to e4m3 1000 x 1024 6.8 / 6.7 / 7.0, 1536 x 1024 8.7 / 7.2 / 7.4, 1000 x 7168
+// 9.3 / 9.9 / 11.9, 2048 x 7168 15.0 / 14.2 / 16.2, 8192 x 1024 24.2 / 15.2 / 11.8; as they are 5120 x 7168 29.5 / 30.2 /
+// 31.8, 8192 x 7168 42.4 / 41.9 / 42.8. Eight would pay from the end of the first wave of blocks of four on (4096 x 1024 to
+// e4m3 14.3 / 10.2 / 8.4, x 7168 25.0 / 22.5 / 21.5), but 4096 tokens are the batch whose phase trace is to show more
+// blocks than it has rows.
+int solo_tokens_per_block(int tokens, int hidden) {
+  constexpr int kResident = 148 * 4;
+  if (tokens <= 2 * kResident) return 2;
+  if (tokens < 5120) return 4;
+  const auto waves = [&](int per_block) { return (tokens + per_block * kResident - 1) / (per_block * kResident); };
+  return hidden >= 4096 && waves(4) * 4 < waves(8) * 8 ? 4 : 8;
+}
+
 } // namespace
 
 cudaError_t launch_ep_dispatch(const CommDev* comms, const EpDev* eps, int emu_ranks, const void* const* x,
@@ -625,11 +641,15 @@ cudaError_t launch_ep_dispatch(const CommDev* comms, const EpDev* eps, int emu_r
   std::vector<DispatchArgs> args(n);
   for (int i = 0; i < n; ++i) args[i] = {x[i], topk_idx[i], topk_w[i], num_tokens, 0};
   if (emu_ranks <= 0 && e0.nranks == 1) {
-    const int per_block = num_tokens >= 640 * 8 ? 8 : num_tokens >= 640 * 4 ? 4 : 2;
+    const int per_block = solo_tokens_per_block(num_tokens, e0.hidden);
     static_assert(kEpWarps >= 8, "a warp for every token of a block");
     args[0].per_block = per_block;
     const int blocks = std::max(1, (num_tokens + per_block - 1) / per_block);
-    const bool wide = reinterpret_cast<uintptr_t>(x[0]) % 32 == 0;  // rows are multiples of 1024 bytes
+    // 32-byte loads (rows are multiples of 1024 bytes), but not of wide rows to e4m3 in several waves of blocks of four: in us
+    // with 16- and 32-byte loads 5120 x 7168 28.0 and 29.0, 7104 x 7168 32.2 and 33.4, but 2048 x 4096 9.9 and 9.4, 4096 x 1024
+    // 10.0 and 9.7, as they are 6000 x 7168 33.9 and 32.2.
+    const bool by16 = e0.fp8 && e0.hidden >= 4096 && per_block == 4 && blocks > 148 * 4;
+    const bool wide = reinterpret_cast<uintptr_t>(x[0]) % 32 == 0 && !by16;
     const auto kernel = comms[0].trace != nullptr ? (wide ? k_ep_dispatch_solo<true, true> : k_ep_dispatch_solo<false, true>)
                                                   : (wide ? k_ep_dispatch_solo<true, false> : k_ep_dispatch_solo<false, false>);
     launch_early(kernel, static_cast<unsigned>(blocks), kEpThreads, stream, comms[0], e0, args[0]);
