@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "wide_access.cuh"
+
 namespace b200c {
 
 constexpr int kMaxRanks = 8;        // one NVSwitch domain
@@ -134,19 +136,6 @@ __device__ __forceinline__ uint4 ld16_stream(const void* p) {
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
-}
-
-// 32 bytes in one access; the address on a 32-byte boundary. Lanes that each take 32 neighbouring bytes in two accesses of
-// 16 touch every sector twice.
-__device__ __forceinline__ void ld32_stream(const void* p, uint4& lo, uint4& hi) {
-  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w)
-               : "l"(p));
-}
-__device__ __forceinline__ void st32(void* p, uint4 lo, uint4 hi) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y),
-               "r"(hi.z), "r"(hi.w)
-               : "memory");
 }
 
 // NVLS: one load that returns the sum over every rank's copy of the address.

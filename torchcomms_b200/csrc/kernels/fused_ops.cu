@@ -13,6 +13,7 @@
 
 #include "early_launch.cuh"
 #include "launch_count.h"
+#include "wide_access.cuh"
 
 namespace b200c {
 
@@ -707,14 +708,6 @@ __global__ void __launch_bounds__(256) k_scale_bf16(const __nv_bfloat16* in, __n
 
 // ------------------------------------------------- row quantisation (e4m3) ---
 
-// 32 bytes of global memory in one access; the address on a 32-byte boundary.
-__device__ __forceinline__ void ld32(const void* p, uint4* v) {
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w)
-               : "l"(p)
-               : "memory");
-}
-
 // q[r, :] = e4m3(x[r, :] / scale[r]) with scale[r] = max(amax_r, 1e-8) / 448. A block per row, which stays in
 // registers between the maximum and the division (longer rows re-read the rest from L2): 2 bytes in and 1 byte
 // out per element is all that moves. The maximum is taken on the bit patterns, where NaN is above infinity and
@@ -735,7 +728,7 @@ __global__ void __launch_bounds__(256) k_quantize_rows(const __nv_bfloat16* x, i
   uint4 keep[KEEP][kQuads];
   uint32_t mx = 0;  // two 16-bit lanes
   auto fetch = [&](int v, uint4* to) {
-    if constexpr (VEC == 16) ld32(row + static_cast<int64_t>(v) * 16, to);
+    if constexpr (VEC == 16) ld32(row + static_cast<int64_t>(v) * 16, to[0], to[1]);
     else to[0] = reinterpret_cast<const uint4*>(row)[v];
   };
   auto look = [&](const uint4* v) {

@@ -27,6 +27,7 @@
 #include "launch_count.h"
 #include "tc_gemm.cuh"
 #include "tc_gemm.h"
+#include "wide_access.cuh"
 
 namespace b200c {
 
@@ -108,12 +109,6 @@ __device__ __forceinline__ uint32_t map_shared(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void st_async_f4(uint32_t addr, const uint32_t* r, uint32_t bar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(r[0]),
                "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(bar)
-               : "memory");
-}
-// 32 bytes to global memory in one access; the address on a 32-byte boundary.
-__device__ __forceinline__ void st_global_32(void* p, const uint32_t* r) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]),
-               "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -318,11 +313,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
 #pragma unroll
       for (int i = 0; i < 8; ++i) o[i] = pack_bf16(__float_as_uint(sum[2 * i]), __float_as_uint(sum[2 * i + 1]));
       if (row < rows) {
+        const uint4 lo = make_uint4(o[0], o[1], o[2], o[3]), hi = make_uint4(o[4], o[5], o[6], o[7]);
         if (first && second && wide && at % 2 == 0) {
-          st_global_32(out + at * 8, o);
+          st32(out + at * 8, lo, hi);
         } else {
-          if (first) *reinterpret_cast<uint4*>(out + at * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-          if (second) *reinterpret_cast<uint4*>(out + at * 8 + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+          if (first) *reinterpret_cast<uint4*>(out + at * 8) = lo;
+          if (second) *reinterpret_cast<uint4*>(out + at * 8 + 8) = hi;
         }
       }
       __syncwarp();
