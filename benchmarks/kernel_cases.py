@@ -71,7 +71,7 @@ def main():
         us2 = timed(lambda: _comms.ops.gemm_bf16_nt_pair(a, b), args.warmup, args.iters, flush)
         ref = timed(lambda: torch.matmul(a, b.t()), args.warmup, args.iters, flush)
         fl = 2.0 * m * n * k / 1e6
-        print(f"gemm tcgen05 {m}x{n}x{k}: one CTA per tile {us:.1f} us {fl / us:.1f} TFLOP/s; CTA pairs {us2:.1f} us {fl / us2:.1f} TFLOP/s; "
+        print(f"gemm tcgen05 {m}x{n}x{k}: the kernel picked for it {us:.1f} us {fl / us:.1f} TFLOP/s; CTA pairs {us2:.1f} us {fl / us2:.1f} TFLOP/s; "
               f"cuBLAS {ref:.1f} us {fl / ref:.1f} TFLOP/s")
     elif args.case in ("ag_gemm", "gemm_rs"):
         from torchcomms_b200.ops.tp import AllGatherGemm, GemmReduceScatter

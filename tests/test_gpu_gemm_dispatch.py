@@ -35,9 +35,10 @@ def test_plain_product(m, n, k, fp8):
         first = c
 
 
-# A wave less on single CTAs than on pairs: one wave, with rows off the lines and a long sum, and three; as many waves; more
-# tiles than SMs for the split kernel, and fewer with unshared sums on and off the lines; boxes of 1, 5, 67 and all rows of A.
-@pytest.mark.parametrize("m,n,k", [(1, 28672, 256), (67, 28672, 576), (128, 22016, 1096), (640, 7168, 1152), (300, 10240, 1032), (384, 28672, 128),
+# A wave less on single CTAs than on pairs: one wave, with rows off the lines and a long sum, and three; four, with a last
+# column tile of eight columns and further tiles behind it; as many waves; more tiles than SMs for the split kernel, and
+# fewer with unshared sums on and off the lines; boxes of 1, 5, 67 and all rows of A.
+@pytest.mark.parametrize("m,n,k", [(3190, 5640, 64), (1, 28672, 256), (67, 28672, 576), (128, 22016, 1096), (640, 7168, 1152), (300, 10240, 1032), (384, 28672, 128),
                                    (384, 28672, 136), (5, 14336, 1088), (100, 14336, 1096), (128, 14336, 1032), (256, 9472, 2112), (5, 9472, 1032)])
 @pytest.mark.parametrize("fp8", [False, True])
 def test_plain_product_by_waves(m, n, k, fp8):

@@ -1,6 +1,7 @@
 """Fused tensor-parallel layers (all-gather -> GEMM, GEMM -> reduce-scatter):
-single-rank numerics on one GPU, then the real multi-process path, both
-against an fp32 PyTorch reference."""
+a single rank's layers (plain products), the fused single-CTA kernels with
+emulated ranks on one GPU (those on CTA pairs: test_gpu_tp_pairs.py), then the
+real multi-process path, all against an fp32 PyTorch reference."""
 import os
 from datetime import timedelta
 
@@ -22,7 +23,7 @@ def test_ag_gemm_single_rank(m, n, k):
     from torchcomms_b200.ops.tp import AllGatherGemm
 
     layer = AllGatherGemm(None, m, k)
-    for it in range(3):  # repeated calls exercise the device-side epoch
+    for it in range(3):  # the layer keeps nothing from call to call
         x, w = _rand((m, k), 10 + it), _rand((n, k), 20 + it, scale=0.05)
         y = layer(w, x)
         torch.cuda.synchronize()
@@ -192,7 +193,7 @@ def test_fp8_fused_layers_emulated_ranks(nranks):
 def test_fp8_layers_single_rank_api():
     from torchcomms_b200.ops.tp import AllGatherGemm, GemmReduceScatter, quantize_rows
 
-    m, n, k = 512, 768, 1024   # m % 256 == 0: the CTA-pair kernels
+    m, n, k = 512, 768, 1024
     x, w = _rand((m, k), 5), _rand((n, k), 6, scale=0.05)
     qw, sw = quantize_rows(w)
     qx, sx = quantize_rows(x)

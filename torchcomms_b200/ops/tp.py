@@ -21,8 +21,9 @@ DTensor over NCCL all-gather / reduce-scatter plus cuBLAS
 (comms/torchcomms/tests/integration/py/TPCommTest.py:71), which is the
 baseline arm of ``benchmarks/tp_layer_perf.py``.  When the token shard is a
 multiple of 256 rows the kernels run on CTA pairs (tcgen05 ``cta_group::2``).
-``comm=None`` builds a single-rank layer on
-the current device (no peers; tests and profiling).
+``comm=None`` builds a single-rank layer on the current device.  A single rank
+has nothing to exchange: its layers are plain products, and the gather reads
+the activations where they are (``input`` holds a copy of them afterwards).
 
 ``fp8=True`` runs the same kernels on e4m3 operands (``tcgen05.mma
 kind::f8f6f4``, twice the tensor throughput and half the all-gather bytes):
