@@ -41,7 +41,7 @@ def test_dispatch(tokens, hidden, fp8, offset, monkeypatch):
 
 
 # Both sides of the lines between 2 and 4 and, for wide rows, between 4 and 8 tokens.
-@pytest.mark.parametrize("tokens,hidden", [(1184, 512), (1185, 512), (5121, 4096), (7105, 4096)])
+@pytest.mark.parametrize("tokens,hidden", [(1184, 512), (1185, 512), (5121, 4096), (7697, 4096)])
 @pytest.mark.parametrize("fp8", [False, True])
 def test_dispatch_at_the_lines_between_block_sizes(tokens, hidden, fp8, monkeypatch):
     test_dispatch(tokens, hidden, fp8, 0, monkeypatch)

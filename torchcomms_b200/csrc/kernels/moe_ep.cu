@@ -613,7 +613,8 @@ cudaError_t launch_coop(void* real_kernel, void* emu_kernel, const CommDev* comm
 
 // Tokens of a block of the single-rank dispatch, which share its start and its atomic and divide over its warps. Two as long
 // as all blocks are resident at once (a second wave costs about what the first does), then four. Eight from 5120 on; for
-// rows of 4096 and more only where blocks of four would not leave the last wave fuller. In us, replayed from a graph
+// rows of 4096 and more only where blocks of four would not leave the last wave fuller (one of theirs that is at most a quarter
+// full does not count: 7105 x 7168 to e4m3 35.0 us with eight). In us, replayed from a graph
 // with what a captured call adds, 2 / 4 / 8: to e4m3 1000 x 1024 6.8 / 6.7 / 7.0, 1536 x 1024 8.7 / 7.2 / 7.4, 1000 x 7168
 // 9.3 / 9.9 / 11.9, 2048 x 7168 15.0 / 14.2 / 16.2, 8192 x 1024 24.2 / 15.2 / 11.8; as they are 5120 x 7168 29.5 / 30.2 /
 // 31.8, 8192 x 7168 42.4 / 41.9 / 42.8. Eight would pay from the end of the first wave of blocks of four on (4096 x 1024 to
@@ -623,8 +624,8 @@ int solo_tokens_per_block(int tokens, int hidden) {
   constexpr int kResident = 148 * 4;
   if (tokens <= 2 * kResident) return 2;
   if (tokens < 5120) return 4;
-  const auto waves = [&](int per_block) { return (tokens + per_block * kResident - 1) / (per_block * kResident); };
-  return hidden >= 4096 && waves(4) * 4 < waves(8) * 8 ? 4 : 8;
+  const int waves8 = (tokens - 1) / (8 * kResident) + 1, waves4 = (tokens - 1 - kResident) / (4 * kResident) + 1;
+  return hidden >= 4096 && waves4 * 4 < waves8 * 8 ? 4 : 8;
 }
 
 } // namespace
