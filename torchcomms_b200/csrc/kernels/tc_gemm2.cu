@@ -5,9 +5,9 @@
 // so the pair reads every B element once instead of twice; the leader CTA
 // issues one 256 x 256 x 16 MMA for both, accumulating into the tensor memory
 // of both. The smaller per-CTA stage (32 KB) also buys a 6-deep TMA ring.
-// Tensor cores bound it: 4096 x 28672 x 4096 in e4m3 341 us (2.8 PFLOP/s before
-// the power cap sets in; tiles of 128 x 256 on single CTAs 365), 4096 x 14336 x
-// 4096 in bf16 317 (337). Tiles of 128 columns are for products whose tiles all
+// Tensor cores bound it: 4096 x 28672 x 4096 in e4m3 301 us (3.2 PFLOP/s before
+// the power cap sets in; tiles of 128 x 256 on single CTAs 343), 4096 x 14336 x
+// 4096 in bf16 309 (334). Tiles of 128 columns are for products whose tiles all
 // find a pair at once; a K step takes them as long, so a second wave does not pay.
 //
 // Roles per CTA (192 threads): warp 0 lane 0 TMA producer (both CTAs), warp 1

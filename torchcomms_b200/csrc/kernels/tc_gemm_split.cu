@@ -12,10 +12,10 @@
 // atomics, a fixed order of summation: the same bits at every call. Shares of K
 // make shorter fp32 chains than the other kernels', so some results round
 // differently and fewer of them away from the exact product's bf16 value (0.07 % of
-// 128 x 3584 x 4096, there 0.24 %). 128 x 3584 x 4096 in bf16, operands in L2, in us from the start: loads issued 4.5,
-// accumulators complete 5.9, shares sent 7.5 and received 8.6, done 9.7; when the cluster met, read one another's
-// accumulators and met again, 11.4. In e4m3 128 x 6144 x 4096 8.8, before 13. Behind another kernel the set-up
-// (barriers, tensor memory) overlaps with that one's end.
+// 128 x 3584 x 4096, there 0.24 %). 128 x 3584 x 4096 in bf16, operands in L2, in us from the start: loads issued 4.3,
+// accumulators complete 5.7, shares sent 7.1 and received 8.1, done 9.1; when the cluster met, read one another's
+// accumulators and met again, 11.4. Replayed from a graph, then and now: this 13.4 and 11.2, in e4m3 128 x 6144 x 4096 12.8
+// and 10.4. Behind another kernel the set-up (barriers, tensor memory) overlaps with that one's end.
 //   warp 0, one lane : TMA producer
 //   warp 1           : allocates tensor memory; one lane issues tcgen05.mma
 //   warps 2..5       : accumulators -> their owners, then the own columns
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
     tc_fence_after_sync();
     cluster_wait();  // the peers' barriers exist
     if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 4);
-    // Every CTA runs this part once: a chain of latencies, and some 30 bytes per ns between the CTAs' shared memories. (From
+    // Every CTA runs this part once: a chain of latencies, and some 35 bytes per ns between the CTAs' shared memories. (From
     // there to there by bulk copies: 2.4 us for what takes 1.6 straight from the registers.) Two groups of columns at a
     // time, from `at` on; the last two where one remains. Warps without rows have nothing to do.
     const bool live = q * 32 < rows;
