@@ -1,0 +1,91 @@
+"""Loss and gradients of a head on the logits kernel: edges of its tiles and vectors, chunks, ignored rows."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _head(rows, dim, vocab, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(rows, dim, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(vocab, dim, generator=g, device="cuda") * 0.3).bfloat16()
+    t = torch.randint(vocab, (rows,), generator=g, device="cuda")
+    return x, w, t
+
+
+def _reference(x, w, t):
+    xd, wd = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    loss = F.cross_entropy(xd @ wd.t(), t, reduction="none", ignore_index=-1).sum() / x.shape[0]
+    return (loss.detach(), *torch.autograd.grad(loss, (xd, wd)))
+
+
+@pytest.mark.parametrize("rows,dim,vocab", [(1, 8, 1), (3, 64, 7), (127, 72, 8), (128, 64, 9), (129, 136, 127), (257, 64, 129),
+                                            (255, 64, 255), (256, 64, 257), (513, 200, 4095), (700, 64, 4097), (33, 264, 16385),
+                                            (2049, 64, 1000), (20, 64, 40003), (1030, 128, 9475)])
+def test_head_against_64_bits(rows, dim, vocab):
+    from torchcomms_b200 import _comms
+
+    x, w, t = _head(rows, dim, vocab, 5)
+    t[-1], t[0] = vocab - 1, 0
+    t[rows // 3] = -1
+    ref = _reference(x, w, t)
+    for chunk in (4096, 100):
+        out = _comms.ops.head(x, w, t, chunk)
+        # Sums of `dim` products in fp32: dim x 2^-24 of the products' magnitudes, which are below 0.3 sqrt(dim) x 5 here;
+        # then fp32 exponentials and sums, 1e-5 as for the loss kernel that makes its own statistics.
+        assert abs(float(out[0].double() - ref[0])) < 1e-5 + dim**1.5 * 1.5 * 2**-24
+        # bf16 logits off by 2^-9 of up to 0.3 sqrt(dim) x 5 move a probability by as much; their gradients and the results
+        # are rounded to 2^-9. One number in a row of one has nothing to average over, hence the maximum, not a norm.
+        for a, b in zip(out[1:], ref[1:]):
+            assert float((a.double() - b).norm()) <= (2**-8 + 2**-9 * 1.5 * dim**0.5) * float(b.norm()) + 1e-12
+    again = _comms.ops.head(x, w, t, 4096)
+    assert all(torch.equal(a, b) for a, b in zip(again, _comms.ops.head(x, w, t, 4096)))  # the same bits every time
+
+
+def test_head_all_rows_ignored_and_infinities():
+    from torchcomms_b200 import _comms
+
+    x, w, t = _head(300, 64, 1003, 6)
+    loss, dx, dw = _comms.ops.head(x, w, torch.full_like(t, -1), 4096)
+    assert float(loss) == 0 and not dx.any() and not dw.any()
+    loss, dx, dw = _comms.ops.head(x, w, torch.full_like(t, 1003), 4096)  # past the vocabulary, as in the loss kernel
+    assert float(loss) == 0 and not dx.any() and not dw.any()
+    x[7, 3] = float("inf")
+    loss, dx, _ = _comms.ops.head(x, w, t, 4096)
+    bad = torch.isnan(dx.float()).any(dim=1)
+    assert torch.isnan(loss) and bool(bad[7]) and int(bad.sum()) == 1  # its own row, as with separate operators
+
+
+def test_head_of_large_logits():
+    """Logits whose exponentials overflow by themselves, and rows with one logit far above the rest."""
+    from torchcomms_b200 import _comms
+
+    x, w, t = _head(200, 64, 2051, 7)
+    x *= 100
+    ref = _reference(x, w, t)
+    loss, _, _ = _comms.ops.head(x, w, t, 4096)
+    # fp32 logits of up to 1500: 2^-24 of that, 64 times over in the worst order
+    assert abs(float(loss.double() - ref[0])) < 1500 * 64 * 2**-24
+
+
+def test_what_the_head_leaves_to_operators():
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops import fused
+
+    x, w, t = _head(40, 64, 99, 8)
+    assert _comms.ops.head(x, w, t, 4096) is not None
+    assert _comms.ops.head(x[:, :63], w[:, :63], t, 4096) is None                      # strides
+    assert _comms.ops.head(x[:, :60].contiguous(), w[:, :60].contiguous(), t, 4096) is None  # no multiple of 8
+    assert _comms.ops.head(x.float(), w.float(), t, 4096) is None
+    assert _comms.ops.head(x, w, t.int(), 4096) is None
+    with torch.autocast("cuda", torch.bfloat16):
+        assert _comms.ops.head(x, w, t, 4096) is None
+    for cols in (64, 60):  # both ways through the public entry point
+        xs, ws = x[:, :cols].contiguous().requires_grad_(True), w[:, :cols].contiguous().requires_grad_(True)
+        loss = fused.linear_cross_entropy(xs, ws, t)
+        dx, dw = torch.autograd.grad(loss, (xs, ws))
+        ref = _reference(xs.detach(), ws.detach(), t)
+        assert abs(float(loss.detach().double() - ref[0])) < 2e-2  # the operators' logits are rounded first
+        for a, b in zip((dx, dw), ref[1:]):
+            assert float((a.double() - b).norm() / b.norm()) < 2**-8 + 2**-9 * 12

@@ -673,13 +673,177 @@ __global__ void __launch_bounds__(kCeMaxThreads, 2) k_cross_entropy(__nv_bfloat1
   }
 }
 
+// Rows whose shares' maxima and sums of exponentials are known (launch_head_logits): the gradient in one look, bound by one
+// read and one write of the logits. A block takes a vector of 16 logits per thread and the grid covers the logits once,
+// in the order of their addresses: 4096 x 128256 302 us by itself (6.9 TB/s); blocks that walk a row of their own take 338,
+// columns from the last, which L2 still holds, to the first 327. Up to kGradFused blocks each puts the log-sum-exp of its
+// row together while its logits are on their way (64 x 2000 4.0 us, 512 x 11008 7.4); more of them leave that to k_head_rows
+// (5.3 and 8.2 with both; 4096 x 1000 9.0 against 15.2, 4096 x 8000 26.5 against 34).
+constexpr int kGradThreads = 256, kGradFused = 2048;
+
+struct HeadGrad {
+  __nv_bfloat16* logits;
+  int64_t ld;
+  const int64_t* targets;
+  const float2* stats;
+  const float* target_logit;
+  float* row_lse;   // [rows], where k_head_rows runs
+  float* row_loss;
+  float* loss;
+  uint32_t* words;
+  int rows, shares, vocab, parts, first;
+  float grad_scale, loss_scale;
+};
+
+// What several shares of a row are together.
+__device__ __forceinline__ void head_join(float2& a, float2 b) {
+  const float top = fmaxf(a.x, b.x);
+  a.y = (a.x == -INFINITY ? a.y : a.y * __expf(a.x - top)) + (b.x == -INFINITY ? b.y : b.y * __expf(b.x - top));
+  a.x = top;
+}
+__device__ __forceinline__ float head_lse(const HeadGrad& a, float2 row) {
+  return a.words[0] != 0u ? NAN : row.x + logf(row.y);  // the product gave up a wait: its logits are not to be used
+}
+
+__device__ __forceinline__ bool head_ignores(const HeadGrad& a, int64_t target) { return target < 0 || target >= a.vocab; }
+
+// Counts `rows` rows whose loss threads of this block have written and fenced; the block that finds all counted adds them up, in an
+// order that does not depend on which block it is. Every thread of the block calls it.
+__device__ __forceinline__ void head_add_up(const HeadGrad& a, int rows, float* scratch) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(a.words + 2, static_cast<uint32_t>(rows)) + static_cast<uint32_t>(rows) == static_cast<uint32_t>(a.rows);
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  float total = 0.0f;
+  for (int i = threadIdx.x; i < a.rows; i += blockDim.x) total += __ldcg(a.row_loss + i);
+  total = block_sum(total, scratch) * a.loss_scale;
+  if (threadIdx.x == 0) *a.loss = a.first != 0 ? total : *a.loss + total;
+}
+
+// 32 rows a block, one per lane; the warps take the shares in turn.
+__global__ void __launch_bounds__(512) k_head_rows(HeadGrad a) {
+  __shared__ float scratch[32];
+  __shared__ float2 part[16][32];
+  grid_release();
+  grid_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
+  float2 sum = make_float2(-INFINITY, 0.0f);
+  if (r < a.rows) {
+#pragma unroll 4
+    for (int t = warp; t < a.shares; t += 16) head_join(sum, a.stats[static_cast<size_t>(t) * a.rows + r]);
+  }
+  part[warp][lane] = sum;
+  __syncthreads();
+  if (warp == 0 && r < a.rows) {
+    for (int w = 1; w < 16; ++w) head_join(sum, part[w][lane]);
+    const float lse = head_lse(a, sum);
+    a.row_lse[r] = lse;
+    a.row_loss[r] = head_ignores(a, a.targets[r]) ? 0.0f : lse - a.target_logit[r];
+    __threadfence();
+  }
+  head_add_up(a, min(32, a.rows - static_cast<int>(blockIdx.x) * 32), scratch);
+}
+
+template <bool LSE_KNOWN>
+__global__ void __launch_bounds__(kGradThreads) k_head_gradient(HeadGrad a) {
+  __shared__ float scratch[32];
+  __shared__ float shared_lse;
+  grid_release();
+  grid_wait();
+  const int r = blockIdx.x / a.parts, part = blockIdx.x - r * a.parts, v = part * blockDim.x + threadIdx.x;
+  const bool there = v < (a.vocab + 15) / 16;
+  __nv_bfloat16* at = a.logits + static_cast<int64_t>(r) * a.ld + static_cast<int64_t>(v) * 16;
+  uint4 q[2];
+  if (there) ld32(at, q[0], q[1]);
+  const int64_t tgt = a.targets[r];
+  const bool ignore = head_ignores(a, tgt);
+  if (!LSE_KNOWN) {
+    if (threadIdx.x < 32) {
+      float2 sum = make_float2(-INFINITY, 0.0f);
+      for (int t = threadIdx.x; t < a.shares; t += 32) head_join(sum, a.stats[static_cast<size_t>(t) * a.rows + r]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        head_join(sum, make_float2(__shfl_xor_sync(0xffffffffu, sum.x, o), __shfl_xor_sync(0xffffffffu, sum.y, o)));
+      }
+      if (threadIdx.x == 0) {
+        shared_lse = head_lse(a, sum);
+        if (part == 0) {
+          a.row_loss[r] = ignore ? 0.0f : shared_lse - a.target_logit[r];
+          __threadfence();
+        }
+      }
+    }
+    __syncthreads();
+  }
+  const float lse = LSE_KNOWN ? a.row_lse[r] : shared_lse;
+  const float gs = ignore ? 0.0f : a.grad_scale;
+  if (there) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float f[8];
+      unpack8(q[h], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = __expf(f[i] - lse);
+      if (!ignore && v * 2 + h == static_cast<int>(tgt / 8)) {
+        const int c = static_cast<int>(tgt % 8);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] -= i == c ? 1.0f : 0.0f;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] *= gs;
+      q[h] = pack8(f);
+    }
+    st32(at, q[0], q[1]);
+  }
+  if (!LSE_KNOWN && part == 0) head_add_up(a, 1, scratch);
+}
+
+// dx[r, :] = bf16(part[r, :] + sum over j < depth of grad[r, j] * w[j, :]): the last few (depth < 8) columns of a vocabulary
+// that is no multiple of 8, whose product with the others would lose its tiled loads and, summed by itself and rounded,
+// its accuracy (512 x 4096 x 6007: 1.78e-3 off, so 1.66e-3 like any product of 8 columns more). Columns in vectors of 8.
+__global__ void __launch_bounds__(256) k_head_tail(const float* part, const __nv_bfloat16* grad, int64_t ld, const __nv_bfloat16* w,
+                                                    __nv_bfloat16* dx, uint32_t total, FastDiv per_row, int depth) {
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= total) return;
+  const uint32_t r = fast_div(i, per_row), c = i - r * per_row.d;
+  float sum[8];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float4 p = reinterpret_cast<const float4*>(part)[2 * static_cast<size_t>(i) + h];
+    sum[4 * h] = p.x;
+    sum[4 * h + 1] = p.y;
+    sum[4 * h + 2] = p.z;
+    sum[4 * h + 3] = p.w;
+  }
+  for (int j = 0; j < depth; ++j) {
+    const float g = __bfloat162float(grad[r * ld + j]);
+    float f[8];
+    unpack8(reinterpret_cast<const uint4*>(w)[static_cast<size_t>(j) * per_row.d + c], f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sum[k] = __fmaf_rn(g, f[k], sum[k]);
+  }
+  reinterpret_cast<uint4*>(dx)[i] = pack8(sum);
+}
+
 // out = in * bf16(*factor) for n bf16 values, the factor on the device. Both pointers 16-byte aligned; out may be
 // in, and then a factor of one (the gradient of a loss that is differentiated directly) leaves nothing to do.
 // Blocks stride over the data: with nothing to do, the 64 thousand blocks that cover a 1 GB gradient once take 45 us
 // to start and end, these 5.
-__global__ void __launch_bounds__(256) k_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* __restrict__ factor,
-                                                     size_t n) {
+struct ScaleSpan {
+  const __nv_bfloat16* in;
+  __nv_bfloat16* out;
+  size_t n;
+};
+__global__ void __launch_bounds__(256) k_scale_bf16(ScaleSpan a, ScaleSpan b, const float* __restrict__ factor) {
   const float f = __bfloat162float(__float2bfloat16_rn(*factor));
+  const ScaleSpan span = blockIdx.y == 0 ? a : b;
+  const __nv_bfloat16* in = span.in;
+  __nv_bfloat16* out = span.out;
+  const size_t n = span.n;
   if (f == 1.0f && in == out) return;
   const size_t nvec = n / 8, stride = static_cast<size_t>(gridDim.x) * 256;
   size_t v = blockIdx.x * static_cast<size_t>(256) + threadIdx.x;
@@ -1167,10 +1331,43 @@ cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, int64_t ld, cons
   return cudaGetLastError();
 }
 
-cudaError_t launch_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* factor, size_t n, cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) return cudaErrorMisalignedAddress;
-  k_scale_bf16<<<std::min<unsigned>(covering_grid(n / 8, 256 * 4), kSms * 8), 256, 0, s>>>(in, out, factor, n);
+cudaError_t launch_head_gradient(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, const float2* stats, int shares,
+                                 const float* target_logit, float* row_scratch, float* loss, uint32_t* words, int rows, int vocab,
+                                 float grad_scale, float loss_scale, bool first, cudaStream_t s) {
+  if (rows <= 0 || vocab <= 0 || shares <= 0 || ld % 16 != 0 || ld < vocab) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(logits) & 31u) != 0) return cudaErrorMisalignedAddress;
+  const int nvec = (vocab + 15) / 16, threads = std::min(kGradThreads, (nvec + 31) / 32 * 32), parts = (nvec + threads - 1) / threads;
+  if (static_cast<int64_t>(rows) * parts > INT32_MAX) return cudaErrorInvalidValue;
+  const HeadGrad a{logits, ld, targets, stats, target_logit, row_scratch, row_scratch + rows, loss, words, rows, shares, vocab, parts,
+                   first ? 1 : 0, grad_scale, loss_scale};
+  const unsigned grid = static_cast<unsigned>(rows) * static_cast<unsigned>(parts);
+  if (grid > kGradFused) {
+    launch_early(k_head_rows, static_cast<unsigned>((rows + 31) / 32), 512, s, a);
+    note_kernel_launch();
+    launch_early(k_head_gradient<true>, grid, threads, s, a);
+  } else {
+    launch_early(k_head_gradient<false>, grid, threads, s, a);
+  }
+  note_kernel_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_head_tail(const float* part, const __nv_bfloat16* grad, int64_t ld, const __nv_bfloat16* w, __nv_bfloat16* dx, int rows,
+                             int cols, int depth, cudaStream_t s) {
+  if (cols <= 0 || cols % 8 != 0) return cudaErrorInvalidValue;
+  if (misaligned16(part, w, dx)) return cudaErrorMisalignedAddress;
+  return for_row_slices(rows, cols / 8, [&](size_t r0, uint32_t total) {
+    k_head_tail<<<covering_grid(total, 256), 256, 0, s>>>(part + r0 * cols, grad + static_cast<int64_t>(r0) * ld, ld, w, dx + r0 * cols, total,
+                                                          make_fast_div(cols / 8), depth);
+  });
+}
+
+cudaError_t launch_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* factor, size_t n, cudaStream_t s,
+                              const __nv_bfloat16* in2, __nv_bfloat16* out2, size_t n2) {
+  if (n == 0 && n2 == 0) return cudaSuccess;
+  if (misaligned16(in, out, in2, out2)) return cudaErrorMisalignedAddress;
+  const dim3 grid(std::min<unsigned>(covering_grid(std::max(n, n2) / 8, 256 * 4), kSms * 8), n2 != 0 ? 2 : 1);
+  k_scale_bf16<<<grid, 256, 0, s>>>(ScaleSpan{in, out, n}, ScaleSpan{in2, out2, n2}, factor);
   note_kernel_launch();
   return cudaGetLastError();
 }

@@ -61,8 +61,22 @@ cudaError_t launch_swiglu_bwd(const __nv_bfloat16* dh, const __nv_bfloat16* gate
 cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, float* loss, int rows,
                                          int vocab, float grad_scale, cudaStream_t s);
 
-// out = in * bf16(*factor) on n bf16 values, the factor read from device memory; in and out 16-byte aligned.
-cudaError_t launch_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* factor, size_t n, cudaStream_t s);
+// The same where launch_head_logits (tc_gemm.h) left the logits with their statistics: row stride `ld` a multiple of 16,
+// logits on a 32-byte boundary; up to 15 elements past a row's last, within its stride, are overwritten. `row_scratch`:
+// 2 * rows; *loss becomes loss_scale times the sum of the rows' losses, added to what it holds unless `first`.
+cudaError_t launch_head_gradient(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, const float2* stats, int shares,
+                                 const float* target_logit, float* row_scratch, float* loss, uint32_t* words, int rows, int vocab,
+                                 float grad_scale, float loss_scale, bool first, cudaStream_t s);
+
+// dx[rows, cols] (bf16) = part (fp32) + grad[rows, depth] (row stride `ld`) x w[depth, cols], both bf16; cols % 8 == 0,
+// part, w and dx 16-byte aligned.
+cudaError_t launch_head_tail(const float* part, const __nv_bfloat16* grad, int64_t ld, const __nv_bfloat16* w, __nv_bfloat16* dx, int rows,
+                             int cols, int depth, cudaStream_t s);
+
+// out = in * bf16(*factor) on n bf16 values, the factor read from device memory; in and out 16-byte aligned. Optionally
+// a second tensor by the same factor.
+cudaError_t launch_scale_bf16(const __nv_bfloat16* in, __nv_bfloat16* out, const float* factor, size_t n, cudaStream_t s,
+                              const __nv_bfloat16* in2 = nullptr, __nv_bfloat16* out2 = nullptr, size_t n2 = 0);
 
 // AdamW on flat fp32 tensors, 16-byte aligned from four elements on. `grad_scale` multiplies the gradient first
 // (loss scaling / averaging); `step` starts at 1.

@@ -48,11 +48,12 @@ inline EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-inline bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+// `ld`: elements from row to row, a multiple of 8 (0: rows follow one another).
+inline bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint64_t ld = 0) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr) return false;
   const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * 2};
+  const cuuint64_t strides[1] = {(ld != 0 ? ld : cols) * 2};
   const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBlockK), box_rows};
   const cuuint32_t elem[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,

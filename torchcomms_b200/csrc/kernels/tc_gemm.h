@@ -52,6 +52,14 @@ cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, in
 int pairs_at_once(bool fp8);
 bool pair_tiles_fit(int m, int n, bool fp8);
 
+// Logits of a head on CTA pairs: logits[m, n] (bf16, row stride `ld`, a multiple of 8) = x[m, k] x w[n, k]^T, any n, k % 8 ==
+// 0. Also, from the fp32 accumulators, for each of head_row_shares(m, n) shares of a row the maximum and the sum of
+// exp(logit - maximum) (`stats`, [shares, m]), and the logit of the row's target (`target_logit`, where targets[row] is in
+// [0, n)). `words`: status as above, then a counter that launch_head_gradient counts rows in; all cleared by the kernel.
+int head_row_shares(int m, int n);
+cudaError_t launch_head_logits(const void* x, const void* w, void* logits, int64_t ld, const int64_t* targets, int m, int n, int k,
+                               float2* stats, float* target_logit, uint32_t* words, cudaStream_t stream);
+
 // Column-parallel layer fused with the all-gather of its input.
 // x_shards[r] is rank r's [m_local, k] bf16 activation shard in symmetric
 // memory (x_shards[rank] local); `x_full` is local scratch [nranks*m_local, k]

@@ -18,6 +18,12 @@
 // the leader's commits (arrival delivered to both CTAs); `acc_empty` lives in
 // the leader and collects the eight epilogue warps of the pair.
 // No load uses cluster multicast.
+//
+// With STATS the product is a head's logits, and the epilogue, which holds a row of the tile in every thread, also leaves
+// each row's maximum and sum of exponentials over the tile and the logit of its target: the loss then needs one look
+// at the logits instead of two. One set of epilogue warps takes 405 us for 4096 x 128256 x 256 with one barrier more a chunk,
+// two sets that share a tile's columns 348, two that take the tiles in turn 315 (the plain product 257); 4096 x 128256 x 4096
+// 2700 to 2790, by the clock that the exponentials' power leaves (plain 2650).
 #include "tc_gemm.h"
 
 #include <algorithm>
@@ -36,18 +42,27 @@ using namespace tc;
 constexpr int kABytes = kBlockM * kBlockK * 2;  // 16 KB: this CTA's 128 rows of A
 constexpr int kOutChunkCols = 64;
 constexpr int kOutChunkBytes = kBlockM * kOutChunkCols * 2;
-constexpr int kThreads = 192;
+// Warps of the epilogue: four, one for each quarter of the tensor memory's lanes, or two such sets that take the tiles, and
+// with them the two accumulators, in turn.
+template <bool STATS>
+constexpr int epilogue_sets() { return STATS ? 2 : 1; }
+template <bool STATS>
+constexpr int pair_threads() { return 64 + 128 * epilogue_sets<STATS>(); }
 constexpr int kAccCols = 256;  // tensor-memory columns of one accumulator
 
-constexpr int kStages = 6;
+// Stages of the TMA ring. With two sets of epilogue warps one of six makes room for two staging buffers each: with six stages
+// and one buffer 4096 x 128256 x 256 takes 361 us, so 315; x 4096 the same either way.
+template <bool STATS>
+constexpr int pair_stages() { return STATS ? 5 : 6; }
 
 // Shared memory for tiles of BN columns: each CTA holds half of the B tile. (Eight stages, which tiles of 128 columns
 // leave room for, gain nothing: 512 x 4096 x 4096 in e4m3 15.1 us either way.)
-template <int BN>
+template <int BN, bool STATS>
 struct PairTile {
+  static constexpr int kStages = pair_stages<STATS>(), kOutBuffers = 2 * epilogue_sets<STATS>();
   static constexpr int kBHalfBytes = (BN / 2) * kBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBHalfBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 2 * kOutChunkBytes + 1024 + 256 + BN * 4;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kOutBuffers * kOutChunkBytes + 1024 + 256 + BN * 4;
 };
 
 struct PairBarriers {
@@ -74,6 +89,70 @@ struct PairParams {
   int m, n, k, gm;  // k in 16-bit units
   int clear;        // the status words are this call's own
   int stage_bytes;  // of one K step's loads, both CTAs together
+  float2* stats;    // STATS: [shares of a row, m] maximum and sum of exponentials; per row its target and the target's logit
+  const int64_t* targets;
+  float* target_logit;
+};
+
+// Maximum and sum of exp(x - maximum) of what a row has shown so far, NaN where one was among it. Two elements per
+// addition and product, two per maximum: the exponentials then take more of the time than what is around them.
+struct RowStats {
+  float mx = -INFINITY, sum = 0.0f;
+  __device__ __forceinline__ void feed(const uint32_t (&r)[32]) {
+    float m[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = fmaxf(__uint_as_float(r[i]), __uint_as_float(r[i + 4]));
+#pragma unroll
+    for (int i = 8; i < 32; i += 8) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) m[j] = max3(m[j], __uint_as_float(r[i + j]), __uint_as_float(r[i + j + 4]));
+    }
+    const float top = fmaxf(max3(m[0], m[1], m[2]), m[3]);
+    if (top > mx) {
+      if (mx != -INFINITY) sum *= __expf(mx - top);
+      mx = top;
+    }
+    constexpr float kLog2e = 1.44269504f;
+    const float shift = mx == -INFINITY ? 0.0f : -mx;
+    float2 s[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      const float2 x = mul2(add2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), make_float2(shift, shift)),
+                            make_float2(kLog2e, kLog2e));
+      s[i / 2 % 2] = add2(s[i / 2 % 2], make_float2(exp2_fast(x.x), exp2_fast(x.y)));
+    }
+    sum += (s[0].x + s[0].y) + (s[1].x + s[1].y);
+  }
+  static __device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+  }
+  static __device__ __forceinline__ float exp2_fast(float x) {
+    float d;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(x));
+    return d;
+  }
+  static __device__ __forceinline__ unsigned long long both(float2 v) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(v.x), "f"(v.y));
+    return d;
+  }
+  static __device__ __forceinline__ float2 apart(unsigned long long v) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+    return d;
+  }
+  static __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(both(a)), "l"(both(b)));
+    return apart(d);
+  }
+  static __device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(both(a)), "l"(both(b)));
+    return apart(d);
+  }
 };
 
 // Pair-tile `t` of the schedule: groups of `gm` 256-row tiles, n-major inside a group.
@@ -87,16 +166,23 @@ __device__ __forceinline__ void pair_tile_at(int t, int tiles_m, int tiles_n, in
   *pn = rem / gsz;
 }
 
-template <bool FP8, int BN>
-__global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant__ PairMaps maps, PairParams p) {
+// The 128 threads of one set of epilogue warps.
+__device__ __forceinline__ void epilogue_sync(int set) {
+  if (set == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+  else asm volatile("bar.sync 2, 128;" ::: "memory");
+}
+
+template <bool FP8, int BN, bool STATS>
+__global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __grid_constant__ PairMaps maps, PairParams p) {
   constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(2 * kBlockM, BN) : make_idesc_bf16(2 * kBlockM, BN);
-  constexpr int kStageBytes = PairTile<BN>::kStageBytes;
+  using Tile = PairTile<BN, STATS>;
+  constexpr int kStages = Tile::kStages, kStageBytes = Tile::kStageBytes, kOutBuffers = Tile::kOutBuffers;
   extern __shared__ char smem_raw[];
   // The carve-up must be identical in both CTAs (the MMA addresses both with one descriptor).
   char* stages = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   char* obuf = stages + kStages * kStageBytes;
-  PairBarriers* bars = reinterpret_cast<PairBarriers*>(obuf + 2 * kOutChunkBytes);
-  float* col_scales = reinterpret_cast<float*>(obuf + 2 * kOutChunkBytes + 256);  // e4m3: of the tile in the epilogue
+  PairBarriers* bars = reinterpret_cast<PairBarriers*>(obuf + kOutBuffers * kOutChunkBytes);
+  float* col_scales = reinterpret_cast<float*>(obuf + kOutBuffers * kOutChunkBytes + 256);  // e4m3: of the tile in the epilogue
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();  // 0 leads
   const bool leader = cta == 0;
@@ -129,6 +215,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
   grid_release();
   grid_wait();  // everything above may run while the kernel in front still does
   if (p.clear != 0) clear_status(p.status);
+  if (STATS && blockIdx.x == 0 && threadIdx.x == 2) p.status[2] = 0u;  // rows whose loss is known
   if (threadIdx.x == 0) trace_stamp_ns(p.trace, 0);
 
   if (warp == 0) {
@@ -197,43 +284,83 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
     // ---------------- epilogue (both CTAs, own 128 rows)
     const int q = warp & 3;
     const int row_in_tile = q * 32 + lane;
-    const bool issuer = warp == 2 && lane == 0;
-    const int et = static_cast<int>(threadIdx.x) - 64;
-    const auto first_col = [&](int t) {
+    constexpr int kSets = epilogue_sets<STATS>();
+    const int set = kSets == 1 ? 0 : (warp - 2) >> 2;
+    const bool issuer = (warp & 3) == 2 && lane == 0;
+    const int et = static_cast<int>(threadIdx.x) - 64;  // (one set: the column scales)
+    // What a row brings along is fetched a tile ahead: its scale, or the column its target has in the tile's row of tiles.
+    const auto rows_of = [&](int t) {
       int pm, pn;
       pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
-      return pn * BN;
+      return make_int2((pm * 2 + static_cast<int>(cta)) * kBlockM, pn * BN);
     };
     ColScales<BN> fetched;
-    if (FP8 && cluster_id < total_tiles) fetched.fetch(p.scale_b, first_col(cluster_id), p.n, et);
-    uint32_t tile_iter = 0, chunk_iter = 0;
-    for (int t = cluster_id; t < total_tiles; t += nclusters, ++tile_iter) {
+    float next_scale = 0.0f;
+    int64_t next_target = -1;
+    const auto fetch = [&](int t) {
+      const int2 at = rows_of(t);
+      const int row = at.x + row_in_tile;
+      if (FP8) {
+        fetched.fetch(p.scale_b, at.y, p.n, et);
+        next_scale = row < p.m ? p.scale_a[row] : 0.0f;
+      }
+      if (STATS) next_target = row < p.m ? p.targets[row] : -1;
+    };
+    const int first = cluster_id + set * nclusters, step = kSets * nclusters;
+    if (first < total_tiles) fetch(first);
+    uint32_t tile_iter = static_cast<uint32_t>(set), chunk_iter = 0;
+    for (int t = first; t < total_tiles; t += step, tile_iter += kSets) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
-      int pm, pn;
-      pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
+      const int2 at = rows_of(t);
+      const int out_row = at.x, out_col = at.y;
+      const float row_scale = next_scale;
+      const int target = next_target >= 0 && next_target < p.n ? static_cast<int>(next_target) - out_col : -1;  // column of the tile
       if (FP8) {
         fetched.put(col_scales, et);
-        if (t + nclusters < total_tiles) fetched.fetch(p.scale_b, first_col(t + nclusters), p.n, et);
+        epilogue_sync(set);
       }
+      if (t + step < total_tiles) fetch(t + step);
       if (!mbar_wait(&bars->acc_full[as], aph)) {
         bars->failed = 1;
         break;
       }
       tc_fence_after_sync();
-      const int out_row = (pm * 2 + static_cast<int>(cta)) * kBlockM;
-      const float row_scale = FP8 && out_row + row_in_tile < p.m ? p.scale_a[out_row + row_in_tile] : 0.0f;
+      RowStats row_stats;
+      const bool row_there = STATS && out_row + row_in_tile < p.m;
       for (int j = 0; j < BN / kOutChunkCols; ++j, ++chunk_iter) {
-        char* buf = obuf + (chunk_iter & 1u) * kOutChunkBytes;
-        if (issuer) tma_store_wait_read<1>();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        char* buf = obuf + (2 * set + (chunk_iter & 1u)) * kOutChunkBytes;
+        uint32_t acc[2][32];
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-          uint32_t r[32];
           tmem_ld_32x32(tmem_base + as * kAccCols + (static_cast<uint32_t>(q * 32) << 16) +
                             static_cast<uint32_t>(j * kOutChunkCols + half * 32),
-                        r);
-          tmem_ld_wait();
+                        acc[half]);
+        }
+        tmem_ld_wait();
+        if (j == BN / kOutChunkCols - 1) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_leader(&bars->acc_empty[as]);
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t(&r)[32] = acc[half];
           if (FP8) scale_acc32(r, row_scale, col_scales + j * kOutChunkCols + half * 32);
+          if constexpr (STATS) {
+            const int col = j * kOutChunkCols + half * 32;
+            const int past = p.n - out_col - col;  // columns beyond the last are zeros of the tile, not logits
+            if (past < 32) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) r[i] = i < past ? r[i] : 0xff800000u;
+            }
+            if (row_there) row_stats.feed(r);
+            if (row_there && target >= col && target < col + 32) {
+              float z = 0.0f;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) z = target == col + i ? __uint_as_float(r[i]) : z;
+              p.target_logit[out_row + row_in_tile] = z;
+            }
+          }
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             const int chunk16 = half * 4 + v;
@@ -242,18 +369,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_pair(const __grid_constant
                               pack_bf16(r[8 * v + 4], r[8 * v + 5]), pack_bf16(r[8 * v + 6], r[8 * v + 7]));
           }
         }
-        if (j == BN / kOutChunkCols - 1) {
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_leader(&bars->acc_empty[as]);
-        }
         fence_proxy_async_smem();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (issuer) {
-          if (out_row < p.m && pn * BN + j * kOutChunkCols < p.n) tma_store_2d(&maps.out, buf, pn * BN + j * kOutChunkCols, out_row);
-          // Nothing to store outside the matrix, but an empty group all the same: the wait above counts groups.
+        // The other buffer is free once the store before this one has been read: one meeting per chunk says both that
+        // and that this one is full.
+        if (issuer) tma_store_wait_read<0>();
+        epilogue_sync(set);
+        if (issuer && out_row < p.m && out_col + j * kOutChunkCols < p.n) {
+          tma_store_2d(&maps.out, buf, out_col + j * kOutChunkCols, out_row);
           tma_store_commit();
         }
+      }
+      if (row_there) {
+        p.stats[static_cast<size_t>(out_col / BN) * p.m + out_row + row_in_tile] = make_float2(row_stats.mx, row_stats.sum);
       }
     }
     if (issuer) {
@@ -276,7 +403,7 @@ constexpr int kDevices = 64;  // whose answers are kept
 
 // Pairs that the current GPU holds at once (each CTA fills an SM), or 0 after an error. Kept per device; a query that
 // failed is asked again at the next call.
-template <bool FP8, int BN>
+template <bool FP8, int BN, bool STATS = false>
 int resident_pairs() {
   static std::atomic<int> known[kDevices];
   int device = 0, n = 0;
@@ -284,35 +411,36 @@ int resident_pairs() {
   std::atomic<int>* kept = device >= 0 && device < kDevices ? &known[device] : nullptr;
   if (kept != nullptr) n = kept->load(std::memory_order_acquire);
   if (n > 0) return n;
-  if (cudaFuncSetAttribute(k_gemm_pair<FP8, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairTile<BN>::kSmemBytes) != cudaSuccess) return 0;
+  if (cudaFuncSetAttribute(k_gemm_pair<FP8, BN, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairTile<BN, STATS>::kSmemBytes) != cudaSuccess) return 0;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = PairTile<BN>::kSmemBytes;
+  cfg.blockDim = dim3(pair_threads<STATS>());
+  cfg.dynamicSmemBytes = PairTile<BN, STATS>::kSmemBytes;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, k_gemm_pair<FP8, BN>, &cfg) != cudaSuccess || n < 1) return 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_gemm_pair<FP8, BN, STATS>, &cfg) != cudaSuccess || n < 1) return 0;
   if (kept != nullptr) kept->store(n, std::memory_order_release);
   return n;
 }
 
-template <bool FP8, int BN>
-cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cudaStream_t stream) {
-  const int pairs = resident_pairs<FP8, BN>();
+// `ldc`: row stride of the output in elements (0: n).
+template <bool FP8, int BN, bool STATS = false>
+cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cudaStream_t stream, int64_t ldc = 0) {
+  const int pairs = resident_pairs<FP8, BN, STATS>();
   if (pairs < 1) {
     const cudaError_t e = cudaGetLastError();
     return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
   }
   PairMaps maps;
-  if (!make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m)) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.out, c, p.m, p.n, kBlockM)) {
+  if (!make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m)) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.out, c, p.m, p.n, kBlockM, ldc)) {
     return cudaErrorInvalidValue;
   }
-  p.stage_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN>::kBHalfBytes);
+  p.stage_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN, STATS>::kBHalfBytes);
   const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / BN + 1;
   // A rows of a group stay in L2 while the pairs sweep over n: at most 8 pair-tiles and ~40 MB. Every group reads B again,
   // so where L2 does not keep that either (above 48 MB) groups are of up to 16 pair-tiles and 32 MB. In us under the power
@@ -323,8 +451,8 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
   p.gm = std::max(1, std::min({b_again ? 16 : 8, tiles_m, static_cast<int>((b_again ? 32u << 20 : 40u << 20) / std::max<size_t>(a_tile_bytes, 1))}));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(pairs, static_cast<int64_t>(tiles_m) * tiles_n)));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = PairTile<BN>::kSmemBytes;
+  cfg.blockDim = dim3(pair_threads<STATS>());
+  cfg.dynamicSmemBytes = PairTile<BN, STATS>::kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -335,7 +463,7 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gemm_pair<FP8, BN>, maps, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gemm_pair<FP8, BN, STATS>, maps, p);
   note_kernel_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -366,6 +494,30 @@ cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, in
   p.k = k;
   if (narrow) return scale_a != nullptr ? launch_pair<true, 128>(a, b, c, p, stream) : launch_pair<false, 128>(a, b, c, p, stream);
   return scale_a != nullptr ? launch_pair<true, 256>(a, b, c, p, stream) : launch_pair<false, 256>(a, b, c, p, stream);
+}
+
+int head_row_shares(int m, int n) {
+  const int bn = pair_tiles_fit(m, n, false) ? 128 : 256;
+  return (n - 1) / bn + 1;
+}
+
+cudaError_t launch_head_logits(const void* x, const void* w, void* logits, int64_t ld, const int64_t* targets, int m, int n, int k,
+                               float2* stats, float* target_logit, uint32_t* words, cudaStream_t stream) {
+  if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || ld % 8 != 0 || ld < n) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(logits)) & 15u) {
+    return cudaErrorMisalignedAddress;
+  }
+  PairParams p{};
+  p.status = words;
+  p.clear = 1;
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  p.stats = stats;
+  p.targets = targets;
+  p.target_logit = target_logit;
+  return pair_tiles_fit(m, n, false) ? launch_pair<false, 128, true>(x, w, logits, p, stream, ld)
+                                     : launch_pair<false, 256, true>(x, w, logits, p, stream, ld);
 }
 
 } // namespace b200c

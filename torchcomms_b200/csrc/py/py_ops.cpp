@@ -2,6 +2,7 @@
 #include "py_common.hpp"
 
 #include <ATen/SavedTensorHooks.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -293,6 +294,62 @@ struct RopeFn : torch::autograd::Function<RopeFn> {
   }
 };
 
+// Loss and gradients of a head, (loss, dx, dweight), on the framework's own logits kernel. Logits have rows of whole
+// 128-byte lines, so that every vocabulary's products are tiled ones: at odd row strides the tensor library's fall
+// back to two-element accesses. x: [rows, dim].
+bool head_applies(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& targets, int64_t chunk_rows) {
+  auto matrix = [&](const at::Tensor& t) {
+    return plain_call(t) && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.is_contiguous() && on16(t) && t.device() == x.device();
+  };
+  return matrix(x) && matrix(weight) && x.size(1) == weight.size(1) && x.size(1) % 8 == 0 && x.numel() > 0 && weight.size(0) > 0 &&
+      x.size(0) <= INT32_MAX && x.size(1) <= INT32_MAX && weight.size(0) <= INT32_MAX - 256 && chunk_rows >= 1 &&
+      !at::autocast::is_autocast_enabled(at::kCUDA) && plain_call(targets) && targets.scalar_type() == at::kLong &&
+      targets.dim() == 1 && targets.size(0) == x.size(0) && targets.is_contiguous() && targets.device() == x.device();
+}
+
+std::tuple<at::Tensor, at::Tensor, at::Tensor> head(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& targets,
+                                                    int64_t chunk_rows) {
+  c10::cuda::CUDAGuard g(x.device());
+  const int64_t rows = x.size(0), dim = x.size(1), vocab = weight.size(0), chunk = std::min(rows, chunk_rows), ld = (vocab + 63) / 64 * 64;
+  at::Tensor dx = at::empty_like(x), dw = at::empty_like(weight), loss = at::empty({}, x.options().dtype(at::kFloat));
+  const at::Tensor logits = at::empty({chunk, ld}, x.options());
+  // Statistics (the last chunk may take narrower tiles), then a target's logit and two words of scratch per row, then the
+  // kernels' words.
+  const int64_t last = rows - (rows - 1) / chunk * chunk;
+  const int64_t stat_words = 2 * std::max(chunk * head_row_shares(static_cast<int>(chunk), static_cast<int>(vocab)),
+                                          last * head_row_shares(static_cast<int>(last), static_cast<int>(vocab)));
+  const at::Tensor scratch = at::empty({stat_words + 3 * chunk + 4}, x.options().dtype(at::kFloat));
+  float* stats = scratch.data_ptr<float>();
+  float *target_logit = stats + stat_words, *row_scratch = target_logit + chunk;
+  auto* words = reinterpret_cast<uint32_t*>(row_scratch + 2 * chunk);
+  const float mean = 1.0f / static_cast<float>(rows);
+  for (int64_t r0 = 0; r0 < rows; r0 += chunk) {
+    const int n = static_cast<int>(std::min(chunk, rows - r0));
+    const int64_t* t = targets.data_ptr<int64_t>() + r0;
+    const at::Tensor xs = r0 == 0 && n == rows ? x : x.narrow(0, r0, n);
+    at::Tensor dxs = r0 == 0 && n == rows ? dx : dx.narrow(0, r0, n);
+    auto* z = reinterpret_cast<__nv_bfloat16*>(logits.data_ptr());
+    B200C_CUDA_CHECK(launch_head_logits(xs.data_ptr(), weight.data_ptr(), z, ld, t, n, static_cast<int>(vocab), static_cast<int>(dim),
+                                        reinterpret_cast<float2*>(stats), target_logit, words, cur(x)));
+    B200C_CUDA_CHECK(launch_head_gradient(z, ld, t, reinterpret_cast<float2*>(stats), head_row_shares(n, static_cast<int>(vocab)),
+                                          target_logit, row_scratch, loss.data_ptr<float>(), words, n, static_cast<int>(vocab), mean, mean,
+                                          r0 == 0, cur(x)));
+    const at::Tensor grad = logits.as_strided({n, vocab}, {ld, 1});
+    // A depth that is no multiple of 8 costs the product its tiled loads: the last few columns are added to its fp32 result.
+    const int64_t even = vocab / 8 * 8;
+    if (even == vocab || even == 0) {
+      at::mm_out(dxs, grad, weight);
+    } else {
+      const at::Tensor part = at::mm(grad.narrow(1, 0, even), weight.narrow(0, 0, even), at::kFloat);
+      B200C_CUDA_CHECK(launch_head_tail(part.data_ptr<float>(), z + even, ld, bf(weight) + even * dim, bf_mut(dxs), n, static_cast<int>(dim),
+                                        static_cast<int>(vocab - even), cur(x)));
+    }
+    if (r0 == 0) at::mm_out(dw, grad.t(), xs);  // the first chunk needs no zeroed gradient to add to
+    else dw.addmm_(grad.t(), xs);
+  }
+  return {loss, dx, dw};
+}
+
 } // namespace
 
 void bind_ops(py::module_& m) {
@@ -376,13 +433,29 @@ void bind_ops(py::module_& m) {
     return loss;
   });
 
+  // (loss, dx, dweight) of a head, or None where its kernels do not apply.
+  ops.def("head", [](const at::Tensor& x, const at::Tensor& weight, const at::Tensor& targets, int64_t chunk_rows)
+              -> std::optional<std::tuple<at::Tensor, at::Tensor, at::Tensor>> {
+    if (!head_applies(x, weight, targets, chunk_rows)) return std::nullopt;
+    return head(x, weight, targets, chunk_rows);
+  });
+
   // t * factor.to(t.dtype) for a 0-d factor on the device (the gradient of a loss). `consume`: nobody reads t
-  // afterwards, so the product may take its place.
+  // afterwards, so the product may take its place. scale_both_by: two tensors by one factor, in one launch.
+  static const auto scalable = [](const at::Tensor& t, const at::Tensor& factor) {
+    return plain_call(t) && plain_call(factor) && t.scalar_type() == at::kBFloat16 && t.is_non_overlapping_and_dense() && on16(t) &&
+        factor.dim() == 0 && factor.scalar_type() == at::kFloat && factor.device() == t.device();
+  };
+  ops.def("scale_both_by", [](const at::Tensor& t, const at::Tensor& u, const at::Tensor& factor, bool consume) {
+    if (!scalable(t, factor) || !scalable(u, factor)) return std::make_pair(t * factor.to(t.scalar_type()), u * factor.to(u.scalar_type()));
+    c10::cuda::CUDAGuard g(t.device());
+    at::Tensor a = consume ? t : at::empty_like(t), b = consume ? u : at::empty_like(u);
+    B200C_CUDA_CHECK(launch_scale_bf16(bf(t), bf_mut(a), factor.data_ptr<float>(), static_cast<size_t>(t.numel()), cur(t), bf(u), bf_mut(b),
+                                       static_cast<size_t>(u.numel())));
+    return std::make_pair(a, b);
+  });
   ops.def("scale_by", [](const at::Tensor& t, const at::Tensor& factor, bool consume) {
-    const bool direct = plain_call(t) && plain_call(factor) && t.scalar_type() == at::kBFloat16 &&
-        t.is_non_overlapping_and_dense() && on16(t) && factor.dim() == 0 &&
-        factor.scalar_type() == at::kFloat && factor.device() == t.device();
-    if (!direct) return t * factor.to(t.scalar_type());
+    if (!scalable(t, factor)) return t * factor.to(t.scalar_type());
     c10::cuda::CUDAGuard g(t.device());
     at::Tensor out = consume ? t : at::empty_like(t);  // same strides: dense tensors map element by element
     B200C_CUDA_CHECK(launch_scale_bf16(bf(t), bf_mut(out), factor.data_ptr<float>(), static_cast<size_t>(t.numel()), cur(t)));

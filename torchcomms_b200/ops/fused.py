@@ -174,11 +174,18 @@ class _LinearCrossEntropy(torch.autograd.Function):
     turns it in place into its own gradient while emitting the per-row loss,
     and two more GEMMs fold that gradient into ``dx`` and ``dW``.  The
     gradients are therefore ready when forward returns; backward only scales
-    them by the incoming gradient of the loss.
+    them by the incoming gradient of the loss.  bf16 heads on the GPU take
+    ``_comms.ops.head``, whose first GEMM leaves the statistics that the
+    gradient needs; what it does not take goes operator by operator.
     """
 
     @staticmethod
     def forward(ctx, x, weight, targets, chunk_rows):
+        out = _k.head(x, weight, targets, chunk_rows) if x.is_cuda and _native(x, weight, targets) else None
+        if out is not None:
+            ctx.save_for_backward(out[1], out[2])
+            ctx.own = not _k.saved_tensor_hooks_active()
+            return out[0]
         rows = x.shape[0]
         # Mean over all rows; rows with a negative target contribute zero.
         scale = 1.0 / max(rows, 1)
@@ -224,7 +231,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
             # A backward that frees the graph hands them out themselves; the gradient of the weight is the size of the
             # weight, and a copy of it would take longer than the loss kernel.
             last = ctx.own and not torch._C._autograd._get_current_graph_task_keep_graph()
-            return _k.scale_by(dx, dloss, last), _k.scale_by(dw, dloss, last), None, None
+            return *_k.scale_both_by(dx, dw, dloss, last), None, None
         return dx * dloss.to(dx.dtype), dw * dloss.to(dw.dtype), None, None
 
 
@@ -232,8 +239,8 @@ def linear_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: torch.T
     """Mean token cross-entropy of the logits ``x @ weight.T`` (``x``: [rows, dim]).
 
     The forward pass holds the logits of ``chunk_rows`` rows and the gradient of the weight; for a bf16 vocabulary that is
-    no multiple of 8 also, from the sizes of ``_worth_padding`` on, a padded copy of the weight (1 GB at 128257 x 4096).
-    A vocabulary padded by the caller needs none.
+    no multiple of 8 also their ``dx`` in fp32, and where the width is no multiple of 8 either, from the sizes of
+    ``_worth_padding`` on, a padded copy of the weight. A vocabulary padded by the caller needs neither.
     """
     return _LinearCrossEntropy.apply(x.contiguous(), weight, targets, chunk_rows)
 
