@@ -47,6 +47,14 @@ def test_dispatch_at_the_lines_between_block_sizes(tokens, hidden, fp8, monkeypa
     test_dispatch(tokens, hidden, fp8, 0, monkeypatch)
 
 
+# Both sides of the lines between shapes of blocks; rows of a quarter piece to three pieces and a bit.
+@pytest.mark.parametrize("tokens,hidden", [(592, 512), (593, 2560), (1185, 1536), (1186, 1024), (2072, 2048), (2073, 2560),
+                                           (2368, 1536), (2369, 4608), (2370, 6656)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_dispatch_at_the_lines_between_blocks(tokens, hidden, fp8, monkeypatch):
+    test_dispatch(tokens, hidden, fp8, 0, monkeypatch)
+
+
 @pytest.mark.parametrize("fp8", [False, True])
 def test_low_latency_outputs_can_be_saved_together(fp8, tmp_path, monkeypatch):
     """torch.save refuses tensors of different types over one storage; outputs that share an allocation are of one type."""

@@ -37,7 +37,7 @@ struct DispatchArgs {
   const int* topk_idx;    // [num_tokens, topk]
   const float* topk_w;    // [num_tokens, topk]
   int num_tokens;
-  int per_block;          // single rank: tokens of a block, at most kEpWarps
+  int per_block;          // single rank: tokens of a block, at most one per warp
 };
 
 // 16 bf16 of a lane to e4m3, with one scale per 128 elements (8 neighbouring lanes). Returns the scale.
@@ -248,25 +248,24 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_emu(const CommDev* c
 // A single rank: rows may stand in any order from 0, so a block numbers its own tokens with one atomic and sends them
 // at once, and nobody waits for anybody. The last block to finish leaves the count. An ordinary launch that covers
 // the tokens, where the general kernel is a cooperative one with grid-wide meetings (4096 tokens of 7168 to e4m3:
-// 23.3 us there, 21.1 us (4.2 TB/s) here; as they are 22.6 (5.2 TB/s), and 24.9 with two accesses of 16 bytes for a lane's
-// 32). How many tokens a block takes: solo_tokens_per_block(). Started early, a dispatch and a combine of 128 x 7168 to e4m3
-// through a communicator take 1.3 us less in a graph and 0.8 on the stream (11.2 and 20.1 us), of 4096 x 7168 2.0 and 3.1
-// (45.0 and 43.2).
+// 23.3 us there, 18.5 us (4.8 TB/s) here; as they are 20.4 (5.8 TB/s)). How many tokens a block takes: solo_blocks().
+// Started early, a dispatch and a combine of 128 x 7168 to e4m3 through a communicator take 1.3 us less in a graph and 0.8 on
+// the stream, of 4096 x 7168 2.0 and 3.1.
 
-template <bool WIDE, bool TRACE>
-__global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDev e, DispatchArgs a) {
-  constexpr int kSteps = kEpChunkCols / 512;
-  __shared__ int s_slot[kEpWarps];
+template <int THREADS, int COLS, bool WIDE, bool TRACE>
+__global__ void __launch_bounds__(THREADS) k_ep_dispatch_solo(CommDev c, EpDev e, DispatchArgs a) {
+  constexpr int kWarps = THREADS / 32, kSteps = COLS / 512;
+  __shared__ int s_slot[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t0 = blockIdx.x * a.per_block, here = min(a.per_block, a.num_tokens - t0);
-  const int groups = e.hidden / 128, nchunks = (e.hidden + kEpChunkCols - 1) / kEpChunkCols;
+  const int groups = e.hidden / 128, nchunks = (e.hidden + COLS - 1) / COLS;
   const size_t row_bytes = e.fp8 ? static_cast<size_t>(e.hidden) : static_cast<size_t>(e.hidden) * 2;
   grid_release();
   grid_wait();
   trace_mark<TRACE>(c, 0);  // the marks of the general kernel
   uint4 v0[kSteps], v1[kSteps];
   auto load = [&](int item) {
-    const int t = t0 + item / nchunks, col0 = (item % nchunks) * kEpChunkCols + lane * 16;
+    const int t = t0 + item / nchunks, col0 = (item % nchunks) * COLS + lane * 16;
     const __nv_bfloat16* xr = static_cast<const __nv_bfloat16*>(a.x) + static_cast<size_t>(t) * e.hidden;
 #pragma unroll
     for (int i = 0; i < kSteps; ++i) {
@@ -323,7 +322,7 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
     }
   }
   while (item < here * nchunks) {
-    const int slot = s_slot[item / nchunks], col0 = (item % nchunks) * kEpChunkCols + lane * 16;
+    const int slot = s_slot[item / nchunks], col0 = (item % nchunks) * COLS + lane * 16;
     if (slot >= 0) {
 #pragma unroll
       for (int i = 0; i < kSteps; ++i) {
@@ -339,7 +338,7 @@ __global__ void __launch_bounds__(kEpThreads) k_ep_dispatch_solo(CommDev c, EpDe
         }
       }
     }
-    item += kEpWarps;
+    item += kWarps;
     if (item < here * nchunks) load(item);
   }
   trace_mark<TRACE>(c, 3);
@@ -611,21 +610,31 @@ cudaError_t launch_coop(void* real_kernel, void* emu_kernel, const CommDev* comm
   return err != cudaSuccess ? err : e2;
 }
 
-// Tokens of a block of the single-rank dispatch, which share its start and its atomic and divide over its warps. Two as long
-// as all blocks are resident at once (a second wave costs about what the first does), then four. Eight from 5120 on; for
-// rows of 4096 and more only where blocks of four would not leave the last wave fuller (one of theirs that is at most a quarter
-// full does not count: 7105 x 7168 to e4m3 35.0 us with eight). In us, replayed from a graph
-// with what a captured call adds, 2 / 4 / 8: to e4m3 1000 x 1024 6.8 / 6.7 / 7.0, 1536 x 1024 8.7 / 7.2 / 7.4, 1000 x 7168
-// 9.3 / 9.9 / 11.9, 2048 x 7168 15.0 / 14.2 / 16.2, 8192 x 1024 24.2 / 15.2 / 11.8; as they are 5120 x 7168 29.5 / 30.2 /
-// 31.8, 8192 x 7168 42.4 / 41.9 / 42.8. Eight would pay from the end of the first wave of blocks of four on (4096 x 1024 to
-// e4m3 14.3 / 10.2 / 8.4, x 7168 25.0 / 22.5 / 21.5), but 4096 tokens are the batch whose phase trace is to show more
-// blocks than it has rows.
-int solo_tokens_per_block(int tokens, int hidden) {
-  constexpr int kResident = 148 * 4;
-  if (tokens <= 2 * kResident) return 2;
-  if (tokens < 5120) return 4;
-  const int waves8 = (tokens - 1) / (8 * kResident) + 1, waves4 = (tokens - 1 - kResident) / (4 * kResident) + 1;
-  return hidden >= 4096 && waves4 * 4 < waves8 * 8 ? 4 : 8;
+// Blocks of the single-rank dispatch. Tokens of a block share its start and its atomic, and a wave of blocks costs that
+// start once more. So while there is a shape whose blocks are all resident at once, it is the one with the fewest tokens a
+// block: blocks of eight warps that take pieces of 1024 columns, four per SM, with one, two or four tokens; between two and
+// four, blocks of four warps with two, which take pieces of 2048 columns, seven per SM (not for rows of 1024, which are half a
+// piece). Above, where several waves run anyway, blocks of four warps: more of them start while others move rows, with half as
+// many bytes again in flight; four tokens a block, two for bf16 rows of more than 4096 columns, which have more to move. In us a
+// launch, replayed from a graph of 24, on eight warps with the best of 2, 4 and 8 tokens, and so: to e4m3 64 x 7168 5.1 and 4.2,
+// 2048 x 7168 12.4 and 11.2, 3000 x 4096 12.4 and 10.8, 4096 x 7168 20.5 and 18.5, 6000 x 7168 28.7 and 26.8, 8192 x 4096 23.4
+// and 20.3; as they are 4096 x 7168 21.9 and 20.4, 8192 x 2560 17.8 and 16.3. Around the lines, to e4m3: 1185 x 7168 8.8 with
+// two tokens on four warps, 8.9 with four on eight, 2072 x 7168 11.5 and 12.7, 2200 x 7168 14.2 and 12.8, 2600 x 4096 10.0 (four
+// tokens on four warps) and 10.9, 2048 x 1024 5.3 and 4.8.
+struct SoloBlocks {
+  int threads, tokens;
+};
+SoloBlocks solo_blocks(int tokens, int hidden, bool fp8) {
+  constexpr int kWide = 148 * 4, kSlim = 148 * 7;  // resident at once: blocks of 256 and of 128 threads
+  if (tokens <= 2 * kWide) return {256, tokens <= kWide ? 1 : 2};
+  if (tokens <= 4 * kWide) return tokens <= 2 * kSlim && hidden > 1024 ? SoloBlocks{128, 2} : SoloBlocks{256, 4};
+  return {128, !fp8 && hidden > 4096 ? 2 : 4};
+}
+
+template <bool TRACE>
+auto solo_dispatch_kernel(int threads, bool wide) {
+  if (threads == 256) return wide ? k_ep_dispatch_solo<256, 1024, true, TRACE> : k_ep_dispatch_solo<256, 1024, false, TRACE>;
+  return wide ? k_ep_dispatch_solo<128, 2048, true, TRACE> : k_ep_dispatch_solo<128, 2048, false, TRACE>;
 }
 
 } // namespace
@@ -642,18 +651,13 @@ cudaError_t launch_ep_dispatch(const CommDev* comms, const EpDev* eps, int emu_r
   std::vector<DispatchArgs> args(n);
   for (int i = 0; i < n; ++i) args[i] = {x[i], topk_idx[i], topk_w[i], num_tokens, 0};
   if (emu_ranks <= 0 && e0.nranks == 1) {
-    const int per_block = solo_tokens_per_block(num_tokens, e0.hidden);
-    static_assert(kEpWarps >= 8, "a warp for every token of a block");
-    args[0].per_block = per_block;
-    const int blocks = std::max(1, (num_tokens + per_block - 1) / per_block);
-    // 32-byte loads (rows are multiples of 1024 bytes), but not of wide rows to e4m3 in several waves of blocks of four: in us
-    // with 16- and 32-byte loads 5120 x 7168 28.0 and 29.0, 7104 x 7168 32.2 and 33.4, but 2048 x 4096 9.9 and 9.4, 4096 x 1024
-    // 10.0 and 9.7, as they are 6000 x 7168 33.9 and 32.2.
-    const bool by16 = e0.fp8 && e0.hidden >= 4096 && per_block == 4 && blocks > 148 * 4;
-    const bool wide = reinterpret_cast<uintptr_t>(x[0]) % 32 == 0 && !by16;
-    const auto kernel = comms[0].trace != nullptr ? (wide ? k_ep_dispatch_solo<true, true> : k_ep_dispatch_solo<false, true>)
-                                                  : (wide ? k_ep_dispatch_solo<true, false> : k_ep_dispatch_solo<false, false>);
-    launch_early(kernel, static_cast<unsigned>(blocks), kEpThreads, stream, comms[0], e0, args[0]);
+    const SoloBlocks by = solo_blocks(num_tokens, e0.hidden, e0.fp8 != 0);  // at most a token per warp
+    args[0].per_block = by.tokens;
+    const int blocks = std::max(1, (num_tokens + by.tokens - 1) / by.tokens);
+    // 32-byte loads (rows are multiples of 1024 bytes).
+    const bool wide = reinterpret_cast<uintptr_t>(x[0]) % 32 == 0;
+    const auto kernel = comms[0].trace != nullptr ? solo_dispatch_kernel<true>(by.threads, wide) : solo_dispatch_kernel<false>(by.threads, wide);
+    launch_early(kernel, static_cast<unsigned>(blocks), static_cast<unsigned>(by.threads), stream, comms[0], e0, args[0]);
     note_kernel_launch();
     return cudaGetLastError();
   }
