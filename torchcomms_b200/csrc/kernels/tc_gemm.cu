@@ -387,7 +387,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
 
   if (warp == 0) {
     // ---------------- TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int t = blockIdx.x; t < total_tiles && !bars->failed; t += G) {
         const TileCoord tc_ = tile_at(t, tiles_m, tiles_n, p.gm);
@@ -429,7 +429,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, tile_iter = 0;
       for (int t = blockIdx.x; t < total_tiles && !bars->failed; t += G, ++tile_iter) {
         const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
@@ -800,7 +800,7 @@ __device__ __forceinline__ void tp_gemm_pair_body(const TpMaps& maps, const Comm
 
   if (warp == 0) {
     // ---------------- TMA producer: own A rows, own half of the B tile
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int t = cluster_id; t < total_tiles && !bars->failed; t += nclusters) {
         int ord, ni;
@@ -842,7 +842,7 @@ __device__ __forceinline__ void tp_gemm_pair_body(const TpMaps& maps, const Comm
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader only)
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       uint32_t it = 0, tile_iter = 0;
       for (int t = cluster_id; t < total_tiles && !bars->failed; t += nclusters, ++tile_iter) {
         const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;

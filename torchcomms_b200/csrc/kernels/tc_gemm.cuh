@@ -73,6 +73,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One thread of a converged warp, which the compiler knows to be one. TMA and tcgen05 instructions take their operands from
+// uniform registers; under `lane == 0` each of them is wrapped in a loop over the threads that might be there, and a K step of
+// four MMAs took 290 ns whatever the tile's width: in a pair kernel of one tile of 128 columns 290 ns and now 144, of 192 290 and
+// 214, of 256, which the tensor pipe bounds, 291 and 284.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier --
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

@@ -10,7 +10,7 @@
 // 4096 in bf16 309 (334). Tiles of 128 columns are for products whose tiles all
 // find a pair at once; a K step takes them as long, so a second wave does not pay.
 //
-// Roles per CTA (192 threads): warp 0 lane 0 TMA producer (both CTAs), warp 1
+// Roles per CTA (192 threads): warp 0 (one thread) TMA producer (both CTAs), warp 1
 // tensor-memory allocation (both CTAs) and MMA issue (leader only), warps 2-5
 // epilogue (both CTAs: tcgen05.ld -> bf16 -> swizzled staging -> TMA store).
 // Barriers: `full` lives in the leader and counts the bytes of all four loads
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
 
   if (warp == 0) {
     // ---------------- TMA producer (each CTA loads its own A rows and its half of B)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int t = cluster_id; t < total_tiles && !bars->failed; t += nclusters) {
         int pm, pn;
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       uint32_t it = 0, tile_iter = 0;
       for (int t = cluster_id; t < total_tiles && !bars->failed; t += nclusters, ++tile_iter) {
         const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;

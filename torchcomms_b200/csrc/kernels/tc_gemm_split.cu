@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
   if (TRACE && threadIdx.x == 0) trace_stamp_ns(p.trace, 0);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const int s = it % kSplitStages;
         const uint32_t ph = (it / kSplitStages) & 1u;
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
       if (TRACE) trace_stamp_ns(p.trace, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const int s = it % kSplitStages;
         const uint32_t ph = (it / kSplitStages) & 1u;
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
       if (TRACE) trace_stamp_ns(p.trace, 2);
     }
   } else {
-    if (p.copy_a != 0 && warp == 2 && lane == 0) {
+    if (p.copy_a != 0 && warp == 2 && elect_one()) {
       // Every column of tiles has all of A pass by; each passes the steps on whose turn it is.
       const int tiles_n = static_cast<int>(gridDim.x) / splits / p.tiles_m;
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
