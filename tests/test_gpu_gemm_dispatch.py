@@ -45,6 +45,49 @@ def test_plain_product_by_waves(m, n, k, fp8):
     test_plain_product(m, n, k, fp8)
 
 
+# Pairs in tiles of 192, 192, 224, 224 and 192 columns, the last tile of a few columns, of a row and of a K step's part; narrow
+# pairs where a shared sum would not pay, and where it does; unshared sums of few steps, and of few rows in many tiles.
+@pytest.mark.parametrize("m,n,k", [(1000, 6144, 136), (1000, 6152, 1096), (1500, 5000, 200), (257, 14344, 1096), (300, 20488, 72),
+                                   (256, 2816, 1280), (128, 4096, 1792), (3, 408, 376), (256, 1536, 192), (100, 6000, 320)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_plain_product_by_tile_width(m, n, k, fp8):
+    test_plain_product(m, n, k, fp8)
+
+
+# Tiles of 112, 96 and 128 columns of gate and of up, one of them in a row, ragged ends of rows, columns and K steps.
+@pytest.mark.parametrize("m,n,k", [(700, 5000, 768), (300, 4808, 72), (1000, 2056, 200), (1, 8, 8), (257, 120, 64), (2049, 232, 136)])
+def test_gated_product(m, n, k):
+    from torchcomms_b200 import _comms
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(2 * n, k, generator=g, device="cuda") * k**-0.5).to(torch.bfloat16)
+    gate_up, act, status = _comms.ops.gemm_gated(x, w)
+    assert int(status[0]) == 0
+    torch.testing.assert_close(gate_up.double(), x.double() @ w.double().t(), rtol=2**-8, atol=1e-6 * k)
+    # The activation from the rounded gate and up: an fp32 expression of five roundings, the exponential's and reciprocal's 2 ulp
+    # among them, then one to bf16, which may fall either way.
+    gate, up = gate_up.double().chunk(2, dim=-1)
+    torch.testing.assert_close(act.double(), torch.nn.functional.silu(gate) * up, rtol=2**-8, atol=1e-12)
+    again = _comms.ops.gemm_gated(x, w)
+    assert torch.equal(again[0], gate_up) and torch.equal(again[1], act)
+
+
+def test_gated_product_of_extremes():
+    """Gates whose exponential overflows or vanishes, zeros, infinities and NaN come out as from the activation kernel."""
+    from torchcomms_b200 import _comms
+
+    values = torch.tensor([0.0, -0.0, 1e-30, 87.0, -87.0, -89.0, -104.0, 300.0, -300.0, 1e38, -1e38, float("inf"), float("-inf"), float("nan")],
+                          device="cuda").to(torch.bfloat16)
+    x = torch.zeros(16, 8, device="cuda", dtype=torch.bfloat16)
+    x[: len(values), 0] = values
+    x[:, 1] = 1.0
+    w = torch.zeros(16, 8, device="cuda", dtype=torch.bfloat16)
+    w[:8, 0], w[8:, 1] = 1.0, 3.0
+    gate_up, act, _ = _comms.ops.gemm_gated(x, w)
+    torch.testing.assert_close(act, _comms.ops.swiglu_fwd(gate_up), rtol=2**-7, atol=0, equal_nan=True)
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 256, 64), (128, 3584, 4096), (384, 512, 704), (512, 5120, 512)])
 def test_gather_layer_leaves_its_input_behind(m, n, k):
     """A single rank's layer reads the activations where they are; its input buffer holds them afterwards all the same."""

@@ -1229,27 +1229,28 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   bool done = false;
   cudaError_t e = launch_gemm_nt_split(a, b, c, m, n, k, scale_a, scale_b, status, stream, &done, layer, a_copy);
   if (e != cudaSuccess || done) return e;
-  if (a_copy != nullptr) {
+  if (a_copy != nullptr && a_copy != a) {
     e = cudaMemcpyAsync(a_copy, a, static_cast<size_t>(m) * k * 2, cudaMemcpyDeviceToDevice, stream);
     if (e != cudaSuccess) return e;
   }
-  // A K step is 0.27 us of either, and a pair's covers twice the tile: so pairs, of 128 columns as long as each finds a pair
-  // at once, or else of 256. But pairs work in units of 256 rows, and where half of the last one is empty they may need a
-  // wave more than single CTAs; those are left with these products, as long as a wave counts (up to four; off the 128-byte
-  // lines, where they load more slowly, two), and with short sums whose tiles fill the GPU once. In us, replayed from a graph, single /
-  // pairs of 256 / pairs of 128 columns: e4m3 256 x 6144 x 8192 24.5 / 24.2 / 24.0; 1000 x 6144 x 8192 51.1 / 44.7 / 61.6, x
-  // 8208 79.3 / 56.7 / 63.3; 768 x 6144 x 512 6.7 / 7.6 / 7.8; bf16 1000 x 4096 x 1024 9.7 / 10.4 / 14.4, x 2048 14.8 /
-  // 15.4 / 24.1. With a wave less: bf16 128 x 28672 x 4096 45.4 / 52.7 / 79.6, 640 x 7168 x 4096 29.9 / 43.2 / 60.7, 300 x 28672
-  // x 4096 86.2 / 89.4 / 136.2 (three waves and four), 384 x 28672 x 4104 128.3 / 110.4 / 139.7, 796 x 9496 x 2144 30.4 /
-  // 36.4 / 54.4 (two and three), 3874 x 11928 x 1920 138.4 / 129.4 / 240.
+  // Pairs, in tiles as wide as their waves are cheapest, or single CTAs. Both take a K step in about the same time, and a pair
+  // covers twice the tile; but pairs work in units of 256 rows, where half of the last one may be empty. A wave of single
+  // CTAs, which load half as much again for the same work, costs 1.2 of a pair's widest, off the 128-byte lines, where they
+  // load more slowly still, 1.45; a pair's longer start and end are worth a fifth of a short sum that is done in one wave, or of
+  // a very short one. In us, replayed from a graph, single CTAs / pairs: bf16 640 x 7168 x 4096 31.7 / 36.8, 128 x 28672 x 4096
+  // 45.4 / 50.8, 128 x 19968 x 2304 22.8 / 25.7, 1000 x 4096 x 1024 9.5 / 10.2, 256 x 11520 x 1024 11.3 / 9.3, 256 x 19456 x 768
+  // 15.9 / 12.4; e4m3 768 x 6144 x 512 6.6 / 7.2, 1920 x 4864 x 384 9.1 / 10.5, 896 x 15104 x 4608 57.6 / 54.2, 657 x 8648 x 4064
+  // (off the lines) 32.9 / 25.2. Over 152 drawn sizes and both types 1 % above the best of all kernels on average, the line by
+  // waves of whole tiles that was here before 3.3 %.
   const bool fp8 = scale_a != nullptr, on_lines = k % kBlockK == 0;
-  if (pair_tiles_fit(m, n, fp8)) return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, true, layer);
-  const int64_t tiles_n = (n - 1) / kTpBN + 1, singles = ((m - 1) / kBlockM + 1) * tiles_n, pairs = ((m - 1) / (2 * kBlockM) + 1) * tiles_n;
-  const int64_t sms = sm_count(), at_once = std::max(1, pairs_at_once(fp8));
-  const int64_t waves = (singles - 1) / sms + 1;
-  const bool wave_less = waves < (pairs - 1) / at_once + 1 && waves <= (on_lines ? 4 : 2);
-  const bool short_sum = k <= 16 * kBlockK && on_lines && waves == 1;
-  if (!wave_less && !short_sum) return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, false, layer);
+  const int64_t sms = sm_count(), singles = static_cast<int64_t>((m - 1) / kBlockM + 1) * ((n - 1) / kTpBN + 1);
+  double pair_cost = 0.0;
+  const int columns = pair_columns(m, n, false, &pair_cost);
+  const bool short_sum = on_lines && k <= (singles <= sms ? 16 : 4) * kBlockK;
+  const double single_cost = wave_cost(singles, sms) * (on_lines ? 1.2 : 1.45) * (short_sum ? 0.8 : 1.0);
+  if (pair_tiles_fit(m, n, fp8) || pair_cost <= single_cost) {
+    return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, columns, layer);
+  }
   TpMaps maps;
   if (!make_map(&maps.a_local, a, m, k, a_box_rows(m)) || !make_map(&maps.b, b, n, k, kTpBN) ||
       !make_map(&maps.out[0], c, m, n, kBlockM)) {
@@ -1440,7 +1441,7 @@ cudaError_t launch_allgather_gemm(const CommDev& comm, const AgGemmArgs& a, cuda
   if (comm.nranks == 1) {  // nothing to gather
     if (a.m_local <= 0 || a.m_local % kBlockM != 0) return cudaErrorInvalidValue;
     return layer_product(comm, a.x_src != nullptr ? a.x_src : a.x_shards[0], a.w, a.y, a.m_local, a.n, a.k, a.fp8, a.scale_x_shards[0],
-                         a.scale_w, a.x_src != nullptr ? const_cast<void*>(a.x_shards[0]) : nullptr, stream);
+                         a.scale_w, a.fp8 ? nullptr : const_cast<void*>(a.x_shards[0]), stream);
   }
   if (a.x_src != nullptr) return cudaErrorInvalidValue;  // peers read the shard where it is
   TpMaps maps;

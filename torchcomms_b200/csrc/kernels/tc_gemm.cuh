@@ -49,15 +49,17 @@ inline EncodeTiledFn encode_tiled_fn() {
 }
 
 // `ld`: elements from row to row, a multiple of 8 (0: rows follow one another).
-inline bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint64_t ld = 0) {
+// `box_cols`: other boxes than of 64 columns are not swizzled.
+inline bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint64_t ld = 0,
+                     uint32_t box_cols = kBlockK) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr) return false;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {(ld != 0 ? ld : cols) * 2};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kBlockK), box_rows};
+  const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t elem[2] = {1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == kBlockK ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -353,23 +355,24 @@ __device__ __forceinline__ void scale_acc32(uint32_t (&r)[32], float row_scale, 
 }
 
 // The column scales of a tile of BN columns on their way to shared memory: each of the 128 epilogue threads fetches BN / 128
-// of them a tile ahead, so that the epilogue does not wait for global memory (zero past column `n`). In e4m3, pairs, in us with every thread
+// of them (rounded up) a tile ahead, so that the epilogue does not wait for global memory (zero past column `n`). In e4m3, pairs, in us with every thread
 // reading each scale from global memory, and so: 300 x 28672 x 2048 31.1 and 27.1, 384 x 28672 x 512 20.4 and 15.8, 1000 x
 // 14336 x 512 19.8 and 15.8.
 template <int BN>
 struct ColScales {
-  float v[BN / 128];
+  static constexpr int kEach = (BN + 127) / 128;
+  float v[kEach];
   __device__ __forceinline__ void fetch(const float* col_scale, int col0, int n, int thread) {
 #pragma unroll
-    for (int i = 0; i < BN / 128; ++i) {
-      const int col = col0 + thread * (BN / 128) + i;
+    for (int i = 0; i < kEach; ++i) {
+      const int col = col0 + thread * kEach + i;
       v[i] = col < n ? col_scale[col] : 0.0f;
     }
   }
-  // To `to`, which nobody reads any more; it may be read after the epilogue's next barrier.
+  // To `to` (kEach * 128 floats), which nobody reads any more; it may be read after the epilogue's next barrier.
   __device__ __forceinline__ void put(float* to, int thread) const {
 #pragma unroll
-    for (int i = 0; i < BN / 128; ++i) to[thread * (BN / 128) + i] = v[i];
+    for (int i = 0; i < kEach; ++i) to[thread * kEach + i] = v[i];
   }
 };
 

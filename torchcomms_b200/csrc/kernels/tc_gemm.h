@@ -25,7 +25,8 @@ cudaError_t launch_gemm_e4m3_nt(const void* a, const void* b, void* c, int m, in
 // Common entry of the two above (k in 16-bit units, scales null = bf16), which picks the kernel. `status`: two words, which
 // the kernel clears before it reports into them. `layer`: the communicator of a fused layer on one rank, whose status
 // words are not the call's own and keep what they hold, and whose phase trace is stamped (start, loads issued, MMAs
-// committed, tiles stored, CTA done). `a_copy`: a second [m, k] buffer (16-byte aligned, not overlapping `a`) that receives a copy of A.
+// committed, tiles stored, CTA done). `a_copy`: a second [m, k] buffer (16-byte aligned, not overlapping `a`) that receives a copy of A, or
+// `a` itself, where it is there already: the same kernel then, and the same bits.
 cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                            const float* scale_b, uint32_t* status, cudaStream_t stream, const CommDev* layer = nullptr,
                            void* a_copy = nullptr);
@@ -42,15 +43,25 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
                                  const CommDev* layer = nullptr, void* a_copy = nullptr);
 
 // The same product on CTA pairs (clusters of two CTAs, tcgen05 cta_group::2):
-// each pair owns a tile of 256 rows and 256 (`narrow`: 128) columns and reads every
+// each pair owns a tile of 256 rows and `columns` (128, 192, 224 or 256; 0: pair_columns()) columns and reads every
 // B element once. Any m, n % 8 == 0, k % 8 == 0 (in 16-bit units); scales
 // non-null = e4m3 operands. `layer`: as above.
 cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                                const float* scale_b, uint32_t* status, cudaStream_t stream, bool narrow = false,
+                                const float* scale_b, uint32_t* status, cudaStream_t stream, int columns = 0,
                                 const CommDev* layer = nullptr);
 // Pairs that the GPU holds at once (0 after an error), and whether the narrow tiles of an m x n product are at most as many.
 int pairs_at_once(bool fp8);
+// Waves of tiles, of which `at_once` run at a time, in time: a last, partial wave costs half a wave and half of the share it
+// fills, since few tiles have the memory to themselves.
+double wave_cost(int64_t tiles, int64_t at_once);
+// Columns of a pair's tile for a product, or a gated one of n columns each, and what its waves cost.
+int pair_columns(int m, int n, bool gated = false, double* cost = nullptr);
 bool pair_tiles_fit(int m, int n, bool fp8);
+
+// The first half of a gated MLP on CTA pairs, bf16: gate_up[m, 2 n] = x[m, k] x w[2 n, k]^T (gate columns first) and, from its
+// rounded values, act[m, n] = silu(gate) * up. n and k multiples of 8. `status`: as above.
+cudaError_t launch_gemm_gated(const void* x, const void* w, void* gate_up, void* act, int m, int n, int k, uint32_t* status,
+                              cudaStream_t stream, int columns = 0);
 
 // Logits of a head on CTA pairs: logits[m, n] (bf16, row stride `ld`, a multiple of 8) = x[m, k] x w[n, k]^T, any n, k % 8 ==
 // 0. Also, from the fp32 accumulators, for each of head_row_shares(m, n) shares of a row the maximum and the sum of

@@ -5,10 +5,11 @@
 // so the pair reads every B element once instead of twice; the leader CTA
 // issues one 256 x 256 x 16 MMA for both, accumulating into the tensor memory
 // of both. The smaller per-CTA stage (32 KB) also buys a 6-deep TMA ring.
-// Tensor cores bound it: 4096 x 28672 x 4096 in e4m3 301 us (3.2 PFLOP/s before
-// the power cap sets in; tiles of 128 x 256 on single CTAs 343), 4096 x 14336 x
-// 4096 in bf16 309 (334). Tiles of 128 columns are for products whose tiles all
-// find a pair at once; a K step takes them as long, so a second wave does not pay.
+// The tensor pipe bounds a pair with the memory to itself (a K step of 64 units
+// in 284 ns), operand traffic from L2 to the SMs all of them together: 4096 x
+// 28672 x 4096 in e4m3 318 us in a burst and 369 under the power cap, in bf16
+// 584 and 680. Tiles are 256, 224, 192 or 128 columns wide, whichever leaves the
+// last wave of pairs fuller (pair_columns).
 //
 // Roles per CTA (192 threads): warp 0 (one thread) TMA producer (both CTAs), warp 1
 // tensor-memory allocation (both CTAs) and MMA issue (leader only), warps 2-5
@@ -19,15 +20,21 @@
 // the leader and collects the eight epilogue warps of the pair.
 // No load uses cluster multicast.
 //
-// With STATS the product is a head's logits, and the epilogue, which holds a row of the tile in every thread, also leaves
+// With kStats the product is a head's logits, and the epilogue, which holds a row of the tile in every thread, also leaves
 // each row's maximum and sum of exponentials over the tile and the logit of its target: the loss then needs one look
 // at the logits instead of two. One set of epilogue warps takes 405 us for 4096 x 128256 x 256 with one barrier more a chunk,
 // two sets that share a tile's columns 348, two that take the tiles in turn 315 (the plain product 257); 4096 x 128256 x 4096
 // 2700 to 2790, by the clock that the exponentials' power leaves (plain 2650).
+//
+// With kGated the product is the first half of a gated MLP: the second CTA's half of a B tile are the rows of `up` that go with
+// the first one's of `gate`, and the epilogue, which then has both of a column, also writes silu(gate) * up. 4096 x 14336 x 4096
+// 609 us, the plain product 584 and with the activation kernel behind it 630; 1000 x 14336 x 4096 165, 157 and 170. Staging the
+// activation as well costs a stage of the ring (644 us for the first, 638 with plain stores of it).
 #include "tc_gemm.h"
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "early_launch.cuh"
 #include "launch_count.h"
@@ -40,29 +47,34 @@ namespace {
 using namespace tc;
 
 constexpr int kABytes = kBlockM * kBlockK * 2;  // 16 KB: this CTA's 128 rows of A
-constexpr int kOutChunkCols = 64;
-constexpr int kOutChunkBytes = kBlockM * kOutChunkCols * 2;
+constexpr int kOutChunkBytes = kBlockM * 64 * 2;  // of the widest chunk
+// What the epilogue does besides storing the product.
+enum Epilogue { kPlain, kStats, kGated };
 // Warps of the epilogue: four, one for each quarter of the tensor memory's lanes, or two such sets that take the tiles, and
 // with them the two accumulators, in turn.
-template <bool STATS>
-constexpr int epilogue_sets() { return STATS ? 2 : 1; }
-template <bool STATS>
-constexpr int pair_threads() { return 64 + 128 * epilogue_sets<STATS>(); }
+template <Epilogue EPI>
+constexpr int epilogue_sets() { return EPI == kStats ? 2 : 1; }
+template <Epilogue EPI>
+constexpr int pair_threads() { return 64 + 128 * epilogue_sets<EPI>(); }
 constexpr int kAccCols = 256;  // tensor-memory columns of one accumulator
 
 // Stages of the TMA ring. With two sets of epilogue warps one of six makes room for two staging buffers each: with six stages
 // and one buffer 4096 x 128256 x 256 takes 361 us, so 315; x 4096 the same either way.
-template <bool STATS>
-constexpr int pair_stages() { return STATS ? 5 : 6; }
+template <Epilogue EPI>
+constexpr int pair_stages() { return EPI == kStats ? 5 : 6; }
 
 // Shared memory for tiles of BN columns: each CTA holds half of the B tile. (Eight stages, which tiles of 128 columns
 // leave room for, gain nothing: 512 x 4096 x 4096 in e4m3 15.1 us either way.)
-template <int BN, bool STATS>
+template <int BN, Epilogue EPI>
 struct PairTile {
-  static constexpr int kStages = pair_stages<STATS>(), kOutBuffers = 2 * epilogue_sets<STATS>();
+  static constexpr int kStages = pair_stages<EPI>(), kOutBuffers = 2 * epilogue_sets<EPI>();
+  // Columns that are staged and stored at a time: a quarter of the tile, of narrow tiles half. Only whole swizzle rows of 64
+  // are swizzled; rows of 56 lie on different banks anyway, rows of 48 two by two on the same.
+  static constexpr int kChunk = BN == 128 ? 64 : BN / 4;
+  static_assert(kChunk % 8 == 0 && kChunk > 32 && kChunk <= 64, "two reads of 32 columns each");
   static constexpr int kBHalfBytes = (BN / 2) * kBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBHalfBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kOutBuffers * kOutChunkBytes + 1024 + 256 + BN * 4;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kOutBuffers * kOutChunkBytes + 1024 + 256 + 256 * 4;
 };
 
 struct PairBarriers {
@@ -75,10 +87,16 @@ struct PairBarriers {
 };
 static_assert(sizeof(PairBarriers) <= 256, "the column scales lie behind them");
 
+template <Epilogue EPI>
 struct PairMaps {
   CUtensorMap a;    // box 128 rows x 64 columns
   CUtensorMap b;    // box BN / 2 rows x 64 columns (half of the B tile)
   CUtensorMap out;  // box 128 rows x 64 columns
+};
+// B and the product in halves, gate and up, of n columns each: a tile has BN / 2 columns of both.
+template <>
+struct PairMaps<kGated> : PairMaps<kPlain> {
+  CUtensorMap b_up, out_up;
 };
 
 struct PairParams {
@@ -89,9 +107,10 @@ struct PairParams {
   int m, n, k, gm;  // k in 16-bit units
   int clear;        // the status words are this call's own
   int stage_bytes;  // of one K step's loads, both CTAs together
-  float2* stats;    // STATS: [shares of a row, m] maximum and sum of exponentials; per row its target and the target's logit
+  float2* stats;    // kStats: [shares of a row, m] maximum and sum of exponentials; per row its target and the target's logit
   const int64_t* targets;
   float* target_logit;
+  __nv_bfloat16* act;  // kGated: [m, n] silu(gate) * up
 };
 
 // Maximum and sum of exp(x - maximum) of what a row has shown so far, NaN where one was among it. Two elements per
@@ -166,16 +185,33 @@ __device__ __forceinline__ void pair_tile_at(int t, int tiles_m, int tiles_n, in
   *pn = rem / gsz;
 }
 
+// silu(gate) * up of two columns, from the rounded values as k_swiglu_fwd has it. The reciprocal is the hardware's (1 ulp): the
+// correctly rounded one branches, and a warp alone on its scheduler then has one element at a time in work.
+__device__ __forceinline__ uint32_t gated_pair(uint32_t gate, uint32_t up) {
+  float o[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float g = __uint_as_float(i == 0 ? gate << 16 : gate & 0xffff0000u), u = __uint_as_float(i == 0 ? up << 16 : up & 0xffff0000u);
+    float sigmoid;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(sigmoid) : "f"(1.0f + __expf(-g)));
+    o[i] = g * sigmoid * u;
+  }
+  return pack_bf16(__float_as_uint(o[0]), __float_as_uint(o[1]));
+}
+
 // The 128 threads of one set of epilogue warps.
 __device__ __forceinline__ void epilogue_sync(int set) {
   if (set == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
   else asm volatile("bar.sync 2, 128;" ::: "memory");
 }
 
-template <bool FP8, int BN, bool STATS>
-__global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __grid_constant__ PairMaps maps, PairParams p) {
+template <bool FP8, int BN, Epilogue EPI>
+__global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __grid_constant__ PairMaps<EPI> maps, PairParams p) {
+  constexpr bool STATS = EPI == kStats, GATED = EPI == kGated;
+  constexpr int kTileCols = GATED ? BN / 2 : BN;  // of the output
   constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(2 * kBlockM, BN) : make_idesc_bf16(2 * kBlockM, BN);
-  using Tile = PairTile<BN, STATS>;
+  using Tile = PairTile<BN, EPI>;
+  constexpr int kChunk = Tile::kChunk;
   constexpr int kStages = Tile::kStages, kStageBytes = Tile::kStageBytes, kOutBuffers = Tile::kOutBuffers;
   extern __shared__ char smem_raw[];
   // The carve-up must be identical in both CTAs (the MMA addresses both with one descriptor).
@@ -187,7 +223,7 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
   const uint32_t cta = cluster_ctarank();  // 0 leads
   const bool leader = cta == 0;
   const int cluster_id = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
-  const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / BN + 1;
+  const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / kTileCols + 1;
   const int total_tiles = tiles_m * tiles_n;
   const int k_iters = (p.k + kBlockK - 1) / kBlockK;
 
@@ -226,7 +262,10 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
         int pm, pn;
         pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
         const int a_row = (pm * 2 + static_cast<int>(cta)) * kBlockM;
-        const int b_row = pn * BN + static_cast<int>(cta) * (BN / 2);
+        // Each CTA loads one half of the B tile: the second one its last rows, or its rows of the second half of B.
+        const int b_row = GATED ? pn * kTileCols : pn * BN + static_cast<int>(cta) * (BN / 2);
+        const CUtensorMap* b_map = &maps.b;
+        if constexpr (GATED) b_map = leader ? &maps.b : &maps.b_up;
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
@@ -238,7 +277,7 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
           if (leader) mbar_expect_tx(&bars->full[s], static_cast<uint32_t>(p.stage_bytes));
           char* sa = stages + s * kStageBytes;
           tma_load_2d_pair(sa, &maps.a, &bars->full[s], kb * kBlockK, a_row);
-          tma_load_2d_pair(sa + kABytes, &maps.b, &bars->full[s], kb * kBlockK, b_row);
+          tma_load_2d_pair(sa + kABytes, b_map, &bars->full[s], kb * kBlockK, b_row);
         }
       }
       trace_stamp_ns(p.trace, 1);
@@ -284,15 +323,17 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
     // ---------------- epilogue (both CTAs, own 128 rows)
     const int q = warp & 3;
     const int row_in_tile = q * 32 + lane;
-    constexpr int kSets = epilogue_sets<STATS>();
+    constexpr int kSets = epilogue_sets<EPI>();
     const int set = kSets == 1 ? 0 : (warp - 2) >> 2;
     const bool issuer = (warp & 3) == 2 && lane == 0;
     const int et = static_cast<int>(threadIdx.x) - 64;  // (one set: the column scales)
+    // Where 16 bytes of a row lie in a staged chunk.
+    const auto staged = [](int row, int piece) { return kChunk == 64 ? row * 128 + ((piece ^ (row & 7)) << 4) : row * kChunk * 2 + piece * 16; };
     // What a row brings along is fetched a tile ahead: its scale, or the column its target has in the tile's row of tiles.
     const auto rows_of = [&](int t) {
       int pm, pn;
       pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
-      return make_int2((pm * 2 + static_cast<int>(cta)) * kBlockM, pn * BN);
+      return make_int2((pm * 2 + static_cast<int>(cta)) * kBlockM, pn * kTileCols);
     };
     ColScales<BN> fetched;
     float next_scale = 0.0f;
@@ -327,17 +368,65 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
       tc_fence_after_sync();
       RowStats row_stats;
       const bool row_there = STATS && out_row + row_in_tile < p.m;
-      for (int j = 0; j < BN / kOutChunkCols; ++j, ++chunk_iter) {
+      if constexpr (GATED) {
+        static_assert(!GATED || kSets == 1, "");
+        for (int j = 0; j < kTileCols / kChunk; ++j) {
+          if (issuer) tma_store_wait_read<0>();
+          epilogue_sync(0);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t g[32], u[32];
+            const uint32_t from = tmem_base + as * kAccCols + (static_cast<uint32_t>(q * 32) << 16) +
+                static_cast<uint32_t>(j * kChunk + half * 32);
+            tmem_ld_32x32(from, g);
+            tmem_ld_32x32(from + BN / 2, u);
+            tmem_ld_wait();
+            if (j == kTileCols / kChunk - 1 && half == 1) {
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_leader(&bars->acc_empty[as]);
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              uint32_t pg[4], pu[4], pa[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                pg[i] = pack_bf16(g[8 * v + 2 * i], g[8 * v + 2 * i + 1]);
+                pu[i] = pack_bf16(u[8 * v + 2 * i], u[8 * v + 2 * i + 1]);
+                pa[i] = gated_pair(pg[i], pu[i]);
+              }
+              if (half * 4 + v >= kChunk / 8) continue;
+              const int at = staged(row_in_tile, half * 4 + v);
+              *reinterpret_cast<uint4*>(obuf + at) = make_uint4(pg[0], pg[1], pg[2], pg[3]);
+              *reinterpret_cast<uint4*>(obuf + kOutChunkBytes + at) = make_uint4(pu[0], pu[1], pu[2], pu[3]);
+              const int col = out_col + j * kChunk + half * 32 + v * 8;
+              if (out_row + row_in_tile < p.m && col < p.n) {
+                *reinterpret_cast<uint4*>(p.act + static_cast<size_t>(out_row + row_in_tile) * p.n + col) = make_uint4(pa[0], pa[1], pa[2], pa[3]);
+              }
+            }
+          }
+          fence_proxy_async_smem();
+          epilogue_sync(0);
+          const int col = out_col + j * kChunk;
+          if (issuer && out_row < p.m && col < p.n) {
+            tma_store_2d(&maps.out, obuf, col, out_row);
+            tma_store_2d(&maps.out_up, obuf + kOutChunkBytes, col, out_row);
+            tma_store_commit();
+          }
+        }
+        continue;
+      }
+      for (int j = 0; j < BN / kChunk; ++j, ++chunk_iter) {
         char* buf = obuf + (2 * set + (chunk_iter & 1u)) * kOutChunkBytes;
         uint32_t acc[2][32];
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           tmem_ld_32x32(tmem_base + as * kAccCols + (static_cast<uint32_t>(q * 32) << 16) +
-                            static_cast<uint32_t>(j * kOutChunkCols + half * 32),
+                            static_cast<uint32_t>(j * kChunk + half * 32),
                         acc[half]);
         }
         tmem_ld_wait();
-        if (j == BN / kOutChunkCols - 1) {
+        if (j == BN / kChunk - 1) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive_leader(&bars->acc_empty[as]);
@@ -345,9 +434,9 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           uint32_t(&r)[32] = acc[half];
-          if (FP8) scale_acc32(r, row_scale, col_scales + j * kOutChunkCols + half * 32);
+          if (FP8) scale_acc32(r, row_scale, col_scales + j * kChunk + half * 32);
           if constexpr (STATS) {
-            const int col = j * kOutChunkCols + half * 32;
+            const int col = j * kChunk + half * 32;
             const int past = p.n - out_col - col;  // columns beyond the last are zeros of the tile, not logits
             if (past < 32) {
 #pragma unroll
@@ -363,9 +452,8 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
           }
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            const int chunk16 = half * 4 + v;
-            uint4* dst = reinterpret_cast<uint4*>(buf + row_in_tile * 128 + ((chunk16 ^ (row_in_tile & 7)) << 4));
-            *dst = make_uint4(pack_bf16(r[8 * v], r[8 * v + 1]), pack_bf16(r[8 * v + 2], r[8 * v + 3]),
+            if (half * 4 + v >= kChunk / 8) continue;
+            *reinterpret_cast<uint4*>(buf + staged(row_in_tile, half * 4 + v)) = make_uint4(pack_bf16(r[8 * v], r[8 * v + 1]), pack_bf16(r[8 * v + 2], r[8 * v + 3]),
                               pack_bf16(r[8 * v + 4], r[8 * v + 5]), pack_bf16(r[8 * v + 6], r[8 * v + 7]));
           }
         }
@@ -374,8 +462,8 @@ __global__ void __launch_bounds__(pair_threads<STATS>(), 1) k_gemm_pair(const __
         // and that this one is full.
         if (issuer) tma_store_wait_read<0>();
         epilogue_sync(set);
-        if (issuer && out_row < p.m && out_col + j * kOutChunkCols < p.n) {
-          tma_store_2d(&maps.out, buf, out_col + j * kOutChunkCols, out_row);
+        if (issuer && out_row < p.m && out_col + j * kChunk < p.n) {
+          tma_store_2d(&maps.out, buf, out_col + j * kChunk, out_row);
           tma_store_commit();
         }
       }
@@ -403,7 +491,7 @@ constexpr int kDevices = 64;  // whose answers are kept
 
 // Pairs that the current GPU holds at once (each CTA fills an SM), or 0 after an error. Kept per device; a query that
 // failed is asked again at the next call.
-template <bool FP8, int BN, bool STATS = false>
+template <bool FP8, int BN, Epilogue EPI = kPlain>
 int resident_pairs() {
   static std::atomic<int> known[kDevices];
   int device = 0, n = 0;
@@ -411,48 +499,56 @@ int resident_pairs() {
   std::atomic<int>* kept = device >= 0 && device < kDevices ? &known[device] : nullptr;
   if (kept != nullptr) n = kept->load(std::memory_order_acquire);
   if (n > 0) return n;
-  if (cudaFuncSetAttribute(k_gemm_pair<FP8, BN, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairTile<BN, STATS>::kSmemBytes) != cudaSuccess) return 0;
+  if (cudaFuncSetAttribute(k_gemm_pair<FP8, BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairTile<BN, EPI>::kSmemBytes) != cudaSuccess) return 0;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2);
-  cfg.blockDim = dim3(pair_threads<STATS>());
-  cfg.dynamicSmemBytes = PairTile<BN, STATS>::kSmemBytes;
+  cfg.blockDim = dim3(pair_threads<EPI>());
+  cfg.dynamicSmemBytes = PairTile<BN, EPI>::kSmemBytes;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, k_gemm_pair<FP8, BN, STATS>, &cfg) != cudaSuccess || n < 1) return 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_gemm_pair<FP8, BN, EPI>, &cfg) != cudaSuccess || n < 1) return 0;
   if (kept != nullptr) kept->store(n, std::memory_order_release);
   return n;
 }
 
 // `ldc`: row stride of the output in elements (0: n).
-template <bool FP8, int BN, bool STATS = false>
+template <bool FP8, int BN, Epilogue EPI = kPlain>
 cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cudaStream_t stream, int64_t ldc = 0) {
-  const int pairs = resident_pairs<FP8, BN, STATS>();
+  const int pairs = resident_pairs<FP8, BN, EPI>();
   if (pairs < 1) {
     const cudaError_t e = cudaGetLastError();
     return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
   }
-  PairMaps maps;
-  if (!make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m)) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.out, c, p.m, p.n, kBlockM, ldc)) {
+  constexpr int kTileCols = EPI == kGated ? BN / 2 : BN;
+  PairMaps<EPI> maps;
+  if (!make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m)) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.out, c, p.m, p.n, kBlockM, ldc, PairTile<BN, EPI>::kChunk)) {
     return cudaErrorInvalidValue;
   }
-  p.stage_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN, STATS>::kBHalfBytes);
-  const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / BN + 1;
+  if constexpr (EPI == kGated) {
+    const auto* up = static_cast<const char*>(b) + static_cast<size_t>(p.n) * p.k * 2;
+    if (!make_map(&maps.b_up, up, p.n, p.k, BN / 2) ||
+        !make_map(&maps.out_up, static_cast<char*>(c) + static_cast<size_t>(p.n) * 2, p.m, p.n, kBlockM, ldc, PairTile<BN, EPI>::kChunk)) {
+      return cudaErrorInvalidValue;
+    }
+  }
+  p.stage_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN, EPI>::kBHalfBytes);
+  const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / kTileCols + 1;
   // A rows of a group stay in L2 while the pairs sweep over n: at most 8 pair-tiles and ~40 MB. Every group reads B again,
   // so where L2 does not keep that either (above 48 MB) groups are of up to 16 pair-tiles and 32 MB. In us under the power
   // cap with 8 and 16: 4096 x 28672 x 4096 in e4m3 (B of 117 MB) 397 and 390, 8192 x 14336 x 4096 (59 MB) 400 and 392; 4096 x
   // 8192 x 1024 (8 MB) 43.4 and 45.8.
   const size_t a_tile_bytes = static_cast<size_t>(2 * kBlockM) * p.k * 2;
-  const bool b_again = static_cast<size_t>(p.n) * p.k * 2 > (48u << 20);
+  const bool b_again = static_cast<size_t>(p.n) * p.k * 2 * (BN / kTileCols) > (48u << 20);
   p.gm = std::max(1, std::min({b_again ? 16 : 8, tiles_m, static_cast<int>((b_again ? 32u << 20 : 40u << 20) / std::max<size_t>(a_tile_bytes, 1))}));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(pairs, static_cast<int64_t>(tiles_m) * tiles_n)));
-  cfg.blockDim = dim3(pair_threads<STATS>());
-  cfg.dynamicSmemBytes = PairTile<BN, STATS>::kSmemBytes;
+  cfg.blockDim = dim3(pair_threads<EPI>());
+  cfg.dynamicSmemBytes = PairTile<BN, EPI>::kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -463,7 +559,7 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gemm_pair<FP8, BN, STATS>, maps, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gemm_pair<FP8, BN, EPI>, maps, p);
   note_kernel_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -472,13 +568,40 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
 
 int pairs_at_once(bool fp8) { return fp8 ? resident_pairs<true, 256>() : resident_pairs<false, 256>(); }
 
+double wave_cost(int64_t tiles, int64_t at_once) {
+  const int64_t part = tiles % at_once;
+  return static_cast<double>(tiles / at_once) + (part > 0 ? 0.5 + 0.5 * static_cast<double>(part) / static_cast<double>(at_once) : 0.0);
+}
+
+// The width whose waves take least. A wave of full width costs 1 and one of half the width 0.575 (the rows of A come in either
+// way). 256 unless another is 1 % ahead. Of 39 sizes, types and epilogues this takes the best of 256, 224, 192, 160 and 128
+// everywhere but once (0.4 % behind). In us with 256 / 224 / 192 columns: bf16 1000 x 6144 x 4096 45.3 / 42.0 / 39.0, 1000 x 28672 x
+// 4096 161.7 / 157.0 / 166.3, 1500 x 5000 x 2992 37.5 / 34.7 / 42.6, 4096 x 4096 x 14336 328 / 346 / 334; e4m3 1000 x 6144 x 4096
+// 26.8 / 24.7 / 22.4, 4096 x 2560 x 2560 25.6 / 23.7 / 24.9; gated 1000 x 14336 x 4096 168.9 / 165.3 / 173.4.
+int pair_columns(int m, int n, bool gated, double* cost) {
+  const int64_t pairs = std::max(1, pairs_at_once(false)), tiles_m = (m - 1) / (2 * kBlockM) + 1;
+  int best = 256;
+  double least = 0.0;
+  for (const int columns : {256, 224, 192, 128}) {
+    if (gated && columns == 128) break;
+    const double waves = wave_cost(tiles_m * ((n - 1) / (gated ? columns / 2 : columns) + 1), pairs);
+    const double here = waves * (0.15 + 0.85 * columns / 256.0) * (columns == 256 ? 0.99 : 1.0);
+    if (columns == 256 || here < least) {
+      best = columns;
+      least = here;
+    }
+  }
+  if (cost != nullptr) *cost = least;
+  return best;
+}
+
 bool pair_tiles_fit(int m, int n, bool fp8) {
   const int pairs = fp8 ? resident_pairs<true, 128>() : resident_pairs<false, 128>();
   return static_cast<int64_t>((m - 1) / (2 * kBlockM) + 1) * ((n - 1) / 128 + 1) <= pairs;
 }
 
 cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                                const float* scale_b, uint32_t* status, cudaStream_t stream, bool narrow, const CommDev* layer) {
+                                const float* scale_b, uint32_t* status, cudaStream_t stream, int columns, const CommDev* layer) {
   if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || n % 8 != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) {
     return cudaErrorInvalidValue;
@@ -492,8 +615,15 @@ cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, in
   p.m = m;
   p.n = n;
   p.k = k;
-  if (narrow) return scale_a != nullptr ? launch_pair<true, 128>(a, b, c, p, stream) : launch_pair<false, 128>(a, b, c, p, stream);
-  return scale_a != nullptr ? launch_pair<true, 256>(a, b, c, p, stream) : launch_pair<false, 256>(a, b, c, p, stream);
+  const auto launch = [&](auto fp8) {
+    switch (columns != 0 ? columns : pair_columns(m, n, false)) {
+      case 128: return launch_pair<fp8(), 128>(a, b, c, p, stream);
+      case 192: return launch_pair<fp8(), 192>(a, b, c, p, stream);
+      case 224: return launch_pair<fp8(), 224>(a, b, c, p, stream);
+      default: return launch_pair<fp8(), 256>(a, b, c, p, stream);
+    }
+  };
+  return scale_a != nullptr ? launch(std::true_type()) : launch(std::false_type());
 }
 
 int head_row_shares(int m, int n) {
@@ -516,8 +646,29 @@ cudaError_t launch_head_logits(const void* x, const void* w, void* logits, int64
   p.stats = stats;
   p.targets = targets;
   p.target_logit = target_logit;
-  return pair_tiles_fit(m, n, false) ? launch_pair<false, 128, true>(x, w, logits, p, stream, ld)
-                                     : launch_pair<false, 256, true>(x, w, logits, p, stream, ld);
+  return pair_tiles_fit(m, n, false) ? launch_pair<false, 128, kStats>(x, w, logits, p, stream, ld)
+                                     : launch_pair<false, 256, kStats>(x, w, logits, p, stream, ld);
+}
+
+cudaError_t launch_gemm_gated(const void* x, const void* w, void* gate_up, void* act, int m, int n, int k, uint32_t* status,
+                              cudaStream_t stream, int columns) {
+  if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || n % 8 != 0) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(act)) & 15u) {
+    return cudaErrorMisalignedAddress;
+  }
+  PairParams p{};
+  p.status = status;
+  p.clear = 1;
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  p.act = static_cast<__nv_bfloat16*>(act);
+  const int64_t ld = 2 * static_cast<int64_t>(n);
+  switch (columns != 0 ? columns : pair_columns(m, n, true)) {
+    case 192: return launch_pair<false, 192, kGated>(x, w, gate_up, p, stream, ld);
+    case 224: return launch_pair<false, 224, kGated>(x, w, gate_up, p, stream, ld);
+    default: return launch_pair<false, 256, kGated>(x, w, gate_up, p, stream, ld);
+  }
 }
 
 } // namespace b200c

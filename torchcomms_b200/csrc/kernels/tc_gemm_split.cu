@@ -90,6 +90,7 @@ struct SplitParams {
   long long* trace;
   int m, n, k, k_iters, tiles_m;  // k in 16-bit units
   int copy_a, per_split;
+  int always;  // (host) this kernel whether it pays or not
   int clear;        // the status words are this call's own
   int stage_bytes;  // of one K step's loads
 };
@@ -375,21 +376,29 @@ int resident_clusters(int device, int splits) {
   return n;
 }
 
-// Whether the split kernel beats the others (tc_gemm.cu has their rule). Sending shares to their owners costs it 2 us
-// more than a kernel that has its tile to itself; a K step of 64 units (16 bits) is 0.27 us of the others' time and 0.2 us
-// of this one's, over the CTAs that share K. Replayed from a graph, best of the others / split in us:
-//   K shared (from 8 steps on): e4m3 128 x 4096 x 2048 (16 steps) 8.9 / 7.9, x 8192 (64) 23.1 / 11.8; bf16 64 x 1024 x 512 (8)
-//   5.7 / 5.2, 128 x 1024 x 512 5.9 / 5.8, 384 x 2560 x 512 6.4 / 6.7, 128 x 6144 x 1024 (16) 8.9 / 7.8, 128 x 1024 x 4096
-//   (64) 21.9 / 9.2
-//   not shared, more tiles than pairs: bf16 128 x 14336 x 1024 9.4 / 9.1, x 2048 15.2 / 14.0, x 4096 27.8 / 26.9, x 8192 50.6 /
-//   48.5; off the 128-byte lines x 1032 (17 steps) 12.0 / 11.4, x 2056 18.2 / 19.5, x 4104 31.7 / 38.2
-//   not shared, at most as many: bf16 256 x 9472 x 2048 (32) 14.0 / 14.4, x 8192 43.5 / 45.2; over such sizes split takes
-//   0.96 to 1.0 of the others' time up to 32 steps, 1.0 at 64 and 1.02 at 128; off the lines 1.02 at 5 steps, 1.1 at 17
-bool split_pays(int m, int n, int k, int k_iters, bool fp8, bool shares_k) {
-  if (shares_k) return fp8 || m <= 64 || k_iters >= 10;
-  const bool fit = pair_tiles_fit(m, n, fp8);
-  if (k % kBlockK == 0) return !fit || k_iters <= 32;
-  return k_iters <= (fit ? 8 : 17);
+// Whether the split kernel beats the others (tc_gemm.cu has their rule), K being shared by `splits` CTAs. Sending shares to
+// their owners costs it 2 us more than a kernel that has its tile to itself, as long as 11 K steps take a pair, or 7 with up to
+// 64 rows, which send less; weights from DRAM, as here, favour the kernel with more CTAs to fetch them. Without shares it is ahead
+// where pairs are mostly start and end, or leave their second half of rows empty in more tiles than a quarter of the SMs.
+// Replayed from a graph over 320 MB of weights, narrow pairs / split in us:
+//   K shared, by the steps that a CTA is spared: bf16 256 x 2816 x 1280 (10) 7.7 / 9.0, 384 x 768 x 1024 (12) 6.5 / 7.0, 128 x 4096 x
+//   1792 (21) 9.7 / 9.1, 128 x 3584 x 4096 (48) 17.9 / 12.0; e4m3 128 x 4096 x 1408 (6) 6.3 / 6.7, 1152 x 768 x 2304 (9) 7.3 / 7.3, 640 x
+//   1792 x 3072 (12) 9.0 / 8.5, 256 x 4608 x 3712 (15) 10.5 / 10.0, 67 x 6144 x 4096 (16) 11.4 / 10.2; few rows: bf16 55 x 4848 x 768
+//   (6) 6.0 / 6.1, e4m3 28 x 6440 x 1808 (8) 7.6 / 7.3, 4 x 272 x 1600 (9) 5.7 / 4.9, 1 x 1712 x 3040 (20) 8.2 / 6.0
+//   not shared, at most as many tiles as pairs: e4m3 256 x 4352 x 512 (4) 4.8 / 4.6, 640 x 3072 x 896 (7) 6.0 / 5.8, 768 x 2048 x 1152
+//   (9) 6.0 / 6.1, 119 x 8376 x 480 (off the lines) 5.8 / 5.0; bf16 1280 x 1536 x 1792 (28) 9.4 / 9.9, 1280 x 1792 x 5120 (80) 21.3 /
+//   22.8; off the lines 1014 x 1400 x 3952 (31) 13.3 / 15.9
+//   not shared, more tiles than pairs, best of the others / split, weights in L2: bf16 384 x 5376 x 1536 10.5 / 9.5, 128 x 12032 x
+//   2304 16.2 / 15.4; e4m3 300 x 6144 x 4096 13.8 / 13.1; off the lines 259 x 5560 x 1872 (15) 10.7 / 10.5, x 2056 in bf16 (33) 18.2 /
+//   19.5
+bool split_pays(int m, int n, int k, int k_iters, bool fp8, int splits) {
+  const bool on_lines = k % kBlockK == 0;
+  if (pair_tiles_fit(m, n, fp8)) {
+    if (splits == 1) return (on_lines && k_iters <= 7) || (m <= kBlockM && n > 40 * kSplitBN);
+    return k_iters - k_iters / splits >= (m > 64 ? 11 : 7);
+  }
+  if (splits > 1) return fp8 || m <= 64 || k_iters >= 10;
+  return on_lines || k_iters <= 17;
 }
 
 template <bool FP8>
@@ -417,7 +426,7 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
     if (resident_clusters<FP8>(device, s) >= tiles) splits = s;
   }
   if (splits == 0) return cudaSuccess;  // more tiles than SMs after all: not this kernel's case
-  if (p.copy_a == 0 && !split_pays(p.m, p.n, p.k, p.k_iters, FP8, splits > 1)) return cudaSuccess;
+  if (!p.always && !split_pays(p.m, p.n, p.k, p.k_iters, FP8, splits)) return cudaSuccess;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = split_config(tiles, splits, stream, attr);
   // Clusters of three and five do not pack into the SMs as the kernel in front leaves them, so that fewer are resident than
@@ -444,9 +453,10 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   SplitMaps maps;
   if (!make_map(&maps.a, a, m, k, a_box_rows(m)) || !make_map(&maps.b, b, n, k, kSplitBN)) return cudaErrorInvalidValue;
   maps.a_copy = maps.a;
-  if (a_copy != nullptr && !make_map(&maps.a_copy, a_copy, m, k, a_box_rows(m))) return cudaErrorInvalidValue;
+  if (a_copy != nullptr && a_copy != a && !make_map(&maps.a_copy, a_copy, m, k, a_box_rows(m))) return cudaErrorInvalidValue;
   SplitParams p{};
-  p.copy_a = a_copy != nullptr ? 1 : 0;
+  p.copy_a = a_copy != nullptr && a_copy != a ? 1 : 0;
+  p.always = a_copy != nullptr ? 1 : 0;
   p.c = static_cast<__nv_bfloat16*>(c);
   p.status = status;
   p.clear = layer == nullptr && status != nullptr ? 1 : 0;

@@ -541,6 +541,20 @@ void bind_ops(py::module_& m) {
     return std::make_pair(c, status);
   });
 
+  // (x w^T, silu(gate) * up of it), bf16, gate columns first.
+  ops.def("gemm_gated", [](const at::Tensor& x, const at::Tensor& w) {
+    want(x, at::kBFloat16, "x");
+    want(w, at::kBFloat16, "w");
+    TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && w.size(0) % 2 == 0, "x: [m, k], w: [2 n, k]");
+    c10::cuda::CUDAGuard g(x.device());
+    at::Tensor gate_up = at::empty({x.size(0), w.size(0)}, x.options()), act = at::empty({x.size(0), w.size(0) / 2}, x.options());
+    at::Tensor status = status_words(x);
+    B200C_CUDA_CHECK(launch_gemm_gated(x.data_ptr(), w.data_ptr(), gate_up.data_ptr(), act.data_ptr(), static_cast<int>(x.size(0)),
+                                       static_cast<int>(w.size(0) / 2), static_cast<int>(x.size(1)),
+                                       reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(x)));
+    return std::make_tuple(gate_up, act, status);
+  });
+
   ops.def("kernel_launch_count", []() { return kernel_launch_count(); });
 }
 
