@@ -1,0 +1,116 @@
+"""The two nodes of a decoder block against the separate operations in 64 bits: edges of the gated product's tiles, gradients
+that nobody asks for, and what they leave to the separate nodes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape, seed, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device="cuda") * scale).bfloat16()
+
+
+def _norm64(x, w, eps=1e-5):
+    return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w
+
+
+def _off(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+# Row tiles of 256 and column tiles of 128 with and without a remainder, one column vector, depths below and above a K step; few
+# rows of large weights, which take the activation kernel.
+@pytest.mark.parametrize("rows,dim,ffn,width", [(1, 64, 8, 64), (127, 72, 120, 64), (256, 128, 128, 192), (257, 200, 136, 128),
+                                                (300, 256, 1032, 256), (1000, 512, 2048, 512), (130, 1024, 9480, 1024),
+                                                (40, 3200, 8192, 64)])
+def test_block_out(rows, dim, ffn, width):
+    from torchcomms_b200 import _comms
+
+    ins = [_rand(rows, dim, seed=1), _rand(rows, width, seed=2), _rand(dim, width, seed=3, scale=width**-0.5),
+           _rand(dim, seed=4, scale=0.1) + 1, _rand(2 * ffn, dim, seed=5, scale=dim**-0.5), _rand(dim, ffn, seed=6, scale=ffn**-0.5)]
+    dy = _rand(rows, dim, seed=7)
+    ins = [t.requires_grad_(True) for t in ins]
+    y = _comms.ops.block_out(*ins, 1e-5)
+    grads = torch.autograd.grad(y, ins, dy)
+    wide = [t.detach().double().requires_grad_(True) for t in ins]
+    x, o, wo, norm, w13, w2 = wide
+    s = x + o @ wo.t()
+    gate, up = (_norm64(s, norm) @ w13.t()).chunk(2, dim=-1)
+    ref = s + (torch.nn.functional.silu(gate) * up) @ w2.t()
+    ref_grads = torch.autograd.grad(ref, wide, dy.double())
+    # Forward: seven roundings to bf16 (2^-9 each, of numbers of about the result's size); backward: three or four more on the way.
+    assert _off(y.detach(), ref.detach()) < 7 * 2**-9
+    for a, b in zip(grads, ref_grads):
+        assert _off(a, b) < 12 * 2**-9
+
+
+@pytest.mark.parametrize("rows,dim,heads,kv_heads,hd", [(1, 64, 1, 1, 8), (129, 200, 4, 2, 32), (1000, 512, 8, 2, 64)])
+def test_block_in(rows, dim, heads, kv_heads, hd):
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops import fused
+
+    x, norm = _rand(rows, dim, seed=1).requires_grad_(True), (_rand(dim, seed=2, scale=0.1) + 1).requires_grad_(True)
+    w = _rand((heads + 2 * kv_heads) * hd, dim, seed=3, scale=dim**-0.5).requires_grad_(True)
+    cos_t, sin_t = fused.rope_tables(64, hd, 10000.0, "cuda")
+    pos = torch.arange(rows, dtype=torch.int32, device="cuda") % 64
+    got = _comms.ops.block_in(x, norm, w, pos, cos_t, sin_t, heads, kv_heads, 1e-5)
+    # The same kernels as the separate nodes, but for a product of sums in another order.
+    x2, h = fused.rms_norm_skip(x, norm, 1e-5)
+    want = (x2, *fused.split_rope(torch.nn.functional.linear(h, w), pos, cos_t, sin_t, heads, kv_heads))
+    douts = [_rand(*t.shape, seed=10 + i) for i, t in enumerate(want)]
+    assert torch.equal(got[0], want[0]) and got[0].data_ptr() == x.data_ptr()
+    # Products that differ by the order of their fp32 sums are rounded to bf16 (2^-9) on one side of a tie or the other, rotated
+    # and rounded again.
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and _off(a.detach(), b.detach()) < 2**-8
+    # Backward takes nothing from the forward product: the same bits.
+    for a, b in zip(torch.autograd.grad(got, (x, norm, w), douts), torch.autograd.grad(want, (x, norm, w), douts)):
+        assert torch.equal(a, b)
+
+
+def test_only_what_is_asked_for():
+    """Frozen weights and partial gradients: the others come out the same."""
+    from torchcomms_b200 import _comms
+
+    ins = [_rand(64, 128, seed=1), _rand(64, 128, seed=2), _rand(128, 128, seed=3, scale=0.1), _rand(128, seed=4, scale=0.1) + 1,
+           _rand(512, 128, seed=5, scale=0.1), _rand(128, 256, seed=6, scale=0.1)]
+    dy = _rand(64, 128, seed=7)
+    full = [t.clone().requires_grad_(True) for t in ins]
+    grads = torch.autograd.grad(_comms.ops.block_out(*full, 1e-5), full, dy)
+    frozen = [t.clone().requires_grad_(i in (0, 3)) for i, t in enumerate(ins)]
+    a, b = torch.autograd.grad(_comms.ops.block_out(*frozen, 1e-5), (frozen[0], frozen[3]), dy)
+    assert torch.equal(a, grads[0]) and torch.equal(b, grads[3])
+    y = _comms.ops.block_out(*full, 1e-5)
+    one = torch.autograd.grad(y, full[4], dy, retain_graph=True)[0]
+    two = torch.autograd.grad(y, full[1], dy)[0]
+    assert torch.equal(one, grads[4]) and torch.equal(two, grads[1])
+    with torch.no_grad():
+        assert not _comms.ops.block_out(*full, 1e-5).requires_grad
+
+
+def test_block_takes_and_leaves():
+    """What the nodes do not take runs as before: other types, autocast, transforms."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.models.llama import Block, LlamaConfig
+    from torchcomms_b200.ops import fused
+
+    cfg = LlamaConfig(dim=128, n_layers=1, n_heads=4, n_kv_heads=2, ffn_dim=200, vocab_size=64, max_seq_len=64)
+    torch.manual_seed(0)
+    block = Block(cfg).cuda().bfloat16()
+    cos_t, sin_t = fused.rope_tables(64, cfg.head_dim, cfg.rope_theta, "cuda")
+    pos = torch.arange(48, dtype=torch.int32, device="cuda")
+    x = _rand(1, 48, 128, seed=1)
+    y = block(x, pos, cos_t, sin_t)
+    with torch.autocast("cuda", torch.bfloat16):
+        assert _off(block(x, pos, cos_t, sin_t).detach(), y.detach()) < 2**-7
+    kept = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.append(t) or t, lambda t: t):
+        (block(x, pos, cos_t, sin_t).float().sum()).backward()
+    assert kept and all(p.grad is not None for p in block.parameters())
+    n = block.ffn_norm
+    assert _comms.ops.block_out(x[0], x[0], block.wo, n, block.w13, block.w2[:, :199], 1e-5) is None
+    assert _comms.ops.block_out(x[0].float(), x[0], block.wo, n, block.w13, block.w2, 1e-5) is None
+    assert _comms.ops.block_in(x[0, :, :64], n, block.wqkv, pos, cos_t, sin_t, 4, 2, 1e-5) is None
+    out = torch.func.functional_call(block, dict(block.named_parameters()), (x, pos, cos_t, sin_t))
+    assert torch.equal(out, y)

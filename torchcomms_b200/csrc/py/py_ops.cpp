@@ -236,14 +236,18 @@ struct SplitRopeFn : torch::autograd::Function<SplitRopeFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
+    return {packed_gradient(std::move(grads), saved[0], saved[1], saved[2]), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+  }
+  // The gradient of the projection's output from those of queries, keys and values.
+  static at::Tensor packed_gradient(variable_list grads, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t) {
     for (auto& t : grads) {
       if (!followable(t)) t = t.clone(at::MemoryFormat::Contiguous);
       TORCH_CHECK(t.scalar_type() == at::kBFloat16, "split_rope: bf16 gradients expected");
     }
     c10::cuda::CUDAGuard g(grads[0].device());
     at::Tensor dqkv = at::empty({grads[0].size(0), (grads[0].size(1) + 2 * grads[1].size(1)) * grads[0].size(2)}, grads[0].options());
-    launch(dqkv, grads, saved[0], saved[1], saved[2], true);
-    return {dqkv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+    launch(dqkv, grads, pos, cos_t, sin_t, true);
+    return dqkv;
   }
   static void launch(const at::Tensor& packed, const variable_list& part, const at::Tensor& pos, const at::Tensor& cos_t,
                      const at::Tensor& sin_t, bool backward) {
@@ -261,14 +265,19 @@ struct SplitRopeFn : torch::autograd::Function<SplitRopeFn> {
   }
   static bool applies(const at::Tensor& qkv, const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t, int64_t heads,
                       int64_t kv_heads) {
-    if (!plain_call(qkv, true) || !plain_call(pos) || !plain_call(cos_t) || !plain_call(sin_t)) return false;
-    if (heads < 1 || kv_heads < 1 || qkv.dim() != 2 || qkv.numel() == 0 || qkv.size(1) % (8 * (heads + 2 * kv_heads)) != 0) return false;
-    const int64_t hd = qkv.size(1) / (heads + 2 * kv_heads);
+    return plain_call(qkv, true) && qkv.dim() == 2 && qkv.numel() > 0 && qkv.scalar_type() == at::kBFloat16 && qkv.stride(1) == 1 &&
+        qkv.stride(0) % 8 == 0 && on16(qkv) && heads >= 1 && kv_heads >= 1 &&
+        applies_to(qkv.size(0), qkv.size(1), qkv.device(), pos, cos_t, sin_t, heads, kv_heads);
+  }
+  // The same for a projection that is yet to be made, contiguous.
+  static bool applies_to(int64_t tokens, int64_t cols, at::Device device, const at::Tensor& pos, const at::Tensor& cos_t,
+                         const at::Tensor& sin_t, int64_t heads, int64_t kv_heads) {
+    if (!plain_call(pos) || !plain_call(cos_t) || !plain_call(sin_t) || cols % (8 * (heads + 2 * kv_heads)) != 0) return false;
+    const int64_t hd = cols / (heads + 2 * kv_heads);
     auto table = [&](const at::Tensor& t) {
-      return t.scalar_type() == at::kFloat && t.is_contiguous() && t.dim() == 2 && t.size(1) == hd / 2 && t.device() == qkv.device() && on16(t);
+      return t.scalar_type() == at::kFloat && t.is_contiguous() && t.dim() == 2 && t.size(1) == hd / 2 && t.device() == device && on16(t);
     };
-    return qkv.scalar_type() == at::kBFloat16 && qkv.stride(1) == 1 && qkv.stride(0) % 8 == 0 && on16(qkv) && table(cos_t) && table(sin_t) && pos.scalar_type() == at::kInt &&
-        pos.is_contiguous() && pos.numel() == qkv.size(0) && pos.device() == qkv.device();
+    return table(cos_t) && table(sin_t) && pos.scalar_type() == at::kInt && pos.is_contiguous() && pos.numel() == tokens && pos.device() == device;
   }
 };
 
@@ -291,6 +300,117 @@ struct RopeFn : torch::autograd::Function<RopeFn> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     return {rope(grads[0], saved[0], saved[1], saved[2], true), at::Tensor(), at::Tensor(), at::Tensor()};
+  }
+};
+
+// The two halves of a decoder block around its attention, as one node each: what the separate nodes of norms, projections,
+// rotary embedding and activation launch, without an allocation, a graph edge and a trip through the engine for each, and with
+// the activation in its projection's epilogue. Both take what those nodes take: contiguous bf16 matrices on the
+// 16-byte grid, widths that are multiples of 8.
+bool block_matrix(const at::Tensor& t, int64_t rows, int64_t cols, const at::Tensor& like) {
+  return plain_call(t, true) && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.size(0) == rows && t.size(1) == cols &&
+      t.is_contiguous() && on16(t) && t.device() == like.device();
+}
+// x w^T of contiguous matrices on the 16-byte grid, widths multiples of 8: this library's product, whose call costs half the
+// tensor library's host time (6.5 and 11.5 us) and which starts early, up to a depth of 4096. Deeper sums that fill the GPU less
+// than once the tensor library splits better, and so products of more than a few million weights whose last unit of 256 rows
+// is mostly empty. In us, both from the host, the library's / this one's: 64 x 512 x 512 11.5 / 7.9, 1000 x 3072 x 2048 13.1 / 13.1,
+// 1000 x 6144 x 4096 37.5 / 38.5, 4096 x 6144 x 4096 137.7 / 131.8; 300 x 4096 x 4096 14.8 / 18.6, 700 x 4096 x 14336 62.1 / 65.6.
+bool mostly_empty_rows(int64_t rows) { return rows > 128 && rows * 10 < (rows + 255) / 256 * 256 * 7; }
+at::Tensor product(const at::Tensor& x, const at::Tensor& w) {
+  const int64_t m = x.size(0), n = w.size(0), k = x.size(1);
+  if (k > 4096 || (mostly_empty_rows(m) && n * k > 12 << 20)) return at::mm(x, w.t());
+  at::Tensor y = at::empty({m, n}, x.options()), status = status_words(x);
+  B200C_CUDA_CHECK(launch_gemm_bf16_nt(x.data_ptr(), w.data_ptr(), y.data_ptr(), static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
+                                       reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(x)));
+  return y;
+}
+// (x w^T, its activation): in one kernel, but for large weights where most of a unit of 256 rows would be empty (300 x 14336 x 4096
+// 88 us, product and activation kernel 67; 64 x 14336 x 4096 54 and 46).
+std::pair<at::Tensor, at::Tensor> gated_product(const at::Tensor& x, const at::Tensor& w) {
+  const int64_t m = x.size(0), n = w.size(0) / 2, k = x.size(1);
+  if ((m <= 128 || mostly_empty_rows(m)) && 2 * n * k > 48 << 20) {
+    at::Tensor gate_up = product(x, w);
+    at::Tensor act = swiglu_fwd(gate_up);
+    return {gate_up, act};
+  }
+  at::Tensor gate_up = at::empty({m, 2 * n}, x.options()), act = at::empty({m, n}, x.options()), status = status_words(x);
+  B200C_CUDA_CHECK(launch_gemm_gated(x.data_ptr(), w.data_ptr(), gate_up.data_ptr(), act.data_ptr(), static_cast<int>(m), static_cast<int>(n),
+                                     static_cast<int>(k), reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(x)));
+  return {gate_up, act};
+}
+// What the products of a node's backward need not be made for.
+at::Tensor product_unless(bool unwanted, const at::Tensor& a, const at::Tensor& b) { return unwanted ? at::Tensor() : at::mm(a, b); }
+
+// (x, queries, keys, values) of x [tokens, dim]: norm, fused projection, rotary embedding. x is returned for the residual.
+struct BlockInFn : torch::autograd::Function<BlockInFn> {
+  static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& norm, const at::Tensor& wqkv,
+                               const at::Tensor& pos, const at::Tensor& cos_t, const at::Tensor& sin_t, int64_t heads, int64_t kv_heads,
+                               double eps) {
+    auto [h, rstd] = rmsnorm_fwd(x, norm, eps);
+    c10::cuda::CUDAGuard g(x.device());
+    const at::Tensor qkv = product(h, wqkv);
+    const int64_t tokens = x.size(0), hd = wqkv.size(0) / (heads + 2 * kv_heads);
+    variable_list out{at::empty({tokens, heads, hd}, x.options()), at::empty({tokens, kv_heads, hd}, x.options()),
+                      at::empty({tokens, kv_heads, hd}, x.options())};
+    SplitRopeFn::launch(qkv, out, pos, cos_t, sin_t, false);
+    ctx->save_for_backward({x, norm, rstd, h, wqkv, pos, cos_t, sin_t});
+    return {x, out[0], out[1], out[2]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const at::Tensor &h = saved[3], &wqkv = saved[4];
+    const at::Tensor dqkv = SplitRopeFn::packed_gradient({grads[1], grads[2], grads[3]}, saved[5], saved[6], saved[7]);
+    const at::Tensor dw = product_unless(!ctx->needs_input_grad(2), dqkv.t(), h);
+    at::Tensor dnorm;
+    const variable_list dx = norm_with_skip_backward({grads[0], at::mm(dqkv, wqkv)}, {saved[0], saved[1], saved[2]}, &dnorm);
+    return {dx[0], dnorm, dw, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+  }
+  static bool applies(const at::Tensor& x, const at::Tensor& norm, const at::Tensor& wqkv, const at::Tensor& pos, const at::Tensor& cos_t,
+                      const at::Tensor& sin_t, int64_t heads, int64_t kv_heads) {
+    if (heads < 1 || kv_heads < 1 || at::autocast::is_autocast_enabled(at::kCUDA) || !norm_with_skip_applies(x, norm)) return false;
+    return x.dim() == 2 && block_matrix(x, x.size(0), x.size(1), x) && wqkv.dim() == 2 && block_matrix(wqkv, wqkv.size(0), x.size(1), x) &&
+        SplitRopeFn::applies_to(x.size(0), wqkv.size(0), x.device(), pos, cos_t, sin_t, heads, kv_heads);
+  }
+};
+
+// x + o wo^T, and on it the norm and the gated MLP: y = s + (silu(gate) * up) w2^T, [gate, up] = norm(s) w13^T, s = x + o wo^T.
+struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
+  static at::Tensor forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& o, const at::Tensor& wo, const at::Tensor& norm,
+                            const at::Tensor& w13, const at::Tensor& w2, double eps) {
+    const int cols = static_cast<int>(x.size(1)), rows = static_cast<int>(x.size(0));
+    c10::cuda::CUDAGuard g(x.device());
+    const at::Tensor delta = product(o, wo);
+    at::Tensor sum = at::empty_like(x), h = at::empty_like(x), rstd = at::empty({rows}, x.options().dtype(at::kFloat));
+    B200C_CUDA_CHECK(launch_rmsnorm_fwd(bf(x), bf(norm), bf_mut(h), rstd.data_ptr<float>(), rows, cols, static_cast<float>(eps), cur(x),
+                                        bf(delta), bf_mut(sum)));
+    const auto [gate_up, act] = gated_product(h, w13);
+    at::Tensor y = product(act, w2);
+    y.add_(sum);
+    ctx->save_for_backward({sum, norm, rstd, o, wo, h, w13, gate_up, act, w2});
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const at::Tensor &o = saved[3], &wo = saved[4], &h = saved[5], &w13 = saved[6], &gate_up = saved[7], &act = saved[8], &w2 = saved[9];
+    const at::Tensor dy = grads[0].contiguous();
+    const at::Tensor dw2 = product_unless(!ctx->needs_input_grad(5), dy.t(), act);
+    const at::Tensor dgate_up = swiglu_bwd(at::mm(dy, w2), gate_up);
+    const at::Tensor dw13 = product_unless(!ctx->needs_input_grad(4), dgate_up.t(), h);
+    at::Tensor dnorm;
+    const at::Tensor ds = norm_with_skip_backward({dy, at::mm(dgate_up, w13)}, {saved[0], saved[1], saved[2]}, &dnorm)[0];
+    const at::Tensor dwo = product_unless(!ctx->needs_input_grad(2), ds.t(), o);
+    return {ds, product_unless(!ctx->needs_input_grad(1), ds, wo), dwo, dnorm, dw13, dw2, at::Tensor()};
+  }
+  static bool applies(const at::Tensor& x, const at::Tensor& o, const at::Tensor& wo, const at::Tensor& norm, const at::Tensor& w13,
+                      const at::Tensor& w2) {
+    if (at::autocast::is_autocast_enabled(at::kCUDA) || !norm_with_skip_applies(x, norm) || x.dim() != 2 || o.dim() != 2 || w2.dim() != 2) {
+      return false;
+    }
+    const int64_t rows = x.size(0), dim = x.size(1), ffn = w2.size(1);
+    return ffn > 0 && ffn % 8 == 0 && o.size(1) > 0 && o.size(1) % 8 == 0 && rows <= INT32_MAX / 2 && ffn <= INT32_MAX / 2 && block_matrix(x, rows, dim, x) &&
+        block_matrix(o, rows, o.size(1), x) && block_matrix(wo, dim, o.size(1), x) && block_matrix(w13, 2 * ffn, dim, x) &&
+        block_matrix(w2, dim, ffn, x);
   }
 };
 
@@ -405,6 +525,16 @@ void bind_ops(py::module_& m) {
                            int64_t heads, int64_t kv_heads) -> std::optional<std::vector<at::Tensor>> {
     if (!SplitRopeFn::applies(qkv, pos, cos_t, sin_t, heads, kv_heads)) return std::nullopt;
     return SplitRopeFn::apply(qkv, pos, cos_t, sin_t, heads, kv_heads);
+  });
+  ops.def("block_in", [](const at::Tensor& x, const at::Tensor& norm, const at::Tensor& wqkv, const at::Tensor& pos, const at::Tensor& cos_t,
+                         const at::Tensor& sin_t, int64_t heads, int64_t kv_heads, double eps) -> std::optional<std::vector<at::Tensor>> {
+    if (!BlockInFn::applies(x, norm, wqkv, pos, cos_t, sin_t, heads, kv_heads)) return std::nullopt;
+    return BlockInFn::apply(x, norm, wqkv, pos, cos_t, sin_t, heads, kv_heads, eps);
+  });
+  ops.def("block_out", [](const at::Tensor& x, const at::Tensor& o, const at::Tensor& wo, const at::Tensor& norm, const at::Tensor& w13,
+                          const at::Tensor& w2, double eps) -> std::optional<at::Tensor> {
+    if (!BlockOutFn::applies(x, o, wo, norm, w13, w2)) return std::nullopt;
+    return BlockOutFn::apply(x, o, wo, norm, w13, w2, eps);
   });
   ops.def("swiglu", [](const at::Tensor& gate_up) -> std::optional<at::Tensor> {
     if (!plain_call(gate_up, true)) return std::nullopt;

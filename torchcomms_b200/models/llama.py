@@ -4,8 +4,9 @@ SwiGLU) used as the flagship training workload.
 The model is written as separate stages - embedding, N identical blocks, head -
 so that a sharded-data-parallel engine can gather, run and free one stage at a
 time.  Norms, rotary embedding, SwiGLU and the loss use the hand-written
-kernels of ``torchcomms_b200.ops``; projections are plain GEMMs and attention
-is PyTorch's fused scaled-dot-product attention.
+kernels of ``torchcomms_b200.ops``, on both sides of attention as one autograd
+node each; the other projections are plain GEMMs and attention is PyTorch's
+fused scaled-dot-product attention.
 """
 from __future__ import annotations
 
@@ -87,16 +88,13 @@ class Block(nn.Module):
         cfg = self.cfg
         b, s, d = x.shape
         hd, nh, nkv = cfg.head_dim, cfg.n_heads, cfg.n_kv_heads
-        x, h = fused.rms_norm_skip(x.reshape(b * s, d), self.attn_norm, cfg.norm_eps)
-        q, k, v = fused.split_rope(F.linear(h, self.wqkv), pos, cos_t, sin_t, nh, nkv)
+        x, q, k, v = fused.block_in(x.reshape(b * s, d), self.attn_norm, self.wqkv, pos, cos_t, sin_t, nh, nkv, cfg.norm_eps)
         q, k, v = q.view(b, s, nh, hd), k.view(b, s, nkv, hd), v.view(b, s, nkv, hd)
         o = F.scaled_dot_product_attention(
             q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True, enable_gqa=(nkv != nh)
         )
         o = o.transpose(1, 2).reshape(b * s, nh * hd)
-        x, h = fused.add_rms_norm(x, F.linear(o, self.wo), self.ffn_norm, cfg.norm_eps)
-        h = fused.swiglu(F.linear(h, self.w13))
-        return (x + F.linear(h, self.w2)).view(b, s, d)
+        return fused.block_out(x, o, self.wo, self.ffn_norm, self.w13, self.w2, cfg.norm_eps).view(b, s, d)
 
 
 class Head(nn.Module):

@@ -149,6 +149,33 @@ def split_rope(qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t:
             v.reshape(t, kv_heads, hd))
 
 
+# ------------------------------------------------------- decoder block
+
+
+def block_in(x: torch.Tensor, norm: torch.Tensor, wqkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor,
+             heads: int, kv_heads: int, eps: float = 1e-5) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
+    """What a decoder block does before attention: ``x = [tokens, dim]`` (for the residual), and queries, keys and values of
+    ``split_rope(rms_norm(x) @ wqkv.T)``."""
+    if x.is_cuda and _native(x, norm, wqkv, pos, cos_t, sin_t):
+        out = _k.block_in(x, norm, wqkv, pos, cos_t, sin_t, heads, kv_heads, eps)
+        if out is not None:
+            return out[0], out[1], out[2], out[3]
+    x, h = rms_norm_skip(x, norm, eps)
+    return (x, *split_rope(F.linear(h, wqkv), pos, cos_t, sin_t, heads, kv_heads))
+
+
+def block_out(x: torch.Tensor, o: torch.Tensor, wo: torch.Tensor, norm: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor,
+              eps: float = 1e-5) -> torch.Tensor:
+    """What a decoder block does after attention (``o = [tokens, heads * head_dim]``): ``s + swiglu(rms_norm(s) @ w13.T) @ w2.T``
+    with ``s = x + o @ wo.T``."""
+    if x.is_cuda and _native(x, o, wo, norm, w13, w2):
+        y = _k.block_out(x, o, wo, norm, w13, w2, eps)
+        if y is not None:
+            return y
+    x, h = add_rms_norm(x, F.linear(o, wo), norm, eps)
+    return x + F.linear(swiglu(F.linear(h, w13)), w2)
+
+
 # ------------------------------------------------- linear + cross entropy
 
 
