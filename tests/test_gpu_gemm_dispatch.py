@@ -54,8 +54,17 @@ def test_plain_product_by_tile_width(m, n, k, fp8):
     test_plain_product(m, n, k, fp8)
 
 
-# Tiles of 112, 96 and 128 columns of gate and of up, one of them in a row, ragged ends of rows, columns and K steps.
-@pytest.mark.parametrize("m,n,k", [(700, 5000, 768), (300, 4808, 72), (1000, 2056, 200), (1, 8, 8), (257, 120, 64), (2049, 232, 136)])
+# A last wave in halves of tiles of 256, of 224 and of 192 columns, one of them past the last column; no whole tile at all.
+@pytest.mark.parametrize("m,n,k", [(4096, 2560, 200), (2049, 2312, 136), (1025, 3784, 520), (1793, 5344, 72), (4096, 1288, 1032)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_plain_product_with_half_tiles(m, n, k, fp8):
+    test_plain_product(m, n, k, fp8)
+
+
+# Tiles of 112, 96 and 128 columns of gate and of up, one of them in a row, ragged ends of rows, columns and K steps,
+# halves of tiles.
+@pytest.mark.parametrize("m,n,k", [(700, 5000, 768), (300, 4808, 72), (1000, 2056, 200), (1, 8, 8), (257, 120, 64), (2049, 232, 136),
+                                   (1000, 2568, 136), (2048, 1160, 72), (512, 9480, 264)])
 def test_gated_product(m, n, k):
     from torchcomms_b200 import _comms
 

@@ -8,8 +8,9 @@
 // The tensor pipe bounds a pair with the memory to itself (a K step of 64 units
 // in 284 ns), operand traffic from L2 to the SMs all of them together: 4096 x
 // 28672 x 4096 in e4m3 318 us in a burst and 369 under the power cap, in bf16
-// 584 and 680. Tiles are 256, 224, 192 or 128 columns wide, whichever leaves the
-// last wave of pairs fuller (pair_columns).
+// 577 and 680. Tiles are 256, 224, 192 or 128 columns wide, whichever leaves the
+// last wave of pairs fuller (pair_columns), and a wave that stays mostly empty
+// all the same is worked on in halves of tiles.
 //
 // Roles per CTA (192 threads): warp 0 (one thread) TMA producer (both CTAs), warp 1
 // tensor-memory allocation (both CTAs) and MMA issue (leader only), warps 2-5
@@ -28,7 +29,7 @@
 //
 // With kGated the product is the first half of a gated MLP: the second CTA's half of a B tile are the rows of `up` that go with
 // the first one's of `gate`, and the epilogue, which then has both of a column, also writes silu(gate) * up. 4096 x 14336 x 4096
-// 609 us, the plain product 584 and with the activation kernel behind it 630; 1000 x 14336 x 4096 165, 157 and 170. Staging the
+// 605 us, the plain product 577 and with the activation kernel behind it 623; 1000 x 14336 x 4096 164, 156 and 169. Staging the
 // activation as well costs a stage of the ring (644 us for the first, 638 with plain stores of it).
 #include "tc_gemm.h"
 
@@ -92,11 +93,12 @@ struct PairMaps {
   CUtensorMap a;    // box 128 rows x 64 columns
   CUtensorMap b;    // box BN / 2 rows x 64 columns (half of the B tile)
   CUtensorMap out;  // box 128 rows x 64 columns
+  CUtensorMap b_tail;  // box BN / 4 rows x 64 columns
 };
 // B and the product in halves, gate and up, of n columns each: a tile has BN / 2 columns of both.
 template <>
 struct PairMaps<kGated> : PairMaps<kPlain> {
-  CUtensorMap b_up, out_up;
+  CUtensorMap b_up, out_up, b_up_tail;
 };
 
 struct PairParams {
@@ -106,7 +108,8 @@ struct PairParams {
   long long* trace;
   int m, n, k, gm;  // k in 16-bit units
   int clear;        // the status words are this call's own
-  int stage_bytes;  // of one K step's loads, both CTAs together
+  int stage_bytes, tail_bytes;  // of one K step's loads, both CTAs together, of a tile and of half a tile
+  int whole;        // tiles that are worked on whole; the others, too few to keep half of the pairs busy, in halves of their columns
   float2* stats;    // kStats: [shares of a row, m] maximum and sum of exponentials; per row its target and the target's logit
   const int64_t* targets;
   float* target_logit;
@@ -185,6 +188,20 @@ __device__ __forceinline__ void pair_tile_at(int t, int tiles_m, int tiles_n, in
   *pn = rem / gsz;
 }
 
+// Item `i` of the work of a product: a tile, or half of one of the last.
+struct PairItem {
+  int pm, col;  // 256-row tile, first column of the output
+  bool tail;
+};
+template <int TILE_COLS>
+__device__ __forceinline__ PairItem pair_item(int i, int whole, int tiles_m, int tiles_n, int gm) {
+  const bool tail = i >= whole;
+  const int half = tail ? (i - whole) & 1 : 0;
+  int pm, pn;
+  pair_tile_at(tail ? whole + ((i - whole) >> 1) : i, tiles_m, tiles_n, gm, &pm, &pn);
+  return PairItem{pm, pn * TILE_COLS + half * (TILE_COLS / 2), tail};
+}
+
 // silu(gate) * up of two columns, from the rounded values as k_swiglu_fwd has it. The reciprocal is the hardware's (1 ulp): the
 // correctly rounded one branches, and a warp alone on its scheduler then has one element at a time in work.
 __device__ __forceinline__ uint32_t gated_pair(uint32_t gate, uint32_t up) {
@@ -210,6 +227,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
   constexpr bool STATS = EPI == kStats, GATED = EPI == kGated;
   constexpr int kTileCols = GATED ? BN / 2 : BN;  // of the output
   constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(2 * kBlockM, BN) : make_idesc_bf16(2 * kBlockM, BN);
+  constexpr uint32_t idesc_tail = FP8 ? make_idesc_e4m3(2 * kBlockM, BN / 2) : make_idesc_bf16(2 * kBlockM, BN / 2);
   using Tile = PairTile<BN, EPI>;
   constexpr int kChunk = Tile::kChunk;
   constexpr int kStages = Tile::kStages, kStageBytes = Tile::kStageBytes, kOutBuffers = Tile::kOutBuffers;
@@ -224,7 +242,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
   const bool leader = cta == 0;
   const int cluster_id = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
   const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / kTileCols + 1;
-  const int total_tiles = tiles_m * tiles_n;
+  const int items = p.whole + 2 * (tiles_m * tiles_n - p.whole);
   const int k_iters = (p.k + kBlockK - 1) / kBlockK;
 
   if (threadIdx.x == 0) {
@@ -258,14 +276,16 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     // ---------------- TMA producer (each CTA loads its own A rows and its half of B)
     if (elect_one()) {
       uint32_t it = 0;
-      for (int t = cluster_id; t < total_tiles && !bars->failed; t += nclusters) {
-        int pm, pn;
-        pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
-        const int a_row = (pm * 2 + static_cast<int>(cta)) * kBlockM;
+      for (int i = cluster_id; i < items && !bars->failed; i += nclusters) {
+        const PairItem at = pair_item<kTileCols>(i, p.whole, tiles_m, tiles_n, p.gm);
+        const int a_row = (at.pm * 2 + static_cast<int>(cta)) * kBlockM;
         // Each CTA loads one half of the B tile: the second one its last rows, or its rows of the second half of B.
-        const int b_row = GATED ? pn * kTileCols : pn * BN + static_cast<int>(cta) * (BN / 2);
-        const CUtensorMap* b_map = &maps.b;
-        if constexpr (GATED) b_map = leader ? &maps.b : &maps.b_up;
+        const int b_row = GATED ? at.col : at.col + static_cast<int>(cta) * (at.tail ? BN / 4 : BN / 2);
+        const CUtensorMap* b_map = at.tail ? &maps.b_tail : &maps.b;
+        if constexpr (GATED) {
+          if (!leader) b_map = at.tail ? &maps.b_up_tail : &maps.b_up;
+        }
+        const uint32_t bytes = static_cast<uint32_t>(at.tail ? p.tail_bytes : p.stage_bytes);
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
@@ -274,7 +294,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
             break;
           }
           // The leader's barrier counts all four loads of the stage.
-          if (leader) mbar_expect_tx(&bars->full[s], static_cast<uint32_t>(p.stage_bytes));
+          if (leader) mbar_expect_tx(&bars->full[s], bytes);
           char* sa = stages + s * kStageBytes;
           tma_load_2d_pair(sa, &maps.a, &bars->full[s], kb * kBlockK, a_row);
           tma_load_2d_pair(sa + kABytes, b_map, &bars->full[s], kb * kBlockK, b_row);
@@ -286,7 +306,8 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     // ---------------- MMA issuer (leader CTA only)
     if (leader && elect_one()) {
       uint32_t it = 0, tile_iter = 0;
-      for (int t = cluster_id; t < total_tiles && !bars->failed; t += nclusters, ++tile_iter) {
+      for (int i = cluster_id; i < items && !bars->failed; i += nclusters, ++tile_iter) {
+        const uint32_t shape = i >= p.whole ? idesc_tail : idesc;
         const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
         if (!mbar_wait(&bars->acc_empty[as], aph ^ 1u)) {
           bars->failed = 1;
@@ -308,9 +329,9 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           for (int kk = 0; kk < kBlockK / kUmmaK; ++kk) {
             // 16 bf16 (or 32 e4m3) = 32 bytes further along K inside the swizzled row
             if (FP8) {
-              umma_f8_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), idesc, (kb | kk) != 0);
+              umma_f8_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), shape, (kb | kk) != 0);
             } else {
-              umma_bf16_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), idesc, (kb | kk) != 0);
+              umma_bf16_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), shape, (kb | kk) != 0);
             }
           }
           umma_commit_pair(&bars->empty[s], 3);  // both CTAs may refill the stage
@@ -330,16 +351,15 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     // Where 16 bytes of a row lie in a staged chunk.
     const auto staged = [](int row, int piece) { return kChunk == 64 ? row * 128 + ((piece ^ (row & 7)) << 4) : row * kChunk * 2 + piece * 16; };
     // What a row brings along is fetched a tile ahead: its scale, or the column its target has in the tile's row of tiles.
-    const auto rows_of = [&](int t) {
-      int pm, pn;
-      pair_tile_at(t, tiles_m, tiles_n, p.gm, &pm, &pn);
-      return make_int2((pm * 2 + static_cast<int>(cta)) * kBlockM, pn * kTileCols);
+    const auto place_of = [&](int i) {
+      const PairItem at = pair_item<kTileCols>(i, p.whole, tiles_m, tiles_n, p.gm);
+      return make_int2((at.pm * 2 + static_cast<int>(cta)) * kBlockM, at.col);
     };
     ColScales<BN> fetched;
     float next_scale = 0.0f;
     int64_t next_target = -1;
-    const auto fetch = [&](int t) {
-      const int2 at = rows_of(t);
+    const auto fetch = [&](int i) {
+      const int2 at = place_of(i);
       const int row = at.x + row_in_tile;
       if (FP8) {
         fetched.fetch(p.scale_b, at.y, p.n, et);
@@ -348,19 +368,20 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
       if (STATS) next_target = row < p.m ? p.targets[row] : -1;
     };
     const int first = cluster_id + set * nclusters, step = kSets * nclusters;
-    if (first < total_tiles) fetch(first);
+    if (first < items) fetch(first);
     uint32_t tile_iter = static_cast<uint32_t>(set), chunk_iter = 0;
-    for (int t = first; t < total_tiles; t += step, tile_iter += kSets) {
+    for (int i = first; i < items; i += step, tile_iter += kSets) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
-      const int2 at = rows_of(t);
+      const int2 at = place_of(i);
       const int out_row = at.x, out_col = at.y;
+      const bool tail = i >= p.whole;
       const float row_scale = next_scale;
       const int target = next_target >= 0 && next_target < p.n ? static_cast<int>(next_target) - out_col : -1;  // column of the tile
       if (FP8) {
         fetched.put(col_scales, et);
         epilogue_sync(set);
       }
-      if (t + step < total_tiles) fetch(t + step);
+      if (i + step < items) fetch(i + step);
       if (!mbar_wait(&bars->acc_full[as], aph)) {
         bars->failed = 1;
         break;
@@ -370,7 +391,9 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
       const bool row_there = STATS && out_row + row_in_tile < p.m;
       if constexpr (GATED) {
         static_assert(!GATED || kSets == 1, "");
-        for (int j = 0; j < kTileCols / kChunk; ++j) {
+        const int chunks = kTileCols / kChunk / (tail ? 2 : 1);
+        const uint32_t to_up = tail ? BN / 4 : BN / 2;
+        for (int j = 0; j < chunks; ++j) {
           if (issuer) tma_store_wait_read<0>();
           epilogue_sync(0);
 #pragma unroll
@@ -379,9 +402,9 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
             const uint32_t from = tmem_base + as * kAccCols + (static_cast<uint32_t>(q * 32) << 16) +
                 static_cast<uint32_t>(j * kChunk + half * 32);
             tmem_ld_32x32(from, g);
-            tmem_ld_32x32(from + BN / 2, u);
+            tmem_ld_32x32(from + to_up, u);
             tmem_ld_wait();
-            if (j == kTileCols / kChunk - 1 && half == 1) {
+            if (j == chunks - 1 && half == 1) {
               tc_fence_before_sync();
               __syncwarp();
               if (lane == 0) mbar_arrive_leader(&bars->acc_empty[as]);
@@ -416,7 +439,8 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
         }
         continue;
       }
-      for (int j = 0; j < BN / kChunk; ++j, ++chunk_iter) {
+      const int chunks = BN / kChunk / (tail ? 2 : 1);
+      for (int j = 0; j < chunks; ++j, ++chunk_iter) {
         char* buf = obuf + (2 * set + (chunk_iter & 1u)) * kOutChunkBytes;
         uint32_t acc[2][32];
 #pragma unroll
@@ -426,7 +450,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
                         acc[half]);
         }
         tmem_ld_wait();
-        if (j == BN / kChunk - 1) {
+        if (j == chunks - 1) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive_leader(&bars->acc_empty[as]);
@@ -487,6 +511,15 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
   if (threadIdx.x == 0) trace_stamp_ns(p.trace, 7);
 }
 
+// Whether the tiles of a last, partial wave are worked on in halves of their columns: where at most half of the pairs would
+// have one. In us without and so: bf16 4096 x 4096 x 14336 (34 of 74 pairs) 328 and 317, 4096 x 2560 x 2560 (12) 43.0 and 38.7, 1000
+// x 28672 x 4096 (4) 161.7 and 156.6; e4m3 4096 x 4096 x 14336 175.7 and 168.2, 640 x 20480 x 2048 (18) 28.7 and 26.8; gated 2048 x
+// 14336 x 4096 (8) 313 and 308, 512 x 14336 x 4096 (2) 99.1 and 94.0.
+bool tail_in_halves(int64_t tiles, int64_t pairs, int columns) {
+  const int64_t rest = tiles % pairs;
+  return columns > 128 && rest > 0 && 2 * rest <= pairs;
+}
+
 constexpr int kDevices = 64;  // whose answers are kept
 
 // Pairs that the current GPU holds at once (each CTA fills an SM), or 0 after an error. Kept per device; a query that
@@ -526,18 +559,22 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
   }
   constexpr int kTileCols = EPI == kGated ? BN / 2 : BN;
   PairMaps<EPI> maps;
-  if (!make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m)) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.out, c, p.m, p.n, kBlockM, ldc, PairTile<BN, EPI>::kChunk)) {
+  if (!make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m)) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.b_tail, b, p.n, p.k, BN / 4) || !make_map(&maps.out, c, p.m, p.n, kBlockM, ldc, PairTile<BN, EPI>::kChunk)) {
     return cudaErrorInvalidValue;
   }
   if constexpr (EPI == kGated) {
     const auto* up = static_cast<const char*>(b) + static_cast<size_t>(p.n) * p.k * 2;
-    if (!make_map(&maps.b_up, up, p.n, p.k, BN / 2) ||
+    if (!make_map(&maps.b_up, up, p.n, p.k, BN / 2) || !make_map(&maps.b_up_tail, up, p.n, p.k, BN / 4) ||
         !make_map(&maps.out_up, static_cast<char*>(c) + static_cast<size_t>(p.n) * 2, p.m, p.n, kBlockM, ldc, PairTile<BN, EPI>::kChunk)) {
       return cudaErrorInvalidValue;
     }
   }
   p.stage_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN, EPI>::kBHalfBytes);
+  p.tail_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN, EPI>::kBHalfBytes / 2);
   const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / kTileCols + 1;
+  const int64_t tiles = static_cast<int64_t>(tiles_m) * tiles_n;
+  const bool halves = EPI != kStats && tail_in_halves(tiles, pairs, BN);
+  p.whole = static_cast<int>(halves ? tiles - tiles % pairs : tiles);
   // A rows of a group stay in L2 while the pairs sweep over n: at most 8 pair-tiles and ~40 MB. Every group reads B again,
   // so where L2 does not keep that either (above 48 MB) groups are of up to 16 pair-tiles and 32 MB. In us under the power
   // cap with 8 and 16: 4096 x 28672 x 4096 in e4m3 (B of 117 MB) 397 and 390, 8192 x 14336 x 4096 (59 MB) 400 and 392; 4096 x
@@ -546,7 +583,7 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
   const bool b_again = static_cast<size_t>(p.n) * p.k * 2 * (BN / kTileCols) > (48u << 20);
   p.gm = std::max(1, std::min({b_again ? 16 : 8, tiles_m, static_cast<int>((b_again ? 32u << 20 : 40u << 20) / std::max<size_t>(a_tile_bytes, 1))}));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(pairs, static_cast<int64_t>(tiles_m) * tiles_n)));
+  cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(pairs, halves ? tiles + tiles % pairs : tiles)));
   cfg.blockDim = dim3(pair_threads<EPI>());
   cfg.dynamicSmemBytes = PairTile<BN, EPI>::kSmemBytes;
   cfg.stream = stream;
@@ -574,18 +611,21 @@ double wave_cost(int64_t tiles, int64_t at_once) {
 }
 
 // The width whose waves take least. A wave of full width costs 1 and one of half the width 0.575 (the rows of A come in either
-// way). 256 unless another is 1 % ahead. Of 39 sizes, types and epilogues this takes the best of 256, 224, 192, 160 and 128
-// everywhere but once (0.4 % behind). In us with 256 / 224 / 192 columns: bf16 1000 x 6144 x 4096 45.3 / 42.0 / 39.0, 1000 x 28672 x
-// 4096 161.7 / 157.0 / 166.3, 1500 x 5000 x 2992 37.5 / 34.7 / 42.6, 4096 x 4096 x 14336 328 / 346 / 334; e4m3 1000 x 6144 x 4096
-// 26.8 / 24.7 / 22.4, 4096 x 2560 x 2560 25.6 / 23.7 / 24.9; gated 1000 x 14336 x 4096 168.9 / 165.3 / 173.4.
+// way), a last wave of halves a tenth more. 256 unless another is 1 % ahead. Of 39 sizes, types and epilogues this takes the
+// best width or one at most 2 % behind it. In us with 256 / 224 / 192 columns: bf16 1000 x 6144 x 4096 40.1 / 43.0 / 38.9, 1500 x 5000 x
+// 2992 38.3 / 34.9 / 40.7, 1024 x 8192 x 1024 16.2 / 15.2 / 15.9, 4096 x 4096 x 14336 318 / 333 / 331; e4m3 1500 x 5000 x 2992 28.0 /
+// 26.6 / 31.4, 4096 x 2560 x 2560 23.0 / 24.1 / 23.4; gated 700 x 5000 x 768 16.8 / 15.4 / 16.0.
 int pair_columns(int m, int n, bool gated, double* cost) {
   const int64_t pairs = std::max(1, pairs_at_once(false)), tiles_m = (m - 1) / (2 * kBlockM) + 1;
   int best = 256;
   double least = 0.0;
+  const auto width_cost = [](int columns) { return 0.15 + 0.85 * columns / 256.0; };
   for (const int columns : {256, 224, 192, 128}) {
     if (gated && columns == 128) break;
-    const double waves = wave_cost(tiles_m * ((n - 1) / (gated ? columns / 2 : columns) + 1), pairs);
-    const double here = waves * (0.15 + 0.85 * columns / 256.0) * (columns == 256 ? 0.99 : 1.0);
+    const int64_t tiles = tiles_m * ((n - 1) / (gated ? columns / 2 : columns) + 1), rest = tiles % pairs;
+    const double here = (tail_in_halves(tiles, pairs, columns)
+                             ? static_cast<double>(tiles / pairs) * width_cost(columns) + 1.1 * wave_cost(2 * rest, pairs) * width_cost(columns / 2)
+                             : wave_cost(tiles, pairs) * width_cost(columns)) * (columns == 256 ? 0.99 : 1.0);
     if (columns == 256 || here < least) {
       best = columns;
       least = here;
