@@ -97,6 +97,27 @@ def test_gated_product_of_extremes():
     torch.testing.assert_close(act, _comms.ops.swiglu_fwd(gate_up), rtol=2**-7, atol=0, equal_nan=True)
 
 
+# K in the rows of both operands, or in the rows of b alone: one row, one column unit, K steps that end anywhere, narrow and wide
+# tiles, a last wave in halves; rows of a that are apart.
+@pytest.mark.parametrize("m,n,k", [(8, 8, 1), (1, 8, 8), (257, 136, 65), (1000, 520, 1003), (2049, 2312, 136), (4096, 2560, 200), (130, 9480, 77)])
+@pytest.mark.parametrize("by_columns", [False, True])
+def test_product_along_rows(m, n, k, by_columns):
+    from torchcomms_b200 import _comms
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    rows, cols = (k, m) if by_columns else (m, k)
+    wide = torch.randn(rows, (cols + 63) // 64 * 64, generator=g, device="cuda").to(torch.bfloat16)
+    wide[:, cols:] = float("nan")  # between the rows, not read
+    a = wide[:, :cols]
+    b = torch.randn(k, n, generator=g, device="cuda").to(torch.bfloat16)
+    c, status = _comms.ops.gemm_bf16_mn(a, b, by_columns)
+    assert int(status[0]) == 0
+    ref = (a.t() if by_columns else a).double() @ b.double()
+    # Half a bf16 ulp (2^-9 relative), and k fp32 additions of terms of size 1 before it.
+    torch.testing.assert_close(c.double(), ref, rtol=2**-8, atol=4e-6 * k)
+    assert torch.equal(c, _comms.ops.gemm_bf16_mn(a, b, by_columns)[0])
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 256, 64), (128, 3584, 4096), (384, 512, 704), (512, 5120, 512)])
 def test_gather_layer_leaves_its_input_behind(m, n, k):
     """A single rank's layer reads the activations where they are; its input buffer holds them afterwards all the same."""

@@ -326,11 +326,26 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
   return d;
 }
 
-// Instruction descriptor: bf16 x bf16 -> fp32, both operands K-major.
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n) {
+// The same for an MN-major tile: 64 rows of K of 64 bf16 each (128 bytes, swizzled), one such block of 8 KB after the other along
+// M or N. Eight rows of K are 1024 bytes; stepping along K adds 128 bytes a row.
+constexpr int kMnBlock = 64;
+constexpr int kMnBlockBytes = kBlockK * kMnBlock * 2;
+__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>(kMnBlockBytes >> 4) << 16;       // leading byte offset: from block to block
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;                // stride byte offset: 8 rows of K
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(2) << 61;
+  return d;
+}
+
+// Instruction descriptor: bf16 x bf16 -> fp32, operands K-major or MN-major.
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, bool a_mn = false, bool b_mn = false) {
   return (1u << 4)                              // D format: fp32
       | (1u << 7)                               // A format: bf16
       | (1u << 10)                              // B format: bf16
+      | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u)
       | (static_cast<uint32_t>(n >> 3) << 17)   // N / 8
       | (static_cast<uint32_t>(m >> 4) << 24);  // M / 16
 }

@@ -49,6 +49,9 @@ using namespace tc;
 
 constexpr int kABytes = kBlockM * kBlockK * 2;  // 16 KB: this CTA's 128 rows of A
 constexpr int kOutChunkBytes = kBlockM * 64 * 2;  // of the widest chunk
+// How the operands lie in memory, K being the rows of B and of A or its columns: A [m, k] and B [n, k], A [m, k] and B [k, n], A [k,
+// m] and B [k, n]. The tensor pipe takes either; only the boxes that bring the operands differ.
+enum class PairLayout { kNT, kNN, kTN };
 // What the epilogue does besides storing the product.
 enum Epilogue { kPlain, kStats, kGated };
 // Warps of the epilogue: four, one for each quarter of the tensor memory's lanes, or two such sets that take the tiles, and
@@ -222,12 +225,14 @@ __device__ __forceinline__ void epilogue_sync(int set) {
   else asm volatile("bar.sync 2, 128;" ::: "memory");
 }
 
-template <bool FP8, int BN, Epilogue EPI>
+template <bool FP8, int BN, Epilogue EPI, PairLayout LAYOUT>
 __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __grid_constant__ PairMaps<EPI> maps, PairParams p) {
   constexpr bool STATS = EPI == kStats, GATED = EPI == kGated;
+  constexpr bool A_MN = LAYOUT == PairLayout::kTN, B_MN = LAYOUT != PairLayout::kNT;
+  static_assert(!B_MN || (!FP8 && EPI == kPlain && BN % 128 == 0), "whole blocks of 64 columns for each CTA");
   constexpr int kTileCols = GATED ? BN / 2 : BN;  // of the output
-  constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(2 * kBlockM, BN) : make_idesc_bf16(2 * kBlockM, BN);
-  constexpr uint32_t idesc_tail = FP8 ? make_idesc_e4m3(2 * kBlockM, BN / 2) : make_idesc_bf16(2 * kBlockM, BN / 2);
+  constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(2 * kBlockM, BN) : make_idesc_bf16(2 * kBlockM, BN, A_MN, B_MN);
+  constexpr uint32_t idesc_tail = FP8 ? make_idesc_e4m3(2 * kBlockM, BN / 2) : make_idesc_bf16(2 * kBlockM, BN / 2, A_MN, B_MN);
   using Tile = PairTile<BN, EPI>;
   constexpr int kChunk = Tile::kChunk;
   constexpr int kStages = Tile::kStages, kStageBytes = Tile::kStageBytes, kOutBuffers = Tile::kOutBuffers;
@@ -296,8 +301,23 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           // The leader's barrier counts all four loads of the stage.
           if (leader) mbar_expect_tx(&bars->full[s], bytes);
           char* sa = stages + s * kStageBytes;
-          tma_load_2d_pair(sa, &maps.a, &bars->full[s], kb * kBlockK, a_row);
-          tma_load_2d_pair(sa + kABytes, b_map, &bars->full[s], kb * kBlockK, b_row);
+          if constexpr (A_MN) {
+#pragma unroll
+            for (int j = 0; j < kBlockM / kMnBlock; ++j) {
+              tma_load_2d_pair(sa + j * kMnBlockBytes, &maps.a, &bars->full[s], a_row + j * kMnBlock, kb * kBlockK);
+            }
+          } else {
+            tma_load_2d_pair(sa, &maps.a, &bars->full[s], kb * kBlockK, a_row);
+          }
+          if constexpr (B_MN) {
+#pragma unroll
+            for (int j = 0; j < BN / 2 / kMnBlock; ++j) {
+              if (j > 0 && at.tail) break;  // half a tile: half the columns
+              tma_load_2d_pair(sa + kABytes + j * kMnBlockBytes, &maps.b, &bars->full[s], b_row + j * kMnBlock, kb * kBlockK);
+            }
+          } else {
+            tma_load_2d_pair(sa + kABytes, b_map, &bars->full[s], kb * kBlockK, b_row);
+          }
         }
       }
       trace_stamp_ns(p.trace, 1);
@@ -324,14 +344,16 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           }
           tc_fence_after_sync();
           const uint32_t sa = smem_u32(stages + s * kStageBytes);
-          const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + kABytes);
+          const uint64_t da = A_MN ? make_smem_desc_mn(sa) : make_smem_desc(sa);
+          const uint64_t db = B_MN ? make_smem_desc_mn(sa + kABytes) : make_smem_desc(sa + kABytes);
+          // 16 bf16 (or 32 e4m3) further along K: 32 bytes inside the swizzled row, or 16 rows of 128 bytes.
+          constexpr uint64_t kNextA = (A_MN ? kUmmaK * 128 : 32) >> 4, kNextB = (B_MN ? kUmmaK * 128 : 32) >> 4;
 #pragma unroll
           for (int kk = 0; kk < kBlockK / kUmmaK; ++kk) {
-            // 16 bf16 (or 32 e4m3) = 32 bytes further along K inside the swizzled row
             if (FP8) {
-              umma_f8_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), shape, (kb | kk) != 0);
+              umma_f8_pair(tmem_acc, da + kk * kNextA, db + kk * kNextB, shape, (kb | kk) != 0);
             } else {
-              umma_bf16_pair(tmem_acc, da + static_cast<uint64_t>(kk * 2), db + static_cast<uint64_t>(kk * 2), shape, (kb | kk) != 0);
+              umma_bf16_pair(tmem_acc, da + kk * kNextA, db + kk * kNextB, shape, (kb | kk) != 0);
             }
           }
           umma_commit_pair(&bars->empty[s], 3);  // both CTAs may refill the stage
@@ -524,7 +546,7 @@ constexpr int kDevices = 64;  // whose answers are kept
 
 // Pairs that the current GPU holds at once (each CTA fills an SM), or 0 after an error. Kept per device; a query that
 // failed is asked again at the next call.
-template <bool FP8, int BN, Epilogue EPI = kPlain>
+template <bool FP8, int BN, Epilogue EPI = kPlain, PairLayout LAYOUT = PairLayout::kNT>
 int resident_pairs() {
   static std::atomic<int> known[kDevices];
   int device = 0, n = 0;
@@ -532,7 +554,10 @@ int resident_pairs() {
   std::atomic<int>* kept = device >= 0 && device < kDevices ? &known[device] : nullptr;
   if (kept != nullptr) n = kept->load(std::memory_order_acquire);
   if (n > 0) return n;
-  if (cudaFuncSetAttribute(k_gemm_pair<FP8, BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairTile<BN, EPI>::kSmemBytes) != cudaSuccess) return 0;
+  if (cudaFuncSetAttribute(k_gemm_pair<FP8, BN, EPI, LAYOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairTile<BN, EPI>::kSmemBytes) !=
+      cudaSuccess) {
+    return 0;
+  }
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2);
@@ -544,22 +569,27 @@ int resident_pairs() {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, k_gemm_pair<FP8, BN, EPI>, &cfg) != cudaSuccess || n < 1) return 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_gemm_pair<FP8, BN, EPI, LAYOUT>, &cfg) != cudaSuccess || n < 1) return 0;
   if (kept != nullptr) kept->store(n, std::memory_order_release);
   return n;
 }
 
-// `ldc`: row stride of the output in elements (0: n).
-template <bool FP8, int BN, Epilogue EPI = kPlain>
-cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cudaStream_t stream, int64_t ldc = 0) {
-  const int pairs = resident_pairs<FP8, BN, EPI>();
+// `ldc`: row stride of the output in elements (0: n), `lda`, `ldb`: of the operands as they lie in memory (0: rows follow one another).
+template <bool FP8, int BN, Epilogue EPI = kPlain, PairLayout LAYOUT = PairLayout::kNT>
+cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cudaStream_t stream, int64_t ldc = 0, int64_t lda = 0,
+                        int64_t ldb = 0) {
+  const int pairs = resident_pairs<FP8, BN, EPI, LAYOUT>();
   if (pairs < 1) {
     const cudaError_t e = cudaGetLastError();
     return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
   }
   constexpr int kTileCols = EPI == kGated ? BN / 2 : BN;
   PairMaps<EPI> maps;
-  if (!make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m)) || !make_map(&maps.b, b, p.n, p.k, BN / 2) || !make_map(&maps.b_tail, b, p.n, p.k, BN / 4) || !make_map(&maps.out, c, p.m, p.n, kBlockM, ldc, PairTile<BN, EPI>::kChunk)) {
+  constexpr bool A_MN = LAYOUT == PairLayout::kTN, B_MN = LAYOUT != PairLayout::kNT;
+  const bool mapped_a = A_MN ? make_map(&maps.a, a, p.k, p.m, kBlockK, lda) : make_map(&maps.a, a, p.m, p.k, a_box_rows(p.m), lda);
+  const bool mapped_b = B_MN ? make_map(&maps.b, b, p.k, p.n, kBlockK, ldb)
+                             : make_map(&maps.b, b, p.n, p.k, BN / 2, ldb) && make_map(&maps.b_tail, b, p.n, p.k, BN / 4, ldb);
+  if (!mapped_a || !mapped_b || !make_map(&maps.out, c, p.m, p.n, kBlockM, ldc, PairTile<BN, EPI>::kChunk)) {
     return cudaErrorInvalidValue;
   }
   if constexpr (EPI == kGated) {
@@ -569,8 +599,9 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
       return cudaErrorInvalidValue;
     }
   }
-  p.stage_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN, EPI>::kBHalfBytes);
-  p.tail_bytes = 2 * (a_box_rows(p.m) * kBlockK * 2 + PairTile<BN, EPI>::kBHalfBytes / 2);
+  const int a_bytes = A_MN ? kABytes : a_box_rows(p.m) * kBlockK * 2;
+  p.stage_bytes = 2 * (a_bytes + PairTile<BN, EPI>::kBHalfBytes);
+  p.tail_bytes = 2 * (a_bytes + PairTile<BN, EPI>::kBHalfBytes / 2);
   const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / kTileCols + 1;
   const int64_t tiles = static_cast<int64_t>(tiles_m) * tiles_n;
   const bool halves = EPI != kStats && tail_in_halves(tiles, pairs, BN);
@@ -596,7 +627,7 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gemm_pair<FP8, BN, EPI>, maps, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gemm_pair<FP8, BN, EPI, LAYOUT>, maps, p);
   note_kernel_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -664,6 +695,32 @@ cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, in
     }
   };
   return scale_a != nullptr ? launch(std::true_type()) : launch(std::false_type());
+}
+
+// Tiles of 128 columns where they are at most a wave, otherwise of 256: the blocks of 64 columns that each CTA brings allow no width
+// between. A step brings its operands in up to four boxes, and the tensor pipe takes them as fast as along K: 4096 x 14336 x 4096
+// 290 us with both along rows, 294 with one (the tensor library 324 and 319), 1000 x 28672 x 4096 156 (183).
+cudaError_t launch_gemm_pair_mn(const void* a, int64_t lda, bool a_by_columns, const void* b, int64_t ldb, void* c, int m, int n, int k,
+                                uint32_t* status, cudaStream_t stream) {
+  if (m <= 0 || n <= 0 || k <= 0 || lda % 8 != 0 || ldb % 8 != 0 || n % 8 != 0 || lda < (a_by_columns ? m : k) || ldb < n) {
+    return cudaErrorInvalidValue;
+  }
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) {
+    return cudaErrorMisalignedAddress;
+  }
+  PairParams p{};
+  p.status = status;
+  p.clear = status != nullptr ? 1 : 0;
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  const bool narrow = pair_tiles_fit(m, n, false);
+  if (a_by_columns) {
+    return narrow ? launch_pair<false, 128, kPlain, PairLayout::kTN>(a, b, c, p, stream, 0, lda, ldb)
+                  : launch_pair<false, 256, kPlain, PairLayout::kTN>(a, b, c, p, stream, 0, lda, ldb);
+  }
+  return narrow ? launch_pair<false, 128, kPlain, PairLayout::kNN>(a, b, c, p, stream, 0, lda, ldb)
+                : launch_pair<false, 256, kPlain, PairLayout::kNN>(a, b, c, p, stream, 0, lda, ldb);
 }
 
 int head_row_shares(int m, int n) {

@@ -339,8 +339,47 @@ std::pair<at::Tensor, at::Tensor> gated_product(const at::Tensor& x, const at::T
                                      static_cast<int>(k), reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(x)));
   return {gate_up, act};
 }
-// What the products of a node's backward need not be made for.
-at::Tensor product_unless(bool unwanted, const at::Tensor& a, const at::Tensor& b) { return unwanted ? at::Tensor() : at::mm(a, b); }
+// Which products of a backward pass this library makes. With K in both operands' rows (a weight's gradient): all but those of
+// few tiles and a long sum, which the tensor library shares out. With K in A's columns (an input's): short sums, which end
+// before the next call is made, and from 700 rows on those of up to 96 steps, or 48 where the tiles are few. In us, both from
+// the host, the tensor library's / this one's: weights' gradients (columns x columns, rows) 512 x 512, 64 11.1 / 5.7; 28672 x 4096, 1000
+// 183 / 156; 4096 x 14336, 4096 324 / 290; 512 x 512, 4096 11.3 / 13.8. Inputs' gradients (rows x K x columns) 64 x 2048 x 8192 11.6 / 10.6,
+// 1000 x 4096 x 14336 82.4 / 82.8, 4096 x 4096 x 14336 319 / 294; 300 x 3072 x 2048 9.0 / 12.1, 1000 x 4096 x 512 13.9 / 15.2, 64 x 28672 x
+// 4096 42 / 94.
+constexpr int64_t kKStep = 64;
+bool few_tiles(int64_t m, int64_t n) { return pair_tiles_fit(static_cast<int>(m), static_cast<int>(n), false); }
+bool own_by_columns(int64_t m, int64_t n, int64_t k) { return !few_tiles(m, n) || k <= 48 * kKStep; }
+bool own_by_rows(int64_t m, int64_t n, int64_t k) {
+  if (mostly_empty_rows(m) && n * k > 12 << 20) return false;
+  return k <= 32 * kKStep || (m >= 700 && k <= (few_tiles(m, n) ? 48 : 96) * kKStep);
+}
+void mn_product_into(at::Tensor& c, const at::Tensor& a, bool by_columns, const at::Tensor& b) {
+  at::Tensor status = status_words(b);
+  B200C_CUDA_CHECK(launch_gemm_pair_mn(a.data_ptr(), a.stride(0), by_columns, b.data_ptr(), b.stride(0), c.data_ptr(),
+                                       static_cast<int>(c.size(0)), static_cast<int>(c.size(1)), static_cast<int>(b.size(0)),
+                                       reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(b)));
+}
+// dy [rows, n] w [n, k] and dy^T x [rows, k], the gradients of a product's operands. The tensor library's where the backward pass is
+// itself differentiated, and where a hook has put something else in a tensor's place.
+bool plain_rows(const at::Tensor& t, const at::Tensor& like) {
+  return plain_call(t) && block_matrix(t, t.size(0), t.size(1), like) && t.size(1) % 8 == 0;
+}
+at::Tensor input_gradient(const at::Tensor& dy, const at::Tensor& w) {
+  if (!plain_rows(dy, dy) || !plain_rows(w, dy) || dy.size(1) != w.size(0) || !own_by_rows(dy.size(0), w.size(1), w.size(0))) {
+    return at::mm(dy, w);
+  }
+  at::Tensor dx = at::empty({dy.size(0), w.size(1)}, w.options());
+  mn_product_into(dx, dy, false, w);
+  return dx;
+}
+at::Tensor weight_gradient(const at::Tensor& dy, const at::Tensor& x) {
+  if (!plain_rows(dy, dy) || !plain_rows(x, dy) || dy.size(0) != x.size(0) || !own_by_columns(dy.size(1), x.size(1), x.size(0))) {
+    return at::mm(dy.t(), x);
+  }
+  at::Tensor dw = at::empty({dy.size(1), x.size(1)}, x.options());
+  mn_product_into(dw, dy, true, x);
+  return dw;
+}
 
 // (x, queries, keys, values) of x [tokens, dim]: norm, fused projection, rotary embedding. x is returned for the residual.
 struct BlockInFn : torch::autograd::Function<BlockInFn> {
@@ -361,9 +400,9 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     const auto saved = ctx->get_saved_variables();
     const at::Tensor &h = saved[3], &wqkv = saved[4];
     const at::Tensor dqkv = SplitRopeFn::packed_gradient({grads[1], grads[2], grads[3]}, saved[5], saved[6], saved[7]);
-    const at::Tensor dw = product_unless(!ctx->needs_input_grad(2), dqkv.t(), h);
+    const at::Tensor dw = ctx->needs_input_grad(2) ? weight_gradient(dqkv, h) : at::Tensor();
     at::Tensor dnorm;
-    const variable_list dx = norm_with_skip_backward({grads[0], at::mm(dqkv, wqkv)}, {saved[0], saved[1], saved[2]}, &dnorm);
+    const variable_list dx = norm_with_skip_backward({grads[0], input_gradient(dqkv, wqkv)}, {saved[0], saved[1], saved[2]}, &dnorm);
     return {dx[0], dnorm, dw, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
   }
   static bool applies(const at::Tensor& x, const at::Tensor& norm, const at::Tensor& wqkv, const at::Tensor& pos, const at::Tensor& cos_t,
@@ -394,13 +433,14 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
     const auto saved = ctx->get_saved_variables();
     const at::Tensor &o = saved[3], &wo = saved[4], &h = saved[5], &w13 = saved[6], &gate_up = saved[7], &act = saved[8], &w2 = saved[9];
     const at::Tensor dy = grads[0].contiguous();
-    const at::Tensor dw2 = product_unless(!ctx->needs_input_grad(5), dy.t(), act);
-    const at::Tensor dgate_up = swiglu_bwd(at::mm(dy, w2), gate_up);
-    const at::Tensor dw13 = product_unless(!ctx->needs_input_grad(4), dgate_up.t(), h);
+    c10::cuda::CUDAGuard g(dy.device());
+    const at::Tensor dw2 = ctx->needs_input_grad(5) ? weight_gradient(dy, act) : at::Tensor();
+    const at::Tensor dgate_up = swiglu_bwd(input_gradient(dy, w2), gate_up);
+    const at::Tensor dw13 = ctx->needs_input_grad(4) ? weight_gradient(dgate_up, h) : at::Tensor();
     at::Tensor dnorm;
-    const at::Tensor ds = norm_with_skip_backward({dy, at::mm(dgate_up, w13)}, {saved[0], saved[1], saved[2]}, &dnorm)[0];
-    const at::Tensor dwo = product_unless(!ctx->needs_input_grad(2), ds.t(), o);
-    return {ds, product_unless(!ctx->needs_input_grad(1), ds, wo), dwo, dnorm, dw13, dw2, at::Tensor()};
+    const at::Tensor ds = norm_with_skip_backward({dy, input_gradient(dgate_up, w13)}, {saved[0], saved[1], saved[2]}, &dnorm)[0];
+    const at::Tensor dwo = ctx->needs_input_grad(2) ? weight_gradient(ds, o) : at::Tensor();
+    return {ds, ctx->needs_input_grad(1) ? input_gradient(ds, wo) : at::Tensor(), dwo, dnorm, dw13, dw2, at::Tensor()};
   }
   static bool applies(const at::Tensor& x, const at::Tensor& o, const at::Tensor& wo, const at::Tensor& norm, const at::Tensor& w13,
                       const at::Tensor& w2) {
@@ -455,17 +495,21 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> head(const at::Tensor& x, const a
                                           target_logit, row_scratch, loss.data_ptr<float>(), words, n, static_cast<int>(vocab), mean, mean,
                                           r0 == 0, cur(x)));
     const at::Tensor grad = logits.as_strided({n, vocab}, {ld, 1});
-    // A depth that is no multiple of 8 costs the product its tiled loads: the last few columns are added to its fp32 result.
+    // A depth that is no multiple of 8 costs the tensor library's product its tiled loads: the last few columns are added to its
+    // fp32 result.
     const int64_t even = vocab / 8 * 8;
-    if (even == vocab || even == 0) {
+    if (own_by_rows(n, dim, vocab)) {
+      mn_product_into(dxs, grad, false, weight);
+    } else if (even == vocab || even == 0) {
       at::mm_out(dxs, grad, weight);
     } else {
       const at::Tensor part = at::mm(grad.narrow(1, 0, even), weight.narrow(0, 0, even), at::kFloat);
       B200C_CUDA_CHECK(launch_head_tail(part.data_ptr<float>(), z + even, ld, bf(weight) + even * dim, bf_mut(dxs), n, static_cast<int>(dim),
                                         static_cast<int>(vocab - even), cur(x)));
     }
-    if (r0 == 0) at::mm_out(dw, grad.t(), xs);  // the first chunk needs no zeroed gradient to add to
-    else dw.addmm_(grad.t(), xs);
+    if (r0 > 0) dw.addmm_(grad.t(), xs);
+    else if (own_by_columns(vocab, dim, n)) mn_product_into(dw, grad, true, xs);  // the first chunk needs no zeroed gradient to add to
+    else at::mm_out(dw, grad.t(), xs);
   }
   return {loss, dx, dw};
 }
@@ -670,6 +714,20 @@ void bind_ops(py::module_& m) {
                                          reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
     return std::make_pair(c, status);
   });
+
+  // a[m, k] b[k, n], or with `by_columns` a[k, m]^T b[k, n], bf16; rows of a may be apart.
+  ops.def("gemm_bf16_mn", [](const at::Tensor& a, const at::Tensor& b, bool by_columns) {
+    want(b, at::kBFloat16, "b");
+    TORCH_CHECK(a.is_cuda() && a.scalar_type() == at::kBFloat16 && a.dim() == 2 && a.stride(1) == 1, "a: bf16 CUDA rows expected");
+    TORCH_CHECK(b.dim() == 2 && a.size(by_columns ? 0 : 1) == b.size(0), "a: [m, k] or, by columns, [k, m]; b: [k, n]");
+    c10::cuda::CUDAGuard g(a.device());
+    const int64_t m = a.size(by_columns ? 1 : 0);
+    at::Tensor c = at::empty({m, b.size(1)}, b.options()), status = status_words(b);
+    B200C_CUDA_CHECK(launch_gemm_pair_mn(a.data_ptr(), a.stride(0), by_columns, b.data_ptr(), b.size(1), c.data_ptr(), static_cast<int>(m),
+                                         static_cast<int>(b.size(1)), static_cast<int>(b.size(0)),
+                                         reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
+    return std::make_pair(c, status);
+  }, py::arg("a"), py::arg("b"), py::arg("by_columns") = false);
 
   // (x w^T, silu(gate) * up of it), bf16, gate columns first.
   ops.def("gemm_gated", [](const at::Tensor& x, const at::Tensor& w) {
