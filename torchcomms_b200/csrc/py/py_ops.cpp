@@ -507,9 +507,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> head(const at::Tensor& x, const a
       B200C_CUDA_CHECK(launch_head_tail(part.data_ptr<float>(), z + even, ld, bf(weight) + even * dim, bf_mut(dxs), n, static_cast<int>(dim),
                                         static_cast<int>(vocab - even), cur(x)));
     }
-    if (r0 > 0) dw.addmm_(grad.t(), xs);
-    else if (own_by_columns(vocab, dim, n)) mn_product_into(dw, grad, true, xs);  // the first chunk needs no zeroed gradient to add to
-    else at::mm_out(dw, grad.t(), xs);
+    if (r0 == 0) at::mm_out(dw, grad.t(), xs);  // the first chunk needs no zeroed gradient to add to
+    else dw.addmm_(grad.t(), xs);
   }
   return {loss, dx, dw};
 }
