@@ -45,6 +45,31 @@ def test_block_out(rows, dim, ffn, width):
         assert _off(a, b) < 12 * 2**-9
 
 
+# The gradient of gate and up in its product's epilogue: narrow and wide tiles, their last columns and rows, a last wave in
+# halves, K steps that end early; gates beyond where exponentials end, and those that are no numbers.
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (257, 136, 72), (1000, 520, 1000), (2049, 2312, 136), (300, 4808, 200)])
+def test_gated_gradient(m, n, k):
+    from torchcomms_b200 import _comms
+
+    dy, w, gate_up = _rand(m, k, seed=1), _rand(k, n, seed=2, scale=k**-0.5), _rand(m, 2 * n, seed=3, scale=2.0)
+    gate_up[:, 3], gate_up[:, 4], gate_up[0, 5], gate_up[0, 6] = 300.0, -300.0, float("nan"), float("-inf")
+    out, status = _comms.ops.gemm_gated_grad(dy, w, gate_up)
+    assert int(status[0]) == 0 and torch.equal(out.isnan(), _comms.ops.swiglu_bwd(_comms.ops.gemm_bf16_mn(dy, w)[0], gate_up).isnan())
+    gate_up[0, 5] = gate_up[0, 6] = 1.0
+    out, _ = _comms.ops.gemm_gated_grad(dy, w, gate_up)
+    d = dy.double() @ w.double()
+    g, u = gate_up.double().chunk(2, dim=1)
+    sig = torch.sigmoid(g)
+    ref = torch.cat([d * u * (sig + g * sig * (1 - sig)), d * g * sig], dim=1)
+    # Half a bf16 ulp (2^-9 relative); before it k fp32 additions of terms of size k^-1/2 and a few operations, of which the
+    # sum of sigmoid and silu x (1 - sigmoid) may cancel, scaled by gates and ups of up to 10, a column's by 300.
+    big = torch.tensor([300.0 if c in (3, n + 3, n + 4) else 10.0 for c in range(2 * n)], device="cuda", dtype=torch.float64)
+    assert bool(((out.double() - ref).abs() <= 2**-8 * ref.abs() + big * (k**0.5 * 2**-23 + 4e-6)).all())
+    for wrong in ((dy[:, :-1].contiguous(), w), (dy, w[:, :-1].contiguous())):
+        with pytest.raises(Exception):
+            _comms.ops.gemm_gated_grad(*wrong, gate_up)
+
+
 @pytest.mark.parametrize("rows,dim,heads,kv_heads,hd", [(1, 64, 1, 1, 8), (129, 200, 4, 2, 32), (1000, 512, 8, 2, 64)])
 def test_block_in(rows, dim, heads, kv_heads, hd):
     from torchcomms_b200 import _comms

@@ -54,6 +54,10 @@ cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, in
 // `lda`, `ldb`: row strides, multiples of 8. Any m and k, n % 8 == 0; all pointers 16-byte aligned. `status`: as above.
 cudaError_t launch_gemm_pair_mn(const void* a, int64_t lda, bool a_by_columns, const void* b, int64_t ldb, void* c, int m, int n, int k,
                                 uint32_t* status, cudaStream_t stream);
+// dgate_up[m, 2 n], the gradient of gate_up, from d = dy[m, k] x w[k, n], that of silu(gate) * up. n, k % 8 == 0; all pointers
+// 16-byte aligned.
+cudaError_t launch_gemm_gated_grad(const void* dy, const void* w, const void* gate_up, void* dgate_up, int m, int n, int k, uint32_t* status,
+                                   cudaStream_t stream);
 // Pairs that the GPU holds at once (0 after an error), and whether the narrow tiles of an m x n product are at most as many.
 int pairs_at_once(bool fp8);
 // Waves of tiles, of which `at_once` run at a time, in time: a last, partial wave costs half a wave and half of the share it

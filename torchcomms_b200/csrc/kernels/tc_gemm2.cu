@@ -53,7 +53,7 @@ constexpr int kOutChunkBytes = kBlockM * 64 * 2;  // of the widest chunk
 // m] and B [k, n]. The tensor pipe takes either; only the boxes that bring the operands differ.
 enum class PairLayout { kNT, kNN, kTN };
 // What the epilogue does besides storing the product.
-enum Epilogue { kPlain, kStats, kGated };
+enum Epilogue { kPlain, kStats, kGated, kGatedGrad };
 // Warps of the epilogue: four, one for each quarter of the tensor memory's lanes, or two such sets that take the tiles, and
 // with them the two accumulators, in turn.
 template <Epilogue EPI>
@@ -62,16 +62,16 @@ template <Epilogue EPI>
 constexpr int pair_threads() { return 64 + 128 * epilogue_sets<EPI>(); }
 constexpr int kAccCols = 256;  // tensor-memory columns of one accumulator
 
-// Stages of the TMA ring. With two sets of epilogue warps one of six makes room for two staging buffers each: with six stages
-// and one buffer 4096 x 128256 x 256 takes 361 us, so 315; x 4096 the same either way.
+// Stages of the TMA ring. With two sets of epilogue warps one of six makes room for two staging buffers each: with six stages and one
+// buffer 4096 x 128256 x 256 takes 361 us, so 315; x 4096 the same either way. So it does for two buffers of gate and two of up.
 template <Epilogue EPI>
-constexpr int pair_stages() { return EPI == kStats ? 5 : 6; }
+constexpr int pair_stages() { return EPI == kStats || EPI == kGatedGrad ? 5 : 6; }
 
 // Shared memory for tiles of BN columns: each CTA holds half of the B tile. (Eight stages, which tiles of 128 columns
 // leave room for, gain nothing: 512 x 4096 x 4096 in e4m3 15.1 us either way.)
 template <int BN, Epilogue EPI>
 struct PairTile {
-  static constexpr int kStages = pair_stages<EPI>(), kOutBuffers = 2 * epilogue_sets<EPI>();
+  static constexpr int kStages = pair_stages<EPI>(), kOutBuffers = EPI == kStats || EPI == kGatedGrad ? 4 : 2;
   // Columns that are staged and stored at a time: a quarter of the tile, of narrow tiles half. Only whole swizzle rows of 64
   // are swizzled; rows of 56 lie on different banks anyway, rows of 48 two by two on the same.
   static constexpr int kChunk = BN == 128 ? 64 : BN / 4;
@@ -86,6 +86,7 @@ struct PairBarriers {
   uint64_t empty[8];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
+  uint64_t gates[2];  // kGatedGrad: a chunk of gate and up has arrived
   uint32_t tmem_base;
   uint32_t failed;
 };
@@ -104,6 +105,12 @@ struct PairMaps<kGated> : PairMaps<kPlain> {
   CUtensorMap b_up, out_up, b_up_tail;
 };
 
+// Gate and up, n columns each, and their gradients: boxes as of `out`.
+template <>
+struct PairMaps<kGatedGrad> : PairMaps<kPlain> {
+  CUtensorMap out_up, gate, up;
+};
+
 struct PairParams {
   uint32_t* status;
   const float* scale_a;  // e4m3: per row of A, per row of B
@@ -117,6 +124,7 @@ struct PairParams {
   const int64_t* targets;
   float* target_logit;
   __nv_bfloat16* act;  // kGated: [m, n] silu(gate) * up
+  const __nv_bfloat16* gate_up;  // (host) kGatedGrad: [m, 2 n]
 };
 
 // Maximum and sum of exp(x - maximum) of what a row has shown so far, NaN where one was among it. Two elements per
@@ -219,6 +227,30 @@ __device__ __forceinline__ uint32_t gated_pair(uint32_t gate, uint32_t up) {
   return pack_bf16(__float_as_uint(o[0]), __float_as_uint(o[1]));
 }
 
+// The gradients of eight columns of gate and up from those of silu(gate) * up, as k_swiglu_bwd has them.
+__device__ __forceinline__ void gated_gradients(const uint32_t* d, uint4 gate, uint4 up, uint4* dgate, uint4* dup) {
+  const uint32_t g[4] = {gate.x, gate.y, gate.z, gate.w}, u[4] = {up.x, up.y, up.z, up.w};
+  uint32_t dg[4], du[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float og[2], ou[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float gf = __uint_as_float(j == 0 ? g[i] << 16 : g[i] & 0xffff0000u), uf = __uint_as_float(j == 0 ? u[i] << 16 : u[i] & 0xffff0000u);
+      const float df = __uint_as_float(d[2 * i + j]);
+      float sigmoid;
+      asm("rcp.approx.f32 %0, %1;" : "=f"(sigmoid) : "f"(1.0f + __expf(-gf)));
+      const float silu = gf * sigmoid;
+      og[j] = df * uf * (sigmoid + silu * (1.0f - sigmoid));
+      ou[j] = df * silu;
+    }
+    dg[i] = pack_bf16(__float_as_uint(og[0]), __float_as_uint(og[1]));
+    du[i] = pack_bf16(__float_as_uint(ou[0]), __float_as_uint(ou[1]));
+  }
+  *dgate = make_uint4(dg[0], dg[1], dg[2], dg[3]);
+  *dup = make_uint4(du[0], du[1], du[2], du[3]);
+}
+
 // The 128 threads of one set of epilogue warps.
 __device__ __forceinline__ void epilogue_sync(int set) {
   if (set == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -227,9 +259,9 @@ __device__ __forceinline__ void epilogue_sync(int set) {
 
 template <bool FP8, int BN, Epilogue EPI, PairLayout LAYOUT>
 __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __grid_constant__ PairMaps<EPI> maps, PairParams p) {
-  constexpr bool STATS = EPI == kStats, GATED = EPI == kGated;
+  constexpr bool STATS = EPI == kStats, GATED = EPI == kGated, GRAD = EPI == kGatedGrad;
   constexpr bool A_MN = LAYOUT == PairLayout::kTN, B_MN = LAYOUT != PairLayout::kNT;
-  static_assert(!B_MN || (!FP8 && EPI == kPlain && BN % 128 == 0), "whole blocks of 64 columns for each CTA");
+  static_assert(!B_MN || (!FP8 && !STATS && !GATED && BN % 128 == 0), "whole blocks of 64 columns for each CTA");
   constexpr int kTileCols = GATED ? BN / 2 : BN;  // of the output
   constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(2 * kBlockM, BN) : make_idesc_bf16(2 * kBlockM, BN, A_MN, B_MN);
   constexpr uint32_t idesc_tail = FP8 ? make_idesc_e4m3(2 * kBlockM, BN / 2) : make_idesc_bf16(2 * kBlockM, BN / 2, A_MN, B_MN);
@@ -258,6 +290,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars->acc_full[s], 1);
       mbar_init(&bars->acc_empty[s], 8);  // four epilogue warps in each CTA of the pair
+      mbar_init(&bars->gates[s], 1);
     }
     bars->failed = 0;
     fence_barrier_init();
@@ -391,6 +424,17 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     };
     const int first = cluster_id + set * nclusters, step = kSets * nclusters;
     if (first < items) fetch(first);
+    // Chunk `n` of gate and up, where its gradients will be: two buffers, the next chunk on its way while one is worked on.
+    const auto load_gates = [&](uint32_t n, int2 at) {
+      if constexpr (GRAD) {
+        char* const to = obuf + 2 * (n & 1u) * kOutChunkBytes;
+        tma_store_wait_read<0>();  // the chunk before the last is out of it
+        mbar_expect_tx(&bars->gates[n & 1u], 2 * kOutChunkBytes);
+        tma_load_2d(to, &maps.gate, &bars->gates[n & 1u], at.y, at.x);
+        tma_load_2d(to + kOutChunkBytes, &maps.up, &bars->gates[n & 1u], at.y, at.x);
+      }
+    };
+    if (GRAD && issuer && first < items) load_gates(0, place_of(first));
     uint32_t tile_iter = static_cast<uint32_t>(set), chunk_iter = 0;
     for (int i = first; i < items; i += step, tile_iter += kSets) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
@@ -406,6 +450,9 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
       if (i + step < items) fetch(i + step);
       if (!mbar_wait(&bars->acc_full[as], aph)) {
         bars->failed = 1;
+        if constexpr (GRAD) {
+          if (issuer) mbar_wait(&bars->gates[chunk_iter & 1u], (chunk_iter >> 1) & 1u);  // nothing is in flight at the end
+        }
         break;
       }
       tc_fence_after_sync();
@@ -456,6 +503,48 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           if (issuer && out_row < p.m && col < p.n) {
             tma_store_2d(&maps.out, obuf, col, out_row);
             tma_store_2d(&maps.out_up, obuf + kOutChunkBytes, col, out_row);
+            tma_store_commit();
+          }
+        }
+        continue;
+      }
+      if constexpr (GRAD) {
+        static_assert(!GRAD || (kSets == 1 && kChunk == 64), "");
+        const int chunks = BN / kChunk / (tail ? 2 : 1);
+        for (int j = 0; j < chunks; ++j, ++chunk_iter) {
+          const uint32_t b = chunk_iter & 1u;
+          if (issuer) {
+            if (j + 1 < chunks) {
+              load_gates(chunk_iter + 1, make_int2(out_row, out_col + (j + 1) * kChunk));
+            } else if (i + step < items) {
+              load_gates(chunk_iter + 1, place_of(i + step));
+            }
+          }
+          if (!mbar_wait(&bars->gates[b], (chunk_iter >> 1) & 1u)) bars->failed = 1;
+          __syncwarp();
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t d[32];
+            tmem_ld_32x32(tmem_base + as * kAccCols + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(j * kChunk + half * 32), d);
+            tmem_ld_wait();
+            if (j == chunks - 1 && half == 1) {
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_leader(&bars->acc_empty[as]);
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              uint4* const gate = reinterpret_cast<uint4*>(obuf + 2 * b * kOutChunkBytes + staged(row_in_tile, half * 4 + v));
+              uint4* const up = gate + kOutChunkBytes / 16;
+              gated_gradients(d + 8 * v, *gate, *up, gate, up);
+            }
+          }
+          fence_proxy_async_smem();
+          epilogue_sync(0);
+          const int col = out_col + j * kChunk;
+          if (issuer && out_row < p.m && col < p.n) {
+            tma_store_2d(&maps.out, obuf + 2 * b * kOutChunkBytes, col, out_row);
+            tma_store_2d(&maps.out_up, obuf + (2 * b + 1) * kOutChunkBytes, col, out_row);
             tma_store_commit();
           }
         }
@@ -599,6 +688,13 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
       return cudaErrorInvalidValue;
     }
   }
+  if constexpr (EPI == kGatedGrad) {
+    constexpr int kCols = PairTile<BN, EPI>::kChunk;
+    if (!make_map(&maps.out_up, static_cast<__nv_bfloat16*>(c) + p.n, p.m, p.n, kBlockM, ldc, kCols) ||
+        !make_map(&maps.gate, p.gate_up, p.m, p.n, kBlockM, ldc, kCols) || !make_map(&maps.up, p.gate_up + p.n, p.m, p.n, kBlockM, ldc, kCols)) {
+      return cudaErrorInvalidValue;
+    }
+  }
   const int a_bytes = A_MN ? kABytes : a_box_rows(p.m) * kBlockK * 2;
   p.stage_bytes = 2 * (a_bytes + PairTile<BN, EPI>::kBHalfBytes);
   p.tail_bytes = 2 * (a_bytes + PairTile<BN, EPI>::kBHalfBytes / 2);
@@ -721,6 +817,28 @@ cudaError_t launch_gemm_pair_mn(const void* a, int64_t lda, bool a_by_columns, c
   }
   return narrow ? launch_pair<false, 128, kPlain, PairLayout::kNN>(a, b, c, p, stream, 0, lda, ldb)
                 : launch_pair<false, 256, kPlain, PairLayout::kNN>(a, b, c, p, stream, 0, lda, ldb);
+}
+
+// What it saves is the product's way through memory and a kernel of memory's speed; gate and up come and their gradients go while
+// the next tile's product runs. Gate and up by boxes into the buffers that their gradients leave from: rows read by one thread each
+// instead were 200 us for 2048 x 14336 x 4096, so 198, and 89 for 2048 x 8192 x 2048, so 67 (two sets of epilogue warps 212 and 91).
+cudaError_t launch_gemm_gated_grad(const void* dy, const void* w, const void* gate_up, void* dgate_up, int m, int n, int k, uint32_t* status,
+                                   cudaStream_t stream) {
+  if (m <= 0 || n <= 0 || k <= 0 || n % 8 != 0 || k % 8 != 0 || n > INT32_MAX / 2) return cudaErrorInvalidValue;
+  if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(gate_up) |
+       reinterpret_cast<uintptr_t>(dgate_up)) & 15u) {
+    return cudaErrorMisalignedAddress;
+  }
+  PairParams p{};
+  p.status = status;
+  p.clear = status != nullptr ? 1 : 0;
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  p.gate_up = static_cast<const __nv_bfloat16*>(gate_up);
+  const int64_t ld = 2 * static_cast<int64_t>(n);
+  return pair_tiles_fit(m, n, false) ? launch_pair<false, 128, kGatedGrad, PairLayout::kNN>(dy, w, dgate_up, p, stream, ld)
+                                     : launch_pair<false, 256, kGatedGrad, PairLayout::kNN>(dy, w, dgate_up, p, stream, ld);
 }
 
 int head_row_shares(int m, int n) {

@@ -372,6 +372,21 @@ at::Tensor input_gradient(const at::Tensor& dy, const at::Tensor& w) {
   mn_product_into(dx, dy, false, w);
   return dx;
 }
+// The gradient of [gate, up] from that of silu(gate) * up w^T. Where this library makes the product, its epilogue does the rest,
+// but for few rows of large weights, whose only tiles end in that epilogue. In us, dy [rows, k] w [k, n], the tensor library's product
+// and the kernel / this library's and the kernel / one kernel: 4096 x 4096 x 14336 504 / 512 / 385, 1000 124 / 129 / 112; 2048 x 2048 x
+// 8192 96 / 90 / 67, 64 13.7 / 14.3 / 15.9; 1000 x 512 x 2048 13.6 / 10.6 / 9.3.
+at::Tensor gated_gradient(const at::Tensor& dy, const at::Tensor& w, const at::Tensor& gate_up) {
+  const int64_t m = dy.size(0), n = w.size(1), k = w.size(0);
+  if (!plain_rows(dy, dy) || !plain_rows(w, dy) || !plain_rows(gate_up, dy) || dy.size(1) != k || gate_up.size(0) != m ||
+      gate_up.size(1) != 2 * n || !own_by_rows(m, n, k) || (m <= 128 && n * k > 12 << 20)) {
+    return swiglu_bwd(input_gradient(dy, w), gate_up);
+  }
+  at::Tensor d = at::empty_like(gate_up), status = status_words(dy);
+  B200C_CUDA_CHECK(launch_gemm_gated_grad(dy.data_ptr(), w.data_ptr(), gate_up.data_ptr(), d.data_ptr(), static_cast<int>(m), static_cast<int>(n),
+                                          static_cast<int>(k), reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(dy)));
+  return d;
+}
 at::Tensor weight_gradient(const at::Tensor& dy, const at::Tensor& x) {
   if (!plain_rows(dy, dy) || !plain_rows(x, dy) || dy.size(0) != x.size(0) || !own_by_columns(dy.size(1), x.size(1), x.size(0))) {
     return at::mm(dy.t(), x);
@@ -435,7 +450,7 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
     const at::Tensor dy = grads[0].contiguous();
     c10::cuda::CUDAGuard g(dy.device());
     const at::Tensor dw2 = ctx->needs_input_grad(5) ? weight_gradient(dy, act) : at::Tensor();
-    const at::Tensor dgate_up = swiglu_bwd(input_gradient(dy, w2), gate_up);
+    const at::Tensor dgate_up = gated_gradient(dy, w2, gate_up);
     const at::Tensor dw13 = ctx->needs_input_grad(4) ? weight_gradient(dgate_up, h) : at::Tensor();
     at::Tensor dnorm;
     const at::Tensor ds = norm_with_skip_backward({dy, input_gradient(dgate_up, w13)}, {saved[0], saved[1], saved[2]}, &dnorm)[0];
@@ -727,6 +742,21 @@ void bind_ops(py::module_& m) {
                                          reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
     return std::make_pair(c, status);
   }, py::arg("a"), py::arg("b"), py::arg("by_columns") = false);
+
+  // The gradient of gate_up[m, 2 n] from dy[m, k] w[k, n], the gradient of silu(gate) * up.
+  ops.def("gemm_gated_grad", [](const at::Tensor& dy, const at::Tensor& w, const at::Tensor& gate_up) {
+    want(dy, at::kBFloat16, "dy");
+    want(w, at::kBFloat16, "w");
+    want(gate_up, at::kBFloat16, "gate_up");
+    TORCH_CHECK(dy.dim() == 2 && w.dim() == 2 && gate_up.dim() == 2 && dy.size(1) == w.size(0) && gate_up.size(0) == dy.size(0) &&
+                    gate_up.size(1) == 2 * w.size(1), "dy: [m, k], w: [k, n], gate_up: [m, 2 n]");
+    c10::cuda::CUDAGuard g(dy.device());
+    at::Tensor d = at::empty_like(gate_up), status = status_words(dy);
+    B200C_CUDA_CHECK(launch_gemm_gated_grad(dy.data_ptr(), w.data_ptr(), gate_up.data_ptr(), d.data_ptr(), static_cast<int>(dy.size(0)),
+                                            static_cast<int>(w.size(1)), static_cast<int>(w.size(0)),
+                                            reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(dy)));
+    return std::make_pair(d, status);
+  });
 
   // (x w^T, silu(gate) * up of it), bf16, gate columns first.
   ops.def("gemm_gated", [](const at::Tensor& x, const at::Tensor& w) {
