@@ -43,6 +43,25 @@ def test_head_against_64_bits(rows, dim, vocab):
     assert all(torch.equal(a, b) for a, b in zip(again, _comms.ops.head(x, w, t, 4096)))  # the same bits every time
 
 
+# Large weights and few rows, or a last unit of 256 rows that is mostly empty: the logits of the tensor library's product; a chunk
+# of each kind.
+@pytest.mark.parametrize("rows,chunk,vocab", [(20, 4096, 65544), (556, 300, 65549)])
+def test_head_of_few_rows_and_large_weights(rows, chunk, vocab):
+    from torchcomms_b200 import _comms
+
+    x, w, t = _head(rows, 2112, vocab, 8)
+    w = w * 0.1
+    t[-1], t[0], t[rows // 3] = vocab - 1, 0, -1
+    ref = _reference(x, w, t)
+    out = _comms.ops.head(x, w, t, chunk)
+    # bf16 logits, of 0.03 sqrt(dim) x 5 at most, are 2^-9 of that off; gradients as above.
+    assert abs(float(out[0].double() - ref[0])) < 2**-9 * 0.15 * 2112**0.5
+    for a, b in zip(out[1:], ref[1:]):
+        assert float((a.double() - b).norm()) <= (2**-8 + 2**-9 * 0.15 * 2112**0.5) * float(b.norm())
+    loss = _comms.ops.head(x, w, torch.full_like(t, -1), chunk)[0]
+    assert loss.shape == () and float(loss) == 0
+
+
 def test_head_all_rows_ignored_and_infinities():
     from torchcomms_b200 import _comms
 

@@ -482,6 +482,18 @@ bool head_applies(const at::Tensor& x, const at::Tensor& weight, const at::Tenso
       targets.dim() == 1 && targets.size(0) == x.size(0) && targets.is_contiguous() && targets.device() == x.device();
 }
 
+// Whether the logits are this library's product, with their statistics: but for large weights where half of a pair's rows would be
+// empty, or with more than a unit of 256 rows and 15 % of all, of widths beyond 2048 5 %. The tensor library's product and the
+// kernel with two looks take as long then or less. A pass of the head in us, that way / this library's, rows x width x vocabulary:
+// 64 x 4096 x 128256 608 / 645, 128 x 2048 x 128256 390 / 397, 128 x 4096 x 32000 215 / 212, 32 x 2048 x 50256 185 / 152; 400 x 4096 x
+// 128256 1346 / 1400, 700 1954 / 1994, 200 909 / 910, 512 1520 / 1513, 400 x 4096 x 32000 365 / 376, 1300 889 / 899; 700 x 2048 x
+// 128256 1130 / 1123, 400 x 2048 x 50256 304 / 306, 1300 792 / 763.
+bool own_logits(int64_t rows, int64_t vocab, int64_t dim) {
+  const int64_t weight = vocab * dim;
+  if (rows <= 256) return rows > 128 || weight <= 128 << 20;
+  return rows * 20 >= (rows + 255) / 256 * 256 * (dim > 2048 ? 19 : 17) || (weight <= 128 << 20 && (dim <= 2048 || weight <= 64 << 20));
+}
+
 std::tuple<at::Tensor, at::Tensor, at::Tensor> head(const at::Tensor& x, const at::Tensor& weight, const at::Tensor& targets,
                                                     int64_t chunk_rows) {
   c10::cuda::CUDAGuard g(x.device());
@@ -504,12 +516,20 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> head(const at::Tensor& x, const a
     const at::Tensor xs = r0 == 0 && n == rows ? x : x.narrow(0, r0, n);
     at::Tensor dxs = r0 == 0 && n == rows ? dx : dx.narrow(0, r0, n);
     auto* z = reinterpret_cast<__nv_bfloat16*>(logits.data_ptr());
-    B200C_CUDA_CHECK(launch_head_logits(xs.data_ptr(), weight.data_ptr(), z, ld, t, n, static_cast<int>(vocab), static_cast<int>(dim),
-                                        reinterpret_cast<float2*>(stats), target_logit, words, cur(x)));
-    B200C_CUDA_CHECK(launch_head_gradient(z, ld, t, reinterpret_cast<float2*>(stats), head_row_shares(n, static_cast<int>(vocab)),
-                                          target_logit, row_scratch, loss.data_ptr<float>(), words, n, static_cast<int>(vocab), mean, mean,
-                                          r0 == 0, cur(x)));
-    const at::Tensor grad = logits.as_strided({n, vocab}, {ld, 1});
+    at::Tensor grad = logits.as_strided({n, vocab}, {ld, 1});
+    if (own_logits(n, vocab, dim)) {
+      B200C_CUDA_CHECK(launch_head_logits(xs.data_ptr(), weight.data_ptr(), z, ld, t, n, static_cast<int>(vocab), static_cast<int>(dim),
+                                          reinterpret_cast<float2*>(stats), target_logit, words, cur(x)));
+      B200C_CUDA_CHECK(launch_head_gradient(z, ld, t, reinterpret_cast<float2*>(stats), head_row_shares(n, static_cast<int>(vocab)),
+                                            target_logit, row_scratch, loss.data_ptr<float>(), words, n, static_cast<int>(vocab), mean, mean,
+                                            r0 == 0, cur(x)));
+    } else {
+      at::mm_out(grad, xs, weight.t());
+      B200C_CUDA_CHECK(launch_cross_entropy_fwd_bwd(z, ld, t, row_scratch, n, static_cast<int>(vocab), mean, cur(x)));
+      const at::Tensor sum = scratch.narrow(0, row_scratch - stats, n).sum().mul_(mean);
+      if (r0 == 0) loss = sum;
+      else loss.add_(sum);
+    }
     // A depth that is no multiple of 8 costs the tensor library's product its tiled loads: the last few columns are added to its
     // fp32 result.
     const int64_t even = vocab / 8 * 8;
