@@ -30,11 +30,16 @@ def test_head_against_64_bits(rows, dim, vocab):
     t[-1], t[0] = vocab - 1, 0
     t[rows // 3] = -1
     ref = _reference(x, w, t)
+    logits = (x.double() @ w.double().t()).bfloat16().double()
+    rounded = F.cross_entropy(logits, t, reduction="none", ignore_index=-1).sum() / rows
     for chunk in (4096, 100):
         out = _comms.ops.head(x, w, t, chunk)
-        # Sums of `dim` products in fp32: dim x 2^-24 of the products' magnitudes, which are below 0.3 sqrt(dim) x 5 here;
-        # then fp32 exponentials and sums, 1e-5 as for the loss kernel that makes its own statistics.
-        assert abs(float(out[0].double() - ref[0])) < 1e-5 + dim**1.5 * 1.5 * 2**-24
+        # The loss is that of the bf16 logits, which are up to 0.3 sqrt(dim) x 5 here: fp32 exponentials and sums, 1e-5 as for the loss
+        # kernel that makes its own statistics; and where a sum of `dim` products in fp32 falls to the other side of a tie (2 in
+        # 10000 do), a target's logit is 2^-8 of itself off: two rows of these at most.
+        top = 1.5 * dim**0.5
+        assert abs(float(out[0].double() - rounded)) < 1e-5 + dim * top * 2**-24 + 2 / rows * top * 2**-8
+        assert abs(float(out[0].double() - ref[0])) < 1e-5 + 2 * top * 2**-9
         # bf16 logits off by 2^-9 of up to 0.3 sqrt(dim) x 5 move a probability by as much; their gradients and the results
         # are rounded to 2^-9. One number in a row of one has nothing to average over, hence the maximum, not a norm.
         for a, b in zip(out[1:], ref[1:]):
@@ -76,6 +81,59 @@ def test_head_all_rows_ignored_and_infinities():
     assert torch.isnan(loss) and bool(bad[7]) and int(bad.sum()) == 1  # its own row, as with separate operators
 
 
+def _by_operators(x, w, t):
+    """Gradients by one product of logits, the loss kernel on them, and two products."""
+    from torchcomms_b200 import _comms
+
+    logits = x @ w.t()
+    _comms.ops.cross_entropy_fwd_bwd_(logits, t, 1.0 / x.shape[0])
+    return logits @ w, logits.t() @ x
+
+
+# Targets that the model has learnt to a degree, up to rows whose gradient all but vanishes, and targets at random among logits of
+# 12 to several hundred; by the logits kernel and by the tensor library's product.
+@pytest.mark.parametrize("rows,dim,vocab,learnt,scale", [
+    (200, 256, 8000, True, 0.05), (200, 256, 8000, True, 0.08), (128, 256, 8000, True, 0.06), (33, 512, 16385, True, 0.03),
+    (200, 64, 2051, False, 1.0), (200, 64, 2051, False, 30.0), (200, 64, 2051, False, 100.0),
+    (20, 2112, 65544, True, 0.008), (300, 2112, 65544, True, 0.01), (20, 2112, 65544, False, 10.0)])
+def test_head_normalises_what_it_differentiates(rows, dim, vocab, learnt, scale):
+    from torchcomms_b200 import _comms
+
+    g = torch.Generator(device="cuda").manual_seed(9)
+    w = torch.randn(vocab, dim, generator=g, device="cuda").bfloat16()
+    t = torch.randint(vocab, (rows,), generator=g, device="cuda")
+    if learnt:
+        x = (w[t].float() * scale).bfloat16()
+    else:
+        x, w = (torch.randn(rows, dim, generator=g, device="cuda") * scale).bfloat16(), (w.float() * 0.3).bfloat16()
+    ref = _reference(x, w, t)
+    out = _comms.ops.head(x, w, t, 4096)
+    # Both round the logits to bf16 and normalise what came out, so that a probability near one stays one and its gradient
+    # small: the same error, but for sums in another order that fall to the other side of a tie.
+    for a, b, r in zip(out[1:], _by_operators(x, w, t), ref[1:]):
+        mine, theirs = float((a.double() - r).norm()), float((b.double() - r).norm())
+        assert mine <= 2 * theirs + 1e-6 * float(r.norm())
+
+
+@pytest.mark.parametrize("vocab", [2051, 8000, 1048600])
+@pytest.mark.parametrize("scale", [0.02, 0.06, 1.0])
+def test_probabilities_of_a_row_sum_to_one(vocab, scale):
+    """Rows that are unit vectors in columns where the weight is zero have the gradient of their logits in those columns of dw."""
+    from torchcomms_b200 import _comms
+
+    rows, dim = 128, 512
+    g = torch.Generator(device="cuda").manual_seed(10)
+    w = torch.randn(vocab, dim, generator=g, device="cuda").bfloat16()
+    w[:, :rows] = 0
+    t = torch.randint(vocab, (rows,), generator=g, device="cuda")
+    x = (w[t].float() * scale).bfloat16()
+    x[:, :rows] = torch.eye(rows, device="cuda")
+    dlogits = _comms.ops.head(x, w, t, 4096)[2][:, :rows].t().double() * rows
+    # A gradient is rounded to bf16, half an ulp of 2^-8 at most; before that fp32 exponentials and sums.
+    assert bool((dlogits.sum(dim=1).abs() <= 1e-3 + 2**-9 * dlogits.abs().sum(dim=1)).all())
+    assert float(dlogits.abs().max()) <= 1 + 1e-3
+
+
 def test_head_of_large_logits():
     """Logits whose exponentials overflow by themselves, and rows with one logit far above the rest."""
     from torchcomms_b200 import _comms
@@ -84,8 +142,10 @@ def test_head_of_large_logits():
     x *= 100
     ref = _reference(x, w, t)
     loss, _, _ = _comms.ops.head(x, w, t, 4096)
-    # fp32 logits of up to 1500: 2^-24 of that, 64 times over in the worst order
-    assert abs(float(loss.double() - ref[0])) < 1500 * 64 * 2**-24
+    # bf16 logits of up to 1500: half an ulp is 4, of a target's and of the highest
+    assert abs(float(loss.double() - ref[0])) < 2 * 4
+    rounded = F.cross_entropy((x.double() @ w.double().t()).bfloat16().double(), t)
+    assert abs(float(loss.double() - rounded)) < 1500 * 64 * 2**-24 + 2 / 200 * 8  # fp32 sums, and two ties that fall the other way
 
 
 def test_what_the_head_leaves_to_operators():

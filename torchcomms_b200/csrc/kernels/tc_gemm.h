@@ -73,7 +73,7 @@ cudaError_t launch_gemm_gated(const void* x, const void* w, void* gate_up, void*
                               cudaStream_t stream, int columns = 0);
 
 // Logits of a head on CTA pairs: logits[m, n] (bf16, row stride `ld`, a multiple of 8) = x[m, k] x w[n, k]^T, any n, k % 8 ==
-// 0. Also, from the fp32 accumulators, for each of head_row_shares(m, n) shares of a row the maximum and the sum of
+// 0. Also, of the rounded logits, for each of head_row_shares(m, n) shares of a row the maximum and the sum of
 // exp(logit - maximum) (`stats`, [shares, m]), and the logit of the row's target (`target_logit`, where targets[row] is in
 // [0, n)). `words`: status as above, then a counter that launch_head_gradient counts rows in; all cleared by the kernel.
 int head_row_shares(int m, int n);

@@ -25,7 +25,10 @@
 // each row's maximum and sum of exponentials over the tile and the logit of its target: the loss then needs one look
 // at the logits instead of two. One set of epilogue warps takes 405 us for 4096 x 128256 x 256 with one barrier more a chunk,
 // two sets that share a tile's columns 348, two that take the tiles in turn 315 (the plain product 257); 4096 x 128256 x 4096
-// 2700 to 2790, by the clock that the exponentials' power leaves (plain 2650).
+// 2700 to 2790, by the clock that the exponentials' power leaves (plain 2650). These are of sums over the accumulators; the
+// sums are of the rounded logits, which costs a pass of the head 2.5 % at a width of 256 (1192 and 1222 us) and 0.9 % at 4096 (9450 and
+// 9540). Accumulators' sums under rounded logits leave rows of probabilities that do not sum to one: where a target has a
+// probability of 0.95 the gradient was 0.26 of itself off (200 x 256 x 8000; so 0.0155), at 0.9999 140 times itself (0.028).
 //
 // With kGated the product is the first half of a gated MLP: the second CTA's half of a B tile are the rows of `up` that go with
 // the first one's of `gate`, and the epilogue, which then has both of a column, also writes silu(gate) * up. 4096 x 14336 x 4096
@@ -127,18 +130,21 @@ struct PairParams {
   const __nv_bfloat16* gate_up;  // (host) kGatedGrad: [m, 2 n]
 };
 
-// Maximum and sum of exp(x - maximum) of what a row has shown so far, NaN where one was among it. Two elements per
-// addition and product, two per maximum: the exponentials then take more of the time than what is around them.
+// Maximum and sum of exp(x - maximum) of what a row has shown so far, NaN where one was among it. Of the logits as they are stored,
+// rounded to bf16: the gradient is made from those, and its probabilities sum to one only if the sum is of the same numbers. Two
+// elements per addition and product, two per maximum: the exponentials then take more of the time than what is around them.
 struct RowStats {
   float mx = -INFINITY, sum = 0.0f;
-  __device__ __forceinline__ void feed(const uint32_t (&r)[32]) {
+  __device__ __forceinline__ void feed(const uint32_t (&packed)[16]) {
+    const auto lo = [&](int i) { return __uint_as_float(packed[i] << 16); };
+    const auto hi = [&](int i) { return __uint_as_float(packed[i] & 0xffff0000u); };
     float m[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = fmaxf(__uint_as_float(r[i]), __uint_as_float(r[i + 4]));
+    for (int i = 0; i < 4; ++i) m[i] = fmaxf(lo(i), hi(i));
 #pragma unroll
-    for (int i = 8; i < 32; i += 8) {
+    for (int i = 4; i < 16; i += 4) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) m[j] = max3(m[j], __uint_as_float(r[i + j]), __uint_as_float(r[i + j + 4]));
+      for (int j = 0; j < 4; ++j) m[j] = max3(m[j], lo(i + j), hi(i + j));
     }
     const float top = fmaxf(max3(m[0], m[1], m[2]), m[3]);
     if (top > mx) {
@@ -149,10 +155,9 @@ struct RowStats {
     const float shift = mx == -INFINITY ? 0.0f : -mx;
     float2 s[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
 #pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-      const float2 x = mul2(add2(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), make_float2(shift, shift)),
-                            make_float2(kLog2e, kLog2e));
-      s[i / 2 % 2] = add2(s[i / 2 % 2], make_float2(exp2_fast(x.x), exp2_fast(x.y)));
+    for (int i = 0; i < 16; ++i) {
+      const float2 x = mul2(add2(make_float2(lo(i), hi(i)), make_float2(shift, shift)), make_float2(kLog2e, kLog2e));
+      s[i % 2] = add2(s[i % 2], make_float2(exp2_fast(x.x), exp2_fast(x.y)));
     }
     sum += (s[0].x + s[0].y) + (s[1].x + s[1].y);
   }
@@ -571,25 +576,29 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           uint32_t(&r)[32] = acc[half];
           if (FP8) scale_acc32(r, row_scale, col_scales + j * kChunk + half * 32);
           if constexpr (STATS) {
-            const int col = j * kChunk + half * 32;
-            const int past = p.n - out_col - col;  // columns beyond the last are zeros of the tile, not logits
+            const int past = p.n - out_col - j * kChunk - half * 32;  // columns beyond the last are zeros of the tile, not logits
             if (past < 32) {
 #pragma unroll
               for (int i = 0; i < 32; ++i) r[i] = i < past ? r[i] : 0xff800000u;
             }
-            if (row_there) row_stats.feed(r);
-            if (row_there && target >= col && target < col + 32) {
-              float z = 0.0f;
+          }
+          uint32_t packed[16];
 #pragma unroll
-              for (int i = 0; i < 32; ++i) z = target == col + i ? __uint_as_float(r[i]) : z;
-              p.target_logit[out_row + row_in_tile] = z;
+          for (int i = 0; i < 16; ++i) packed[i] = pack_bf16(r[2 * i], r[2 * i + 1]);
+          if constexpr (STATS) {
+            const int col = j * kChunk + half * 32;
+            if (row_there) row_stats.feed(packed);
+            if (row_there && target >= col && target < col + 32) {
+              uint32_t z = 0;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) z = target == col + i ? r[i] : z;
+              p.target_logit[out_row + row_in_tile] = __uint_as_float(pack_bf16(z, 0u) << 16);
             }
           }
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             if (half * 4 + v >= kChunk / 8) continue;
-            *reinterpret_cast<uint4*>(buf + staged(row_in_tile, half * 4 + v)) = make_uint4(pack_bf16(r[8 * v], r[8 * v + 1]), pack_bf16(r[8 * v + 2], r[8 * v + 3]),
-                              pack_bf16(r[8 * v + 4], r[8 * v + 5]), pack_bf16(r[8 * v + 6], r[8 * v + 7]));
+            *reinterpret_cast<uint4*>(buf + staged(row_in_tile, half * 4 + v)) = make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
           }
         }
         fence_proxy_async_smem();
