@@ -94,6 +94,38 @@ def test_block_in(rows, dim, heads, kv_heads, hd):
         assert torch.equal(a, b)
 
 
+def test_single_rows_of_any_stride():
+    """A row by itself is contiguous whatever its stride says: a column transposed, for one."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops import fused
+
+    def column(t):
+        return t.detach().as_strided(t.shape, (1, 1))
+
+    ins = [_rand(1, 64, seed=1), _rand(1, 128, seed=2), _rand(64, 128, seed=3, scale=0.1), _rand(64, seed=4, scale=0.1) + 1,
+           _rand(400, 64, seed=5, scale=0.1), _rand(64, 200, seed=6, scale=0.1)]
+    dy = _rand(1, 64, seed=7)
+    assert column(dy).is_contiguous()
+    plain = [t.clone().requires_grad_(True) for t in ins]
+    odd = [(column(t) if i < 2 else t).requires_grad_(True) for i, t in enumerate(ins)]
+    a, b = _comms.ops.block_out(*plain, 1e-5), _comms.ops.block_out(*odd, 1e-5)
+    assert torch.equal(a, b)
+    for p, q in zip(torch.autograd.grad(a, plain, dy), torch.autograd.grad(b, odd, column(dy))):
+        assert torch.equal(p, q)
+
+    cos_t, sin_t = fused.rope_tables(4, 16, 10000.0, "cuda")
+    pos = torch.ones(1, dtype=torch.int32, device="cuda")
+    wqkv = _rand(8 * 16, 64, seed=8, scale=0.1).requires_grad_(True)
+    norm = ins[3].clone().requires_grad_(True)
+    results = []
+    for x in (ins[0].clone(), column(ins[0])):
+        x.requires_grad_(True)
+        out = _comms.ops.block_in(x, norm, wqkv, pos, cos_t, sin_t, 4, 2, 1e-5)
+        douts = [dy if x.stride(0) == 64 else column(dy), *(_rand(*t.shape, seed=10 + i) for i, t in enumerate(out[1:]))]
+        results.append((*out, *torch.autograd.grad(out, (x, norm, wqkv), douts)))
+    assert all(torch.equal(p, q) for p, q in zip(*results))
+
+
 def test_only_what_is_asked_for():
     """Frozen weights and partial gradients: the others come out the same."""
     from torchcomms_b200 import _comms

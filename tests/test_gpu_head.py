@@ -67,6 +67,18 @@ def test_head_of_few_rows_and_large_weights(rows, chunk, vocab):
     assert loss.shape == () and float(loss) == 0
 
 
+@pytest.mark.parametrize("rows,vocab", [(40, 1), (1, 9)])
+def test_head_of_single_rows_of_any_stride(rows, vocab):
+    """A row by itself is contiguous whatever its stride says."""
+    from torchcomms_b200 import _comms
+
+    x, w, t = _head(rows, 64, vocab, 11)
+    odd = [v.as_strided(v.shape, (1, 1)) if v.shape[0] == 1 else v for v in (x, w)]
+    assert all(v.is_contiguous() for v in odd)
+    for a, b in zip(_comms.ops.head(x, w, t, 4096), _comms.ops.head(*odd, t, 4096)):
+        assert torch.equal(a, b)
+
+
 def test_head_all_rows_ignored_and_infinities():
     from torchcomms_b200 import _comms
 

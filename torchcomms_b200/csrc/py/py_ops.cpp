@@ -353,9 +353,11 @@ bool own_by_rows(int64_t m, int64_t n, int64_t k) {
   if (mostly_empty_rows(m) && n * k > 12 << 20) return false;
   return k <= 32 * kKStep || (m >= 700 && k <= (few_tiles(m, n) ? 48 : 96) * kKStep);
 }
+// Elements from row to row. A single row is contiguous whatever its stride says, and then that means nothing.
+int64_t row_stride(const at::Tensor& t) { return t.size(0) > 1 ? t.stride(0) : (t.size(1) + 7) / 8 * 8; }
 void mn_product_into(at::Tensor& c, const at::Tensor& a, bool by_columns, const at::Tensor& b) {
   at::Tensor status = status_words(b);
-  B200C_CUDA_CHECK(launch_gemm_pair_mn(a.data_ptr(), a.stride(0), by_columns, b.data_ptr(), b.stride(0), c.data_ptr(),
+  B200C_CUDA_CHECK(launch_gemm_pair_mn(a.data_ptr(), row_stride(a), by_columns, b.data_ptr(), row_stride(b), c.data_ptr(),
                                        static_cast<int>(c.size(0)), static_cast<int>(c.size(1)), static_cast<int>(b.size(0)),
                                        reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(b)));
 }
@@ -757,7 +759,7 @@ void bind_ops(py::module_& m) {
     c10::cuda::CUDAGuard g(a.device());
     const int64_t m = a.size(by_columns ? 1 : 0);
     at::Tensor c = at::empty({m, b.size(1)}, b.options()), status = status_words(b);
-    B200C_CUDA_CHECK(launch_gemm_pair_mn(a.data_ptr(), a.stride(0), by_columns, b.data_ptr(), b.size(1), c.data_ptr(), static_cast<int>(m),
+    B200C_CUDA_CHECK(launch_gemm_pair_mn(a.data_ptr(), row_stride(a), by_columns, b.data_ptr(), b.size(1), c.data_ptr(), static_cast<int>(m),
                                          static_cast<int>(b.size(1)), static_cast<int>(b.size(0)),
                                          reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(a)));
     return std::make_pair(c, status);
