@@ -70,6 +70,39 @@ def test_gated_gradient(m, n, k):
             _comms.ops.gemm_gated_grad(*wrong, gate_up)
 
 
+@pytest.mark.parametrize("m,n", [(257, 136), (1000, 9480)])
+def test_gated_gradient_of_exact_products(m, n):
+    """Where the product is a bf16 number, the activation's own backward kernel makes the same bits of it."""
+    from torchcomms_b200 import _comms
+
+    w, gate_up = _rand(64, n, seed=2), _rand(m, 2 * n, seed=3, scale=3.0)
+    dy = torch.zeros(m, 64, device="cuda", dtype=torch.bfloat16)
+    dy[torch.arange(m), torch.arange(m) % 64] = 1.0
+    out, _ = _comms.ops.gemm_gated_grad(dy, w, gate_up)
+    assert torch.equal(out, _comms.ops.swiglu_bwd(w[torch.arange(m) % 64], gate_up))
+
+
+def test_activation_of_every_gate():
+    """All bf16 gates: the activation and its gradients as the definition with a correctly rounded division has them."""
+    from torchcomms_b200 import _comms
+
+    gate = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    up = _rand(65536, seed=1)
+    gate_up = torch.cat((gate.view(8, -1), up.view(8, -1)), dim=1)
+    g, u = gate.double(), up.double()
+    act, grads = _comms.ops.swiglu_fwd(gate_up).view(-1), _comms.ops.swiglu_bwd(torch.ones(8, 8192, device="cuda").bfloat16(), gate_up)
+    finite = g.isfinite() & (g.abs() < 80)
+    sig = torch.sigmoid(g)
+    for out, ref in ((act, g * sig * u), (grads[:, 8192:].reshape(-1), g * sig), (grads[:, :8192].reshape(-1), u * (sig + g * sig * (1 - sig)))):
+        # Half a bf16 ulp (2^-9, or 2^-134 where there are no more bits); in fp32 before it the exponential's 2 ulp and its argument's
+        # half (of up to 80), a handful of roundings, and a sum that may cancel.
+        assert bool(((out.double() - ref).abs() <= 2**-8 * ref.abs() + u.abs() * 2**-20 + 2**-133)[finite].all())
+    # Exponentials that overflow end in a zero of the sign of the gate; infinities and NaN as in the expression itself.
+    low = g < -89
+    assert not act[low & g.isfinite()].any()
+    assert torch.equal(act.isnan(), (g * sig * u).isnan())
+
+
 @pytest.mark.parametrize("rows,dim,heads,kv_heads,hd", [(1, 64, 1, 1, 8), (129, 200, 4, 2, 32), (1000, 512, 8, 2, 64)])
 def test_block_in(rows, dim, heads, kv_heads, hd):
     from torchcomms_b200 import _comms

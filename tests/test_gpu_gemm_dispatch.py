@@ -74,6 +74,7 @@ def test_gated_product(m, n, k):
     gate_up, act, status = _comms.ops.gemm_gated(x, w)
     assert int(status[0]) == 0
     torch.testing.assert_close(gate_up.double(), x.double() @ w.double().t(), rtol=2**-8, atol=1e-6 * k)
+    assert torch.equal(act, _comms.ops.swiglu_fwd(gate_up))  # the activation kernel's bits
     # The activation from the rounded gate and up: an fp32 expression of five roundings, the exponential's and reciprocal's 2 ulp
     # among them, then one to bf16, which may fall either way.
     gate, up = gate_up.double().chunk(2, dim=-1)

@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "activation.cuh"
 #include "early_launch.cuh"
 #include "launch_count.h"
 #include "wide_access.cuh"
@@ -507,8 +508,6 @@ __global__ void __launch_bounds__(256) k_split_rope(__nv_bfloat16* packed, int64
 // chain of latencies, which a second vector's arithmetic makes longer: forward / backward of [100, 2 x 8192] 2.9 / 3.5 us
 // with two, 2.3 / 2.8 with one, of [1, 2 x 4096] 2.6 / 3.0 and 2.0 / 2.3; of [700, 2 x 4096] (358 thousand vectors)
 // 4.2 / 5.0 with two.
-__device__ __forceinline__ float sigmoid_of(float g) { return 1.0f / (1.0f + __expf(-g)); }
-
 template <int VECS>
 __global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* gate_up, __nv_bfloat16* h, uint32_t total, FastDiv per_row) {
   const uint32_t base = blockIdx.x * (256u * VECS) + threadIdx.x;
@@ -533,7 +532,7 @@ __global__ void __launch_bounds__(256) k_swiglu_fwd(const __nv_bfloat16* gate_up
       unpack8(gv[k], g);
       unpack8(uv[k], u);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoid_of(g[j]) * u[j];
+      for (int j = 0; j < 8; ++j) o[j] = gated(g[j], u[j]);
       reinterpret_cast<uint4*>(h)[i] = pack8(o);
     }
   }
@@ -566,12 +565,7 @@ __global__ void __launch_bounds__(256) k_swiglu_bwd(const __nv_bfloat16* dh, con
       unpack8(uv[k], u);
       unpack8(dv[k], d);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float sig = sigmoid_of(g[j]);
-        const float silu = g[j] * sig;
-        dg[j] = d[j] * u[j] * (sig + silu * (1.0f - sig));
-        du[j] = d[j] * silu;
-      }
+      for (int j = 0; j < 8; ++j) gated_gradient(d[j], g[j], u[j], &dg[j], &du[j]);
       reinterpret_cast<uint4*>(dgate_up)[at] = pack8(dg);
       reinterpret_cast<uint4*>(dgate_up)[at + per_row.d] = pack8(du);
     }

@@ -40,6 +40,7 @@
 #include <atomic>
 #include <type_traits>
 
+#include "activation.cuh"
 #include "early_launch.cuh"
 #include "launch_count.h"
 #include "tc_gemm.cuh"
@@ -218,21 +219,14 @@ __device__ __forceinline__ PairItem pair_item(int i, int whole, int tiles_m, int
   return PairItem{pm, pn * TILE_COLS + half * (TILE_COLS / 2), tail};
 }
 
-// silu(gate) * up of two columns, from the rounded values as k_swiglu_fwd has it. The reciprocal is the hardware's (1 ulp): the
-// correctly rounded one branches, and a warp alone on its scheduler then has one element at a time in work.
+// silu(gate) * up of two columns, from the rounded values: the bits of k_swiglu_fwd.
 __device__ __forceinline__ uint32_t gated_pair(uint32_t gate, uint32_t up) {
-  float o[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const float g = __uint_as_float(i == 0 ? gate << 16 : gate & 0xffff0000u), u = __uint_as_float(i == 0 ? up << 16 : up & 0xffff0000u);
-    float sigmoid;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(sigmoid) : "f"(1.0f + __expf(-g)));
-    o[i] = g * sigmoid * u;
-  }
-  return pack_bf16(__float_as_uint(o[0]), __float_as_uint(o[1]));
+  const float lo = gated(__uint_as_float(gate << 16), __uint_as_float(up << 16));
+  const float hi = gated(__uint_as_float(gate & 0xffff0000u), __uint_as_float(up & 0xffff0000u));
+  return pack_bf16(__float_as_uint(lo), __float_as_uint(hi));
 }
 
-// The gradients of eight columns of gate and up from those of silu(gate) * up, as k_swiglu_bwd has them.
+// The gradients of eight columns of gate and up as k_swiglu_bwd has them, but from the fp32 sums of silu(gate) * up's gradient.
 __device__ __forceinline__ void gated_gradients(const uint32_t* d, uint4 gate, uint4 up, uint4* dgate, uint4* dup) {
   const uint32_t g[4] = {gate.x, gate.y, gate.z, gate.w}, u[4] = {up.x, up.y, up.z, up.w};
   uint32_t dg[4], du[4];
@@ -242,12 +236,7 @@ __device__ __forceinline__ void gated_gradients(const uint32_t* d, uint4 gate, u
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const float gf = __uint_as_float(j == 0 ? g[i] << 16 : g[i] & 0xffff0000u), uf = __uint_as_float(j == 0 ? u[i] << 16 : u[i] & 0xffff0000u);
-      const float df = __uint_as_float(d[2 * i + j]);
-      float sigmoid;
-      asm("rcp.approx.f32 %0, %1;" : "=f"(sigmoid) : "f"(1.0f + __expf(-gf)));
-      const float silu = gf * sigmoid;
-      og[j] = df * uf * (sigmoid + silu * (1.0f - sigmoid));
-      ou[j] = df * silu;
+      gated_gradient(__uint_as_float(d[2 * i + j]), gf, uf, &og[j], &ou[j]);
     }
     dg[i] = pack_bf16(__float_as_uint(og[0]), __float_as_uint(og[1]));
     du[i] = pack_bf16(__float_as_uint(ou[0]), __float_as_uint(ou[1]));
