@@ -162,3 +162,42 @@ def test_gather_layer_in_a_graph(m, n, k):
         y.zero_()
         graph.replay()
         assert torch.equal(y, ref) and torch.equal(layer.input, x) and layer.status()[0] == 0
+
+
+def test_products_in_threads_that_have_called_nothing_yet():
+    """Every product as the first CUDA call of its thread, whose buffers the allocator has at hand."""
+    import threading
+
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops.tp import AllGatherGemm
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, w = (torch.randn(128, 256, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    big = torch.randn(4096, 256, generator=g, device="cuda").to(torch.bfloat16)
+    gate_up = torch.randn(128, 512, generator=g, device="cuda").to(torch.bfloat16)
+    square = torch.randn(256, 256, generator=g, device="cuda").to(torch.bfloat16)
+    targets = torch.zeros(128, dtype=torch.long, device="cuda")
+    layer = AllGatherGemm(None, m_local=128, k=256)
+    calls = [lambda: _comms.ops.gemm_bf16_nt(x, w)[0], lambda: _comms.ops.gemm_bf16_nt(big, big)[0], lambda: _comms.ops.gemm_bf16_mn(x, square)[0],
+             lambda: _comms.ops.gemm_gated(x, w)[1], lambda: _comms.ops.gemm_gated_grad(x, square, gate_up)[0],
+             lambda: _comms.ops.head(x, w, targets, 4096)[1], lambda: layer(square, x)]
+    for call in calls:
+        first = call().clone()
+        for _ in range(2):  # the cache then has what the thread asks for
+            call()
+        torch.cuda.synchronize()
+        results = []
+
+        def work():
+            try:
+                results.append(call())
+            except Exception as e:
+                results.append(e)
+
+        thread = threading.Thread(target=work)
+        thread.start()
+        thread.join()
+        if isinstance(results[0], Exception):
+            raise results[0]
+        torch.cuda.synchronize()
+        assert torch.equal(results[0], first)

@@ -48,12 +48,22 @@ inline EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
+// The driver encodes maps under the calling thread's context, and refuses where there is none yet: in a thread that has made no call
+// of the runtime that binds one. Buffers from PyTorch's cache and what is kept per device need none, so a product in a new
+// thread can come here first.
+inline void bind_thread() {
+  thread_local bool bound = false;
+  int device = 0;
+  if (!bound) bound = cudaGetDevice(&device) == cudaSuccess && cudaSetDevice(device) == cudaSuccess;
+}
+
 // `ld`: elements from row to row, a multiple of 8 (0: rows follow one another).
 // `box_cols`: other boxes than of 64 columns are not swizzled.
 inline bool make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint64_t ld = 0,
                      uint32_t box_cols = kBlockK) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr) return false;
+  bind_thread();
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {(ld != 0 ? ld : cols) * 2};
   const cuuint32_t box[2] = {box_cols, box_rows};
