@@ -179,6 +179,43 @@ def test_only_what_is_asked_for():
         assert not _comms.ops.block_out(*full, 1e-5).requires_grad
 
 
+def _launches(call):
+    from torchcomms_b200 import _comms
+
+    before = _comms.ops.kernel_launch_count()
+    call()
+    return _comms.ops.kernel_launch_count() - before
+
+
+def test_backward_makes_only_what_is_asked_for():
+    """The last weight's gradient takes one product, the one before it the activation's too; the norm waits for whoever wants it."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops import fused
+
+    ins = [_rand(64, 128, seed=1), _rand(64, 128, seed=2), _rand(128, 128, seed=3, scale=0.1), _rand(128, seed=4, scale=0.1) + 1,
+           _rand(512, 128, seed=5, scale=0.1), _rand(128, 256, seed=6, scale=0.1)]
+    ins = [t.requires_grad_(True) for t in ins]
+    dy = _rand(64, 128, seed=7)
+    y = _comms.ops.block_out(*ins, 1e-5)
+    full = torch.autograd.grad(y, ins, dy, retain_graph=True)
+    # one launch each: a product, the activation's gradients with theirs; the norm's two
+    for wanted, launches in (([5], 1), ([4], 2), ([4, 5], 3), ([3], 4), ([0], 4), ([2], 5), ([1], 5)):
+        some = []
+        assert _launches(lambda: some.extend(torch.autograd.grad(y, [ins[i] for i in wanted], dy, retain_graph=True))) == launches
+        assert all(torch.equal(a, full[i]) for a, i in zip(some, wanted))
+
+    cos_t, sin_t = fused.rope_tables(64, 16, 10000.0, "cuda")
+    pos = torch.arange(64, dtype=torch.int32, device="cuda")
+    wqkv = _rand(8 * 16, 128, seed=8, scale=0.1).requires_grad_(True)
+    out = _comms.ops.block_in(ins[0], ins[3], wqkv, pos, cos_t, sin_t, 4, 2, 1e-5)
+    douts = [_rand(*t.shape, seed=10 + i) for i, t in enumerate(out)]
+    full = torch.autograd.grad(out, (ins[0], ins[3], wqkv), douts, retain_graph=True)
+    for wanted, launches in (((2,), 2), ((1,), 4), ((0,), 4)):
+        some = []
+        assert _launches(lambda: some.extend(torch.autograd.grad(out, [(ins[0], ins[3], wqkv)[i] for i in wanted], douts, retain_graph=True))) == launches
+        assert all(torch.equal(a, full[i]) for a, i in zip(some, wanted))
+
+
 def test_block_takes_and_leaves():
     """What the nodes do not take runs as before: other types, autocast, transforms."""
     from torchcomms_b200 import _comms

@@ -306,7 +306,8 @@ struct RopeFn : torch::autograd::Function<RopeFn> {
 // The two halves of a decoder block around its attention, as one node each: what the separate nodes of norms, projections,
 // rotary embedding and activation launch, without an allocation, a graph edge and a trip through the engine for each, and with
 // the activation in its projection's epilogue. Both take what those nodes take: contiguous bf16 matrices on the
-// 16-byte grid, widths that are multiples of 8.
+// 16-byte grid, widths that are multiples of 8. Backward they make what is asked for and what that takes, as the engine does of
+// separate nodes.
 bool block_matrix(const at::Tensor& t, int64_t rows, int64_t cols, const at::Tensor& like) {
   return plain_call(t, true) && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.size(0) == rows && t.size(1) == cols &&
       t.is_contiguous() && on16(t) && t.device() == like.device();
@@ -418,9 +419,11 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     const at::Tensor &h = saved[3], &wqkv = saved[4];
     const at::Tensor dqkv = SplitRopeFn::packed_gradient({grads[1], grads[2], grads[3]}, saved[5], saved[6], saved[7]);
     const at::Tensor dw = ctx->needs_input_grad(2) ? weight_gradient(dqkv, h) : at::Tensor();
-    at::Tensor dnorm;
-    const variable_list dx = norm_with_skip_backward({grads[0], input_gradient(dqkv, wqkv)}, {saved[0], saved[1], saved[2]}, &dnorm);
-    return {dx[0], dnorm, dw, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+    at::Tensor dx, dnorm;
+    if (ctx->needs_input_grad(0) || ctx->needs_input_grad(1)) {
+      dx = norm_with_skip_backward({grads[0], input_gradient(dqkv, wqkv)}, {saved[0], saved[1], saved[2]}, &dnorm)[0];
+    }
+    return {dx, dnorm, dw, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
   }
   static bool applies(const at::Tensor& x, const at::Tensor& norm, const at::Tensor& wqkv, const at::Tensor& pos, const at::Tensor& cos_t,
                       const at::Tensor& sin_t, int64_t heads, int64_t kv_heads) {
@@ -451,13 +454,17 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
     const at::Tensor &o = saved[3], &wo = saved[4], &h = saved[5], &w13 = saved[6], &gate_up = saved[7], &act = saved[8], &w2 = saved[9];
     const at::Tensor dy = grads[0].contiguous();
     c10::cuda::CUDAGuard g(dy.device());
-    const at::Tensor dw2 = ctx->needs_input_grad(5) ? weight_gradient(dy, act) : at::Tensor();
-    const at::Tensor dgate_up = gated_gradient(dy, w2, gate_up);
-    const at::Tensor dw13 = ctx->needs_input_grad(4) ? weight_gradient(dgate_up, h) : at::Tensor();
-    at::Tensor dnorm;
-    const at::Tensor ds = norm_with_skip_backward({dy, input_gradient(dgate_up, w13)}, {saved[0], saved[1], saved[2]}, &dnorm)[0];
-    const at::Tensor dwo = ctx->needs_input_grad(2) ? weight_gradient(ds, o) : at::Tensor();
-    return {ds, ctx->needs_input_grad(1) ? input_gradient(ds, wo) : at::Tensor(), dwo, dnorm, dw13, dw2, at::Tensor()};
+    at::Tensor ds, d_o, dwo, dnorm, dw13, dw2;
+    if (ctx->needs_input_grad(5)) dw2 = weight_gradient(dy, act);
+    const bool sum_wanted = ctx->needs_input_grad(0) || ctx->needs_input_grad(1) || ctx->needs_input_grad(2) || ctx->needs_input_grad(3);
+    if (sum_wanted || ctx->needs_input_grad(4)) {
+      const at::Tensor dgate_up = gated_gradient(dy, w2, gate_up);
+      if (ctx->needs_input_grad(4)) dw13 = weight_gradient(dgate_up, h);
+      if (sum_wanted) ds = norm_with_skip_backward({dy, input_gradient(dgate_up, w13)}, {saved[0], saved[1], saved[2]}, &dnorm)[0];
+    }
+    if (ctx->needs_input_grad(2)) dwo = weight_gradient(ds, o);
+    if (ctx->needs_input_grad(1)) d_o = input_gradient(ds, wo);
+    return {ds, d_o, dwo, dnorm, dw13, dw2, at::Tensor()};
   }
   static bool applies(const at::Tensor& x, const at::Tensor& o, const at::Tensor& wo, const at::Tensor& norm, const at::Tensor& w13,
                       const at::Tensor& w2) {
