@@ -216,6 +216,48 @@ def test_backward_makes_only_what_is_asked_for():
         assert all(torch.equal(a, full[i]) for a, i in zip(some, wanted))
 
 
+def test_frozen_weights_keep_nothing():
+    """What a forward pass makes on the way is kept only for the gradients that take it, as separate operations keep it."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops import fused
+
+    rows, dim, width, ffn = 40, 128, 64, 256
+    ins = [_rand(rows, dim, seed=1), _rand(rows, width, seed=2), _rand(dim, width, seed=3, scale=0.1), _rand(dim, seed=4, scale=0.1) + 1,
+           _rand(2 * ffn, dim, seed=5, scale=0.1), _rand(dim, ffn, seed=6, scale=0.1)]
+    dy = _rand(rows, dim, seed=7)
+
+    def made(call, args):  # elements kept beside the arguments, and the norm's statistics
+        kept, given = {}, {t.data_ptr() for t in args}
+
+        def pack(t):
+            if t.data_ptr() not in given:
+                kept[t.data_ptr()] = t.numel()
+            return t
+
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+            out = call()
+        return sum(kept.values()) - rows, out
+
+    full = [t.clone().requires_grad_(True) for t in ins]
+    grads = torch.autograd.grad(_comms.ops.block_out(*full, 1e-5), full, dy)
+    # sum and norm's output are rows x dim, gate and up rows x 2 ffn, the activation rows x ffn
+    for wanted, cols in (((0, 1, 2, 3, 4, 5), 2 * dim + 3 * ffn), ((0,), dim + 2 * ffn), ((1, 4), 2 * dim + 2 * ffn), ((5,), ffn), ((4,), dim + 2 * ffn)):
+        some = [t.clone().requires_grad_(i in wanted) for i, t in enumerate(ins)]
+        elements, y = made(lambda: _comms.ops.block_out(*some, 1e-5), some)
+        assert elements == rows * cols
+        for i, g in zip(wanted, torch.autograd.grad(y, [some[i] for i in wanted], dy)):
+            assert torch.equal(g, grads[i])
+
+    cos_t, sin_t = fused.rope_tables(rows, 16, 10000.0, "cuda")
+    pos = torch.arange(rows, dtype=torch.int32, device="cuda")
+    wqkv = _rand(8 * 16, dim, seed=8, scale=0.1)
+    for wanted, cols in (((0, 1, 2), dim), ((0,), 0), ((2,), dim)):
+        some = [t.clone().requires_grad_(i in wanted) for i, t in enumerate((ins[0], ins[3], wqkv))]
+        elements, out = made(lambda: _comms.ops.block_in(*some, pos, cos_t, sin_t, 4, 2, 1e-5), (*some, pos, cos_t, sin_t))
+        assert elements == rows * cols
+        torch.autograd.grad(out[1:], [some[i] for i in wanted], [t.detach() for t in out[1:]])
+
+
 def test_block_takes_and_leaves():
     """What the nodes do not take runs as before: other types, autocast, transforms."""
     from torchcomms_b200 import _comms

@@ -411,7 +411,8 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     variable_list out{at::empty({tokens, heads, hd}, x.options()), at::empty({tokens, kv_heads, hd}, x.options()),
                       at::empty({tokens, kv_heads, hd}, x.options())};
     SplitRopeFn::launch(qkv, out, pos, cos_t, sin_t, false);
-    ctx->save_for_backward({x, norm, rstd, h, wqkv, pos, cos_t, sin_t});
+    const at::Tensor none;
+    ctx->save_for_backward({x, norm, rstd, wqkv.requires_grad() ? h : none, wqkv, pos, cos_t, sin_t});
     return {x, out[0], out[1], out[2]};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -446,7 +447,11 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
     const auto [gate_up, act] = gated_product(h, w13);
     at::Tensor y = product(act, w2);
     y.add_(sum);
-    ctx->save_for_backward({sum, norm, rstd, o, wo, h, w13, gate_up, act, w2});
+    // What was made on the way is kept for whoever has a gradient that takes it.
+    const at::Tensor none;
+    const bool sum_wanted = x.requires_grad() || o.requires_grad() || wo.requires_grad() || norm.requires_grad();
+    ctx->save_for_backward({sum_wanted ? sum : none, norm, rstd, o, wo, w13.requires_grad() ? h : none, w13,
+                            sum_wanted || w13.requires_grad() ? gate_up : none, w2.requires_grad() ? act : none, w2});
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
