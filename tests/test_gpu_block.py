@@ -258,6 +258,56 @@ def test_frozen_weights_keep_nothing():
         torch.autograd.grad(out[1:], [some[i] for i in wanted], [t.detach() for t in out[1:]])
 
 
+def test_gradients_of_gradients():
+    """Second-order gradients are those of the separate operations, also where attention makes one argument from another."""
+    from torchcomms_b200 import _comms
+    from torchcomms_b200.ops import fused
+
+    rows, dim, ffn = 48, 128, 200
+    ins = [_rand(rows, dim, seed=1), _rand(dim, dim, seed=3, scale=0.1), _rand(dim, seed=4, scale=0.1) + 1, _rand(2 * ffn, dim, seed=5, scale=0.1),
+           _rand(dim, ffn, seed=6, scale=0.1)]
+    dy = _rand(rows, dim, seed=7)
+
+    def apart(x, o, wo, norm, w13, w2):
+        s, h = fused.add_rms_norm(x, torch.nn.functional.linear(o, wo), norm, 1e-5)
+        return s + torch.nn.functional.linear(fused.swiglu(torch.nn.functional.linear(h, w13)), w2)
+
+    def orders(f, frozen):
+        x, *weights = [t.clone().requires_grad_(i not in frozen) for i, t in enumerate(ins)]
+        o = x * x  # made from another argument
+        leaves = [t for t in (x, *weights) if t.requires_grad]
+        first = torch.autograd.grad(f(x, o, *weights), leaves, dy, create_graph=True)
+        with_history = [g for g in first if g.requires_grad]
+        assert with_history
+        second = torch.autograd.grad(sum(g.float().square().sum() for g in with_history), leaves, allow_unused=True)
+        return [g.requires_grad for g in first], first, second
+
+    for frozen in ((), (1, 4), (2, 3)):
+        mine, theirs = orders(lambda *a: _comms.ops.block_out(*a, 1e-5), frozen), orders(apart, frozen)
+        assert mine[0] == theirs[0]
+        # The same kernels; the engine adds what meets in an argument, four terms in bf16 at most, in its own order.
+        for a, b in zip(mine[1] + mine[2], theirs[1] + theirs[2]):
+            assert (a is None and b is None) or _off(a.detach(), b.detach()) < 4 * 2**-9
+
+    cos_t, sin_t = fused.rope_tables(rows, 16, 10000.0, "cuda")
+    pos = torch.arange(rows, dtype=torch.int32, device="cuda")
+    wqkv = _rand(8 * 16, dim, seed=8, scale=0.1)
+
+    def apart_in(x, norm, w):
+        x, h = fused.rms_norm_skip(x, norm, 1e-5)
+        return (x, *fused.split_rope(torch.nn.functional.linear(h, w), pos, cos_t, sin_t, 4, 2))
+
+    results = []
+    for f in (lambda *a: _comms.ops.block_in(*a, pos, cos_t, sin_t, 4, 2, 1e-5), apart_in):
+        leaves = [t.clone().requires_grad_(True) for t in (ins[0], ins[2], wqkv)]
+        out = f(*leaves)
+        first = torch.autograd.grad(out, leaves, [_rand(*t.shape, seed=10 + i) for i, t in enumerate(out)], create_graph=True)
+        second = torch.autograd.grad(sum(g.float().square().sum() for g in first if g.requires_grad), leaves, allow_unused=True)
+        results.append((*first, *second))
+    for a, b in zip(*results):
+        assert (a is None and b is None) or (_off(a.detach(), b.detach()) < 4 * 2**-9 and a.requires_grad == b.requires_grad)
+
+
 def test_block_takes_and_leaves():
     """What the nodes do not take runs as before: other types, autocast, transforms."""
     from torchcomms_b200 import _comms

@@ -362,8 +362,8 @@ void mn_product_into(at::Tensor& c, const at::Tensor& a, bool by_columns, const 
                                        static_cast<int>(c.size(0)), static_cast<int>(c.size(1)), static_cast<int>(b.size(0)),
                                        reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(b)));
 }
-// dy [rows, n] w [n, k] and dy^T x [rows, k], the gradients of a product's operands. The tensor library's where the backward pass is
-// itself differentiated, and where a hook has put something else in a tensor's place.
+// dy [rows, n] w [n, k] and dy^T x [rows, k], the gradients of a product's operands. The tensor library's where a mode watches the
+// backward pass, or a hook has put something else in a tensor's place.
 bool plain_rows(const at::Tensor& t, const at::Tensor& like) {
   return plain_call(t) && block_matrix(t, t.size(0), t.size(1), like) && t.size(1) % 8 == 0;
 }
@@ -399,6 +399,26 @@ at::Tensor weight_gradient(const at::Tensor& dy, const at::Tensor& x) {
   return dw;
 }
 
+// A backward pass that is itself differentiated needs its gradients' history, which the nodes below do not have: what they keep was
+// made inside them. There the separate nodes run once more, on the arguments, and the engine differentiates them: the history, and
+// the limits (a norm's or an activation's gradient has none), of a block made of them. `forward` gets the arguments under other
+// names, so that nothing is counted twice where one argument was made from another.
+template <typename F>
+variable_list gradients_with_history(AutogradContext* ctx, const std::vector<at::Tensor>& args, variable_list grads, F&& forward) {
+  std::vector<at::Tensor> own(args.size());
+  variable_list wanted, out(args.size());
+  for (size_t i = 0; i < args.size(); ++i) {
+    own[i] = args[i].view_as(args[i]);
+    if (ctx->needs_input_grad(i)) wanted.push_back(own[i]);
+  }
+  const variable_list made = torch::autograd::grad(forward(own), wanted, grads, /*retain_graph=*/std::nullopt, /*create_graph=*/true,
+                                                   /*allow_unused=*/true);
+  for (size_t i = 0, j = 0; i < args.size(); ++i) {
+    if (ctx->needs_input_grad(i)) out[i] = made[j++];
+  }
+  return out;
+}
+
 // (x, queries, keys, values) of x [tokens, dim]: norm, fused projection, rotary embedding. x is returned for the residual.
 struct BlockInFn : torch::autograd::Function<BlockInFn> {
   static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& norm, const at::Tensor& wqkv,
@@ -413,11 +433,25 @@ struct BlockInFn : torch::autograd::Function<BlockInFn> {
     SplitRopeFn::launch(qkv, out, pos, cos_t, sin_t, false);
     const at::Tensor none;
     ctx->save_for_backward({x, norm, rstd, wqkv.requires_grad() ? h : none, wqkv, pos, cos_t, sin_t});
+    ctx->saved_data["heads"] = heads;
+    ctx->saved_data["kv_heads"] = kv_heads;
+    ctx->saved_data["eps"] = eps;
     return {x, out[0], out[1], out[2]};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const at::Tensor &h = saved[3], &wqkv = saved[4];
+    if (c10::GradMode::is_enabled()) {
+      variable_list out = gradients_with_history(ctx, {saved[0], saved[1], wqkv}, grads, [&](const std::vector<at::Tensor>& a) {
+        const variable_list normed = SkipRmsNormFn::apply(a[0], a[1], ctx->saved_data["eps"].toDouble());
+        variable_list parts = SplitRopeFn::apply(at::linear(normed[1], a[2]), saved[5], saved[6], saved[7], ctx->saved_data["heads"].toInt(),
+                                                 ctx->saved_data["kv_heads"].toInt());
+        parts.insert(parts.begin(), normed[0]);
+        return parts;
+      });
+      out.resize(9);
+      return out;
+    }
     const at::Tensor dqkv = SplitRopeFn::packed_gradient({grads[1], grads[2], grads[3]}, saved[5], saved[6], saved[7]);
     const at::Tensor dw = ctx->needs_input_grad(2) ? weight_gradient(dqkv, h) : at::Tensor();
     at::Tensor dx, dnorm;
@@ -451,12 +485,21 @@ struct BlockOutFn : torch::autograd::Function<BlockOutFn> {
     const at::Tensor none;
     const bool sum_wanted = x.requires_grad() || o.requires_grad() || wo.requires_grad() || norm.requires_grad();
     ctx->save_for_backward({sum_wanted ? sum : none, norm, rstd, o, wo, w13.requires_grad() ? h : none, w13,
-                            sum_wanted || w13.requires_grad() ? gate_up : none, w2.requires_grad() ? act : none, w2});
+                            sum_wanted || w13.requires_grad() ? gate_up : none, w2.requires_grad() ? act : none, w2, x});
+    ctx->saved_data["eps"] = eps;
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const at::Tensor &o = saved[3], &wo = saved[4], &h = saved[5], &w13 = saved[6], &gate_up = saved[7], &act = saved[8], &w2 = saved[9];
+    if (c10::GradMode::is_enabled()) {
+      variable_list out = gradients_with_history(ctx, {saved[10], o, wo, saved[1], w13, w2}, grads, [&](const std::vector<at::Tensor>& a) {
+        const variable_list normed = AddRmsNormFn::apply(a[0], at::linear(a[1], a[2]), a[3], ctx->saved_data["eps"].toDouble());
+        return variable_list{normed[0] + at::linear(SwiGluFn::apply(at::linear(normed[1], a[4])), a[5])};
+      });
+      out.resize(7);
+      return out;
+    }
     const at::Tensor dy = grads[0].contiguous();
     c10::cuda::CUDAGuard g(dy.device());
     at::Tensor ds, d_o, dwo, dnorm, dw13, dw2;
