@@ -201,3 +201,32 @@ def test_products_in_threads_that_have_called_nothing_yet():
             raise results[0]
         torch.cuda.synchronize()
         assert torch.equal(results[0], first)
+
+
+# Loads that are never complete and waits of 20 ms, on every kernel: split, single CTAs, pairs with more tiles than pairs and a last
+# wave in halves, fewer and more K steps than stages; the gated epilogues.
+@pytest.mark.parametrize("kind,m,n,k", [("nt", 128, 4096, 1792), ("nt", 640, 7168, 4096), ("pair", 4096, 2560, 200), ("pair", 300, 264, 1024),
+                                        ("gated", 1000, 5136, 136), ("gated", 200, 272, 1024), ("gated_grad", 300, 4808, 200),
+                                        ("gated_grad", 257, 136, 1024)])
+def test_a_product_that_gives_up_says_so(kind, m, n, k):
+    """Whoever drops the status words, as a decoder block does, finds NaN and not what the memory held."""
+    from torchcomms_b200 import _comms
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(*((k, n) if kind == "gated_grad" else (n, k)), generator=g, device="cuda").to(torch.bfloat16)
+    gate_up = torch.randn(m, 2 * n, generator=g, device="cuda").to(torch.bfloat16) if kind == "gated_grad" else None
+    out, status = _comms.ops.gemm_giving_up(kind, a, w, gate_up, 20)
+    torch.cuda.synchronize()
+    assert int(status[0]) != 0 and bool(out.isnan().all())
+    # The context goes on, and so does the same kernel.
+    if kind == "gated_grad":
+        c, status = _comms.ops.gemm_gated_grad(a, w, gate_up)
+        assert not c.isnan().any()
+    elif kind == "gated":
+        c, _, status = _comms.ops.gemm_gated(a, w)
+        torch.testing.assert_close(c.double(), a.double() @ w.double().t(), rtol=2**-8, atol=4e-6 * k)
+    else:
+        c, status = (_comms.ops.gemm_bf16_nt if kind == "nt" else _comms.ops.gemm_bf16_nt_pair)(a, w)
+        torch.testing.assert_close(c.double(), a.double() @ w.double().t(), rtol=2**-8, atol=4e-6 * k)
+    assert int(status[0]) == 0

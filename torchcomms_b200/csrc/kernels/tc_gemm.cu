@@ -97,6 +97,7 @@ struct TpParams {
   int clear;          // plain mode: the status words are this call's own
   int stage_bytes;    // plain mode: of one K step's loads
   int late;           // plain mode: not launched early
+  unsigned long long wait_ns;  // plain mode: limit of a wait (0: kLocalWaitNs)
   int m_total, m_local, n, k, gm;   // k in 16-bit units: K for bf16, K / 2 for e4m3
   // e4m3 operands: C = (row_scale[m] * col_scale[n]) * (A_q x B_q^T)
   int fp8;
@@ -415,7 +416,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % Cfg::kStages;
           const uint32_t ph = (it / Cfg::kStages) & 1u;
-          if (!mbar_wait(&bars->empty[s], ph ^ 1u)) {
+          if (!mbar_wait(&bars->empty[s], ph ^ 1u, p.wait_ns)) {
             bars->failed = 1;
             break;
           }
@@ -433,7 +434,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
       uint32_t it = 0, tile_iter = 0;
       for (int t = blockIdx.x; t < total_tiles && !bars->failed; t += G, ++tile_iter) {
         const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
-        if (!mbar_wait(&bars->acc_empty[as], aph ^ 1u)) {
+        if (!mbar_wait(&bars->acc_empty[as], aph ^ 1u, p.wait_ns)) {
           bars->failed = 1;
           break;
         }
@@ -442,7 +443,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % Cfg::kStages;
           const uint32_t ph = (it / Cfg::kStages) & 1u;
-          if (!mbar_wait(&bars->full[s], ph)) {
+          if (!mbar_wait(&bars->full[s], ph, p.wait_ns)) {
             bars->failed = 1;
             break;
           }
@@ -460,6 +461,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
           }
           umma_commit(&bars->empty[s]);  // stage reusable once these MMAs have read it
         }
+        if (bars->failed) break;  // not all of K: the epilogue waits in vain
         umma_commit(&bars->acc_full[as]);  // accumulator complete
       }
       trace_stamp_ns(c, 2);
@@ -473,6 +475,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
     ColScales<BN> fetched;
     if (FP8 && static_cast<int>(blockIdx.x) < total_tiles) fetched.fetch(p.scale_b, tile_at(blockIdx.x, tiles_m, tiles_n, p.gm).ni * BN, p.n, et);
     uint32_t tile_iter = 0, chunk_iter = 0;
+    bool lost = false;  // a wait ran out: NaN from here on, see no_acc()
     for (int t = blockIdx.x; t < total_tiles; t += G, ++tile_iter) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
       const TileCoord tc_ = tile_at(t, tiles_m, tiles_n, p.gm);
@@ -482,9 +485,14 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
         fetched.put(col_scales, et);
         if (t + G < total_tiles) fetched.fetch(p.scale_b, tile_at(t + G, tiles_m, tiles_n, p.gm).ni * BN, p.n, et);
       }
-      if (!mbar_wait(&bars->acc_full[as], aph)) {
-        bars->failed = 1;
-        break;
+      if (kFused) {
+        if (!mbar_wait(&bars->acc_full[as], aph)) {
+          bars->failed = 1;
+          break;
+        }
+      } else {
+        lost = lost || !mbar_wait_warp(&bars->acc_full[as], aph, p.wait_ns);
+        if (lost) bars->failed = 1;
       }
       tc_fence_after_sync();
       const float row_scale = FP8 ? row_scale_of<MODE>(p, c, tc_.ord, tiles_per_src, mi * kBlockM + row_in_tile) : 1.0f;
@@ -515,6 +523,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
                             static_cast<uint32_t>(j * kOutChunkCols + half * 32),
                         r);
           tmem_ld_wait();
+          if (lost) no_acc(r);
           if (FP8) scale_acc32(r, row_scale, col_scales + j * kOutChunkCols + half * 32);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
@@ -1221,13 +1230,14 @@ cudaError_t launch_gemm_e4m3_nt(const void* a, const void* b, void* c, int m, in
 
 // k in 16-bit units; scales non-null = e4m3 operands.
 cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                           const float* scale_b, uint32_t* status, cudaStream_t stream, const CommDev* layer, void* a_copy) {
+                           const float* scale_b, uint32_t* status, cudaStream_t stream, const CommDev* layer, void* a_copy,
+                           const GiveUp* give_up) {
   if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || n % 8 != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) {
     return cudaErrorInvalidValue;
   }
   bool done = false;
-  cudaError_t e = launch_gemm_nt_split(a, b, c, m, n, k, scale_a, scale_b, status, stream, &done, layer, a_copy);
+  cudaError_t e = launch_gemm_nt_split(a, b, c, m, n, k, scale_a, scale_b, status, stream, &done, layer, a_copy, give_up);
   if (e != cudaSuccess || done) return e;
   if (a_copy != nullptr && a_copy != a) {
     e = cudaMemcpyAsync(a_copy, a, static_cast<size_t>(m) * k * 2, cudaMemcpyDeviceToDevice, stream);
@@ -1249,7 +1259,7 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   const bool short_sum = on_lines && k <= (singles <= sms ? 16 : 4) * kBlockK;
   const double single_cost = wave_cost(singles, sms) * (on_lines ? 1.2 : 1.45) * (short_sum ? 0.8 : 1.0);
   if (pair_tiles_fit(m, n, fp8) || pair_cost <= single_cost) {
-    return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, columns, layer);
+    return launch_gemm_nt_pair(a, b, c, m, n, k, scale_a, scale_b, status, stream, columns, layer, give_up);
   }
   TpMaps maps;
   if (!make_map(&maps.a_local, a, m, k, a_box_rows(m)) || !make_map(&maps.b, b, n, k, kTpBN) ||
@@ -1265,7 +1275,8 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
   TpParams p{};
   p.status = status;
   p.clear = layer == nullptr && status != nullptr ? 1 : 0;
-  p.stage_bytes = a_box_rows(m) * kBlockK * 2 + TileCfg<kTpBN>::kBBytes;
+  p.stage_bytes = a_box_rows(m) * kBlockK * 2 + TileCfg<kTpBN>::kBBytes + (give_up != nullptr ? give_up->missing : 0);
+  p.wait_ns = give_up != nullptr ? give_up->wait_ns : 0;
   p.m_total = m;
   p.m_local = m;
   p.n = n;

@@ -122,7 +122,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // pipeline stage may legitimately wait while copy warps sit in their own
 // (time-bounded) wait for a slow peer. kLocalWaitNs is far above any peer-wait
 // budget, so a local wait only runs out when the pipeline is truly stuck.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned long long limit_ns = 0) {
   unsigned long long start = 0;
   for (uint32_t i = 0;; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -131,11 +131,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
       if (start == 0) {
         start = now;
-      } else if (now - start > kLocalWaitNs) {
+      } else if (now - start > (limit_ns != 0 ? limit_ns : kLocalWaitNs)) {
         return false;
       }
     }
   }
+}
+// The same for a converged warp, whose lanes all get the one answer: each leaves the wait by itself, and one might give up where
+// the next one still sees the barrier complete.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned long long limit_ns) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit_ns)) != 0;
+}
+// Accumulators that will never be there. A plain product whose wait ran out stores NaN wherever it has nothing else: not every
+// caller reads the status words (a decoder block has no time to), and what was in the output's memory before passes for numbers.
+template <int N>
+__device__ __forceinline__ void no_acc(uint32_t (&r)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) r[i] = 0x7fc00000u;
 }
 // The two status words of a plain product, cleared by its first block (after grid_wait()) and not by a launch of their own
 // in front of it: a kernel node for that costs a captured product 2.5 us (128 x 1024 x 256 in bf16: 7.1 us a replay, with the

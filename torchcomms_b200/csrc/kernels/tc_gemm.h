@@ -22,6 +22,14 @@ cudaError_t launch_gemm_bf16_nt(const void* a, const void* b, void* c, int m, in
 // tiles, tensor maps and pipeline are those of the bf16 kernel; only the tcgen05.mma kind differs.
 cudaError_t launch_gemm_e4m3_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                 const float* scale_b, uint32_t* status, cudaStream_t stream);
+// For tests of waits that run out: every K step's loads are said to be `missing` bytes more than they are, so that none is
+// complete, and each wait of the kernel gives up after `wait_ns`. A product whose waits ran out reports kStatusTimeout and stores NaN
+// for what it does not have.
+struct GiveUp {
+  unsigned long long wait_ns;
+  int missing;
+};
+
 // Common entry of the two above (k in 16-bit units, scales null = bf16), which picks the kernel. `status`: two words, which
 // the kernel clears before it reports into them. `layer`: the communicator of a fused layer on one rank, whose status
 // words are not the call's own and keep what they hold, and whose phase trace is stamped (start, loads issued, MMAs
@@ -29,7 +37,7 @@ cudaError_t launch_gemm_e4m3_nt(const void* a, const void* b, void* c, int m, in
 // `a` itself, where it is there already: the same kernel then, and the same bits.
 cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                            const float* scale_b, uint32_t* status, cudaStream_t stream, const CommDev* layer = nullptr,
-                           void* a_copy = nullptr);
+                           void* a_copy = nullptr, const GiveUp* give_up = nullptr);
 
 // The same product where 128 x 128 tiles are too few to fill the GPU: clusters of CTAs split K and sum in
 // distributed shared memory. Sets *done when it launched; otherwise (more than kSplitMaxTiles tiles, or a product that
@@ -40,7 +48,7 @@ cudaError_t launch_gemm_nt(const void* a, const void* b, void* c, int m, int n, 
 constexpr int kSplitMaxTiles = 148;
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                  const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done,
-                                 const CommDev* layer = nullptr, void* a_copy = nullptr);
+                                 const CommDev* layer = nullptr, void* a_copy = nullptr, const GiveUp* give_up = nullptr);
 
 // The same product on CTA pairs (clusters of two CTAs, tcgen05 cta_group::2):
 // each pair owns a tile of 256 rows and `columns` (128, 192, 224 or 256; 0: pair_columns()) columns and reads every
@@ -48,7 +56,7 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
 // non-null = e4m3 operands. `layer`: as above.
 cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                 const float* scale_b, uint32_t* status, cudaStream_t stream, int columns = 0,
-                                const CommDev* layer = nullptr);
+                                const CommDev* layer = nullptr, const GiveUp* give_up = nullptr);
 // Products whose operands do not lie along K, bf16: c[m, n] = A x b[k, n] with A = a[m, k], or the transpose of a[k, m] where it
 // lies `by_columns`.
 // `lda`, `ldb`: row strides, multiples of 8. Any m and k, n % 8 == 0; all pointers 16-byte aligned. `status`: as above.
@@ -57,7 +65,7 @@ cudaError_t launch_gemm_pair_mn(const void* a, int64_t lda, bool a_by_columns, c
 // dgate_up[m, 2 n], the gradient of gate_up, from d = dy[m, k] x w[k, n], that of silu(gate) * up. n, k % 8 == 0; all pointers
 // 16-byte aligned.
 cudaError_t launch_gemm_gated_grad(const void* dy, const void* w, const void* gate_up, void* dgate_up, int m, int n, int k, uint32_t* status,
-                                   cudaStream_t stream);
+                                   cudaStream_t stream, const GiveUp* give_up = nullptr);
 // Pairs that the GPU holds at once (0 after an error), and whether the narrow tiles of an m x n product are at most as many.
 int pairs_at_once(bool fp8);
 // Waves of tiles, of which `at_once` run at a time, in time: a last, partial wave costs half a wave and half of the share it
@@ -70,7 +78,7 @@ bool pair_tiles_fit(int m, int n, bool fp8);
 // The first half of a gated MLP on CTA pairs, bf16: gate_up[m, 2 n] = x[m, k] x w[2 n, k]^T (gate columns first) and, from its
 // rounded values, act[m, n] = silu(gate) * up. n and k multiples of 8. `status`: as above.
 cudaError_t launch_gemm_gated(const void* x, const void* w, void* gate_up, void* act, int m, int n, int k, uint32_t* status,
-                              cudaStream_t stream, int columns = 0);
+                              cudaStream_t stream, int columns = 0, const GiveUp* give_up = nullptr);
 
 // Logits of a head on CTA pairs: logits[m, n] (bf16, row stride `ld`, a multiple of 8) = x[m, k] x w[n, k]^T, any n, k % 8 ==
 // 0. Also, of the rounded logits, for each of head_row_shares(m, n) shares of a row the maximum and the sum of

@@ -120,9 +120,11 @@ struct PairParams {
   const float* scale_a;  // e4m3: per row of A, per row of B
   const float* scale_b;
   long long* trace;
+  unsigned long long wait_ns;  // limit of a wait (0: kLocalWaitNs)
   int m, n, k, gm;  // k in 16-bit units
   int clear;        // the status words are this call's own
   int stage_bytes, tail_bytes;  // of one K step's loads, both CTAs together, of a tile and of half a tile
+  int missing;      // (host) bytes more that a step's loads are said to be
   int whole;        // tiles that are worked on whole; the others, too few to keep half of the pairs busy, in halves of their columns
   float2* stats;    // kStats: [shares of a row, m] maximum and sum of exponentials; per row its target and the target's logit
   const int64_t* targets;
@@ -321,7 +323,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(&bars->empty[s], ph ^ 1u)) {
+          if (!mbar_wait(&bars->empty[s], ph ^ 1u, p.wait_ns)) {
             bars->failed = 1;
             break;
           }
@@ -356,7 +358,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
       for (int i = cluster_id; i < items && !bars->failed; i += nclusters, ++tile_iter) {
         const uint32_t shape = i >= p.whole ? idesc_tail : idesc;
         const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
-        if (!mbar_wait(&bars->acc_empty[as], aph ^ 1u)) {
+        if (!mbar_wait(&bars->acc_empty[as], aph ^ 1u, p.wait_ns)) {
           bars->failed = 1;
           break;
         }
@@ -365,7 +367,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
         for (int kb = 0; kb < k_iters; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
-          if (!mbar_wait(&bars->full[s], ph)) {
+          if (!mbar_wait(&bars->full[s], ph, p.wait_ns)) {
             bars->failed = 1;
             break;
           }
@@ -385,6 +387,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           }
           umma_commit_pair(&bars->empty[s], 3);  // both CTAs may refill the stage
         }
+        if (bars->failed) break;  // not all of K: the epilogues wait in vain
         umma_commit_pair(&bars->acc_full[as], 3);  // both CTAs' epilogues may read
       }
     }
@@ -419,8 +422,10 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     const int first = cluster_id + set * nclusters, step = kSets * nclusters;
     if (first < items) fetch(first);
     // Chunk `n` of gate and up, where its gradients will be: two buffers, the next chunk on its way while one is worked on.
+    uint32_t gate_loads = 0;  // made by this thread
     const auto load_gates = [&](uint32_t n, int2 at) {
       if constexpr (GRAD) {
+        gate_loads = n + 1;
         char* const to = obuf + 2 * (n & 1u) * kOutChunkBytes;
         tma_store_wait_read<0>();  // the chunk before the last is out of it
         mbar_expect_tx(&bars->gates[n & 1u], 2 * kOutChunkBytes);
@@ -430,6 +435,9 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     };
     if (GRAD && issuer && first < items) load_gates(0, place_of(first));
     uint32_t tile_iter = static_cast<uint32_t>(set), chunk_iter = 0;
+    // After a wait that ran out a warp waits no more, and goes on to the end with the others of its set, which meet it at every
+    // chunk; what it stores is NaN. `gates_lost`: that of a load of gate and up.
+    bool lost = false, gates_lost = false;
     for (int i = first; i < items; i += step, tile_iter += kSets) {
       const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
       const int2 at = place_of(i);
@@ -442,13 +450,8 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
         epilogue_sync(set);
       }
       if (i + step < items) fetch(i + step);
-      if (!mbar_wait(&bars->acc_full[as], aph)) {
-        bars->failed = 1;
-        if constexpr (GRAD) {
-          if (issuer) mbar_wait(&bars->gates[chunk_iter & 1u], (chunk_iter >> 1) & 1u);  // nothing is in flight at the end
-        }
-        break;
-      }
+      lost = lost || !mbar_wait_warp(&bars->acc_full[as], aph, p.wait_ns);
+      if (lost) bars->failed = 1;
       tc_fence_after_sync();
       RowStats row_stats;
       const bool row_there = STATS && out_row + row_in_tile < p.m;
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
             tmem_ld_32x32(from, g);
             tmem_ld_32x32(from + to_up, u);
             tmem_ld_wait();
+            if (lost) no_acc(g), no_acc(u);
             if (j == chunks - 1 && half == 1) {
               tc_fence_before_sync();
               __syncwarp();
@@ -507,20 +511,21 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
         const int chunks = BN / kChunk / (tail ? 2 : 1);
         for (int j = 0; j < chunks; ++j, ++chunk_iter) {
           const uint32_t b = chunk_iter & 1u;
-          if (issuer) {
+          if (issuer && !gates_lost) {
             if (j + 1 < chunks) {
               load_gates(chunk_iter + 1, make_int2(out_row, out_col + (j + 1) * kChunk));
             } else if (i + step < items) {
               load_gates(chunk_iter + 1, place_of(i + step));
             }
           }
-          if (!mbar_wait(&bars->gates[b], (chunk_iter >> 1) & 1u)) bars->failed = 1;
-          __syncwarp();
+          gates_lost = gates_lost || !mbar_wait_warp(&bars->gates[b], (chunk_iter >> 1) & 1u, p.wait_ns);
+          if (gates_lost) bars->failed = 1;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             uint32_t d[32];
             tmem_ld_32x32(tmem_base + as * kAccCols + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(j * kChunk + half * 32), d);
             tmem_ld_wait();
+            if (lost || gates_lost) no_acc(d);
             if (j == chunks - 1 && half == 1) {
               tc_fence_before_sync();
               __syncwarp();
@@ -555,6 +560,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
                         acc[half]);
         }
         tmem_ld_wait();
+        if (lost) no_acc(acc[0]), no_acc(acc[1]);
         if (j == chunks - 1) {
           tc_fence_before_sync();
           __syncwarp();
@@ -606,6 +612,8 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     }
     if (issuer) {
       tma_store_wait_all<0>();
+      // Of loads that nobody waited for in the end, the last of each buffer may still be on its way.
+      for (uint32_t n = gate_loads; n > 0 && n + 2 > gate_loads; --n) mbar_wait(&bars->gates[(n - 1) & 1u], ((n - 1) >> 1) & 1u, p.wait_ns);
       trace_stamp_ns(p.trace, 3);
     }
   }
@@ -661,6 +669,12 @@ int resident_pairs() {
   return n;
 }
 
+void set_limits(PairParams* p, const GiveUp* give_up) {
+  if (give_up == nullptr) return;
+  p->wait_ns = give_up->wait_ns;
+  p->missing = give_up->missing;
+}
+
 // `ldc`: row stride of the output in elements (0: n), `lda`, `ldb`: of the operands as they lie in memory (0: rows follow one another).
 template <bool FP8, int BN, Epilogue EPI = kPlain, PairLayout LAYOUT = PairLayout::kNT>
 cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cudaStream_t stream, int64_t ldc = 0, int64_t lda = 0,
@@ -694,8 +708,8 @@ cudaError_t launch_pair(const void* a, const void* b, void* c, PairParams p, cud
     }
   }
   const int a_bytes = A_MN ? kABytes : a_box_rows(p.m) * kBlockK * 2;
-  p.stage_bytes = 2 * (a_bytes + PairTile<BN, EPI>::kBHalfBytes);
-  p.tail_bytes = 2 * (a_bytes + PairTile<BN, EPI>::kBHalfBytes / 2);
+  p.stage_bytes = 2 * (a_bytes + PairTile<BN, EPI>::kBHalfBytes) + p.missing;
+  p.tail_bytes = 2 * (a_bytes + PairTile<BN, EPI>::kBHalfBytes / 2) + p.missing;
   const int tiles_m = (p.m - 1) / (2 * kBlockM) + 1, tiles_n = (p.n - 1) / kTileCols + 1;
   const int64_t tiles = static_cast<int64_t>(tiles_m) * tiles_n;
   const bool halves = EPI != kStats && tail_in_halves(tiles, pairs, BN);
@@ -766,12 +780,14 @@ bool pair_tiles_fit(int m, int n, bool fp8) {
 }
 
 cudaError_t launch_gemm_nt_pair(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
-                                const float* scale_b, uint32_t* status, cudaStream_t stream, int columns, const CommDev* layer) {
+                                const float* scale_b, uint32_t* status, cudaStream_t stream, int columns, const CommDev* layer,
+                                const GiveUp* give_up) {
   if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || n % 8 != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) {
     return cudaErrorInvalidValue;
   }
   PairParams p{};
+  set_limits(&p, give_up);
   p.status = status;
   p.clear = layer == nullptr && status != nullptr ? 1 : 0;
   p.scale_a = scale_a;
@@ -821,13 +837,14 @@ cudaError_t launch_gemm_pair_mn(const void* a, int64_t lda, bool a_by_columns, c
 // the next tile's product runs. Gate and up by boxes into the buffers that their gradients leave from: rows read by one thread each
 // instead were 200 us for 2048 x 14336 x 4096, so 198, and 89 for 2048 x 8192 x 2048, so 67 (two sets of epilogue warps 212 and 91).
 cudaError_t launch_gemm_gated_grad(const void* dy, const void* w, const void* gate_up, void* dgate_up, int m, int n, int k, uint32_t* status,
-                                   cudaStream_t stream) {
+                                   cudaStream_t stream, const GiveUp* give_up) {
   if (m <= 0 || n <= 0 || k <= 0 || n % 8 != 0 || k % 8 != 0 || n > INT32_MAX / 2) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(gate_up) |
        reinterpret_cast<uintptr_t>(dgate_up)) & 15u) {
     return cudaErrorMisalignedAddress;
   }
   PairParams p{};
+  set_limits(&p, give_up);
   p.status = status;
   p.clear = status != nullptr ? 1 : 0;
   p.m = m;
@@ -864,12 +881,13 @@ cudaError_t launch_head_logits(const void* x, const void* w, void* logits, int64
 }
 
 cudaError_t launch_gemm_gated(const void* x, const void* w, void* gate_up, void* act, int m, int n, int k, uint32_t* status,
-                              cudaStream_t stream, int columns) {
+                              cudaStream_t stream, int columns, const GiveUp* give_up) {
   if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || n % 8 != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(act)) & 15u) {
     return cudaErrorMisalignedAddress;
   }
   PairParams p{};
+  set_limits(&p, give_up);
   p.status = status;
   p.clear = 1;
   p.m = m;

@@ -88,6 +88,7 @@ struct SplitParams {
   const float* scale_a;  // e4m3: per row of A, per row of B
   const float* scale_b;
   long long* trace;
+  unsigned long long wait_ns;  // limit of a wait (0: kLocalWaitNs)
   int m, n, k, k_iters, tiles_m;  // k in 16-bit units
   int copy_a, per_split;
   int always;  // (host) this kernel whether it pays or not
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const int s = it % kSplitStages;
         const uint32_t ph = (it / kSplitStages) & 1u;
-        if (!mbar_wait(&bars->empty[s], ph ^ 1u)) {
+        if (!mbar_wait(&bars->empty[s], ph ^ 1u, p.wait_ns)) {
           bars->failed = 1;
           break;
         }
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const int s = it % kSplitStages;
         const uint32_t ph = (it / kSplitStages) & 1u;
-        if (!mbar_wait(&bars->full[s], ph)) {
+        if (!mbar_wait(&bars->full[s], ph, p.wait_ns)) {
           bars->failed = 1;
           break;
         }
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
         }
         umma_commit(&bars->empty[s]);
       }
-      umma_commit(&bars->acc_full);
+      if (!bars->failed) umma_commit(&bars->acc_full);  // or not all of K is there: the epilogue waits in vain
       if (TRACE) trace_stamp_ns(p.trace, 2);
     }
   } else {
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
       const int tiles_n = static_cast<int>(gridDim.x) / splits / p.tiles_m;
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const int s = it % kSplitStages;
-        if (!mbar_wait(&bars->full[s], (it / kSplitStages) & 1u)) {
+        if (!mbar_wait(&bars->full[s], (it / kSplitStages) & 1u, p.wait_ns)) {
           bars->failed = 1;
           break;
         }
@@ -236,9 +237,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
       bars->scale_b[row] = ni * kSplitBN + row < p.n ? p.scale_b[ni * kSplitBN + row] : 0.0f;
       asm volatile("bar.sync 1, 128;" ::: "memory");
     }
-    // After a failed wait the shares still go out and come in, so that no CTA leaves while another one writes to it.
-    if (!mbar_wait(&bars->acc_full, 0)) bars->failed = 1;
-    __syncwarp();  // every lane leaves the wait by itself; the cluster barrier and the loads below want them together
+    // After a failed wait the shares still go out and come in, as NaN, so that no CTA leaves while another one writes to it and no
+    // tile passes for complete.
+    bool lost = !mbar_wait_warp(&bars->acc_full, 0, p.wait_ns);
+    if (lost) bars->failed = 1;
+    __syncwarp();  // the cluster barrier and the loads below want the lanes together
     tc_fence_after_sync();
     cluster_wait();  // the peers' barriers exist
     if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 4);
@@ -259,6 +262,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
         const int at = min(g, kSplitGroups - 2);
         tmem_ld_32x16(acc + static_cast<uint32_t>(at * 8), r);
         tmem_ld_wait();
+        if (lost) no_acc(r);
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
           const int here = at + v / 2;
@@ -269,7 +273,10 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
     }
     if (TRACE && threadIdx.x == 64) trace_stamp_ns(p.trace, 5);
     if (splits > 1) {
-      if (!mbar_wait(&bars->shares, 0) && !mbar_wait(&bars->shares, 0)) bars->failed = 1;  // longer than a peer's own waits
+      if (!mbar_wait_warp(&bars->shares, 0, p.wait_ns) && !mbar_wait_warp(&bars->shares, 0, p.wait_ns)) {  // longer than a peer's own waits
+        bars->failed = 1;
+        lost = true;
+      }
       asm volatile("fence.acq_rel.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -284,6 +291,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
       const int at = min(g, kSplitGroups - 2);
       tmem_ld_32x16(acc + static_cast<uint32_t>(at * 8), r);
       tmem_ld_wait();
+      if (lost) no_acc(r);
       const float4* from = in + (at - own_lo) * 2 * kBlockM;
       const bool first = at >= g, second = at + 1 < own_hi;  // which of the two are wanted
       float sum[16];
@@ -446,7 +454,7 @@ cudaError_t launch_split(const SplitMaps& maps, const SplitParams& p, int tiles,
 
 cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, int n, int k, const float* scale_a,
                                  const float* scale_b, uint32_t* status, cudaStream_t stream, bool* done, const CommDev* layer,
-                                 void* a_copy) {
+                                 void* a_copy, const GiveUp* give_up) {
   *done = false;
   const int64_t tiles_m = (static_cast<int64_t>(m) + kBlockM - 1) / kBlockM, tiles_n = (static_cast<int64_t>(n) + kSplitBN - 1) / kSplitBN;
   if (tiles_m * tiles_n > kSplitMaxTiles) return cudaSuccess;
@@ -466,7 +474,8 @@ cudaError_t launch_gemm_nt_split(const void* a, const void* b, void* c, int m, i
   p.m = m;
   p.n = n;
   p.k = k;
-  p.stage_bytes = a_box_rows(m) * kBlockK * 2 + kSplitBBytes;
+  p.stage_bytes = a_box_rows(m) * kBlockK * 2 + kSplitBBytes + (give_up != nullptr ? give_up->missing : 0);
+  p.wait_ns = give_up != nullptr ? give_up->wait_ns : 0;
   p.k_iters = (k + kBlockK - 1) / kBlockK;
   p.tiles_m = static_cast<int>(tiles_m);
   const int tiles = static_cast<int>(tiles_m * tiles_n);

@@ -38,7 +38,7 @@ bool on16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr(
 // of a gradient) does not start on such a boundary, and contiguous() leaves it where it is.
 at::Tensor vectorable(const at::Tensor& t) { return on16(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
 
-// The two status words of one product, which its kernel clears.
+// The two status words of one product, which its kernel clears. Whoever drops them sees a wait that ran out all the same: as NaN.
 at::Tensor status_words(const at::Tensor& like) { return at::empty({2}, like.options().dtype(at::kInt)); }
 
 bool quantizable(const at::Tensor& x) {
@@ -848,6 +848,37 @@ void bind_ops(py::module_& m) {
                                        reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(x)));
     return std::make_tuple(gate_up, act, status);
   });
+
+  // For tests: the products' kernels with loads that are never complete and waits of `wait_ms`. `kind`: "nt" (a w^T by the kernel that
+  // its size takes), "pair", "gated" (a, w) or "gated_grad" (a w, gate_up). Output and status words.
+  ops.def("gemm_giving_up", [](const std::string& kind, const at::Tensor& a, const at::Tensor& w, const std::optional<at::Tensor>& gate_up,
+                               int wait_ms) {
+    want(a, at::kBFloat16, "a");
+    want(w, at::kBFloat16, "w");
+    const bool grad = kind == "gated_grad";
+    TORCH_CHECK(a.dim() == 2 && w.dim() == 2 && a.size(1) == w.size(grad ? 0 : 1) && wait_ms >= 1 && wait_ms <= 1000, "a: [m, k], w: [n, k] or [k, n]");
+    const GiveUp give_up{static_cast<unsigned long long>(wait_ms) * 1000000ull, 16};
+    c10::cuda::CUDAGuard g(a.device());
+    const int m = static_cast<int>(a.size(0)), n = static_cast<int>(w.size(grad ? 1 : 0)), k = static_cast<int>(a.size(1));
+    at::Tensor status = status_words(a), out = at::zeros({m, grad ? 2 * n : n}, a.options());
+    auto* words = reinterpret_cast<uint32_t*>(status.data_ptr<int>());
+    if (kind == "nt") {
+      B200C_CUDA_CHECK(launch_gemm_nt(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, nullptr, nullptr, words, cur(a), nullptr, nullptr, &give_up));
+    } else if (kind == "pair") {
+      B200C_CUDA_CHECK(launch_gemm_nt_pair(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, nullptr, nullptr, words, cur(a), 0, nullptr, &give_up));
+    } else if (kind == "gated") {
+      TORCH_CHECK(n % 2 == 0, "w: [2 n, k]");
+      at::Tensor act = at::zeros({m, n / 2}, a.options());
+      B200C_CUDA_CHECK(launch_gemm_gated(a.data_ptr(), w.data_ptr(), out.data_ptr(), act.data_ptr(), m, n / 2, k, words, cur(a), 0, &give_up));
+      out = at::cat({out, act}, 1);
+    } else {
+      TORCH_CHECK(grad && gate_up.has_value(), "kind");
+      want(*gate_up, at::kBFloat16, "gate_up");
+      TORCH_CHECK(gate_up->dim() == 2 && gate_up->size(0) == m && gate_up->size(1) == 2 * n, "gate_up: [m, 2 n]");
+      B200C_CUDA_CHECK(launch_gemm_gated_grad(a.data_ptr(), w.data_ptr(), gate_up->data_ptr(), out.data_ptr(), m, n, k, words, cur(a), &give_up));
+    }
+    return std::make_pair(out, status);
+  }, py::arg("kind"), py::arg("a"), py::arg("w"), py::arg("gate_up") = std::nullopt, py::arg("wait_ms") = 20);
 
   ops.def("kernel_launch_count", []() { return kernel_launch_count(); });
 }
