@@ -237,6 +237,27 @@ def test_scale_by_matches_operators(numel):
     assert _comms.ops.scale_by(t, g).requires_grad  # a gradient of the gradient keeps its graph
 
 
+# Two tensors in one launch, the grid that of the larger: either one the larger, below a vector, empty.
+@pytest.mark.parametrize("first,second", [(1, 3_000_001), (3_000_001, 7), (0, 4099), (4099, 0), (8, 8), (0, 0)])
+@pytest.mark.parametrize("consume", [False, True])
+def test_scale_both_by_matches_operators(first, second, consume):
+    from torchcomms_b200 import _comms
+
+    for value in (1.0, -0.3337, 0.0, float("inf")):
+        t, u, f = _bf(first, seed=12), _bf(second, seed=13), torch.tensor(value, device="cuda")
+        want = [v * f.to(v.dtype) for v in (t, u)]
+        got = _comms.ops.scale_both_by(t, u, f, consume)
+        for v, a, b in zip((t, u), got, want):
+            torch.testing.assert_close(a, b, rtol=0, atol=0, equal_nan=True)
+            assert v.numel() == 0 or (a.data_ptr() == v.data_ptr()) == consume
+    # what the kernel does not take: strides of a transposed matrix it does, a view off the grid and a factor with a gradient it does not
+    m, odd, f = _bf(6, 10, seed=14).t(), _bf(4100, seed=15)[1:], torch.tensor(-0.5, device="cuda")
+    a, b = _comms.ops.scale_both_by(m, odd, f, False)
+    assert torch.equal(a, m * -0.5) and a.stride() == (m * 1).stride() and torch.equal(b, odd * -0.5)
+    g = torch.tensor(3.0, device="cuda", requires_grad=True)
+    assert all(v.requires_grad for v in _comms.ops.scale_both_by(m, odd, g, consume))
+
+
 def test_linear_cross_entropy_matches_unfused():
     from torchcomms_b200.ops import fused
 

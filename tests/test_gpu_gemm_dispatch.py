@@ -61,17 +61,29 @@ def test_plain_product_with_half_tiles(m, n, k, fp8):
     test_plain_product(m, n, k, fp8)
 
 
-# Tiles of 112, 96 and 128 columns of gate and of up, one of them in a row, ragged ends of rows, columns and K steps,
-# halves of tiles.
+# Tiles of 112, 96 and 128 columns of gate and of up, one of them in a row, ragged ends of rows, columns and K steps; a last wave in
+# halves of tiles of 192 columns (1 x 8 to 1000 x 2568), of 224 and of 256.
 @pytest.mark.parametrize("m,n,k", [(700, 5000, 768), (300, 4808, 72), (1000, 2056, 200), (1, 8, 8), (257, 120, 64), (2049, 232, 136),
-                                   (1000, 2568, 136), (2048, 1160, 72), (512, 9480, 264)])
+                                   (1000, 2568, 136), (2048, 1160, 72), (512, 9480, 264), (512, 5288, 136), (768, 4728, 136)])
 def test_gated_product(m, n, k):
+    _gated_product(m, n, k, 0)
+
+
+# Every width with whole tiles and with halves, some of which lie past the last column: one tile, 4 to 6, and 90 to 135 for 74
+# pairs.
+@pytest.mark.parametrize("columns", [192, 224, 256])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (257, 200, 200), (2300, 1000, 72), (2300, 1192, 72), (1000, 2840, 136), (513, 4264, 72)])
+def test_gated_product_of_every_width(m, n, k, columns):
+    _gated_product(m, n, k, columns)
+
+
+def _gated_product(m, n, k, columns):
     from torchcomms_b200 import _comms
 
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     x = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
     w = (torch.randn(2 * n, k, generator=g, device="cuda") * k**-0.5).to(torch.bfloat16)
-    gate_up, act, status = _comms.ops.gemm_gated(x, w)
+    gate_up, act, status = _comms.ops.gemm_gated(x, w, columns)
     assert int(status[0]) == 0
     torch.testing.assert_close(gate_up.double(), x.double() @ w.double().t(), rtol=2**-8, atol=1e-6 * k)
     assert torch.equal(act, _comms.ops.swiglu_fwd(gate_up))  # the activation kernel's bits
@@ -79,7 +91,7 @@ def test_gated_product(m, n, k):
     # among them, then one to bf16, which may fall either way.
     gate, up = gate_up.double().chunk(2, dim=-1)
     torch.testing.assert_close(act.double(), torch.nn.functional.silu(gate) * up, rtol=2**-8, atol=1e-12)
-    again = _comms.ops.gemm_gated(x, w)
+    again = _comms.ops.gemm_gated(x, w, columns)
     assert torch.equal(again[0], gate_up) and torch.equal(again[1], act)
 
 

@@ -835,8 +835,8 @@ void bind_ops(py::module_& m) {
     return std::make_pair(d, status);
   });
 
-  // (x w^T, silu(gate) * up of it), bf16, gate columns first.
-  ops.def("gemm_gated", [](const at::Tensor& x, const at::Tensor& w) {
+  // (x w^T, silu(gate) * up of it), bf16, gate columns first. `columns` of a tile, gate and up together: 192, 224 or 256 (0: by size).
+  ops.def("gemm_gated", [](const at::Tensor& x, const at::Tensor& w, int columns) {
     want(x, at::kBFloat16, "x");
     want(w, at::kBFloat16, "w");
     TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && w.size(0) % 2 == 0, "x: [m, k], w: [2 n, k]");
@@ -845,9 +845,9 @@ void bind_ops(py::module_& m) {
     at::Tensor status = status_words(x);
     B200C_CUDA_CHECK(launch_gemm_gated(x.data_ptr(), w.data_ptr(), gate_up.data_ptr(), act.data_ptr(), static_cast<int>(x.size(0)),
                                        static_cast<int>(w.size(0) / 2), static_cast<int>(x.size(1)),
-                                       reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(x)));
+                                       reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(x), columns));
     return std::make_tuple(gate_up, act, status);
-  });
+  }, py::arg("x"), py::arg("w"), py::arg("columns") = 0);
 
   // For tests: the products' kernels with loads that are never complete and waits of `wait_ms`. `kind`: "nt" (a w^T by the kernel that
   // its size takes), "pair", "gated" (a, w) or "gated_grad" (a w, gate_up). Output and status words.
