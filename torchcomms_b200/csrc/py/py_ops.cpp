@@ -312,25 +312,32 @@ bool block_matrix(const at::Tensor& t, int64_t rows, int64_t cols, const at::Ten
   return plain_call(t, true) && t.scalar_type() == at::kBFloat16 && t.dim() == 2 && t.size(0) == rows && t.size(1) == cols &&
       t.is_contiguous() && on16(t) && t.device() == like.device();
 }
+// Pairs work in units of 256 rows, the tensor library's kernels in finer ones: whether rows fill theirs to so many percent.
+bool filled(int64_t rows, int percent) { return rows * 100 >= (rows + 255) / 256 * 256 * percent; }
+bool mostly_empty_rows(int64_t rows) { return rows > 128 && !filled(rows, 70); }
+constexpr int64_t kLargeWeight = 12 << 20;
 // x w^T of contiguous matrices on the 16-byte grid, widths multiples of 8: this library's product, whose call costs half the
-// tensor library's host time (6.5 and 11.5 us) and which starts early, up to a depth of 4096. Deeper sums that fill the GPU less
-// than once the tensor library splits better, and so products of more than a few million weights whose last unit of 256 rows
-// is mostly empty. In us, both from the host, the library's / this one's: 64 x 512 x 512 11.5 / 7.9, 1000 x 3072 x 2048 13.1 / 13.1,
-// 1000 x 6144 x 4096 37.5 / 38.5, 4096 x 6144 x 4096 137.7 / 131.8; 300 x 4096 x 4096 14.8 / 18.6, 700 x 4096 x 14336 62.1 / 65.6.
-bool mostly_empty_rows(int64_t rows) { return rows > 128 && rows * 10 < (rows + 255) / 256 * 256 * 7; }
+// tensor library's host time (6.5 and 11.5 us) and which starts early, up to a depth of 4096 (deeper sums that fill the GPU less
+// than once the tensor library splits better), where that is most of it or units of 256 rows are nine tenths full, and of large
+// weights from 450 rows on. In us, both from the host over weights from DRAM, the library's / this one's: 64 x 2048 x 2048 10.0 / 7.7,
+// 1000 x 3072 x 2048 13.1 / 13.1, 1552 x 2048 x 2048 17 / 21; 160 x 6144 x 4096 16 / 23, 520 25 / 33, 784 38 / 45, 1000 45 / 47, 1288 59 / 63,
+// 1536 68 / 66, 4096 169 / 150; 304 x 4096 x 4096 15 / 19, 1552 52 / 61, 4096 114 / 100.
 at::Tensor product(const at::Tensor& x, const at::Tensor& w) {
   const int64_t m = x.size(0), n = w.size(0), k = x.size(1);
-  if (k > 4096 || (mostly_empty_rows(m) && n * k > 12 << 20)) return at::mm(x, w.t());
+  const bool own = k <= 4096 && (n * k > kLargeWeight ? m >= 450 && filled(m, 90) : m * n * k <= 6000000000 || filled(m, 90));
+  if (!own) return at::mm(x, w.t());
   at::Tensor y = at::empty({m, n}, x.options()), status = status_words(x);
   B200C_CUDA_CHECK(launch_gemm_bf16_nt(x.data_ptr(), w.data_ptr(), y.data_ptr(), static_cast<int>(m), static_cast<int>(n), static_cast<int>(k),
                                        reinterpret_cast<uint32_t*>(status.data_ptr<int>()), cur(x)));
   return y;
 }
-// (x w^T, its activation): in one kernel, but for large weights where most of a unit of 256 rows would be empty (300 x 14336 x 4096
-// 88 us, product and activation kernel 67; 64 x 14336 x 4096 54 and 46).
+// (x w^T, its activation): in one kernel, but of large weights for up to 128 rows and where units of 256 rows are too empty: less
+// than 77 % full, from 768 rows on, where the activation kernel is less of it, 83 %. In us, the tensor library's product and the
+// activation kernel / one kernel: 64 x 14336 x 4096 49 / 53, 160 54 / 56, 208 61 / 57, 304 74 / 86, 400 92 / 90, 568 115 / 132, 592
+// 172 / 138, 784 159 / 173, 832 184 / 174, 1032 214 / 227, 1288 267 / 254; 64 x 8192 x 2048 20 / 26, 208 24 / 25, 304 31 / 35, 592 41 / 40.
 std::pair<at::Tensor, at::Tensor> gated_product(const at::Tensor& x, const at::Tensor& w) {
   const int64_t m = x.size(0), n = w.size(0) / 2, k = x.size(1);
-  if ((m <= 128 || mostly_empty_rows(m)) && 2 * n * k > 48 << 20) {
+  if (2 * n * k > kLargeWeight && (m <= 128 || !filled(m, m < 768 ? 77 : 83))) {
     at::Tensor gate_up = product(x, w);
     at::Tensor act = swiglu_fwd(gate_up);
     return {gate_up, act};
@@ -351,7 +358,7 @@ constexpr int64_t kKStep = 64;
 bool few_tiles(int64_t m, int64_t n) { return pair_tiles_fit(static_cast<int>(m), static_cast<int>(n), false); }
 bool own_by_columns(int64_t m, int64_t n, int64_t k) { return !few_tiles(m, n) || k <= 48 * kKStep; }
 bool own_by_rows(int64_t m, int64_t n, int64_t k) {
-  if (mostly_empty_rows(m) && n * k > 12 << 20) return false;
+  if (mostly_empty_rows(m) && n * k > kLargeWeight) return false;
   return k <= 32 * kKStep || (m >= 700 && k <= (few_tiles(m, n) ? 48 : 96) * kKStep);
 }
 // Elements from row to row. A single row is contiguous whatever its stride says, and then that means nothing.
@@ -382,7 +389,7 @@ at::Tensor input_gradient(const at::Tensor& dy, const at::Tensor& w) {
 at::Tensor gated_gradient(const at::Tensor& dy, const at::Tensor& w, const at::Tensor& gate_up) {
   const int64_t m = dy.size(0), n = w.size(1), k = w.size(0);
   if (!plain_rows(dy, dy) || !plain_rows(w, dy) || !plain_rows(gate_up, dy) || dy.size(1) != k || gate_up.size(0) != m ||
-      gate_up.size(1) != 2 * n || !own_by_rows(m, n, k) || (m <= 128 && n * k > 12 << 20)) {
+      gate_up.size(1) != 2 * n || !own_by_rows(m, n, k) || (m <= 128 && n * k > kLargeWeight)) {
     return swiglu_bwd(input_gradient(dy, w), gate_up);
   }
   at::Tensor d = at::empty_like(gate_up), status = status_words(dy);
