@@ -30,16 +30,11 @@ def test_head_against_64_bits(rows, dim, vocab):
     t[-1], t[0] = vocab - 1, 0
     t[rows // 3] = -1
     ref = _reference(x, w, t)
-    logits = (x.double() @ w.double().t()).bfloat16().double()
-    rounded = F.cross_entropy(logits, t, reduction="none", ignore_index=-1).sum() / rows
     for chunk in (4096, 100):
         out = _comms.ops.head(x, w, t, chunk)
-        # The loss is that of the bf16 logits, which are up to 0.3 sqrt(dim) x 5 here: fp32 exponentials and sums, 1e-5 as for the loss
-        # kernel that makes its own statistics; and where a sum of `dim` products in fp32 falls to the other side of a tie (2 in
-        # 10000 do), a target's logit is 2^-8 of itself off: two rows of these at most.
-        top = 1.5 * dim**0.5
-        assert abs(float(out[0].double() - rounded)) < 1e-5 + dim * top * 2**-24 + 2 / rows * top * 2**-8
-        assert abs(float(out[0].double() - ref[0])) < 1e-5 + 2 * top * 2**-9
+        # Sums of `dim` products in fp32: dim x 2^-24 of the products' magnitudes, which are below 0.3 sqrt(dim) x 5 here;
+        # then fp32 exponentials and sums, 1e-5 as for the loss kernel that makes its own statistics.
+        assert abs(float(out[0].double() - ref[0])) < 1e-5 + dim**1.5 * 1.5 * 2**-24
         # bf16 logits off by 2^-9 of up to 0.3 sqrt(dim) x 5 move a probability by as much; their gradients and the results
         # are rounded to 2^-9. One number in a row of one has nothing to average over, hence the maximum, not a norm.
         for a, b in zip(out[1:], ref[1:]):
@@ -154,10 +149,32 @@ def test_head_of_large_logits():
     x *= 100
     ref = _reference(x, w, t)
     loss, _, _ = _comms.ops.head(x, w, t, 4096)
-    # bf16 logits of up to 1500: half an ulp is 4, of a target's and of the highest
-    assert abs(float(loss.double() - ref[0])) < 2 * 4
-    rounded = F.cross_entropy((x.double() @ w.double().t()).bfloat16().double(), t)
-    assert abs(float(loss.double() - rounded)) < 1500 * 64 * 2**-24 + 2 / 200 * 8  # fp32 sums, and two ties that fall the other way
+    # fp32 logits of up to 1500: 2^-24 of that, 64 times over in the worst order
+    assert abs(float(loss.double() - ref[0])) < 1500 * 64 * 2**-24
+
+
+@pytest.mark.parametrize("vocab", [99, 2051])
+@pytest.mark.parametrize("scale", [0.3, 3.0, 30.0, 1e30])
+def test_head_loss_of_unrounded_logits(vocab, scale):
+    """Around the line at which the loss takes exponentials of what rounding took off, and with logits far below all others."""
+    from torchcomms_b200 import _comms
+
+    x, w, t = _head(130, 64, vocab, 12)
+    x[:, 0], w[:, 0] = 1, 0
+    w[::7, 0] = -scale if scale < 1e3 else -1e30  # lows: no exponential is left of them at the last scale
+    t = t // 7 * 7 + 1 if scale > 1e3 else t
+    t.clamp_(max=vocab - 2)
+    if scale > 1e3:
+        t[t % 7 == 0] += 1
+    else:
+        x[:, 1:] *= scale
+    ref = _reference(x, w, t)
+    out = _comms.ops.head(x, w, t, 4096)
+    size = float((x.double().abs() @ w.double().abs().t())[:, 1::7].max()) if scale < 1e3 else 1.5 * 64**0.5
+    # Products of that size in sum, 2^-24 of it per addition in the worst order; exponentials and sums as above.
+    assert abs(float(out[0].double() - ref[0])) < 1e-5 + 64 * size * 2**-24
+    for a, b in zip(out[1:], ref[1:]):
+        assert bool(a.isfinite().all()) and float((a.double() - b).norm()) <= 0.1 * float(b.norm())
 
 
 def test_what_the_head_leaves_to_operators():

@@ -680,6 +680,7 @@ struct HeadGrad {
   int64_t ld;
   const int64_t* targets;
   const float2* stats;
+  const float* fine;
   const float* target_logit;
   float* row_lse;   // [rows], where k_head_rows runs
   float* row_loss;
@@ -689,14 +690,27 @@ struct HeadGrad {
   float grad_scale, loss_scale;
 };
 
-// What several shares of a row are together.
-__device__ __forceinline__ void head_join(float2& a, float2 b) {
-  const float top = fmaxf(a.x, b.x);
-  a.y = (a.x == -INFINITY ? a.y : a.y * __expf(a.x - top)) + (b.x == -INFINITY ? b.y : b.y * __expf(b.x - top));
-  a.x = top;
+// What several shares of a row are together: maximum and sum of exponentials of the rounded logits, and what the sum of the
+// unrounded ones has more.
+struct HeadShare {
+  float mx = -INFINITY, sum = 0.0f, fine = 0.0f;
+};
+__device__ __forceinline__ void head_join(HeadShare& a, HeadShare b) {
+  const float top = fmaxf(a.mx, b.mx);
+  const float by_a = a.mx == -INFINITY ? 1.0f : __expf(a.mx - top), by_b = b.mx == -INFINITY ? 1.0f : __expf(b.mx - top);
+  a = HeadShare{top, a.sum * by_a + b.sum * by_b, a.fine * by_a + b.fine * by_b};
 }
-__device__ __forceinline__ float head_lse(const HeadGrad& a, float2 row) {
-  return a.words[0] != 0u ? NAN : row.x + logf(row.y);  // the product gave up a wait: its logits are not to be used
+__device__ __forceinline__ HeadShare head_share(const HeadGrad& a, int share, int row) {
+  const size_t at = static_cast<size_t>(share) * a.rows + row;
+  const float2 s = a.stats[at];
+  return HeadShare{s.x, s.y, a.fine[at]};
+}
+// The log-sum-exp that the gradient is made with, of the rounded logits, and the loss's, of the unrounded ones.
+__device__ __forceinline__ float head_lse(const HeadGrad& a, HeadShare row) {
+  return a.words[0] != 0u ? NAN : row.mx + logf(row.sum);  // the product gave up a wait: its logits are not to be used
+}
+__device__ __forceinline__ float head_loss(const HeadGrad& a, HeadShare row, int r) {
+  return (a.words[0] != 0u ? NAN : row.mx + logf(row.sum + row.fine)) - a.target_logit[r];
 }
 
 __device__ __forceinline__ bool head_ignores(const HeadGrad& a, int64_t target) { return target < 0 || target >= a.vocab; }
@@ -721,22 +735,21 @@ __device__ __forceinline__ void head_add_up(const HeadGrad& a, int rows, float* 
 // 32 rows a block, one per lane; the warps take the shares in turn.
 __global__ void __launch_bounds__(512) k_head_rows(HeadGrad a) {
   __shared__ float scratch[32];
-  __shared__ float2 part[16][32];
+  __shared__ HeadShare part[16][32];
   grid_release();
   grid_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
-  float2 sum = make_float2(-INFINITY, 0.0f);
+  HeadShare sum;
   if (r < a.rows) {
 #pragma unroll 4
-    for (int t = warp; t < a.shares; t += 16) head_join(sum, a.stats[static_cast<size_t>(t) * a.rows + r]);
+    for (int t = warp; t < a.shares; t += 16) head_join(sum, head_share(a, t, r));
   }
   part[warp][lane] = sum;
   __syncthreads();
   if (warp == 0 && r < a.rows) {
     for (int w = 1; w < 16; ++w) head_join(sum, part[w][lane]);
-    const float lse = head_lse(a, sum);
-    a.row_lse[r] = lse;
-    a.row_loss[r] = head_ignores(a, a.targets[r]) ? 0.0f : lse - a.target_logit[r];
+    a.row_lse[r] = head_lse(a, sum);
+    a.row_loss[r] = head_ignores(a, a.targets[r]) ? 0.0f : head_loss(a, sum, r);
     __threadfence();
   }
   head_add_up(a, min(32, a.rows - static_cast<int>(blockIdx.x) * 32), scratch);
@@ -757,16 +770,17 @@ __global__ void __launch_bounds__(kGradThreads) k_head_gradient(HeadGrad a) {
   const bool ignore = head_ignores(a, tgt);
   if (!LSE_KNOWN) {
     if (threadIdx.x < 32) {
-      float2 sum = make_float2(-INFINITY, 0.0f);
-      for (int t = threadIdx.x; t < a.shares; t += 32) head_join(sum, a.stats[static_cast<size_t>(t) * a.rows + r]);
+      HeadShare sum;
+      for (int t = threadIdx.x; t < a.shares; t += 32) head_join(sum, head_share(a, t, r));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
-        head_join(sum, make_float2(__shfl_xor_sync(0xffffffffu, sum.x, o), __shfl_xor_sync(0xffffffffu, sum.y, o)));
+        head_join(sum, HeadShare{__shfl_xor_sync(0xffffffffu, sum.mx, o), __shfl_xor_sync(0xffffffffu, sum.sum, o),
+                                 __shfl_xor_sync(0xffffffffu, sum.fine, o)});
       }
       if (threadIdx.x == 0) {
         shared_lse = head_lse(a, sum);
         if (part == 0) {
-          a.row_loss[r] = ignore ? 0.0f : shared_lse - a.target_logit[r];
+          a.row_loss[r] = ignore ? 0.0f : head_loss(a, sum, r);
           __threadfence();
         }
       }
@@ -1325,14 +1339,14 @@ cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, int64_t ld, cons
   return cudaGetLastError();
 }
 
-cudaError_t launch_head_gradient(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, const float2* stats, int shares,
+cudaError_t launch_head_gradient(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, const float2* stats, const float* fine, int shares,
                                  const float* target_logit, float* row_scratch, float* loss, uint32_t* words, int rows, int vocab,
                                  float grad_scale, float loss_scale, bool first, cudaStream_t s) {
   if (rows <= 0 || vocab <= 0 || shares <= 0 || ld % 16 != 0 || ld < vocab) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(logits) & 31u) != 0) return cudaErrorMisalignedAddress;
   const int nvec = (vocab + 15) / 16, threads = std::min(kGradThreads, (nvec + 31) / 32 * 32), parts = (nvec + threads - 1) / threads;
   if (static_cast<int64_t>(rows) * parts > INT32_MAX) return cudaErrorInvalidValue;
-  const HeadGrad a{logits, ld, targets, stats, target_logit, row_scratch, row_scratch + rows, loss, words, rows, shares, vocab, parts,
+  const HeadGrad a{logits, ld, targets, stats, fine, target_logit, row_scratch, row_scratch + rows, loss, words, rows, shares, vocab, parts,
                    first ? 1 : 0, grad_scale, loss_scale};
   const unsigned grid = static_cast<unsigned>(rows) * static_cast<unsigned>(parts);
   if (grid > kGradFused) {

@@ -64,7 +64,7 @@ cudaError_t launch_cross_entropy_fwd_bwd(__nv_bfloat16* logits, int64_t ld, cons
 // The same where launch_head_logits (tc_gemm.h) left the logits with their statistics: row stride `ld` a multiple of 16,
 // logits on a 32-byte boundary; up to 15 elements past a row's last, within its stride, are overwritten. `row_scratch`:
 // 2 * rows; *loss becomes loss_scale times the sum of the rows' losses, added to what it holds unless `first`.
-cudaError_t launch_head_gradient(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, const float2* stats, int shares,
+cudaError_t launch_head_gradient(__nv_bfloat16* logits, int64_t ld, const int64_t* targets, const float2* stats, const float* fine, int shares,
                                  const float* target_logit, float* row_scratch, float* loss, uint32_t* words, int rows, int vocab,
                                  float grad_scale, float loss_scale, bool first, cudaStream_t s);
 

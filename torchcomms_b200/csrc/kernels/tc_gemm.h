@@ -82,11 +82,11 @@ cudaError_t launch_gemm_gated(const void* x, const void* w, void* gate_up, void*
 
 // Logits of a head on CTA pairs: logits[m, n] (bf16, row stride `ld`, a multiple of 8) = x[m, k] x w[n, k]^T, any n, k % 8 ==
 // 0. Also, of the rounded logits, for each of head_row_shares(m, n) shares of a row the maximum and the sum of
-// exp(logit - maximum) (`stats`, [shares, m]), and the logit of the row's target (`target_logit`, where targets[row] is in
-// [0, n)). `words`: status as above, then a counter that launch_head_gradient counts rows in; all cleared by the kernel.
+// exp(logit - maximum) (`stats`, [shares, m]), what the sum of the unrounded ones has more (`fine`, the same), and the unrounded
+// logit of the row's target (`target_logit`, where targets[row] is in [0, n)). `words`: status as above, then a counter that launch_head_gradient counts rows in; all cleared by the kernel.
 int head_row_shares(int m, int n);
 cudaError_t launch_head_logits(const void* x, const void* w, void* logits, int64_t ld, const int64_t* targets, int m, int n, int k,
-                               float2* stats, float* target_logit, uint32_t* words, cudaStream_t stream);
+                               float2* stats, float* fine, float* target_logit, uint32_t* words, cudaStream_t stream);
 
 // Column-parallel layer fused with the all-gather of its input.
 // x_shards[r] is rank r's [m_local, k] bf16 activation shard in symmetric

@@ -25,10 +25,12 @@
 // each row's maximum and sum of exponentials over the tile and the logit of its target: the loss then needs one look
 // at the logits instead of two. One set of epilogue warps takes 405 us for 4096 x 128256 x 256 with one barrier more a chunk,
 // two sets that share a tile's columns 348, two that take the tiles in turn 315 (the plain product 257); 4096 x 128256 x 4096
-// 2700 to 2790, by the clock that the exponentials' power leaves (plain 2650). These are of sums over the accumulators; the
-// sums are of the rounded logits, which costs a pass of the head 2.5 % at a width of 256 (1192 and 1222 us) and 0.9 % at 4096 (9450 and
-// 9540). Accumulators' sums under rounded logits leave rows of probabilities that do not sum to one: where a target has a
-// probability of 0.95 the gradient was 0.26 of itself off (200 x 256 x 8000; so 0.0155), at 0.9999 140 times itself (0.028).
+// 2700 to 2790, by the clock that the exponentials' power leaves (plain 2650). These are of one sum, over the
+// accumulators. There are two now: of the rounded logits for the gradient, and what the unrounded ones have more for the loss. Both cost
+// a pass of the head 8 % at a width of 256 (1230 and 1335 us) and 0.9 % at 4096 (9900 and 9990), where the exponentials do not
+// bound the kernel. With the accumulators' sum under rounded logits a row of probabilities does not sum to one: where a target has
+// a probability of 0.95 the gradient was 0.26 of itself off (200 x 256 x 8000; so 0.0155), at 0.9999 140 times itself (0.028); with
+// the rounded sum in the loss that is 2.5e-5 off at 4096 x 1024 x 32000, so 1.2e-6.
 //
 // With kGated the product is the first half of a gated MLP: the second CTA's half of a B tile are the rows of `up` that go with
 // the first one's of `gate`, and the epilogue, which then has both of a column, also writes silu(gate) * up. 4096 x 14336 x 4096
@@ -126,43 +128,85 @@ struct PairParams {
   int stage_bytes, tail_bytes;  // of one K step's loads, both CTAs together, of a tile and of half a tile
   int missing;      // (host) bytes more that a step's loads are said to be
   int whole;        // tiles that are worked on whole; the others, too few to keep half of the pairs busy, in halves of their columns
-  float2* stats;    // kStats: [shares of a row, m] maximum and sum of exponentials; per row its target and the target's logit
+  float2* stats;    // kStats: [shares of a row, m] maximum and sum of exponentials of rounded logits; per row its target and the target's logit
+  float* fine;      // [shares of a row, m] what the sum of unrounded ones has more
   const int64_t* targets;
   float* target_logit;
   __nv_bfloat16* act;  // kGated: [m, n] silu(gate) * up
   const __nv_bfloat16* gate_up;  // (host) kGatedGrad: [m, 2 n]
 };
 
-// Maximum and sum of exp(x - maximum) of what a row has shown so far, NaN where one was among it. Of the logits as they are stored,
-// rounded to bf16: the gradient is made from those, and its probabilities sum to one only if the sum is of the same numbers. Two
-// elements per addition and product, two per maximum: the exponentials then take more of the time than what is around them.
+// Maximum and sum of exp(x - maximum) of what a row has shown so far, NaN where one was among it. `sum` is of the logits as they
+// are stored, rounded to bf16: the gradient is made from those, and its probabilities sum to one only if the sum is of the same
+// numbers. `fine` is what the sum of the unrounded ones, which the loss is made from, has more. Two elements per addition and
+// product, two per maximum: the exponentials then take more of the time than what is around them.
 struct RowStats {
-  float mx = -INFINITY, sum = 0.0f;
-  __device__ __forceinline__ void feed(const uint32_t (&packed)[16]) {
+  float mx = -INFINITY, sum = 0.0f, fine = 0.0f;
+  __device__ __forceinline__ void feed(const uint32_t (&r)[32], const uint32_t (&packed)[16]) {
     const auto lo = [&](int i) { return __uint_as_float(packed[i] << 16); };
     const auto hi = [&](int i) { return __uint_as_float(packed[i] & 0xffff0000u); };
-    float m[4];
+    float m[4], l[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = fmaxf(lo(i), hi(i));
+    for (int i = 0; i < 4; ++i) {
+      m[i] = fmaxf(lo(i), hi(i));
+      l[i] = fminf(lo(i), hi(i));
+    }
 #pragma unroll
     for (int i = 4; i < 16; i += 4) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) m[j] = max3(m[j], lo(i + j), hi(i + j));
+      for (int j = 0; j < 4; ++j) {
+        m[j] = max3(m[j], lo(i + j), hi(i + j));
+        l[j] = min3(l[j], lo(i + j), hi(i + j));
+      }
     }
-    const float top = fmaxf(max3(m[0], m[1], m[2]), m[3]);
+    const float top = fmaxf(max3(m[0], m[1], m[2]), m[3]), bottom = fminf(min3(l[0], l[1], l[2]), l[3]);
     if (top > mx) {
-      if (mx != -INFINITY) sum *= __expf(mx - top);
+      if (mx != -INFINITY) {
+        const float less = __expf(mx - top);
+        sum *= less;
+        fine *= less;
+      }
       mx = top;
     }
     constexpr float kLog2e = 1.44269504f;
     const float shift = mx == -INFINITY ? 0.0f : -mx;
-    float2 s[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+    float2 s[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)}, f[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+    // What rounding took off an element.
+    const auto rest = [&](int i, float2 x) {
+      return fma2(x, make_float2(-1.0f, -1.0f), make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
+    };
+    if (fabsf(mx) <= 32.0f && bottom >= -1e4f) {
+      // exp(d) - 1 to the third order: d is 2^-9 of the element at most, the fourth order 6e-7 of the exponential. (Where d is larger,
+      // far below the maximum, nothing is left of that.)
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float2 x = mul2(add2(make_float2(lo(i), hi(i)), make_float2(shift, shift)), make_float2(kLog2e, kLog2e));
-      s[i % 2] = add2(s[i % 2], make_float2(exp2_fast(x.x), exp2_fast(x.y)));
+      for (int i = 0; i < 16; ++i) {
+        const float2 x = make_float2(lo(i), hi(i)), d = rest(i, x);
+        const float2 y = mul2(add2(x, make_float2(shift, shift)), make_float2(kLog2e, kLog2e));
+        const float2 e = make_float2(exp2_fast(y.x), exp2_fast(y.y));
+        s[i % 2] = add2(s[i % 2], e);
+        const float2 q = fma2(fma2(d, make_float2(1.0f / 6.0f, 1.0f / 6.0f), make_float2(0.5f, 0.5f)), d, make_float2(1.0f, 1.0f));
+        f[i % 2] = fma2(mul2(e, d), q, f[i % 2]);
+      }
+    } else {
+      // An infinity less an infinity is no number, and its exponential zero or none either; logits above 32768 lose up to more than
+      // 64, of which the rest stays off.
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 x = make_float2(lo(i), hi(i)), d = rest(i, x);
+        const float2 y = mul2(add2(x, make_float2(shift, shift)), make_float2(kLog2e, kLog2e));
+        const float2 e = make_float2(exp2_fast(y.x), exp2_fast(y.y));
+        s[i % 2] = add2(s[i % 2], e);
+        f[i % 2].x += e.x * (__expf(fminf(d.x, 64.0f)) - 1.0f);
+        f[i % 2].y += e.y * (__expf(fminf(d.y, 64.0f)) - 1.0f);
+      }
     }
     sum += (s[0].x + s[0].y) + (s[1].x + s[1].y);
+    fine += (f[0].x + f[0].y) + (f[1].x + f[1].y);
+  }
+  static __device__ __forceinline__ float min3(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
   }
   static __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
@@ -187,6 +231,11 @@ struct RowStats {
   static __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     unsigned long long d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(both(a)), "l"(both(b)));
+    return apart(d);
+  }
+  static __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(both(a)), "l"(both(b)), "l"(both(c)));
     return apart(d);
   }
   static __device__ __forceinline__ float2 add2(float2 a, float2 b) {
@@ -582,12 +631,12 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           for (int i = 0; i < 16; ++i) packed[i] = pack_bf16(r[2 * i], r[2 * i + 1]);
           if constexpr (STATS) {
             const int col = j * kChunk + half * 32;
-            if (row_there) row_stats.feed(packed);
+            if (row_there) row_stats.feed(r, packed);
             if (row_there && target >= col && target < col + 32) {
               uint32_t z = 0;
 #pragma unroll
               for (int i = 0; i < 32; ++i) z = target == col + i ? r[i] : z;
-              p.target_logit[out_row + row_in_tile] = __uint_as_float(pack_bf16(z, 0u) << 16);
+              p.target_logit[out_row + row_in_tile] = __uint_as_float(z);
             }
           }
 #pragma unroll
@@ -607,7 +656,9 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
         }
       }
       if (row_there) {
-        p.stats[static_cast<size_t>(out_col / BN) * p.m + out_row + row_in_tile] = make_float2(row_stats.mx, row_stats.sum);
+        const size_t at = static_cast<size_t>(out_col / BN) * p.m + out_row + row_in_tile;
+        p.stats[at] = make_float2(row_stats.mx, row_stats.sum);
+        p.fine[at] = row_stats.fine;
       }
     }
     if (issuer) {
@@ -862,7 +913,7 @@ int head_row_shares(int m, int n) {
 }
 
 cudaError_t launch_head_logits(const void* x, const void* w, void* logits, int64_t ld, const int64_t* targets, int m, int n, int k,
-                               float2* stats, float* target_logit, uint32_t* words, cudaStream_t stream) {
+                               float2* stats, float* fine, float* target_logit, uint32_t* words, cudaStream_t stream) {
   if (m <= 0 || n <= 0 || k <= 0 || k % 8 != 0 || ld % 8 != 0 || ld < n) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(logits)) & 15u) {
     return cudaErrorMisalignedAddress;
@@ -874,6 +925,7 @@ cudaError_t launch_head_logits(const void* x, const void* w, void* logits, int64
   p.n = n;
   p.k = k;
   p.stats = stats;
+  p.fine = fine;
   p.targets = targets;
   p.target_logit = target_logit;
   return pair_tiles_fit(m, n, false) ? launch_pair<false, 128, kStats>(x, w, logits, p, stream, ld)

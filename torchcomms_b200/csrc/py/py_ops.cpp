@@ -567,11 +567,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> head(const at::Tensor& x, const a
   // Statistics (the last chunk may take narrower tiles), then a target's logit and two words of scratch per row, then the
   // kernels' words.
   const int64_t last = rows - (rows - 1) / chunk * chunk;
-  const int64_t stat_words = 2 * std::max(chunk * head_row_shares(static_cast<int>(chunk), static_cast<int>(vocab)),
-                                          last * head_row_shares(static_cast<int>(last), static_cast<int>(vocab)));
-  const at::Tensor scratch = at::empty({stat_words + 3 * chunk + 4}, x.options().dtype(at::kFloat));
-  float* stats = scratch.data_ptr<float>();
-  float *target_logit = stats + stat_words, *row_scratch = target_logit + chunk;
+  const int64_t shares = std::max(chunk * head_row_shares(static_cast<int>(chunk), static_cast<int>(vocab)),
+                                  last * head_row_shares(static_cast<int>(last), static_cast<int>(vocab)));
+  const at::Tensor scratch = at::empty({3 * shares + 3 * chunk + 4}, x.options().dtype(at::kFloat));
+  float *stats = scratch.data_ptr<float>(), *fine = stats + 2 * shares;
+  float *target_logit = fine + shares, *row_scratch = target_logit + chunk;
   auto* words = reinterpret_cast<uint32_t*>(row_scratch + 2 * chunk);
   const float mean = 1.0f / static_cast<float>(rows);
   for (int64_t r0 = 0; r0 < rows; r0 += chunk) {
@@ -583,8 +583,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> head(const at::Tensor& x, const a
     at::Tensor grad = logits.as_strided({n, vocab}, {ld, 1});
     if (own_logits(n, vocab, dim)) {
       B200C_CUDA_CHECK(launch_head_logits(xs.data_ptr(), weight.data_ptr(), z, ld, t, n, static_cast<int>(vocab), static_cast<int>(dim),
-                                          reinterpret_cast<float2*>(stats), target_logit, words, cur(x)));
-      B200C_CUDA_CHECK(launch_head_gradient(z, ld, t, reinterpret_cast<float2*>(stats), head_row_shares(n, static_cast<int>(vocab)),
+                                          reinterpret_cast<float2*>(stats), fine, target_logit, words, cur(x)));
+      B200C_CUDA_CHECK(launch_head_gradient(z, ld, t, reinterpret_cast<float2*>(stats), fine, head_row_shares(n, static_cast<int>(vocab)),
                                             target_logit, row_scratch, loss.data_ptr<float>(), words, n, static_cast<int>(vocab), mean, mean,
                                             r0 == 0, cur(x)));
     } else {
