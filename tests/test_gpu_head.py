@@ -175,6 +175,9 @@ def test_head_loss_of_unrounded_logits(vocab, scale):
     assert abs(float(out[0].double() - ref[0])) < 1e-5 + 64 * size * 2**-24
     for a, b in zip(out[1:], ref[1:]):
         assert bool(a.isfinite().all()) and float((a.double() - b).norm()) <= 0.1 * float(b.norm())
+    # A logit of minus infinity has no probability.
+    w[5], w[5, 0], t[t == 5] = 0, float("-inf"), 6
+    assert abs(float(_comms.ops.head(x, w, t, 4096)[0].double() - _reference(x, w, t)[0])) < 1e-5 + 64 * size * 2**-24
 
 
 def test_what_the_head_leaves_to_operators():

@@ -503,7 +503,8 @@ __global__ void __launch_bounds__(256) k_split_rope(__nv_bfloat16* packed, int64
 
 // Both directions stream their operands once and are bound by memory: every thread takes VECS vectors of each
 // operand, all loads before the first use, and finds its row with a multiply instead of a 64-bit division.
-// [4096, 2 x 14336]: forward 60.8 us, now 53.8 (6.5 TB/s); backward 101.2 us, now 83.5 (7.0 TB/s). Two vectors per
+// [4096, 2 x 14336]: forward 60.8 us, now 53.8 (6.5 TB/s); backward 101.2 us, now 83.5 (7.0 TB/s); a pass of both through autograd
+// 146.7 us with a division in the sigmoid, which branches, and 142.5. Two vectors per
 // thread once every vector cannot have a resident thread of its own (148 x 2048 threads); below that a pass is one
 // chain of latencies, which a second vector's arithmetic makes longer: forward / backward of [100, 2 x 8192] 2.9 / 3.5 us
 // with two, 2.3 / 2.8 with one, of [1, 2 x 4096] 2.6 / 3.0 and 2.0 / 2.3; of [700, 2 x 4096] (358 thousand vectors)

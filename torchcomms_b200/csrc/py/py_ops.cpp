@@ -564,8 +564,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> head(const at::Tensor& x, const a
   const int64_t rows = x.size(0), dim = x.size(1), vocab = weight.size(0), chunk = std::min(rows, chunk_rows), ld = (vocab + 63) / 64 * 64;
   at::Tensor dx = at::empty_like(x), dw = at::empty_like(weight), loss = at::empty({}, x.options().dtype(at::kFloat));
   const at::Tensor logits = at::empty({chunk, ld}, x.options());
-  // Statistics (the last chunk may take narrower tiles), then a target's logit and two words of scratch per row, then the
-  // kernels' words.
+  // Statistics and what the loss's sums have more (the last chunk may take narrower tiles), then a target's logit and two words of
+  // scratch per row, then the kernels' words.
   const int64_t last = rows - (rows - 1) / chunk * chunk;
   const int64_t shares = std::max(chunk * head_row_shares(static_cast<int>(chunk), static_cast<int>(vocab)),
                                   last * head_row_shares(static_cast<int>(last), static_cast<int>(vocab)));
