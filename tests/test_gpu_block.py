@@ -297,15 +297,20 @@ def test_gradients_of_gradients():
         x, h = fused.rms_norm_skip(x, norm, 1e-5)
         return (x, *fused.split_rope(torch.nn.functional.linear(h, w), pos, cos_t, sin_t, 4, 2))
 
-    results = []
-    for f in (lambda *a: _comms.ops.block_in(*a, pos, cos_t, sin_t, 4, 2, 1e-5), apart_in):
-        leaves = [t.clone().requires_grad_(True) for t in (ins[0], ins[2], wqkv)]
-        out = f(*leaves)
-        first = torch.autograd.grad(out, leaves, [_rand(*t.shape, seed=10 + i) for i, t in enumerate(out)], create_graph=True)
-        second = torch.autograd.grad(sum(g.float().square().sum() for g in first if g.requires_grad), leaves, allow_unused=True)
-        results.append((*first, *second))
-    for a, b in zip(*results):
-        assert (a is None and b is None) or (_off(a.detach(), b.detach()) < 4 * 2**-9 and a.requires_grad == b.requires_grad)
+    for frozen in ((), (0, 1), (2,), (1, 2)):
+        results = []
+        for f in (lambda *a: _comms.ops.block_in(*a, pos, cos_t, sin_t, 4, 2, 1e-5), apart_in):
+            args = [t.clone().requires_grad_(i not in frozen) for i, t in enumerate((ins[0], ins[2], wqkv))]
+            leaves = [t for t in args if t.requires_grad]
+            out = f(*args)
+            used = [(t, _rand(*t.shape, seed=10 + i)) for i, t in enumerate(out) if i > 0 or 0 not in frozen]
+            first = torch.autograd.grad([t for t, _ in used], leaves, [d for _, d in used], create_graph=True)
+            with_history = [g for g in first if g.requires_grad]
+            second = torch.autograd.grad(sum(g.float().square().sum() for g in with_history), leaves, allow_unused=True) if with_history else ()
+            results.append((*first, *second))
+        assert len(results[0]) == len(results[1])
+        for a, b in zip(*results):
+            assert (a is None and b is None) or (_off(a.detach(), b.detach()) < 4 * 2**-9 and a.requires_grad == b.requires_grad)
 
 
 def test_block_takes_and_leaves():

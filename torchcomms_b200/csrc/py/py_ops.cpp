@@ -418,7 +418,14 @@ variable_list gradients_with_history(AutogradContext* ctx, const std::vector<at:
     own[i] = args[i].view_as(args[i]);
     if (ctx->needs_input_grad(i)) wanted.push_back(own[i]);
   }
-  const variable_list made = torch::autograd::grad(forward(own), wanted, grads, /*retain_graph=*/std::nullopt, /*create_graph=*/true,
+  variable_list results, of_results;
+  const variable_list all = forward(own);
+  for (size_t i = 0; i < all.size(); ++i) {
+    if (!all[i].requires_grad()) continue;  // the residual stream where only the projection is trained
+    results.push_back(all[i]);
+    of_results.push_back(grads[i]);
+  }
+  const variable_list made = torch::autograd::grad(results, wanted, of_results, /*retain_graph=*/std::nullopt, /*create_graph=*/true,
                                                    /*allow_unused=*/true);
   for (size_t i = 0, j = 0; i < args.size(); ++i) {
     if (ctx->needs_input_grad(i)) out[i] = made[j++];
