@@ -432,6 +432,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
     // ---------------- MMA issuer
     if (elect_one()) {
       uint32_t it = 0, tile_iter = 0;
+      bool cut_short = false;
       for (int t = blockIdx.x; t < total_tiles && !bars->failed; t += G, ++tile_iter) {
         const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
         if (!mbar_wait(&bars->acc_empty[as], aph ^ 1u, p.wait_ns)) {
@@ -445,6 +446,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
           const uint32_t ph = (it / Cfg::kStages) & 1u;
           if (!mbar_wait(&bars->full[s], ph, p.wait_ns)) {
             bars->failed = 1;
+            cut_short = true;
             break;
           }
           tc_fence_after_sync();
@@ -461,7 +463,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpMaps& maps, const CommDev& 
           }
           umma_commit(&bars->empty[s]);  // stage reusable once these MMAs have read it
         }
-        if (bars->failed) break;  // not all of K: the epilogue waits in vain
+        if (cut_short) break;  // not all of K: the epilogue waits in vain
         umma_commit(&bars->acc_full[as]);  // accumulator complete
       }
       trace_stamp_ns(c, 2);

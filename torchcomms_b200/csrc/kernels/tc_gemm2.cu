@@ -404,6 +404,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
     // ---------------- MMA issuer (leader CTA only)
     if (leader && elect_one()) {
       uint32_t it = 0, tile_iter = 0;
+      bool cut_short = false;
       for (int i = cluster_id; i < items && !bars->failed; i += nclusters, ++tile_iter) {
         const uint32_t shape = i >= p.whole ? idesc_tail : idesc;
         const uint32_t as = tile_iter & 1u, aph = (tile_iter >> 1) & 1u;
@@ -418,6 +419,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           const uint32_t ph = (it / kStages) & 1u;
           if (!mbar_wait(&bars->full[s], ph, p.wait_ns)) {
             bars->failed = 1;
+            cut_short = true;
             break;
           }
           tc_fence_after_sync();
@@ -436,7 +438,7 @@ __global__ void __launch_bounds__(pair_threads<EPI>(), 1) k_gemm_pair(const __gr
           }
           umma_commit_pair(&bars->empty[s], 3);  // both CTAs may refill the stage
         }
-        if (bars->failed) break;  // not all of K: the epilogues wait in vain
+        if (cut_short) break;  // not all of K: the epilogues wait in vain
         umma_commit_pair(&bars->acc_full[as], 3);  // both CTAs' epilogues may read
       }
     }

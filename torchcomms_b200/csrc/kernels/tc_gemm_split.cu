@@ -186,11 +186,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
     }
   } else if (warp == 1) {
     if (elect_one()) {
+      bool cut_short = false;
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const int s = it % kSplitStages;
         const uint32_t ph = (it / kSplitStages) & 1u;
         if (!mbar_wait(&bars->full[s], ph, p.wait_ns)) {
           bars->failed = 1;
+          cut_short = true;
           break;
         }
         tc_fence_after_sync();
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_gemm_split(const __grid_co
         }
         umma_commit(&bars->empty[s]);
       }
-      if (!bars->failed) umma_commit(&bars->acc_full);  // or not all of K is there: the epilogue waits in vain
+      if (!cut_short) umma_commit(&bars->acc_full);  // or not all of K is there: the epilogue waits in vain
       if (TRACE) trace_stamp_ns(p.trace, 2);
     }
   } else {
